@@ -1,10 +1,8 @@
 // api.cu -- the C ABI of libeagb.so (declared in include/eagb.h).
 //
-// A context is one job: it owns every device buffer and two streams (the job's
-// and the cluster-uniform generator's), and enqueues the kernels of kernels.cu
+// A context is one job: it owns every device buffer and its stream, and enqueues the kernels of kernels.cu
 // in the order of the reference driver (PROGRAM/src/main.cu:142-230).  No call
 // synchronises the device except the ones that return data to the host.
-#include <cuda.h>
 #include <curand.h>
 
 #include <algorithm>
@@ -20,6 +18,7 @@
 #include "host.hpp"
 #include "batch.cuh"
 #include "kernels.cuh"
+#include "xorwow.cuh"
 
 using namespace eagb;
 
@@ -63,24 +62,12 @@ struct ea_ctx {
   bool have_temps = false;
   bool energies_fresh = false;
   // Houdayer
-  curandGenerator_t gen = nullptr;
   uint64_t cuda_rng_offset = 0, seed_cluster = 0;
   int nclust_cap = 0;
-  // Uniforms of a move: U[set][group].  The generator runs on its own stream
-  // `rs` at the highest priority and draws the next move's set while the
-  // current move and the sweeps after it run on `st`.  Its kernel holds 64
-  // blocks of 64 threads and is bound by FP64 throughput on the SMs it
-  // holds, so it overlaps the integer kernels of the job almost entirely.
-  // The sequence of uniforms is the generator's own, whatever the overlap.
-  cudaStream_t rs = nullptr;
-  // optional SM partition (green contexts): the generator on its own SMs,
-  // the job's kernels on the rest
-  CUgreenCtx part[2] = {nullptr, nullptr};
-  int part_sms = 0;
-  double *U[2][2] = {};
-  cudaEvent_t drawn[2] = {}, used[2] = {};
-  int cur = 0;    // set that holds the uniforms of the next move
-  int ready = 0;  // sets drawn and not yet used by a move (0..2)
+  // Coins of a move (xorwow.cuh)
+  bool xw_ready = false;   // the states hold the sequence of (seed_cluster, cuda_rng_offset)
+  uint32_t *xw_mat = nullptr;
+  int rng_sms = 0;         // see ea_set_rng_sms
   uint32_t *label = nullptr;
   uint32_t *sel = nullptr;
   unsigned long long *Q = nullptr;
@@ -164,59 +151,6 @@ static void prof_collect(ea_ctx *c) {
     }
     c->prof_ev[k].clear();
   }
-}
-
-
-// Driver entry points of the green-context API, looked up at run time so
-// that the library needs no link to the driver library.
-static void *drv_fn(const char *name) {
-  void *fn = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  if (cudaGetDriverEntryPointByVersion(name, &fn, CUDA_VERSION, cudaEnableDefault, &q) != cudaSuccess ||
-      q != cudaDriverEntryPointSuccess)
-    return nullptr;
-  return fn;
-}
-
-// Splits the device into nsm SMs for the cluster-uniform generator and the
-// rest for the job, and creates the two streams there.
-static int make_partition(ea_ctx *c, int nsm) {
-  using GetRes = CUresult (*)(CUdevice, CUdevResource *, CUdevResourceType);
-  using Split = CUresult (*)(CUdevResource *, unsigned *, const CUdevResource *, CUdevResource *, unsigned, unsigned);
-  using GenDesc = CUresult (*)(CUdevResourceDesc *, CUdevResource *, unsigned);
-  using GCreate = CUresult (*)(CUgreenCtx *, CUdevResourceDesc, CUdevice, unsigned);
-  using GStream = CUresult (*)(CUstream *, CUgreenCtx, unsigned, int);
-  using DevGet = CUresult (*)(CUdevice *, int);
-  auto devget = (DevGet)drv_fn("cuDeviceGet");
-  auto getres = (GetRes)drv_fn("cuDeviceGetDevResource");
-  auto split = (Split)drv_fn("cuDevSmResourceSplitByCount");
-  auto gendesc = (GenDesc)drv_fn("cuDevResourceGenerateDesc");
-  auto gcreate = (GCreate)drv_fn("cuGreenCtxCreate");
-  auto gstream = (GStream)drv_fn("cuGreenCtxStreamCreate");
-  if (!devget || !getres || !split || !gendesc || !gcreate || !gstream)
-    return fail(EA_ERR_CUDA, "green contexts are not available from this driver");
-  CUdevice dev;
-  CUdevResource all, grp, rest;
-  unsigned ng = 1;
-  CUdevResourceDesc d[2];
-  CUstream s[2];
-  if (devget(&dev, c->device) || getres(dev, &all, CU_DEV_RESOURCE_TYPE_SM) ||
-      split(&grp, &ng, &all, &rest, 0, (unsigned)nsm) || ng != 1 || gendesc(&d[0], &grp, 1) ||
-      gendesc(&d[1], &rest, 1) || gcreate(&c->part[0], d[0], dev, CU_GREEN_CTX_DEFAULT_STREAM) ||
-      gcreate(&c->part[1], d[1], dev, CU_GREEN_CTX_DEFAULT_STREAM) ||
-      gstream(&s[0], c->part[0], CU_STREAM_NON_BLOCKING, 0) || gstream(&s[1], c->part[1], CU_STREAM_NON_BLOCKING, 0))
-    return fail(EA_ERR_CUDA, "SM partition of %d SMs failed", nsm);
-  c->rs = (cudaStream_t)s[0];
-  c->st = (cudaStream_t)s[1];
-  c->part_sms = (int)grp.sm.smCount;
-  return EA_OK;
-}
-
-static void drop_partition(ea_ctx *c) {
-  using GDestroy = CUresult (*)(CUgreenCtx);
-  auto gdestroy = (GDestroy)drv_fn("cuGreenCtxDestroy");
-  for (CUgreenCtx &g : c->part)
-    if (g && gdestroy) { gdestroy(g); g = nullptr; }
 }
 
 
@@ -392,46 +326,20 @@ int ea_create(const ea_geom *gp, int32_t device, ea_ctx **out) {
 
 int ea_get_rng_sms(const ea_ctx *c, int32_t *nsm) {
   if (!c || !nsm) return fail(EA_ERR_ARG, "null argument");
-  *nsm = c->part_sms;
+  *nsm = c->rng_sms;
   return EA_OK;
 }
 
 int ea_set_rng_sms(ea_ctx *c, int32_t nsm) {
   if (check(c)) return EA_ERR_ARG;
-  if (c->gen) return fail(EA_ERR_STATE, "the SM split is set before the first cluster move");
+  if (c->xw_ready) return fail(EA_ERR_STATE, "the SM split is set before the first cluster move");
   if (set_device(c)) return EA_ERR_CUDA;
   const Geometry &g = c->g;
   int nsms = 0;
   CU(cudaDeviceGetAttribute(&nsms, cudaDevAttrMultiProcessorCount, c->device));
   if (nsm < 0) nsm = (2.0 * g.V * g.NB * g.ns >= (double)(1 << 24) && nsms >= 128) ? 32 : 0;
   if (nsm >= nsms) return fail(EA_ERR_ARG, "SM split %d of %d SMs", nsm, nsms);
-  if (nsm == c->part_sms) return EA_OK;
-  CU(cudaStreamSynchronize(c->st));
-  if (c->rs) CU(cudaStreamSynchronize(c->rs));
-  cudaStream_t old_st = c->st, old_rs = c->rs;
-  CUgreenCtx old_part[2] = {c->part[0], c->part[1]};
-  c->part[0] = c->part[1] = nullptr;
-  c->rs = nullptr;
-  int rc = EA_OK;
-  if (nsm > 0) {
-    rc = make_partition(c, nsm);
-  } else {
-    cudaError_t e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
-    if (e != cudaSuccess) rc = fail(EA_ERR_CUDA, "stream: %s", cudaGetErrorString(e));
-    c->part_sms = 0;
-  }
-  if (rc != EA_OK) {
-    drop_partition(c);
-    c->st = old_st; c->rs = old_rs;
-    c->part[0] = old_part[0]; c->part[1] = old_part[1];
-    return rc;
-  }
-  if (old_rs) cudaStreamDestroy(old_rs);
-  cudaStreamDestroy(old_st);
-  using GDestroy = CUresult (*)(CUgreenCtx);
-  auto gdestroy = (GDestroy)drv_fn("cuGreenCtxDestroy");
-  for (CUgreenCtx gx : old_part)
-    if (gx && gdestroy) gdestroy(gx);
+  c->rng_sms = nsm;
   return EA_OK;
 }
 
@@ -439,26 +347,19 @@ int ea_destroy(ea_ctx *c) {
   if (!c) return EA_OK;
   cudaSetDevice(c->device);
   if (c->st) cudaStreamSynchronize(c->st);
-  if (c->rs) cudaStreamSynchronize(c->rs);
-  if (c->gen) curandDestroyGenerator(c->gen);
   prof_collect(c);
   for (void *p : c->owned) cudaFree(p);
-  for (auto &set : c->U)
-    for (double *u : set)
-      if (u) cudaFree(u);
-  for (int s = 0; s < 2; ++s) {
-    if (c->drawn[s]) cudaEventDestroy(c->drawn[s]);
-    if (c->used[s]) cudaEventDestroy(c->used[s]);
-  }
+  if (c->j.xw_bits) cudaFree(c->j.xw_bits);
+  if (c->j.xw_state) cudaFree(c->j.xw_state);
+  if (c->j.xw_pos) cudaFree(c->j.xw_pos);
+  if (c->xw_mat) cudaFree(c->xw_mat);
   if (c->cs) cudaStreamSynchronize(c->cs);
   if (c->staged) cudaEventDestroy(c->staged);
   if (c->stage_free) cudaEventDestroy(c->stage_free);
   if (c->stage) cudaFree(c->stage);
   if (c->cs) cudaStreamDestroy(c->cs);
-  if (c->rs) cudaStreamDestroy(c->rs);
   if (c->st) cudaStreamDestroy(c->st);
   c->st = nullptr;
-  drop_partition(c);
   if (c->label) cudaFree(c->label);
   if (c->sel) cudaFree(c->sel);
   if (c->Q) cudaFree(c->Q);
@@ -477,21 +378,12 @@ int ea_get_geom(const ea_ctx *c, ea_geom *g) {
 int ea_sync(ea_ctx *c) {
   if (check(c)) return EA_ERR_ARG;
   CU(cudaStreamSynchronize(c->st));
-  if (c->rs) CU(cudaStreamSynchronize(c->rs));
   if (c->cs) CU(cudaStreamSynchronize(c->cs));
   return EA_OK;
 }
 
 int ea_join(ea_ctx *c) {
-  if (check(c)) return EA_ERR_ARG;
-  if (!c->rs) return EA_OK;
-  if (set_device(c)) return EA_ERR_CUDA;
-  cudaEvent_t e;
-  CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  CU(cudaEventRecord(e, c->rs));
-  CU(cudaStreamWaitEvent(c->st, e, 0));
-  CU(cudaEventDestroy(e));
-  return EA_OK;
+  return check(c) ? EA_ERR_ARG : EA_OK;  // all of a job's work runs on its stream
 }
 
 int ea_get_stream(ea_ctx *c, void **stream) {
@@ -608,16 +500,10 @@ int ea_set_generators(ea_ctx *c, const ea_generators *gen, const ea_hq *pt) {
   CU(cudaMemcpyAsync(c->j.rc, &gen->rc, sizeof(ea_hq), cudaMemcpyHostToDevice, c->st));
   CU(cudaMemcpyAsync(c->j.pt, pt, sizeof(ea_hq) * g.ns * g.NR, cudaMemcpyHostToDevice, c->st));
   CU(cudaStreamSynchronize(c->st));
-  // The same cluster seed and offset as the job's own continue its generator
-  // (uniforms drawn ahead included), as the reference process keeps its
-  // generator across bins; other values start a new generator there, as
+  // The same cluster seed and offset as the job's own continue its generator,
+  // as the reference process keeps its generator across bins; other values start a new generator there, as
   // ClusterInit does on a restart.
-  if (c->gen && (gen->seed_cluster != c->seed_cluster || gen->cuda_rng_offset != c->cuda_rng_offset)) {
-    CU(cudaStreamSynchronize(c->rs));
-    curandDestroyGenerator(c->gen);
-    c->gen = nullptr;
-    c->ready = 0;
-  }
+  if (gen->seed_cluster != c->seed_cluster || gen->cuda_rng_offset != c->cuda_rng_offset) c->xw_ready = false;
   c->cuda_rng_offset = gen->cuda_rng_offset;
   c->seed_cluster = gen->seed_cluster;
   return EA_OK;
@@ -715,19 +601,19 @@ int ea_get_counter(ea_ctx *c, int64_t *iter) {
 // Hot path
 // ---------------------------------------------------------------------------
 // Event pair around one launch when profiling is on (ea_profile).
-static cudaEvent_t prof_begin(ea_ctx *c, cudaStream_t st = nullptr) {
+static cudaEvent_t prof_begin(ea_ctx *c) {
   if (!c->prof_on) return nullptr;
   cudaEvent_t e;
   if (cudaEventCreate(&e) != cudaSuccess) return nullptr;
-  cudaEventRecord(e, st ? st : c->st);
+  cudaEventRecord(e, c->st);
   return e;
 }
 
-static void prof_end(ea_ctx *c, int kind, cudaEvent_t b, cudaStream_t st = nullptr) {
+static void prof_end(ea_ctx *c, int kind, cudaEvent_t b) {
   if (!b) return;
   cudaEvent_t e;
   if (cudaEventCreate(&e) != cudaSuccess) return;
-  cudaEventRecord(e, st ? st : c->st);
+  cudaEventRecord(e, c->st);
   c->prof_ev[kind].push_back({b, e});
 }
 
@@ -789,22 +675,27 @@ int ea_parallel_tempering(ea_ctx *c) {
   return pt(c);
 }
 
-static int ensure_cluster(ea_ctx *c, int nclust) {
+// st: the stream the move's kernels run on.
+static int ensure_cluster(ea_ctx *c, int nclust, cudaStream_t st) {
   const Geometry &g = c->g;
-  if (!c->rs) {
-    int least = 0, greatest = 0;
-    CU(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    CU(cudaStreamCreateWithPriority(&c->rs, cudaStreamNonBlocking, greatest));
-  }
-  if (!c->drawn[0]) {
-    for (int s = 0; s < 2; ++s) {
-      CU(cudaEventCreateWithFlags(&c->drawn[s], cudaEventDisableTiming));
-      CU(cudaEventCreateWithFlags(&c->used[s], cudaEventDisableTiming));
+  JobDev &j = c->j;
+  if (!j.xw_bits) {
+    j.xw_n = 2ull * g.V * g.NB * g.ns;
+    if (j.xw_n >> 36) return fail(EA_ERR_NOMEM, "%llu cluster coins a move", j.xw_n);
+    j.xw_seg = xw_segments(j.xw_n);
+    j.xw_w = xw_rows(j.xw_n, j.xw_seg);
+    CU(dalloc(j.xw_bits, xw_words(j.xw_n)));
+    CU(dalloc(j.xw_state, (size_t)j.xw_seg * 6 * kXwStreams));
+    CU(dalloc(j.xw_pos, 2));
+    CU(dalloc(c->xw_mat, 2 * (size_t)kXwMat));
+    j.xw_jump = c->xw_mat;
+    if (j.xw_seg > 1) {
+      std::vector<uint32_t> m(2 * (size_t)kXwMat);
+      xw_jump(j.xw_n / kXwStreams - j.xw_w, m.data());
+      xw_jump(j.xw_w, m.data() + kXwMat);
+      CU(cudaMemcpy(c->xw_mat, m.data(), m.size() * 4, cudaMemcpyHostToDevice));
     }
   }
-  for (auto &set : c->U)
-    for (double *&u : set)
-      if (!u) CU(dalloc(u, (size_t)g.V * g.NB * g.ns));
   if (nclust > c->nclust_cap) {
     CU(cudaStreamSynchronize(c->st));
     if (c->label) cudaFree(c->label);
@@ -821,14 +712,11 @@ static int ensure_cluster(ea_ctx *c, int nclust) {
   c->j.Q = c->Q;
   c->j.nclust = nclust;
   set_dividers(c->j);
-  if (!c->gen) {
+  if (!c->xw_ready) {
     // ClusterInit (HoudayerXEA.cu:174-178): default pseudo generator (XORWOW),
     // seed_Cluster, and the offset already consumed.
-    CR(curandCreateGenerator(&c->gen, CURAND_RNG_PSEUDO_DEFAULT));
-    CR(curandSetPseudoRandomGeneratorSeed(c->gen, (unsigned long long)c->seed_cluster));
-    if (c->cuda_rng_offset > 0) CR(curandSetGeneratorOffset(c->gen, c->cuda_rng_offset));
-    CR(curandSetStream(c->gen, c->rs));
-    c->ready = 0;
+    CU(launch_xw_init(j, (unsigned long long)c->seed_cluster, c->cuda_rng_offset, c->xw_mat + kXwMat, st));
+    c->xw_ready = true;
   }
   return EA_OK;
 }
@@ -838,62 +726,34 @@ static int norm_nclust(const Geometry &g, int nclust) {
   return nclust > g.NB ? g.NB : nclust;
 }
 
-// ClusterStep's uniforms (HoudayerXEA.cu:189-195) for both groups of one move,
-// V*NB*nsamples doubles per group in the reference's call sizes, into set
-// `set` once the move that last read it has finished.
-static int houdayer_draw(ea_ctx *c, int set) {
-  const Geometry &g = c->g;
-  const size_t tot = (size_t)g.V * g.NB * g.ns;
-  CU(cudaStreamWaitEvent(c->rs, c->used[set], 0));
-  cudaEvent_t b = prof_begin(c, c->rs);
-  for (int grp = 0; grp < 2; ++grp) CR(curandGenerateUniformDouble(c->gen, c->U[set][grp], tot));
-  prof_end(c, EA_K_RNG, b, c->rs);
-  CU(cudaEventRecord(c->drawn[set], c->rs));
-  return EA_OK;
-}
-
-// Everything of a move that happens before its kernels: buffers, the
-// generator, and the uniforms of this move (and of the next one, drawn ahead).
-static int houdayer_prepare(ea_ctx *c, int nclust) {
+// Everything of a move that happens before its kernels on stream st: buffers
+// and the generator's states.
+static int houdayer_prepare(ea_ctx *c, int nclust, cudaStream_t st) {
   const Geometry &g = c->g;
   if (g.NR < 4) return fail(EA_ERR_ARG, "the Houdayer move needs at least 2 replicas per group");
-  int rc = ensure_cluster(c, norm_nclust(g, nclust));
-  if (rc) return rc;
-  if (c->ready == 0) {
-    if ((rc = houdayer_draw(c, c->cur))) return rc;
-    c->ready = 1;
-  }
-  if (c->ready == 1) {
-    if ((rc = houdayer_draw(c, c->cur ^ 1))) return rc;
-    c->ready = 2;
-  }
-  return EA_OK;
+  return ensure_cluster(c, norm_nclust(g, nclust), st);
 }
 
-// After the move's kernels were enqueued on stream s.
-static int houdayer_finish(ea_ctx *c, cudaStream_t s) {
-  const Geometry &g = c->g;
-  CU(cudaEventRecord(c->used[c->cur], s));
-  c->cur ^= 1;
-  c->ready = 1;
-  c->cuda_rng_offset += 2 * (uint64_t)g.V * g.NB * g.ns;
+// After the move's kernels were enqueued: ClusterStep's uniforms
+// (HoudayerXEA.cu:189-195), V*NB*nsamples a group, are consumed.
+static void houdayer_finish(ea_ctx *c) {
+  c->cuda_rng_offset += c->j.xw_n;
   c->energies_fresh = false;
-  return EA_OK;
 }
 
 static int houdayer(ea_ctx *c, int nclust) {
-  int rc = houdayer_prepare(c, nclust);
+  int rc = houdayer_prepare(c, nclust, c->st);
   if (rc) return rc;
-  CU(launch_houdayer_pairs(c->j, c->st));
-  CU(cudaStreamWaitEvent(c->st, c->drawn[c->cur], 0));
+  cudaEvent_t b = prof_begin(c);
+  CU(launch_move_start(c->j, c->st));
+  prof_end(c, EA_K_RNG, b);
   for (int grp = 0; grp < 2; ++grp) {
-    JobDev jg = c->j;
-    jg.U = c->U[c->cur][grp];
-    cudaEvent_t b = prof_begin(c);
-    CU(launch_houdayer_group(jg, grp, c->st));
+    b = prof_begin(c);
+    CU(launch_houdayer_group(c->j, grp, c->st));
     prof_end(c, EA_K_CLUSTER, b);
   }
-  return houdayer_finish(c, c->st);
+  houdayer_finish(c);
+  return EA_OK;
 }
 
 int ea_houdayer(ea_ctx *c, int32_t nclust) {
@@ -1031,7 +891,6 @@ struct ea_batch {
   BatchDev bd{};
   cudaGraphExec_t cycle = nullptr;
   int cycle_ptfr = -1;
-  UTable u{};  // uniforms of the current group, by job
   float tuned_ms = 0.f;  // autotuner: two sweeps of the chosen tile width
 };
 
@@ -1084,7 +943,6 @@ static int batch_upload(ea_batch *b) {
   int slab_threads = 32, flip_smem = 0;
   for (int i = 0; i < n; ++i) {
     hj[i] = b->jobs[i]->j;
-    hj[i].U = nullptr;
     uint32_t cnt[KB_COUNT];
     batch_blocks(hj[i], cnt);
     for (int k = 0; k < KB_COUNT; ++k) hp[(size_t)k * (n + 1) + i + 1] = hp[(size_t)k * (n + 1) + i] + cnt[k];
@@ -1124,7 +982,7 @@ static int batch_upload(ea_batch *b) {
   b->bd.ctr = b->d_ctr;
   // chunks of work items a block takes at a time: one heavy item, or several
   // light ones so that the job lookup and the fetch are amortised
-  const uint32_t chunk[KB_COUNT] = {1, 4, 1, 4, 4, 1, 4, 4, 1};
+  const uint32_t chunk[KB_COUNT] = {1, 4, 1, 4, 4, 1, 4, 4, 1, 1};
   for (int k = 0; k < KB_COUNT; ++k) b->bd.chunk[k] = chunk[k];
   if (b->bd.total[KB_SWEEP] >= 8u * 304u) b->bd.chunk[KB_SWEEP] = 2;
   // the cycle graph holds the descriptor by value
@@ -1356,25 +1214,19 @@ static int batch_houdayer(ea_batch *b, int nclust) {
   const int n = (int)b->jobs.size();
   int rc;
   for (ea_ctx *c : b->jobs)
-    if ((rc = houdayer_prepare(c, nclust))) return rc;
+    if ((rc = houdayer_prepare(c, nclust, b->bs))) return rc;
   if ((rc = batch_upload(b))) return rc;
-  for (ea_ctx *c : b->jobs) CU(cudaStreamWaitEvent(b->bs, c->drawn[c->cur], 0));
-  CU(batch_pairs(b->bd, b->bs));
-  UTable &u = b->u;
+  CU(batch_move_start(b->bd, b->bs));
   for (int grp = 0; grp < 2; ++grp) {
-    for (int i = 0; i < n; ++i) u.u[i] = b->jobs[i]->U[b->jobs[i]->cur][grp];
-    CU(batch_houdayer_group(b->bd, u, grp, b->bs));
+    CU(batch_houdayer_group(b->bd, grp, b->bs));
     // jobs whose planes exceed the slab labelling take the one-job path
     for (int i = 0; i < n; ++i) {
       const uint32_t *pre = b->up_pre.data() + (size_t)KB_SLAB * (n + 1);
       if (pre[i + 1] != pre[i]) continue;
-      JobDev jg = b->jobs[i]->j;
-      jg.U = u.u[i];
-      CU(launch_houdayer_group(jg, grp, b->bs));
+      CU(launch_houdayer_group(b->jobs[i]->j, grp, b->bs));
     }
   }
-  for (ea_ctx *c : b->jobs)
-    if ((rc = houdayer_finish(c, b->bs))) return rc;
+  for (ea_ctx *c : b->jobs) houdayer_finish(c);
   return EA_OK;
 }
 
@@ -1412,7 +1264,7 @@ int ea_batch_run_bin(ea_batch *b, const ea_cadence *cad) {
     CU(cudaMemsetAsync(c->avgE, 0, nsr * g.NB * 8, b->bs));
     CU(cudaMemsetAsync(c->hist, 0, nsr * maxit * g.NB, b->bs));
     if (cad->cluster) {
-      const int rc = ensure_cluster(c, norm_nclust(g, cad->nclust));
+      const int rc = ensure_cluster(c, norm_nclust(g, cad->nclust), b->bs);
       if (rc) return rc;
     }
   }
@@ -1534,9 +1386,11 @@ int ea_job_bytes(const ea_geom *gp, const ea_cadence *cad, const double *betas, 
   add(nsr * maxit * NB);                                     // temperature history
   if (cad && cad->cluster) {
     const uint64_t ncl = (uint64_t)norm_nclust(g, cad->nclust);
-    for (int k = 0; k < 4; ++k) add(V * NB * g.ns * 8);      // uniforms: two sets of two groups
+    // Four arrays of uniforms as doubles: what a move's buffers once took, and
+    // what budgets are sized by.  Its coins and generator states take less.
+    for (int k = 0; k < 4; ++k) add(V * NB * g.ns * 8);
     add(V * ncl * g.ns * 4); add(V / 32 * ncl * g.ns * 4); add(2 * half * ncl * g.ns * 8);
-    tot += 4ull << 20;                                       // cuRAND generator state
+    tot += 4ull << 20;
   }
   *bytes = tot + (4ull << 20);                               // streams, events, pages of the small allocations
   return EA_OK;

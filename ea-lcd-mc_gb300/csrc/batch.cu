@@ -11,6 +11,7 @@ void batch_blocks(const JobDev &j, uint32_t out[KB_COUNT]) {
   out[KB_REDUCE] = (nsrb + 255) / 256;
   out[KB_PT] = (uint32_t)(j.ns * ((j.NR + 7) / 8));
   out[KB_MEASURE] = (nsrb + 255) / 256;
+  out[KB_START] = j.nclust > 0 ? 1 + (uint32_t)(j.xw_seg * (kXwStreams / 256)) : 0;
   int D, P, nslab;
   if (j.nclust > 0 && slab_shape(j, &D, &P, &nslab) && flip_smem_bytes(j) <= kFlipMaxSmem) {
     out[KB_OVERLAP] = (uint32_t)((2 * j.half + 255) / 256) * nlat;
@@ -109,11 +110,6 @@ __global__ void kb_measure(const __grid_constant__ BatchDev b, int itm) {
   }
 }
 
-__global__ void kb_pairs(const __grid_constant__ BatchDev b) {
-  const int jb = blockIdx.x * blockDim.x + threadIdx.x;
-  if (jb < b.njobs && b.jobs[jb].nclust > 0) pairs_body(b.jobs[jb]);
-}
-
 __global__ void kb_overlap(const __grid_constant__ BatchDev b, int g) {
   BATCH_LOOP(KB_OVERLAP) {
     const int jb = item_job(pre, b.njobs, v);
@@ -163,13 +159,24 @@ __global__ void kb_cc_compress(const __grid_constant__ BatchDev b) {
   }
 }
 
-__global__ void __launch_bounds__(512) kb_flip(const __grid_constant__ BatchDev b, const __grid_constant__ UTable u,
-                                               int g) {
+__global__ void __launch_bounds__(256) kb_move_start(const __grid_constant__ BatchDev b) {
+  __shared__ __align__(16) uint32_t s_m[kXwMat];
+  BATCH_LOOP(KB_START) {
+    const int jb = item_job(pre, b.njobs, v);
+    const JobDev jd = b.jobs[jb];
+    const int blk = (int)(v - __ldg(pre + jb));
+    if (blk > 0) xw_body(jd, blk - 1, s_m);
+    else if (threadIdx.x == 0) pairs_body(jd);
+  }
+  }
+}
+
+__global__ void __launch_bounds__(512) kb_flip(const __grid_constant__ BatchDev b, int g) {
   extern __shared__ uint32_t s_flip[];
   BATCH_LOOP(KB_FLIP) {
     const int jb = item_job(pre, b.njobs, v);
     const JobDev jd = b.jobs[jb];
-    flip_body(jd, u.u[jb], g, (size_t)(v - __ldg(pre + jb)), s_flip + 64, reinterpret_cast<int *>(s_flip));
+    flip_body(jd, g, (size_t)(v - __ldg(pre + jb)), s_flip + 64, reinterpret_cast<int *>(s_flip));
     __syncthreads();
   }
   }
@@ -270,19 +277,19 @@ cudaError_t batch_measure(const BatchDev &b, int itm, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t batch_pairs(const BatchDev &b, cudaStream_t st) {
-  kb_pairs<<<(b.njobs + 127) / 128, 128, 0, st>>>(b);
+cudaError_t batch_move_start(const BatchDev &b, cudaStream_t st) {
+  if (b.total[KB_START]) kb_move_start<<<grid_for(chunks(b, KB_START), 8), 256, 0, st>>>(b);
   return cudaGetLastError();
 }
 
-cudaError_t batch_houdayer_group(const BatchDev &b, const UTable &u, int g, cudaStream_t st) {
+cudaError_t batch_houdayer_group(const BatchDev &b, int g, cudaStream_t st) {
   if (!b.total[KB_SLAB]) return cudaSuccess;
   kb_overlap<<<grid_for(chunks(b, KB_OVERLAP), 8), 256, 0, st>>>(b, g);
   const int per_sm = b.slab_threads > 0 ? 2048 / b.slab_threads : 1;
   kb_cc_slab<<<grid_for(chunks(b, KB_SLAB), per_sm < 1 ? 1 : per_sm), b.slab_threads, 0, st>>>(b);
   kb_cc_merge<<<grid_for(chunks(b, KB_MERGE), 8), 256, 0, st>>>(b);
   kb_cc_compress<<<grid_for(chunks(b, KB_COMPRESS), 8), 256, 0, st>>>(b);
-  kb_flip<<<grid_for(chunks(b, KB_FLIP), 4), 512, b.flip_smem, st>>>(b, u, g);
+  kb_flip<<<grid_for(chunks(b, KB_FLIP), 4), 512, b.flip_smem, st>>>(b, g);
   return cudaGetLastError();
 }
 

@@ -9,7 +9,7 @@
 namespace eagb {
 
 // Work-list kinds: the blocks of one job for each one-job kernel.
-enum { KB_SWEEP = 0, KB_REDUCE, KB_PT, KB_MEASURE, KB_OVERLAP, KB_SLAB, KB_MERGE, KB_COMPRESS, KB_FLIP, KB_COUNT };
+enum { KB_SWEEP = 0, KB_REDUCE, KB_PT, KB_MEASURE, KB_OVERLAP, KB_SLAB, KB_MERGE, KB_COMPRESS, KB_FLIP, KB_START, KB_COUNT };
 
 constexpr int kBatchMaxJobs = 1024;
 
@@ -29,11 +29,6 @@ struct BatchDev {
   int flip_smem;     // dynamic SMEM of the flip (largest lattice)
 };
 
-// Uniforms of the current group for every job (kernel parameter).
-struct UTable {
-  const double *u[kBatchMaxJobs];
-};
-
 // Blocks of job j for each kind (the one-job launch geometry, flattened).
 void batch_blocks(const JobDev &j, uint32_t out[KB_COUNT]);
 
@@ -47,7 +42,7 @@ cudaError_t batch_sweep(const BatchDev &b, int NR, int KT, int NBmax, int parity
 cudaError_t batch_energy_reduce(const BatchDev &b, cudaStream_t st);
 cudaError_t batch_pt(const BatchDev &b, cudaStream_t st);
 cudaError_t batch_measure(const BatchDev &b, int itm, cudaStream_t st);
-cudaError_t batch_pairs(const BatchDev &b, cudaStream_t st);
-cudaError_t batch_houdayer_group(const BatchDev &b, const UTable &u, int g, cudaStream_t st);
+cudaError_t batch_move_start(const BatchDev &b, cudaStream_t st);
+cudaError_t batch_houdayer_group(const BatchDev &b, int g, cudaStream_t st);
 
 }  // namespace eagb

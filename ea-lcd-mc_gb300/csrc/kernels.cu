@@ -45,8 +45,6 @@ __global__ void k_measure(const __grid_constant__ JobDev j, int itm) {
   measure_body(j, blockIdx.x * blockDim.x + threadIdx.x, itm);
 }
 
-__global__ void k_hou_pairs(const __grid_constant__ JobDev j) { pairs_body(j); }
-
 __global__ void k_hou_overlap(const __grid_constant__ JobDev j, int g) {
   overlap_body(j, g, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
 }
@@ -67,13 +65,13 @@ __global__ void k_cc_compress(const __grid_constant__ JobDev j, int D, int nslab
 
 __global__ void __launch_bounds__(512) k_hou_flip(const __grid_constant__ JobDev j, int g) {
   extern __shared__ uint32_t s_flip[];
-  flip_body(j, j.U, g, blockIdx.x, s_flip + 64, reinterpret_cast<int *>(s_flip));
+  flip_body(j, g, blockIdx.x, s_flip + 64, reinterpret_cast<int *>(s_flip));
 }
 
 size_t flip_smem_bytes(const JobDev &j) { return 256 + (size_t)j.V / 8; }
 
-__global__ void __launch_bounds__(256) k_hou_select(const __grid_constant__ JobDev j) {
-  select_body(j, j.U, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(256) k_hou_select(const __grid_constant__ JobDev j, int g) {
+  select_body(j, g, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
 }
 
 __global__ void __launch_bounds__(256) k_hou_apply(const __grid_constant__ JobDev j, int g) {
@@ -233,11 +231,6 @@ cudaError_t launch_measure(const JobDev &j, int itm, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_houdayer_pairs(const JobDev &j, cudaStream_t st) {
-  k_hou_pairs<<<1, 1, 0, st>>>(j);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_houdayer_group(const JobDev &j, int g, cudaStream_t st) {
   const size_t ns = (size_t)j.ns * j.nclust * j.V;
   const unsigned bs = (unsigned)((ns + 255) / 256);
@@ -272,7 +265,7 @@ cudaError_t launch_houdayer_group(const JobDev &j, int g, cudaStream_t st) {
       k_cc_union<<<bs, 256, 0, st>>>(j);
     }
   }
-  k_hou_select<<<dim3((j.V + 255) / 256, nlat), 256, 0, st>>>(j);
+  k_hou_select<<<dim3((j.V + 255) / 256, nlat), 256, 0, st>>>(j, g);
   k_hou_apply<<<dim3((2 * j.half + 3) / 4, nlat), 256, 0, st>>>(j, g);
   return cudaGetLastError();
 }

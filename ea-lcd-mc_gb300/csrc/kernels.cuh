@@ -65,8 +65,14 @@ struct JobDev {
   unsigned long long *Q;            // [s][nclust][2][half] overlap words
   uint32_t *label;                  // [s][nclust][V] natural order
   uint32_t *sel;                    // [s][nclust][V / 32] cluster selection bits, natural order
-  const double *U;                  // [s][NB][V] uniforms of the current group
   int nclust;
+  // cluster coins (xorwow.cuh): [U < 0.5] of the move's uniforms, both groups
+  uint32_t *xw_bits;                // bit (xw_pos[0] mod 32) + i: coin i of the move
+  uint32_t *xw_state;               // [segment][d, v0..v4][4096] generator states at the next move's rows
+  const uint32_t *xw_jump;          // advances a state from its segment's end to the next move's segment
+  unsigned long long *xw_pos;       // first position of this move, of the next
+  unsigned long long xw_n;          // coins of a move: 2 groups x [s][NB][V]
+  int xw_seg, xw_w;                 // segments, rows of a segment
   // x coordinate against which site 0 tests its periodic -x bond.  The
   // reference computes (ltid-1+nx)%nx with a 32-bit ltid (HoudayerXEA.cu:96),
   // i.e. (2^32-1+L) mod L, which differs from L-1 unless L is a power of two;
@@ -108,7 +114,6 @@ cudaError_t launch_energy(const JobDev &j, cudaStream_t st);
 cudaError_t launch_energy_reduce(const JobDev &j, cudaStream_t st);
 cudaError_t launch_pt(const JobDev &j, cudaStream_t st);
 cudaError_t launch_measure(const JobDev &j, int itm, cudaStream_t st);
-cudaError_t launch_houdayer_pairs(const JobDev &j, cudaStream_t st);
 cudaError_t launch_houdayer_group(const JobDev &j, int group, cudaStream_t st);
 
 }  // namespace eagb

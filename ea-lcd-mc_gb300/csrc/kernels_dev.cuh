@@ -9,6 +9,7 @@
 // relative to the reference project).
 #pragma once
 #include "kernels.cuh"
+#include "xorwow.cuh"
 
 namespace eagb {
 
@@ -409,6 +410,11 @@ __device__ __forceinline__ void pairs_body(const JobDev &j) {
 // q = s_r1 ^ s_r2 per (sample, beta < nclust, parity, half) (main.cu:889-936).
 __device__ __forceinline__ void overlap_body(const JobDev &j, int g, int w, size_t lat) {
   if (w >= 2 * j.half) return;
+  if (g == 0 && lat == 0 && w == 0) {  // the coins are drawn: the next move's continue where they ended
+    const u64 pos = j.xw_pos[1];
+    j.xw_pos[0] = pos;
+    j.xw_pos[1] = pos + j.xw_n;
+  }
   const size_t i = lat * 2 * j.half + w;
   const int p = w >= j.half, k = w - p * j.half;
   const int s = j.fd_nclust.div((uint32_t)lat), b = (int)lat - s * j.nclust;
@@ -603,17 +609,19 @@ __device__ __forceinline__ int word_site0(const JobDev &j, int p, int k) {
 // natural order (coalesced label reads, one ballot per 32 sites); then each
 // word gathers its 64 bits from SMEM, q' = q xor sel, and s_r1 ^= q',
 // s_r2 ^= q'.  s_bits holds V/32 words, s_off 64.
-__device__ __forceinline__ void flip_body(const JobDev &j, const double *U, int g, size_t lat, uint32_t *s_bits,
+__device__ __forceinline__ void flip_body(const JobDev &j, int g, size_t lat, uint32_t *s_bits,
                                           int *s_off) {
   const int t = threadIdx.x, nth = blockDim.x;
   const int s = j.fd_nclust.div((uint32_t)lat), b = (int)lat - s * j.nclust;
   const uint32_t *lab = j.label + lat * j.V;
-  const double *u = U + ((size_t)s * j.NB + b) * j.V;
+  const u64 ub = xw_base(j, g) + ((u64)s * j.NB + b) * (u64)j.V;
+  const uint32_t *u = j.xw_bits + (ub >> 5);
+  const uint32_t us = (uint32_t)ub & 31u;
   if (t < 64) s_off[t] = word_bit_offset(j, t);
   for (int base = 0; base < j.V; base += nth) {
     const int site = base + t;
     bool sel = false;
-    if (site < j.V) sel = __ldg(u + cc_find(lab, (uint32_t)site)) < 0.5;
+    if (site < j.V) sel = xw_coin(u, us + cc_find(lab, (uint32_t)site));
     const unsigned ball = __ballot_sync(0xffffffffu, sel);
     if ((t & 31) == 0 && site < j.V) s_bits[site >> 5] = ball;
   }
@@ -642,12 +650,13 @@ __device__ __forceinline__ void flip_body(const JobDev &j, const double *U, int 
 // [U(root(i)) < 0.5] for site i (HoudayerXEA.cu:358-374).  Consecutive lanes
 // take consecutive sites, so the label reads are coalesced; the decisions of
 // a lattice (V / 8 bytes) then stay in cache for the word-order flip.
-__device__ __forceinline__ void select_body(const JobDev &j, const double *U, int site, size_t lat) {
+__device__ __forceinline__ void select_body(const JobDev &j, int g, int site, size_t lat) {
   const int s = j.fd_nclust.div((uint32_t)lat), b = (int)lat - s * j.nclust;
   bool sel = false;
   if (site < j.V) {
     const uint32_t root = cc_find(j.label + lat * j.V, (uint32_t)site);
-    sel = __ldg(U + ((size_t)s * j.NB + b) * j.V + root) < 0.5;
+    const u64 ub = xw_base(j, g) + ((u64)s * j.NB + b) * (u64)j.V;
+    sel = xw_coin(j.xw_bits + (ub >> 5), ((uint32_t)ub & 31u) + root);
   }
   const unsigned ball = __ballot_sync(0xffffffffu, sel);
   if ((threadIdx.x & 31) == 0 && site < j.V) j.sel[lat * (j.V >> 5) + (site >> 5)] = ball;

@@ -254,9 +254,6 @@ int create_job(ea_server *s, Job *j) {
   ea_ctx *c = nullptr;
   int rc = ea_create(&j->req.geom, s->cfg.device, &c);
   if (rc) return rc;
-  // the batch draws every job's cluster uniforms on the job's own stream;
-  // no SM partition per job
-  if (!rc) rc = ea_set_rng_sms(c, 0);
   if (!rc) rc = ea_set_temperatures(c, j->betas.data(), j->cum.data());
   if (!rc) rc = ea_init_run(c, j->req.masters, nullptr, j->req.iter0, j->req.jobid);
   if (rc) {
