@@ -533,242 +533,338 @@ __device__ __forceinline__ void sp_cluster_body(const SpDev &d, int g, int blk, 
   for (int i = threadIdx.x; i < V; i += blockDim.x) Qb[(size_t)i * 8] = fb[i];
 }
 
-// The same labelling for 4 samples at a time, for lattices up to
-// kSpCluster4MaxV sites: a site's 4 labels sit in one 16-byte SMEM slot and
-// its 4 bond masks in one word (sample l at bits 8l..8l+5), so that one
-// neighbour-table load and one loop step serve the 4 samples (the 1-sample
-// form spends ~600 instructions per site and lattice, mostly on those).
-// Roots, coins and flip bytes are those of sp_cluster_body.
-__device__ __forceinline__ uint32_t spread4(uint32_t x) {
-  return (x & 1u) | ((x & 2u) << 7) | ((x & 4u) << 14) | ((x & 8u) << 21);
-}
-
-__device__ __forceinline__ void sp_cluster4_body(const SpDev &d, int g, int blk, uint32_t *sm) {
-  const unsigned long long key = sp_cluster_key(d);
-  const int V = d.V, nc = d.nclust;
-  uint4 *lab = reinterpret_cast<uint4 *>(sm);                          // [V]
-  uint32_t *lab1 = sm;                                                 // the same, one label per word
-  uint32_t *bond = sm + 4 * (size_t)V;                                 // [V]
-  uint8_t *qb = reinterpret_cast<uint8_t *>(bond + V);                 // [V]
-  uint8_t *fb = qb + V;                                                // [V]
-  const int grp = blk & 7, lat = blk >> 3;
-  const int b = lat % nc, w = lat / nc;
-  uint8_t *Qb = reinterpret_cast<uint8_t *>(d.Q + (size_t)lat * V) + grp;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    qb[i] = Qb[(size_t)i * 8];
-    fb[i] = 0;
-  }
-  __syncthreads();
-  const unsigned long long mv = *d.move;
-  for (int h = 0; h < 2; ++h) {
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const uint32_t qi = (qb[i] >> (4 * h)) & 15u;
-      uint32_t m = 0;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        const int p = __ldg(d.nb + (size_t)i * 6 + q);
-        if (p < i) m |= spread4(~(qi ^ (qb[p] >> (4 * h))) & 15u) << q;
-      }
-      bond[i] = m;
-      lab[i] = make_uint4((uint32_t)i, (uint32_t)i, (uint32_t)i, (uint32_t)i);
-    }
-    __syncthreads();
-    for (;;) {
-      int hooked = 0;
-      for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        const uint32_t m = bond[i];
-        if (!m) continue;
-        const uint4 li4 = lab[i];
-        const uint32_t li[4] = {li4.x, li4.y, li4.z, li4.w};
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-          const uint32_t mq = (m >> q) & 0x01010101u;
-          if (!mq) continue;
-          const int p = __ldg(d.nb + (size_t)i * 6 + q);
-          const uint4 lj4 = lab[p];
-          const uint32_t lj[4] = {lj4.x, lj4.y, lj4.z, lj4.w};
-#pragma unroll
-          for (int l = 0; l < 4; ++l)
-            if (((mq >> (8 * l)) & 1u) && lj[l] != li[l]) {
-              atomicMin(&lab1[4 * (size_t)max(li[l], lj[l]) + l], min(li[l], lj[l]));
-              hooked = 1;
-            }
-        }
-      }
-      if (!__syncthreads_or(hooked)) break;
-      for (;;) {
-        int moved = 0;
-        for (int i = threadIdx.x; i < V; i += blockDim.x) {
-          const uint4 x = lab[i];
-          const uint4 y = make_uint4(lab1[4 * (size_t)x.x], lab1[4 * (size_t)x.y + 1], lab1[4 * (size_t)x.z + 2],
-                                     lab1[4 * (size_t)x.w + 3]);
-          if (y.x != x.x || y.y != x.y || y.z != x.z || y.w != x.w) { lab[i] = y; moved = 1; }
-        }
-        if (!__syncthreads_or(moved)) break;
-      }
-    }
-    // coins of the roots (bits 0..3 of the roots' bond words, no longer needed)
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const uint4 x = lab[i];
-      const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
-      uint32_t c = 0;
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        if (xs[l] != (uint32_t)i) continue;
-        const int lane = grp * 8 + 4 * h + l;
-        const uint32_t tag = (((uint32_t)(w * 64 + lane) << 6 | (uint32_t)b) << 1) | (uint32_t)g;
-        uint32_t v0 = (uint32_t)mv, v1 = (uint32_t)(mv >> 32), v2 = (uint32_t)i, v3 = tag;
-        philox10(v0, v1, v2, v3, (uint32_t)key, (uint32_t)(key >> 32));
-        c |= (v0 & 1u) << l;
-      }
-      bond[i] = c;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const uint4 x = lab[i];
-      const uint32_t f = (bond[x.x] & 1u) | (bond[x.y] & 2u) | (bond[x.z] & 4u) | (bond[x.w] & 8u);
-      fb[i] |= (uint8_t)(f << (4 * h));
-    }
-    __syncthreads();
-  }
-  for (int i = threadIdx.x; i < V; i += blockDim.x) Qb[(size_t)i * 8] = fb[i];
-}
-
-// The same labelling for all 8 samples of the CTA at once, for lattices up
-// to kSpCluster8MaxV sites: 16-bit labels, a site's 8 in one 16-byte SMEM
-// slot, its 8 bond masks in one 64-bit word (sample l at bits 8l..8l+5), so
-// one neighbour-table load and one loop step serve the 8 samples, in a single
-// pass (26 bytes of SMEM per site).  SMEM has no 16-bit atomicMin, so a hook
-// is a plain store: when several threads hook one root in a round, one
-// store stays and the other bonds are hooked again in the next round, as
-// with atomicMin (which keeps one link per root and round as well).  Every
-// value stored is a smaller site of the same cluster, so labels still end at
-// each cluster's smallest site.
-constexpr int kSpCluster8MaxV = 8900;
-
-__device__ __forceinline__ unsigned long long spread8(uint32_t x) {
-  unsigned long long r = 0;
-#pragma unroll
-  for (int l = 0; l < 8; ++l) r |= (unsigned long long)((x >> l) & 1u) << (8 * l);
+// The labelling by runs.  A "run" is a maximal stretch of equal overlap along z
+// of one (x, y) column of one sample; its sites share a cluster, so only its
+// lowest site -- its smallest index -- carries a label, and the bonds along x
+// and y are needed once per pair of touching runs (a "contact").  A thread
+// holds the q bits of one (sample, column, chunk of at most 31 planes) in a
+// word: run starts and contacts are a few bit operations, and walking them
+// touches 2 to 3 times fewer labels than sites.
+//   hook:  every pending contact whose two labels differ hangs the larger
+//          label below the smaller by a plain store (SMEM has no 16-bit
+//          atomicMin): of several stores to one root one stays, and the other
+//          contacts are still pending in the next round.  A contact whose
+//          labels are equal is done for good: they lie in one tree, or are
+//          joined by the pending contact of the thread that stored one of
+//          them in this round.
+//   jump:  every run walks to its root; roots do not change meanwhile, so one
+//          pass leaves every label a root.
+// until a hook pass finds no difference: 3 passes on overlaps of production
+// tubes.  Labels only decrease and stay inside the cluster, so every run ends
+// labelled by its cluster's smallest site, the root the reference takes.
+// NS samples at a time (lanes: NS samples of 32 / NS neighbouring columns, so
+// one 2 NS-byte label slot serves the NS lanes of a column).
+//
+// Bound by instruction issue (63 % of the slots busy, 38 % of the SMEM path, 21
+// of 32 lanes active in the walks).  The forms it replaces labelled every
+// site, 8 samples in lock step with vector label slots, at 72 % of the SMEM
+// path.  A launch on 6144 x 8 lattices of 12 x 12 x 48: 5.08 -> 2.27 ms; one
+// word of it (96 blocks): 155 -> 62 us; 24 x 24 x 192 in slabs: 1.83 -> 0.83
+// ms a group; a move of 16 x 16 x 64 (once one sample at a time): 4.84 -> 0.77
+// ms.
+struct RunShape {
+  int S, nz, H, nch, nseg;  // sites of a plane, planes, planes of a chunk, chunks, column chunks
+};
+__host__ __device__ inline RunShape run_shape(int L, int nz) {
+  RunShape r;
+  r.S = L * L;
+  r.nz = nz;
+  const int n = (nz + 30) / 31;
+  r.H = (nz + n - 1) / n;
+  r.nch = (nz + r.H - 1) / r.H;
+  r.nseg = r.S * r.nch;
   return r;
 }
-
-__device__ __forceinline__ void unpack8(uint4 v, uint32_t l[8]) {
-  l[0] = v.x & 0xFFFFu; l[1] = v.x >> 16; l[2] = v.y & 0xFFFFu; l[3] = v.y >> 16;
-  l[4] = v.z & 0xFFFFu; l[5] = v.z >> 16; l[6] = v.w & 0xFFFFu; l[7] = v.w >> 16;
+// SMEM: run words and contacts [3][nseg][NS] u32, labels [nz S][NS] u16, the
+// column at x + 1 [S] u16, the 8 samples' q bytes [nz S] and (NS < 8) their
+// flip bytes.
+__host__ __device__ inline size_t run_smem(const RunShape &r, int NS) {
+  return (size_t)12 * r.nseg * NS + (size_t)r.nz * r.S * (2 * NS + (NS < 8 ? 2 : 1)) + (size_t)2 * r.S;
+}
+constexpr size_t kRunSmem = 224 * 1024;  // leaves 3 KB for the static SMEM of the batched and persistent kernels
+// Samples at a time for a whole lattice in SMEM; 0: it does not fit.
+__host__ __device__ inline int run_samples(int L, int Lz) {
+  if (L * L * Lz > kSpClusterMaxV) return 0;
+  const RunShape r = run_shape(L, Lz);
+  for (int ns = 8; ns >= 1; ns >>= 1)
+    if (run_smem(r, ns) <= kRunSmem) return ns;
+  return 0;
 }
 
-__device__ __forceinline__ uint4 pack8(const uint32_t l[8]) {
-  return make_uint4(l[0] | (l[1] << 16), l[2] | (l[3] << 16), l[4] | (l[5] << 16), l[6] | (l[7] << 16));
+__device__ __forceinline__ uint32_t run_mask(const RunShape &r, int ch) {
+  return (1u << min(r.H, r.nz - ch * r.H)) - 1u;
+}
+__device__ __forceinline__ uint32_t run_starts(uint32_t m, uint32_t mask) { return ((m ^ (m << 1)) | 1u) & mask; }
+
+// The 8 x 8 bit matrix with byte i, bit j at bit 8 i + j, transposed.
+__device__ __forceinline__ u64 transpose8(u64 x) {
+  u64 t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull;
+  x ^= t ^ (t << 7);
+  t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull;
+  x ^= t ^ (t << 14);
+  t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull;
+  return x ^ t ^ (t << 28);
 }
 
-// The 8-sample lock-step labelling of the sites [base, base + Vs) (all of
-// the lattice, or one slab of z planes): bonds to sites outside the run are
-// left out; labels are local indices (site - base).  SMEM: lab [Vs] (8
-// labels a site), bond [Vs], qb [Vs] (the group's 8 q bits a site).
-__device__ __forceinline__ void sp_label8(const SpDev &d, const uint8_t *Qb, int base, int Vs, unsigned char *sm) {
-  uint4 *lab = reinterpret_cast<uint4 *>(sm);
-  uint16_t *lab16 = reinterpret_cast<uint16_t *>(sm);
-  unsigned long long *bond = reinterpret_cast<unsigned long long *>(sm + (size_t)16 * Vs);
-  uint8_t *qb = sm + (size_t)24 * Vs;
-  for (int i = threadIdx.x; i < Vs; i += blockDim.x) qb[i] = Qb[(size_t)(base + i) * 8];
-  __syncthreads();
-  for (int i = threadIdx.x; i < Vs; i += blockDim.x) {
-    const uint32_t qi = qb[i];
-    const int gi = base + i;
-    unsigned long long m = 0;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      const int p = __ldg(d.nb + (size_t)gi * 6 + q);
-      if (p >= base && p < gi) m |= spread8(~(qi ^ qb[p - base]) & 0xFFu) << q;
-    }
-    bond[i] = m;
-    const uint32_t ii = (uint32_t)i | ((uint32_t)i << 16);
-    lab[i] = make_uint4(ii, ii, ii, ii);
+template <int NS>
+struct RunLab {
+  RunShape r;
+  int L;
+  uint32_t *qm, *cx, *cy;  // [nseg][NS]: q bits, pending contacts with the column at x + 1 / y + 1 (bit 31 of cy: towards z + H)
+  uint16_t *lab;           // [nz S][NS], valid at run starts
+  uint16_t *nx;            // [S]
+  uint8_t *qb, *fb;        // [nz S]
+
+  __device__ __forceinline__ RunLab(unsigned char *sm, int L_, int nz) : r(run_shape(L_, nz)), L(L_) {
+    qm = reinterpret_cast<uint32_t *>(sm);
+    cx = qm + (size_t)r.nseg * NS;
+    cy = cx + (size_t)r.nseg * NS;
+    lab = reinterpret_cast<uint16_t *>(cy + (size_t)r.nseg * NS);
+    nx = lab + (size_t)r.nz * r.S * NS;
+    qb = reinterpret_cast<uint8_t *>(nx + r.S);
+    fb = qb + (NS < 8 ? (size_t)r.nz * r.S : 0);
   }
-  __syncthreads();
-  const int V = Vs;
-  for (;;) {
+  // the 8 samples' q bytes of the sites from Qb on, one byte of 8 a site
+  __device__ __forceinline__ void load(const uint8_t *Qb) const {
+    for (int i = threadIdx.x; i < r.nz * r.S; i += blockDim.x) qb[i] = Qb[(size_t)i * 8];
+    for (int i = threadIdx.x; i < r.S; i += blockDim.x) nx[i] = (uint16_t)(i % L == L - 1 ? i - (L - 1) : i + 1);
+    __syncthreads();
+  }
+  // the thread's (column chunk, sample) items: body(item, chunk, column)
+  template <class F>
+  __device__ __forceinline__ void items(F &&body) const {
+    const int step = blockDim.x / NS;
+    int sg = threadIdx.x / NS, ch = sg / r.S, col = sg - ch * r.S;
+    for (; sg < r.nseg; sg += step) {
+      body(sg * NS + (int)(threadIdx.x % NS), ch, col);
+      for (col += step; col >= r.S; col -= r.S) ++ch;
+    }
+  }
+  // body(byte of the chunk's plane words, column chunk, chunk, column, planes of that byte)
+  template <class F>
+  __device__ __forceinline__ void bytes(F &&body) const {
+    for (int u = threadIdx.x; u < 4 * r.nseg; u += blockDim.x) {
+      const int j = u / r.nseg, sg = u - j * r.nseg, ch = sg / r.S, col = sg - ch * r.S;
+      body(j, sg, ch, col, min(8, min(r.H, r.nz - ch * r.H) - 8 * j));
+    }
+  }
+  __device__ __forceinline__ uint16_t *slot(int ch, int col) const {
+    return lab + ((size_t)ch * r.H * r.S + col) * NS + threadIdx.x % NS;
+  }
+  __device__ __forceinline__ int next_y(int col) const { return col + L >= r.S ? col + L - r.S : col + L; }
+  // M: the bits of a slot that are its label
+  template <int M = 0xFFFF>
+  __device__ __forceinline__ int root(int x) const {
+    const uint16_t *lane = lab + threadIdx.x % NS;
+    for (int y; (y = lane[x * NS] & M) != x;) x = y;
+    return x;
+  }
+
+  // The pending contacts of two columns: those whose labels still differ.
+  // WALK: the labels may have been hung below others since they were roots.
+  template <bool WALK>
+  __device__ __forceinline__ uint32_t hook(uint32_t c, uint32_t sa, uint32_t sb, const uint16_t *la,
+                                           const uint16_t *lb) const {
+    const int zs = r.S * NS;
+    uint16_t *lane = lab + threadIdx.x % NS;
+    uint32_t keep = 0;
+    while (c) {
+      const uint32_t bit = c & (0u - c), low = bit + (bit - 1u);  // bits up to and with the contact
+      c ^= bit;
+      int a = la[(31 - __clz(sa & low)) * zs], b = lb[(31 - __clz(sb & low)) * zs];
+      if (WALK) {
+        a = root(a);
+        b = root(b);
+      }
+      if (a != b) {
+        keep |= bit;
+        lane[max(a, b) * NS] = (uint16_t)min(a, b);
+      }
+    }
+    return keep;
+  }
+  // One hook pass; whether this thread found labels that differ.
+  template <bool WALK>
+  __device__ __forceinline__ int hooks() const {
+    const int zs = r.S * NS;
     int hooked = 0;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const unsigned long long m = bond[i];
-      if (!m) continue;
-      uint32_t li[8];
-      unpack8(lab[i], li);
-#pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        const unsigned long long mq = (m >> q) & 0x0101010101010101ull;
-        if (!mq) continue;
-        const int p = __ldg(d.nb + (size_t)(base + i) * 6 + q) - base;
-        uint32_t lj[8];
-        unpack8(lab[p], lj);
-#pragma unroll
-        for (int l = 0; l < 8; ++l)
-          if (((mq >> (8 * l)) & 1ull) && lj[l] != li[l]) {
-            lab16[8 * (size_t)max(li[l], lj[l]) + l] = (uint16_t)min(li[l], lj[l]);
-            hooked = 1;
+    items([&](int it, int ch, int col) {
+      uint32_t c = cx[it];
+      const uint32_t d = cy[it];
+      if (!(c | d)) return;
+      const uint32_t mask = run_mask(r, ch), st = run_starts(qm[it], mask);
+      const int row = it - col * NS;  // item of column 0 of the chunk
+      const uint16_t *la = slot(ch, col);
+      if (c) {
+        const int nc = nx[col];
+        c = hook<WALK>(c, st, run_starts(qm[row + nc * NS], mask), la, slot(ch, nc));
+        cx[it] = c;
+        hooked |= c != 0;
+      }
+      if (d) {
+        const int nc = next_y(col);
+        uint32_t e = 0;
+        if (d & 0x7FFFFFFFu)
+          e = hook<WALK>(d & 0x7FFFFFFFu, st, run_starts(qm[row + nc * NS], mask), la, slot(ch, nc));
+        if (d >> 31) {
+          int a = la[(31 - __clz(st)) * zs], b = *slot(ch == r.nch - 1 ? 0 : ch + 1, col);
+          if (WALK) {
+            a = root(a);
+            b = root(b);
           }
-      }
-    }
-    if (!__syncthreads_or(hooked)) break;
-    for (;;) {
-      int moved = 0;
-      for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        uint32_t x[8], y[8];
-        unpack8(lab[i], x);
-        bool ch = false;
-#pragma unroll
-        for (int l = 0; l < 8; ++l) {
-          y[l] = lab16[8 * (size_t)x[l] + l];
-          ch |= y[l] != x[l];
+          if (a != b) {
+            e |= 0x80000000u;
+            lab[max(a, b) * NS + threadIdx.x % NS] = (uint16_t)min(a, b);
+          }
         }
-        if (ch) { lab[i] = pack8(y); moved = 1; }
+        cy[it] = e;
+        hooked |= e != 0;
       }
-      if (!__syncthreads_or(moved)) break;
+    });
+    return __syncthreads_or(hooked);
+  }
+  // Every run's label a root; found(slot of the column, its first index, the
+  // item's roots) may set bits outside M in the roots' slots.
+  template <int M = 0xFFFF, class F>
+  __device__ __forceinline__ void jump(F &&found) const {
+    const int zs = r.S * NS;
+    items([&](int it, int ch, int col) {
+      uint16_t *l = slot(ch, col);
+      const int id = ch * r.H * r.S + col;
+      uint32_t roots = 0;
+      for (uint32_t st = run_starts(qm[it], run_mask(r, ch)); st; st &= st - 1u) {
+        const uint32_t bit = st & (0u - st);
+        const int z = 31 - __clz(bit), x = l[z * zs] & M;
+        if (x == id + z * r.S) {
+          roots |= bit;
+          continue;
+        }
+        const int y = root<M>(x);
+        if (y != x) l[z * zs] = (uint16_t)y;
+      }
+      found(l, id, roots);
+    });
+  }
+
+  // Labels of samples [h NS, (h + 1) NS) from the q bytes; the runs' labels
+  // are left one walk from their roots (jump).  wrap: the last plane is bonded
+  // to the first; corner: only its last column is.
+  __device__ __forceinline__ void label(int h, bool wrap, bool corner) const {
+    const int zs = r.S * NS;
+    bytes([&](int j, int sg, int ch, int col, int n) {
+      const uint8_t *p = qb + (ch * r.H + 8 * j) * r.S + col;
+      u64 x = 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < n) x |= (u64)p[k * r.S] << (8 * k);
+      x = transpose8(x) >> (8 * NS * h);
+      uint8_t *o = reinterpret_cast<uint8_t *>(qm + (size_t)sg * NS) + j;
+#pragma unroll
+      for (int l = 0; l < NS; ++l) o[4 * l] = (uint8_t)(x >> (8 * l));
+    });
+    __syncthreads();
+    items([&](int it, int ch, int col) {
+      const uint32_t mask = run_mask(r, ch), m = qm[it], st = run_starts(m, mask);
+      const int row = it - col * NS, id = ch * r.H * r.S + col;
+      uint16_t *l0 = slot(ch, col);
+      for (uint32_t s = st; s; s &= s - 1u) {
+        const int z = 31 - __clz(s & (0u - s));
+        l0[z * zs] = (uint16_t)(id + z * r.S);
+      }
+      uint32_t n = qm[row + nx[col] * NS], eq = ~(m ^ n) & mask;
+      cx[it] = eq & (st | run_starts(n, mask) | ~(eq << 1));
+      n = qm[row + next_y(col) * NS];
+      eq = ~(m ^ n) & mask;
+      uint32_t c = eq & (st | run_starts(n, mask) | ~(eq << 1));
+      const bool last = ch == r.nch - 1;
+      if (!last || wrap || (corner && col == r.S - 1)) {
+        n = qm[last ? it - ch * r.S * NS : it + r.S * NS];  // the chunk above: its first plane
+        const uint32_t top = (m >> (31 - __clz(mask))) & 1u;
+        if (top == (n & 1u)) c |= 0x80000000u;
+      }
+      cy[it] = c;
+    });
+    __syncthreads();
+    // two rounds on root labels join nearly everything; the few contacts left
+    // walk, which saves a jump pass a round
+    if (!hooks<false>()) return;
+    jump([](uint16_t *, int, uint32_t) {});
+    __syncthreads();
+    if (!hooks<false>()) return;
+    while (hooks<true>()) {
     }
   }
-}
+};
 
-__device__ __forceinline__ void sp_cluster8_body(const SpDev &d, int g, int blk, unsigned char *sm) {
+// One (word, slot, 8 samples) of the move: labels by runs, a coin per root
+// (bit 15 of the root's label: labels are below 2^15), and the flip bytes in
+// place of the overlap bytes.
+template <int NS>
+__device__ __forceinline__ void sp_cluster_runs(const SpDev &d, int g, int blk, unsigned char *sm) {
   const unsigned long long key = sp_cluster_key(d);
-  const int V = d.V, nc = d.nclust;
-  uint4 *lab = reinterpret_cast<uint4 *>(sm);                                  // [V]: 8 labels
-  uint8_t *qb = sm + (size_t)24 * V;                                           // [V] q bits, then coins
-  const int grp = blk & 7, lat = blk >> 3;
+  const int V = d.V, nc = d.nclust, grp = blk & 7, lat = blk >> 3;
   const int b = lat % nc, w = lat / nc;
   uint8_t *Qb = reinterpret_cast<uint8_t *>(d.Q + (size_t)lat * V) + grp;
-  sp_label8(d, Qb, 0, V, sm);
-  // coins of the roots (in qb, no longer needed), then the flip bytes
+  const RunLab<NS> rl(sm, d.L, d.Lz);
+  const RunShape &r = rl.r;
+  const int zs = r.S * NS;
+  rl.load(Qb);
   const unsigned long long mv = *d.move;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    uint32_t x[8];
-    unpack8(lab[i], x);
-    uint32_t c = 0;
+  for (int h = 0; h < 8 / NS; ++h) {
+    rl.label(h, d.bc == EA_PBC, (d.L & 1) != 0);
+    const int lane = grp * 8 + h * NS + (int)(threadIdx.x % NS);
+    const uint32_t tag = (((uint32_t)(w * 64 + lane) << 6 | (uint32_t)b) << 1) | (uint32_t)g;
+    // roots are collected before their coins are drawn: the coins then take as
+    // many steps as the lane with most roots, not one for every run
+    rl.template jump<0x7FFF>([&](uint16_t *l, int id, uint32_t roots) {
+      for (; roots; roots &= roots - 1u) {
+        const int z = 31 - __clz(roots & (0u - roots));
+        uint32_t v0 = (uint32_t)mv, v1 = (uint32_t)(mv >> 32), v2 = (uint32_t)(id + z * r.S), v3 = tag;
+        philox10(v0, v1, v2, v3, (uint32_t)key, (uint32_t)(key >> 32));
+        l[z * zs] = (uint16_t)((uint32_t)(id + z * r.S) | ((v0 & 1u) << 15));
+      }
+    });
+    __syncthreads();
+    rl.items([&](int it, int ch, int col) {
+      const uint16_t *l = rl.slot(ch, col), *ln = rl.lab + threadIdx.x % NS;
+      const uint32_t mask = run_mask(r, ch), s0 = run_starts(rl.qm[it], mask);
+      // the coins' changes from run to run, then summed upwards
+      uint32_t f = 0, prev = 0;
+      for (uint32_t st = s0; st; st &= st - 1u) {
+        const uint32_t bit = st & (0u - st);
+        const uint32_t c = ln[(l[(31 - __clz(bit)) * zs] & 0x7FFF) * NS] >> 15;
+        if (c != prev) f |= bit;
+        prev = c;
+      }
+      f ^= f << 1; f ^= f << 2; f ^= f << 4; f ^= f << 8; f ^= f << 16;
+      rl.cx[it] = f & mask;
+    });
+    __syncthreads();
+    rl.bytes([&](int j, int sg, int ch, int col, int n) {
+      const uint8_t *f = reinterpret_cast<const uint8_t *>(rl.cx + (size_t)sg * NS) + j;
+      u64 x = 0;
 #pragma unroll
-    for (int l = 0; l < 8; ++l) {
-      if (x[l] != (uint32_t)i) continue;
-      const int lane = grp * 8 + l;
-      const uint32_t tag = (((uint32_t)(w * 64 + lane) << 6 | (uint32_t)b) << 1) | (uint32_t)g;
-      uint32_t v0 = (uint32_t)mv, v1 = (uint32_t)(mv >> 32), v2 = (uint32_t)i, v3 = tag;
-      philox10(v0, v1, v2, v3, (uint32_t)key, (uint32_t)(key >> 32));
-      c |= (v0 & 1u) << l;
-    }
-    qb[i] = (uint8_t)c;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    uint32_t x[8];
-    unpack8(lab[i], x);
-    uint32_t f = 0;
+      for (int l = 0; l < NS; ++l) x |= (u64)f[4 * l] << (8 * l);
+      x = transpose8(x) << (NS * h);
+      const int i0 = (ch * r.H + 8 * j) * r.S + col;
 #pragma unroll
-    for (int l = 0; l < 8; ++l) f |= ((uint32_t)(qb[x[l]] >> l) & 1u) << l;
-    Qb[(size_t)i * 8] = (uint8_t)f;
+      for (int k = 0; k < 8; ++k) {
+        if (k >= n) break;
+        const int i = i0 + k * r.S;
+        const uint8_t byte = (uint8_t)(x >> (8 * k));
+        if (NS == 8) Qb[(size_t)i * 8] = byte;
+        else if (h == 0) rl.fb[i] = byte;
+        else if (h < 8 / NS - 1) rl.fb[i] |= byte;
+        else Qb[(size_t)i * 8] = rl.fb[i] | byte;
+      }
+    });
+    __syncthreads();
   }
 }
 
 // ---------------------------------------------------------------------------
 // Lattices above kSpClusterMaxV sites, one-job path: slabs of slabD z planes
-// labelled 8 samples at a time in SMEM (sp_label8), each site's label written
+// labelled by runs in SMEM, slabNS samples at a time, each site's label written
 // as a global site index into slab_lab [unit = lattice * 8 + group][8][V];
 // then the bonds between slabs joined by the lock-free union of the
 // multispin path (cc_unite: a root hung below the smaller one with
@@ -778,19 +874,32 @@ __device__ __forceinline__ void sp_cluster8_body(const SpDev &d, int g, int blk,
 // the smallest site of their cluster, so the roots -- and the coins and
 // flips -- are those of the one-CTA labelling.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void sp_slab8_body(const SpDev &d, int unit, int sl, unsigned char *sm) {
-  const int V = d.V, L2 = d.L * d.L, z0 = sl * d.slabD;
-  const int base = z0 * L2, Vs = min(d.slabD, d.Lz - z0) * L2;
+template <int NS>
+__device__ __forceinline__ void sp_slab_body(const SpDev &d, int unit, int sl, unsigned char *sm) {
+  const int V = d.V, L2 = d.L * d.L, z0 = sl * d.slabD, nz = min(d.slabD, d.Lz - z0);
+  const int base = z0 * L2, Vs = nz * L2;
   const int grp = unit & 7, lat = unit >> 3;
   const uint8_t *Qb = reinterpret_cast<const uint8_t *>(d.Q + (size_t)lat * V) + grp;
-  sp_label8(d, Qb, base, Vs, sm);
-  const uint4 *lab = reinterpret_cast<const uint4 *>(sm);
-  uint32_t *Lu = d.slab_lab + (size_t)unit * 8 * V;
-  for (int i = threadIdx.x; i < Vs; i += blockDim.x) {
-    uint32_t x[8];
-    unpack8(lab[i], x);
+  const RunLab<NS> rl(sm, d.L, nz);
+  const RunShape &r = rl.r;
+  rl.load(Qb + (size_t)base * 8);
+  uint32_t *Lu = d.slab_lab + (size_t)unit * 8 * V + base;
+  for (int h = 0; h < 8 / NS; ++h) {
+    rl.label(h, false, false);
+    rl.jump([](uint16_t *, int, uint32_t) {});
+    __syncthreads();
+    for (int i = threadIdx.x; i < Vs; i += blockDim.x) {
+      const int z = i / L2, col = i - z * L2, ch = z / r.H;
+      const uint32_t low = (2u << (z - ch * r.H)) - 1u;
+      const uint32_t *m = rl.qm + (size_t)(ch * L2 + col) * NS;
+      const uint16_t *l = rl.lab + ((size_t)ch * r.H * L2 + col) * NS;
 #pragma unroll
-    for (int l = 0; l < 8; ++l) Lu[(size_t)l * V + base + i] = (uint32_t)(base + (int)x[l]);
+      for (int s = 0; s < NS; ++s) {
+        const int zr = 31 - __clz(run_starts(m[s], low));
+        Lu[(size_t)(h * NS + s) * V + i] = (uint32_t)(base + l[(size_t)zr * L2 * NS + s]);
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -851,9 +960,13 @@ __device__ __forceinline__ void sp_slab_flip_body(const SpDev &d, long long t) {
 
 // Labelling of one CTA's (word, slot, 8 samples) by lattice size.
 __device__ __forceinline__ void sp_cluster_any(const SpDev &d, int g, int blk, unsigned char *sm) {
-  if (d.V <= kSpCluster8MaxV) sp_cluster8_body(d, g, blk, sm);
-  else if (d.V <= kSpCluster4MaxV) sp_cluster4_body(d, g, blk, reinterpret_cast<uint32_t *>(sm));
-  else sp_cluster_body(d, g, blk, reinterpret_cast<uint32_t *>(sm));
+  switch (run_samples(d.L, d.Lz)) {
+    case 8: sp_cluster_runs<8>(d, g, blk, sm); break;
+    case 4: sp_cluster_runs<4>(d, g, blk, sm); break;
+    case 2: sp_cluster_runs<2>(d, g, blk, sm); break;
+    case 1: sp_cluster_runs<1>(d, g, blk, sm); break;
+    default: sp_cluster_body(d, g, blk, reinterpret_cast<uint32_t *>(sm));  // wide flat lattices; global scratch
+  }
 }
 
 // Both replicas of the group take the flip words: thread per (word, site, slot).
@@ -1028,7 +1141,7 @@ __global__ void kb_sp_flip(const __grid_constant__ SpBatchDev b, int g) {
   sp_flip_body(d, g, (long long)blk * blockDim.x + threadIdx.x);
 }
 
-size_t sp_cluster_smem(int V);
+size_t sp_cluster_smem(int L, int Lz);
 
 // Blocks of job d for each batched kernel kind (the one-job launch geometry).
 void sp_batch_blocks(const SpDev &d, bool cluster, uint32_t out[SPB_COUNT]) {
@@ -1327,9 +1440,10 @@ __global__ void __launch_bounds__(1024, 1) k_sp_cluster(const __grid_constant__ 
   extern __shared__ __align__(16) uint32_t sm[];
   sp_cluster_any(d, g, blockIdx.x, reinterpret_cast<unsigned char *>(sm));
 }
-__global__ void __launch_bounds__(1024, 1) k_sp_slab8(const __grid_constant__ SpDev d) {
+template <int NS>
+__global__ void __launch_bounds__(1024, 1) k_sp_slab(const __grid_constant__ SpDev d) {
   extern __shared__ __align__(16) unsigned char sm8[];
-  sp_slab8_body(d, blockIdx.y, blockIdx.x, sm8);
+  sp_slab_body<NS>(d, blockIdx.y, blockIdx.x, sm8);
 }
 __global__ void k_sp_slab_merge(const __grid_constant__ SpDev d) {
   sp_slab_merge_body(d, (long long)blockIdx.x * blockDim.x + threadIdx.x);
@@ -1350,7 +1464,7 @@ __global__ void k_sp_measure_u2(const __grid_constant__ SpDev d, int from_e) {
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
-size_t sp_cluster_smem(int V);
+size_t sp_cluster_smem(int L, int Lz);
 
 size_t sp_sweep_smem(int NB, int NR, int kt) {
   return (size_t)NB * 256 * 10 + (size_t)3 * NB * kt * NR * 8 + (size_t)kt * 7 * 4;
@@ -1385,14 +1499,14 @@ int sp_kt(int NB, int NR, int nsites_colour) {
 cudaError_t sp_setup() {
   cudaError_t e = cudaFuncSetAttribute(k_sp_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_pass_items, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_sp_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)std::max(sp_cluster_smem(kSpClusterMaxV),
-                                           std::max(sp_cluster_smem(kSpCluster4MaxV), sp_cluster_smem(kSpCluster8MaxV))));
+  const int cl = (int)std::max(kRunSmem, (size_t)kSpClusterMaxV * 7);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, cl);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_sp_permute, cudaFuncAttributeMaxDynamicSharedMemorySize, kPermRows * 65 * 8);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_sp_slab8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp_cluster_smem(kSpCluster8MaxV));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_slab<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_slab<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_slab<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_slab<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
   return e;
 }
 
@@ -1430,24 +1544,44 @@ cudaError_t sp_launch_permute(const SpDev &d, cudaStream_t st) {
 }
 
 
-size_t sp_cluster_smem(int V) {
-  return V <= kSpCluster8MaxV ? (size_t)V * 26 : V <= kSpCluster4MaxV ? (size_t)V * 22 : V <= kSpClusterMaxV ? (size_t)V * 7 : 0;
+size_t sp_cluster_smem(int L, int Lz) {
+  const int ns = run_samples(L, Lz), V = L * L * Lz;
+  return ns ? run_smem(run_shape(L, Lz), ns) : V <= kSpClusterMaxV ? (size_t)V * 7 : 0;
 }
 
-// Block size of the cluster labelling: 1024 threads, 256 for lattices of
-// at most 2048 sites (256 threads measured 20 % slower on 6912 sites, 512 the
-// same as 1024).
-int sp_cluster_threads(int V) { return V <= 2048 ? 256 : 1024; }
+// Block size of the cluster labelling: its (column chunk, sample) items spread
+// evenly over the fewest passes of at most 1024 threads (12 x 12 x 48: 768
+// threads 4.91 ms a move, 1024 4.96, 512 6.51; 8 x 8 x 16: 512 threads 31 us,
+// 256 40; 7 x 7 x 21: 512 threads 38 us, 256 47).
+int sp_cluster_threads(int L, int Lz) {
+  const int ns = run_samples(L, Lz);
+  if (!ns) return 1024;
+  const int items = run_shape(L, Lz).nseg * ns, passes = (items + 1023) / 1024;
+  return std::min(1024, ((items + passes - 1) / passes + 31) / 32 * 32);
+}
 
 // Planes per slab of the slab labelling of lattices above kSpClusterMaxV
-// sites: as many whole planes as the 8-sample SMEM labelling takes; 0 (the
-// one-CTA labelling in global scratch) when a plane alone is too large or
-// the labels of every (word, slot, group) would pass 4 GB.
-int sp_slab_planes(int L, int Lz, int nw, int nclust) {
+// sites, and the samples labelled at a time: 8 when slabs of at least 6
+// planes then fit SMEM (fewer planes leave more bonds to the union across
+// slabs than the wider label slots save), else the fewest that give 6, else
+// the thickest slab of any; 0 (the one-CTA labelling in global scratch) when
+// a plane alone is too large or the labels of every (word, slot, group) would
+// pass 4 GB.
+int sp_slab_planes(int L, int Lz, int nw, int nclust, int *samples) {
   const long long L2 = (long long)L * L, V = L2 * Lz;
-  if (V <= kSpClusterMaxV || L2 > kSpCluster8MaxV) return 0;
+  if (V <= kSpClusterMaxV || L2 > 32768) return 0;
   if ((long long)nw * nclust * 8 * V * 33 > (4ll << 30)) return 0;
-  return (int)std::min<long long>(Lz, kSpCluster8MaxV / L2);
+  int best = 0;
+  for (int ns = 8; ns >= 1 && best < 6; ns >>= 1) {
+    int D = 0;
+    // at least two slabs: the z wrap is left to the union across slabs
+    while (D < Lz - 1 && L2 * (D + 1) <= 65535 && run_smem(run_shape(L, D + 1), ns) <= kRunSmem) ++D;
+    if (D > best) {
+      best = D;
+      if (samples) *samples = ns;
+    }
+  }
+  return best;
 }
 
 cudaError_t sp_launch_houdayer(const SpDev &d, cudaStream_t st) {
@@ -1459,12 +1593,19 @@ cudaError_t sp_launch_houdayer(const SpDev &d, cudaStream_t st) {
     if (d.slabD > 0) {
       const int L2 = d.L * d.L, nslab = (d.Lz + d.slabD - 1) / d.slabD, nunits = d.nw * d.nclust * 8;
       const long long nu = (long long)nunits * d.V;
-      k_sp_slab8<<<dim3((unsigned)nslab, (unsigned)nunits), 1024, sp_cluster_smem(d.slabD * L2), st>>>(d);
+      const dim3 grid((unsigned)nslab, (unsigned)nunits);
+      const size_t sm = run_smem(run_shape(d.L, d.slabD), d.slabNS);
+      switch (d.slabNS) {
+        case 8: k_sp_slab<8><<<grid, 1024, sm, st>>>(d); break;
+        case 4: k_sp_slab<4><<<grid, 1024, sm, st>>>(d); break;
+        case 2: k_sp_slab<2><<<grid, 1024, sm, st>>>(d); break;
+        default: k_sp_slab<1><<<grid, 1024, sm, st>>>(d);
+      }
       k_sp_slab_merge<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d);
       k_sp_slab_roots<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d, g);
       k_sp_slab_flip<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d);
     } else {
-      k_sp_cluster<<<(unsigned)(d.nw * d.nclust * 8), d.cthreads, sp_cluster_smem(d.V), st>>>(d, g);
+      k_sp_cluster<<<(unsigned)(d.nw * d.nclust * 8), d.cthreads, sp_cluster_smem(d.L, d.Lz), st>>>(d, g);
     }
     k_sp_flip<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, g);
   }
@@ -1610,7 +1751,7 @@ int ea_sp_create(const ea_sp_geom *gp, int32_t device, ea_sp **out) {
   int maxc = 0;
   for (int k = 0; k < g.ncol; ++k) maxc = std::max(maxc, g.col_off[k + 1] - g.col_off[k]);
   d.kt = sp_kt(d.NB, d.NR, maxc);
-  d.cthreads = sp_cluster_threads(d.V);
+  d.cthreads = sp_cluster_threads(d.L, d.Lz);
   d.esites = d.V;
   d.epair = 0;
   d.echunk = sp_energy_chunk(d);
@@ -1992,7 +2133,7 @@ int ea_sp_autotune(ea_sp *c, int32_t *tile, int32_t *echunk, int32_t *cthreads) 
     for (int ct : {256, 512, 1024}) {
       const float ms = timed([&] {
         k_sp_noise<<<(unsigned)((nq + 255) / 256), 256, 0, c->st>>>(d.Q, nq);
-        k_sp_cluster<<<(unsigned)(d.nw * d.nclust * 8), ct, sp_cluster_smem(d.V), c->st>>>(d, 0);
+        k_sp_cluster<<<(unsigned)(d.nw * d.nclust * 8), ct, sp_cluster_smem(d.L, d.Lz), c->st>>>(d, 0);
       });
       if (ms < best) { best = ms; best_ct = ct; }
     }
@@ -2088,12 +2229,14 @@ static int sp_cluster_prepare(ea_sp *c, int &nclust) {
     SCU(cudaMalloc((void **)&d.Q, sizeof(unsigned long long) * (size_t)d.nw * nclust * d.V));
     if (d.V > kSpClusterMaxV) {
       SCU(cudaMalloc((void **)&d.cscratch, sizeof(uint32_t) * sp_cluster_words(d.V) * (size_t)d.nw * nclust * 8));
-      const int D = sp_slab_planes(d.L, d.Lz, d.nw, nclust);
+      int ns = 0;
+      const int D = sp_slab_planes(d.L, d.Lz, d.nw, nclust, &ns);
       if (D > 0) {
         const size_t units = (size_t)d.nw * nclust * 8;
         SCU(cudaMalloc((void **)&d.slab_lab, sizeof(uint32_t) * units * 8 * d.V));
         SCU(cudaMalloc((void **)&d.slab_coin, units * d.V));
         d.slabD = D;
+        d.slabNS = ns;
       }
     }
     c->q_cap = nclust;
@@ -2157,7 +2300,7 @@ static int sp_run_persist(ea_sp *c, const ea_cadence *cad) {
   p.bar = c->p_bar;
   p.err = c->p_err;
   size_t smem = std::max(sp_sweep_smem(d.NB, d.NR, d.kt), (size_t)kPermRows * (d.NB | 1) * 8);
-  if (p.cluster) smem = std::max(smem, sp_cluster_smem(d.V));
+  if (p.cluster) smem = std::max(smem, sp_cluster_smem(d.L, d.Lz));
   const int grid = sp_persist_grid(p.b, smem);
   if (grid < 1) return spfail(EA_ERR_CUDA, "persistent bin kernel: no co-resident grid for %zu bytes of shared memory", smem);
   SCU(sp_launch_persist(p, grid, smem, c->st));
@@ -2354,7 +2497,7 @@ int ea_sp_bin_results(ea_sp *c, double *avgE) {
 // geometries into one launch costs more than the launches it saves.)
 struct SpClass {
   std::vector<ea_sp *> jobs;
-  int ncol_max = 0, cl_threads = 1024;
+  int ncol_max = 0, cl_threads = 0;
   SpDev *d_jobs = nullptr;
   uint32_t *d_pre = nullptr;
   std::vector<SpDev> up_jobs;
@@ -2397,7 +2540,7 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
     pass_smem = std::max(pass_smem, (int)(hj[i].pgrid ? sp_items_smem(hj[i].NB)
                                                        : sp_sweep_smem(hj[i].NB, hj[i].NR, hj[i].kt)));
     perm_smem = std::max(perm_smem, kPermRows * (hj[i].NB | 1) * 8);
-    if (cluster) cl_smem = std::max(cl_smem, (int)sp_cluster_smem(hj[i].V));
+    if (cluster) cl_smem = std::max(cl_smem, (int)sp_cluster_smem(hj[i].L, hj[i].Lz));
   }
   if (k.up_jobs.size() != hj.size() || std::memcmp(k.up_jobs.data(), hj.data(), sizeof(SpDev) * n) ||
       k.up_pre != hp) {
@@ -2462,11 +2605,11 @@ int ea_sp_batch_create(ea_sp *const *jobs, int32_t njobs, ea_sp_batch **out) {
     if (q == keys.size()) {
       keys.push_back(key);
       b->classes.emplace_back();
-      b->classes.back().cl_threads = sp_cluster_threads(key.second == 0 ? 2048 : 32768);
     }
     SpClass &k = b->classes[q];
     k.jobs.push_back(c);
     k.ncol_max = std::max(k.ncol_max, c->d.ncol);
+    k.cl_threads = std::max(k.cl_threads, sp_cluster_threads(c->d.L, c->d.Lz));
   }
   cudaError_t e = cudaSetDevice(b->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->bs, cudaStreamNonBlocking);
@@ -2637,7 +2780,7 @@ int ea_sp_job_bytes(const ea_sp_geom *gp, const ea_cadence *cad, const double *b
     const uint64_t nc = (uint64_t)(cad->nclust > 0 ? std::min<int>(cad->nclust, (int)NB) : std::lround(0.5 * NB));
     add(nw * nc * V * 8);
     if (V > (uint64_t)kSpClusterMaxV) add(nw * nc * 8 * sp_cluster_words((int)V) * 4);
-    if (sp_slab_planes(gp->L, gp->Lz, (int)nw, (int)nc) > 0) {   // slab labels and coins
+    if (sp_slab_planes(gp->L, gp->Lz, (int)nw, (int)nc, nullptr) > 0) {   // slab labels and coins
       add(nw * nc * 8 * 8 * V * 4);
       add(nw * nc * 8 * V);
     }

@@ -74,7 +74,7 @@ struct SpDev {
   unsigned long long *move;          // cluster moves so far
   int nclust;
   uint32_t *cscratch;                // labelling arrays of lattices above kSpClusterMaxV, per CTA
-  int slabD;                         // > 0: such lattices labelled in slabs of slabD z planes (one-job path)
+  int slabD, slabNS;                 // > 0: such lattices labelled in slabs of slabD z planes, slabNS samples at a time (one-job path)
   uint32_t *slab_lab;                // [nw*nclust*8 units][8][V] labels of the slab path
   uint8_t *slab_coin;                // [units][V] roots' coins (one bit a sample)
   // exact enumeration
@@ -85,13 +85,10 @@ struct SpDev {
 // site: label, 8 samples' overlap and flip bits, bond mask); larger ones use
 // a global scratch region of sp_cluster_words(V) words per CTA.
 constexpr int kSpClusterMaxV = 32768;
-// Lattices up to this size are labelled 4 samples at a time (22 bytes of
-// SMEM per site; 512 bytes left for static SMEM).
-constexpr int kSpCluster4MaxV = 10500;
 __host__ __device__ inline size_t sp_cluster_words(int V) { return ((size_t)V * 7 + 15) / 16 * 4; }
 
 int sp_kt(int NB, int NR, int nsites_colour);
-int sp_slab_planes(int L, int Lz, int nw, int nclust);
+int sp_slab_planes(int L, int Lz, int nw, int nclust, int *samples);
 int sp_energy_chunk(const SpDev &d);
 size_t sp_sweep_smem(int NB, int NR, int kt);
 size_t sp_items_smem(int NB);
