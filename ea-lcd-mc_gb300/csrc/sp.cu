@@ -222,153 +222,318 @@ __device__ __forceinline__ void sp_pass_any(const SpDev &d, int colour, int blk,
   }
 }
 
+// The 8 x 8 bit matrix with byte i, bit j at bit 8 i + j, transposed.
+__device__ __forceinline__ u64 transpose8(u64 x) {
+  u64 t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull;
+  x ^= t ^ (t << 7);
+  t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull;
+  x ^= t ^ (t << 14);
+  t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull;
+  return x ^ t ^ (t << 28);
+}
+
 // ---------------------------------------------------------------------------
 // Energy: per (word, sample, replica, slot) the number of unsatisfied
 // half-edges U2 (each bond counted from both ends), so E = 3V - U2
-// (main.cu:1379).  A thread owns one (replica, slot) column of a word over a
-// chunk of sites and counts the unsatisfied slots of each sample with
-// bit-sliced counters (one bit plane per power of two, all 64 samples at
-// once), then adds its per-sample totals to U2.
-// ---------------------------------------------------------------------------
-constexpr int kSpChunkMax = 256;  // sites per thread: 6 * 256 < 2^11
-constexpr int kSpPlanes = 11;
-
-// Sites per thread of the energy kernel: enough threads to fill the GPU
-// (152 SMs x 2048), at least 4 sites each (each thread ends with up to 64
-// atomic additions, which small chunks pile on the same counters).  Jobs too
-// small to fill the GPU get the floor: their count is a chain of dependent
-// loads per site, so fewer sites a thread is a shorter chain (16 sites a
-// thread measured 16-21 us per count on one-word jobs).
-int sp_energy_chunk(const SpDev &d) {
-  const double words = (double)d.nw * d.esites * d.NR * d.NB;
-  int c = (int)(words / (152.0 * 2048.0));
-  return c < 4 ? 4 : (c > kSpChunkMax ? kSpChunkMax : c);
-}
-
-// col: the thread's index over nw * nchunk * G (blocks of 256 threads).
+// (main.cu:1379).  A block owns a tile of sites of one word: the sites'
+// neighbours and couplings are staged in SMEM once, lane groups of one lane
+// per (replica, slot) column walk the tile's sites in turn, counting the
+// unsatisfied slots of all 64 samples in bit-sliced counters (one bit plane
+// per power of two), the groups' counts are added up through SMEM, and the
+// block adds one total per (column, sample) to U2.
 // With epair (two colours, both ends of every bond holding its coupling word:
 // checked on the host when the couplings are set) every bond has exactly one
 // colour-1 end, so the count walks the colour-1 sites only and doubles them.
-__device__ __forceinline__ void sp_energy_body(const SpDev &d, long long col) {
-  const int G = d.NR * d.NB, V = d.V, chunk = d.echunk, ns = d.esites;
-  const int nchunk = (ns + chunk - 1) / chunk;
-  if (col >= (long long)d.nw * nchunk * G) return;
-  const int rb = (int)(col % G), ch = (int)((col / G) % nchunk), w = (int)(col / ((long long)G * nchunk));
-  const u64 *Sw = d.S + (size_t)w * V * G + rb;
-  const u64 *Jw = d.J + (size_t)w * V * 6;
-  u64 P[kSpPlanes];
-#pragma unroll
-  for (int p = 0; p < kSpPlanes; ++p) P[p] = 0;
-  const int i0 = ch * chunk, i1 = min(ns, i0 + chunk);
-  const int32_t *c1 = d.col_sites + d.col_off[1];
-  // two sites an iteration, so that the second site's loads are in flight
-  // while the first is counted (the words are read-only here)
-#pragma unroll 2
-  for (int ii = i0; ii < i1; ++ii) {
-    const int i = d.epair ? __ldg(c1 + ii) : ii;
-    const u64 sv = __ldg(Sw + (size_t)i * G);
-    const int *nb = d.nb + (size_t)i * 6;
-    u64 f[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) f[q] = sv ^ __ldg(Jw + (size_t)i * 6 + q) ^ __ldg(Sw + (size_t)__ldg(nb + q) * G);
+//
+// Bound by issue and the latency of the neighbours' loads; the words come from
+// DRAM once (340 MB on 64 words of 12 x 12 x 48, 24 temperatures, 4 replicas:
+// 50 us at the copy rate).  One thread a column and run of sites, each ending
+// in 64 global atomic additions, took 257 us there (190 instructions a word)
+// and 28 us on one word; this form 167 and 12.  Two columns a lane (16-byte loads)
+// took 181 us: 115 registers leave 16 warps an SM.
+// ---------------------------------------------------------------------------
+constexpr int kEnPlanes = 8;
+constexpr int kEnSites = 42;      // sites a lane counts: 6 * 42 < 2^8
+constexpr int kEnMaxThreads = 288;
+
+// Fills the count's launch shape (d.en) for `chunk` sites a lane.
+void sp_energy_shape(SpDev &d, int chunk) {
+  EnShape &e = d.en;
+  const int G = d.NR * d.NB;
+  d.echunk = chunk;
+  e.nslice = (G + kEnMaxThreads - 1) / kEnMaxThreads;
+  e.lanes = (G + e.nslice - 1) / e.nslice;
+  e.threads = (e.lanes + 31) / 32 * 32;
+  for (int t = e.threads; t <= kEnMaxThreads; t += 32)  // the multiple of 32 that lane groups fill best
+    if (t / e.lanes * e.lanes * e.threads >= e.threads / e.lanes * e.lanes * t) e.threads = t;
+  e.tile = std::min(e.threads / e.lanes * chunk, d.esites);
+  e.ntile = (d.esites + e.tile - 1) / e.tile;
+}
+inline size_t en_blocks(const SpDev &d) { return (size_t)d.nw * d.en.ntile * d.en.nslice; }
+// The staged sites; then, in the same bytes, the groups' planes.  `threads` of
+// the launch's blocks.
+inline size_t en_smem(const SpDev &d, int threads) {
+  return std::max((size_t)d.en.tile * 80, (size_t)(threads / d.en.lanes) * d.en.lanes * kEnPlanes * 8);
+}
+
+// Sites per lane of the energy count: at most what the counters take, fewer
+// when the GPU would otherwise get less than about three waves of blocks, at
+// least 4 (the counters take 4 at a time).
+int sp_energy_chunk(const SpDev &d) {
+  const double words = (double)d.nw * d.esites * d.NR * d.NB;
+  const int c = (int)(words / (3 * 152.0 * 1152.0));
+  return c < 4 ? 4 : (c > kEnSites ? kEnSites : c);
+}
+
+// Bit-sliced counters of 64 samples.  site() takes a site's six unsatisfied
+// bits and returns its carry of weight 8; carries are added in pairs and
+// rippled once every 4 sites.
+struct EnCount {
+  u64 P[kEnPlanes];
+  static __device__ __forceinline__ u64 maj(u64 a, u64 b, u64 c) { return (a & b) | (c & (a ^ b)); }
+  __device__ __forceinline__ u64 site(const u64 f[6]) {
     // six bits -> a 3-bit count per sample (two full adders and a merge)
-    const u64 x1 = f[0] ^ f[1] ^ f[2], y1 = (f[0] & f[1]) | (f[2] & (f[0] ^ f[1]));
-    const u64 x2 = f[3] ^ f[4] ^ f[5], y2 = (f[3] & f[4]) | (f[5] & (f[3] ^ f[4]));
-    const u64 z0 = x1 ^ x2, c0 = x1 & x2;
-    const u64 z1 = y1 ^ y2 ^ c0, z2 = (y1 & y2) | (c0 & (y1 ^ y2));
-    // add z0 + 2 z1 + 4 z2 to the counter planes
+    const u64 x1 = f[0] ^ f[1] ^ f[2], y1 = maj(f[0], f[1], f[2]);
+    const u64 x2 = f[3] ^ f[4] ^ f[5], y2 = maj(f[3], f[4], f[5]);
+    const u64 z0 = x1 ^ x2, c0 = x1 & x2, z1 = y1 ^ y2 ^ c0, z2 = maj(y1, y2, c0);
     u64 c = P[0] & z0;
     P[0] ^= z0;
-    u64 s = P[1] ^ z1 ^ c;
-    c = (P[1] & z1) | (c & (P[1] ^ z1));
-    P[1] = s;
-    s = P[2] ^ z2 ^ c;
-    c = (P[2] & z2) | (c & (P[2] ^ z2));
+    const u64 t = P[1] ^ z1 ^ c;
+    c = maj(P[1], z1, c);
+    P[1] = t;
+    const u64 s = P[2] ^ z2 ^ c;
+    c = maj(P[2], z2, c);
     P[2] = s;
+    return c;
+  }
+  __device__ __forceinline__ u64 pair(u64 a, u64 b) {
+    const u64 c = maj(P[3], a, b);
+    P[3] ^= a ^ b;
+    return c;
+  }
+  __device__ __forceinline__ void ripple(u64 a, u64 b) {
+    u64 c = maj(P[4], a, b);
+    P[4] ^= a ^ b;
 #pragma unroll
-    for (int p = 3; p < kSpPlanes; ++p) {
-      const u64 t = P[p] & c;
+    for (int p = 5; p < kEnPlanes; ++p) {
+      const u64 h = P[p] & c;
       P[p] ^= c;
-      c = t;
+      c = h;
     }
   }
-  int32_t *U = d.U2 + (size_t)w * 64 * G + rb;
-  int np = kSpPlanes;
-  while (np > 1 && !P[np - 1]) --np;
-  for (int lane = 0; lane < 64; ++lane) {
-    int cnt = 0;
-    for (int p = 0; p < np; ++p) cnt |= (int)((P[p] >> lane) & 1ull) << p;
-    if (cnt) atomicAdd(U + (size_t)lane * G, cnt << d.epair);
+};
+
+__device__ __forceinline__ void sp_energy_body(const SpDev &d, int blk, unsigned char *sm) {
+  const EnShape &e = d.en;
+  const int G = d.NR * d.NB, V = d.V;
+  const int part = blk / e.nslice, sl = blk - part * e.nslice, w = part / e.ntile, tl = part - w * e.ntile;
+  const int s0 = tl * e.tile, ns = min(e.tile, d.esites - s0);
+  u64 *sJ = reinterpret_cast<u64 *>(sm);                                   // [tile][6]
+  uint32_t *sN = reinterpret_cast<uint32_t *>(sJ + (size_t)6 * e.tile);    // [tile][8]: first words of the 6 neighbours and of the site
+  const int32_t *c1 = d.col_sites + d.col_off[1];
+  const u64 *Jw = d.J + (size_t)w * V * 6;
+  for (int i = threadIdx.x; i < ns * 8; i += blockDim.x) {
+    const int k = i >> 3, f = i & 7, site = d.epair ? __ldg(c1 + s0 + k) : s0 + k;
+    if (f < 6) sJ[k * 6 + f] = __ldg(Jw + (size_t)site * 6 + f);
+    if (f < 7) sN[i] = (uint32_t)(f < 6 ? __ldg(d.nb + (size_t)site * 6 + f) : site) * (uint32_t)G;
+  }
+  __syncthreads();
+  const int groups = blockDim.x / e.lanes, g = threadIdx.x / e.lanes, ln = threadIdx.x - g * e.lanes;
+  const int col = sl * e.lanes + ln;
+  EnCount n;
+#pragma unroll
+  for (int p = 0; p < kEnPlanes; ++p) n.P[p] = 0;
+  if (g < groups && col < G) {
+    const u64 *Sc = d.S + (size_t)w * V * G + col;
+    auto site = [&](int k) -> u64 {
+      const uint4 *nb = reinterpret_cast<const uint4 *>(sN + k * 8);
+      const ulonglong2 *J = reinterpret_cast<const ulonglong2 *>(sJ + k * 6);
+      const uint4 na = nb[0], nc = nb[1];
+      const u64 sv = __ldg(Sc + nc.z);
+      u64 f[6];
+      f[0] = __ldg(Sc + na.x); f[1] = __ldg(Sc + na.y); f[2] = __ldg(Sc + na.z);
+      f[3] = __ldg(Sc + na.w); f[4] = __ldg(Sc + nc.x); f[5] = __ldg(Sc + nc.y);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const ulonglong2 j = J[q];
+        f[2 * q] ^= sv ^ j.x;
+        f[2 * q + 1] ^= sv ^ j.y;
+      }
+      return n.site(f);
+    };
+    int k = g;
+    for (; k + 3 * groups < ns; k += 4 * groups) {
+      u64 a = site(k), b = site(k + groups);
+      const u64 p = n.pair(a, b);
+      a = site(k + 2 * groups);
+      b = site(k + 3 * groups);
+      n.ripple(p, n.pair(a, b));
+    }
+    for (; k < ns; k += groups) n.ripple(n.pair(site(k), 0), 0);
+  }
+  __syncthreads();
+  u64 *pl = reinterpret_cast<u64 *>(sm);  // [group][plane][lane]
+  if (g < groups) {
+#pragma unroll
+    for (int p = 0; p < kEnPlanes; ++p) pl[(g * kEnPlanes + p) * e.lanes + ln] = n.P[p];
+  }
+  __syncthreads();
+  // totals: a task takes 8 samples of a column -- byte j of the 8 planes, an
+  // 8 x 8 bit matrix whose transpose holds the 8 samples' counts -- from every
+  // group, added as 16-bit fields
+  const int cols = min(e.lanes, G - sl * e.lanes);
+  int32_t *U = d.U2 + (size_t)w * 64 * G + sl * e.lanes;
+  for (int t = threadIdx.x; t < cols * 8; t += blockDim.x) {
+    const int j = t / cols, c = t - j * cols;
+    const uint8_t *P = reinterpret_cast<const uint8_t *>(pl + c) + j;
+    u64 even = 0, odd = 0;
+    for (int q = 0; q < groups; ++q, P += (size_t)kEnPlanes * e.lanes * 8) {
+      u64 x = 0;
+#pragma unroll
+      for (int p = 0; p < kEnPlanes; ++p) x |= (u64)P[(size_t)p * e.lanes * 8] << (8 * p);
+      x = transpose8(x);
+      even += x & 0x00FF00FF00FF00FFull;
+      odd += (x >> 8) & 0x00FF00FF00FF00FFull;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int cnt = (int)(((q & 1 ? odd : even) >> (16 * (q >> 1))) & 0xFFFFu);
+      if (cnt) atomicAdd(U + (size_t)(8 * j + q) * G + c, cnt << d.epair);
+    }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Tempering: one thread per (word, sample, replica) chain; the rule of
-// upd.c:3-48 over the slot pairs in order (pt = -(b[i+1]-b[i]) * dE in FP64,
+// Tempering: one block per (word, replica), one lane per sample's chain; the
+// rule of upd.c:3-48 over the slot pairs in order (pt = -(b[i+1]-b[i]) * dE,
 // accept when pt >= 0 or FNORM * u < exp(pt), exp from the host's libm table;
 // beyond the table exp(pt) < 2^-72 and only u = 0 accepts).  The 64-bit
 // uniform u of (step, pair, chain) is Philox4x32-10 keyed by the job's
 // tempering seed -- the reference draws it from a per-chain Parisi-Rapuano
 // generator; sample-packed jobs have 64 chains per word, so a counter-based
-// draw replaces the 2 KB of state per chain.  A warp holds 32 samples of one
-// (word, replica): the accepted swaps of pair i form the lane mask M[i].
+// draw replaces the 2 KB of state per chain.
+//
+// The walk over the pairs is a serial chain, so everything that does not
+// depend on the carried configuration is put in SMEM by the whole block first:
+// energies, slot ids and the uniforms as FNORM * u.  The chain needs no FP64
+// (pt >= 0 exactly when dE has the sign of -(b[i+1]-b[i]), and non-negative
+// doubles order as their bit patterns), and it reads the table only when a
+// single-precision exp(pt) cannot tell: that is within 2e-5 of the true value
+// (pt in [-50, 0) has a relative error of 3 * 2^-24, so its exponential 9e-6;
+// __expf adds 2 + 1.16 |x| ulp, 7e-6), so a uniform more than 1e-4 away from
+// it decides alone, and one draw in some 10^4 looks at the table.
+// A warp's accepted swaps of pair i form half of the lane mask M[i].
+// Bound by latency.  24 temperatures, one word: 31 us with every operand read
+// from global memory on the way, 23 staged with a table read a pair, 12 so.
 // ---------------------------------------------------------------------------
-// wr = (word, replica); lane = sample, 0..63, the 64 lanes two whole warps.
-__device__ __forceinline__ void sp_pt_body(const SpDev &d, int wr, int lane) {
-  const int NB = d.NB, NR = d.NR, G = NR * NB;
-  const int w = wr / NR, r = wr % NR;
-  const int nt = 3 * d.V;
-  const size_t o = ((size_t)w * 64 + lane) * G + (size_t)r * NB;
-  const unsigned long long step = *d.ptstep;
-  const uint32_t chain = (uint32_t)(((size_t)w * 64 + lane) * NR + r);
-  const double FNORM = 5.4210108624275218e-20;
-  uint32_t *acc = d.acc + ((size_t)w * 64 + lane) * NR * (NB - 1) + (size_t)r * (NB - 1);
-  uint32_t *Mh = reinterpret_cast<uint32_t *>(d.M + ((size_t)w * NR + r) * (NB - 1));
-  // The pairs in order: slot i+1 still holds its own configuration when pair
-  // i is decided, slot i holds the one carried up from below (a swap at i
-  // moves it on to i+1).  So the chain keeps only the carried energy and id
-  // in registers; slot i's final values are written as soon as pair i is
-  // decided.
-  int carry_e = nt - d.U2[o];
-  uint8_t carry_p = d.perm[o];
-  for (int i = 0; i < NB - 1; ++i) {
-    const int e1 = nt - d.U2[o + i + 1];
-    const uint8_t p1 = d.perm[o + i + 1];
-    const int dE = e1 - carry_e;
-    const double pt = __dmul_rn(-__dsub_rn(d.betas[i + 1], d.betas[i]), (double)dE);
-    uint32_t v0 = (uint32_t)step, v1 = (uint32_t)(step >> 32), v2 = (uint32_t)i, v3 = chain;
-    philox10(v0, v1, v2, v3, (uint32_t)d.pt_seed, (uint32_t)(d.pt_seed >> 32));
-    const u64 u = ((u64)v0 << 32) | v1;
-    bool change;
-    if (pt >= 0.0) {
-      change = true;
-    } else {
-      const int base = d.expoff[i], m = (-dE) >> 1, nx = d.expoff[i + 1] - base;
-      change = (m >= 1 && m <= nx) ? __dmul_rn(FNORM, __ull2double_rn(u)) < d.exptab[base + m - 1] : u == 0;
-    }
-    if (change) {
-      d.E[o + i] = e1;
-      d.perm[o + i] = p1;
-      acc[i] += 1u;
-    } else {
-      d.E[o + i] = carry_e;
-      d.perm[o + i] = carry_p;
-      carry_e = e1;
-      carry_p = p1;
-    }
-    const unsigned mask = __ballot_sync(0xffffffffu, change);
-    if ((lane & 31) == 0) Mh[2 * i + (lane >> 5)] = mask;
+constexpr int kPtThreads = 256;
+// SMEM: uniforms [NB-1][64] u64, masks [NB-1] u64, energies [NB][65] i32, table
+// offsets [NB], b[i]-b[i+1] [NB] f32, slot ids [NB][64] u8
+__host__ __device__ inline size_t pt_smem(int NB) { return (size_t)8 * 65 * (NB - 1) + 4 * 67 * NB + 64 * NB; }
+
+__device__ __forceinline__ void sp_pt_body(const SpDev &d, int wr, unsigned char *sm) {
+  const int NB = d.NB, NP = NB - 1, NR = d.NR, G = NR * NB;
+  const int w = wr / NR, r = wr % NR, nt = 3 * d.V;
+  u64 *xs = reinterpret_cast<u64 *>(sm), *Ms = xs + 64 * NP;
+  int *es = reinterpret_cast<int *>(Ms + NP), *eo = es + 65 * NB;
+  float *db = reinterpret_cast<float *>(eo + NB);
+  uint8_t *ps = reinterpret_cast<uint8_t *>(db + NB);
+  const size_t row = (size_t)w * 64 * G + (size_t)r * NB;
+#pragma unroll 8
+  for (int t = threadIdx.x; t < 64 * NB; t += blockDim.x) {
+    const int lane = t / NB, b = t - lane * NB;
+    const size_t o = row + (size_t)lane * G + b;
+    es[b * 65 + lane] = nt - __ldg(d.U2 + o);
+    ps[b * 64 + lane] = __ldg(d.perm + o);
   }
-  d.E[o + NB - 1] = carry_e;
-  d.perm[o + NB - 1] = carry_p;
+  for (int i = threadIdx.x; i < NB; i += blockDim.x) {
+    eo[i] = __ldg(d.expoff + i);
+    // betas descend; a difference too small for single precision stays
+    // positive (exp(pt) is then within 1e-4 of 1 and the table decides)
+    const double f = i < NP ? -__dsub_rn(__ldg(d.betas + i + 1), __ldg(d.betas + i)) : 0.0;
+    db[i] = f > 0.0 ? fmaxf((float)f, 1e-30f) : (float)f;
+  }
+  const unsigned long long step = *d.ptstep;
+  const double FNORM = 5.4210108624275218e-20;
+  for (int t = threadIdx.x; t < 64 * NP; t += blockDim.x) {
+    uint32_t v0 = (uint32_t)step, v1 = (uint32_t)(step >> 32), v2 = (uint32_t)(t >> 6);
+    uint32_t v3 = (uint32_t)(((size_t)w * 64 + (t & 63)) * NR + r);
+    philox10(v0, v1, v2, v3, (uint32_t)d.pt_seed, (uint32_t)(d.pt_seed >> 32));
+    xs[t] = (u64)__double_as_longlong(__dmul_rn(FNORM, __ull2double_rn(((u64)v0 << 32) | v1)));
+  }
+  __syncthreads();
+  if (threadIdx.x < 64) {
+    // The pairs in order: slot i+1 still holds its own configuration when pair
+    // i is decided, slot i holds the one carried up from below (a swap at i
+    // moves it on to i+1); slot i's final values are written as soon as pair i
+    // is decided.
+    const int lane = threadIdx.x;
+    uint32_t *Mh = reinterpret_cast<uint32_t *>(Ms) + (lane >> 5);
+    const u64 *tab = reinterpret_cast<const u64 *>(d.exptab);
+    int carry_e = es[lane];
+    uint8_t carry_p = ps[lane];
+#pragma unroll 4
+    for (int i = 0; i < NP; ++i) {
+      const int e1 = es[(i + 1) * 65 + lane];
+      const uint8_t p1 = ps[(i + 1) * 64 + lane];
+      const u64 x = xs[i * 64 + lane];
+      const float f = db[i], xf = (float)__longlong_as_double((long long)x);
+      const int base = eo[i], nx = eo[i + 1] - base;
+      const int dE = e1 - carry_e, m = (-dE) >> 1;
+      const float pt = f * (float)dE, ex = __expf(pt);
+      bool change = pt >= 0.f;
+      if (!change) {
+        change = xf < ex;
+        if (m < 1 || m > nx) change = x == 0;                 // beyond the table: exp(pt) < 2^-72
+        else if (fabsf(xf - ex) <= 1e-4f * ex) change = x < __ldg(tab + base + m - 1);
+      }
+      es[i * 65 + lane] = change ? e1 : carry_e;
+      ps[i * 64 + lane] = change ? p1 : carry_p;
+      carry_e = change ? carry_e : e1;
+      carry_p = change ? carry_p : p1;
+      const unsigned mask = __ballot_sync(0xffffffffu, change);
+      if ((lane & 31) == 0) Mh[2 * i] = mask;
+    }
+    es[NP * 65 + lane] = carry_e;
+    ps[NP * 64 + lane] = carry_p;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 64 * NB; t += blockDim.x) {
+    const int lane = t / NB, b = t - lane * NB;
+    const size_t o = row + (size_t)lane * G + b;
+    d.E[o] = es[b * 65 + lane];
+    d.perm[o] = ps[b * 64 + lane];
+  }
+  uint32_t *acc = d.acc + ((size_t)w * 64 * NR + r) * NP;
+  for (int t = threadIdx.x; t < 64 * NP; t += blockDim.x) {
+    const int lane = t / NP, i = t - lane * NP;
+    if ((Ms[i] >> lane) & 1ull) atomicAdd(acc + (size_t)lane * NR * NP + i, 1u);  // no wait for the old value
+  }
+  for (int i = threadIdx.x; i < NP; i += blockDim.x) d.M[((size_t)w * NR + r) * NP + i] = Ms[i];
 }
 
 // The accepted swaps of the last tempering step, applied to the words in
 // pair order: slot i exchanges the masked samples with slot i+1, and is final
-// after that (one carry word).  A block stages kPermRows consecutive
-// (word, site, replica) rows of NB words through SMEM, so that global loads
-// and stores are coalesced, and each thread then walks one row.
+// after that (one carry word).  A block takes kPermRows consecutive (word,
+// site, replica) rows of NB words, a thread one row.
+// NB a multiple of 4: rows are whole 32-byte sectors, so a thread streams its
+// row through registers with 32-byte loads and stores, the next four words
+// in flight while four are exchanged.  Other NB: the block stages its rows in
+// SMEM so that loads and stores are coalesced.  Both move the words once each
+// way (2 x 340 MB on 64 words of 12 x 12 x 48: 100 us at the copy rate); the
+// staged form took 219 us there, the streamed one 115 (0.87 of the copy rate).
 constexpr int kPermRows = 128;
+
+__device__ __forceinline__ void ld32(u64 v[4], const u64 *p) {
+  asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st32(u64 *p, const u64 v[4]) {
+  asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v[0]), "l"(v[1]), "l"(v[2]), "l"(v[3])
+               : "memory");
+}
+
+inline size_t perm_smem(int NB) { return NB & 3 ? (size_t)kPermRows * (NB | 1) * 8 : 0; }
 
 __device__ __forceinline__ void sp_permute_body(const SpDev &d, int blk, u64 *rows) {
   const int NB = d.NB, NR = d.NR;
@@ -376,20 +541,48 @@ __device__ __forceinline__ void sp_permute_body(const SpDev &d, int blk, u64 *ro
   const long long r0 = (long long)blk * kPermRows;
   if (blk == 0 && threadIdx.x == 0) *d.ptstep += 1ull;
   const int nr = (int)min((long long)kPermRows, nrows - r0);
-  // rows sit in SMEM with an odd stride (in words): the threads' scans then
-  // hit distinct banks (an even stride such as NB = 24 is a 16-way conflict)
-  const int rs = NB | 1;
+  const long long t = r0 + threadIdx.x;
+  const int r = (int)(t % NR), w = (int)(t / ((long long)NR * d.V));
+  const u64 *M = d.M + ((size_t)w * NR + r) * (NB - 1);
   u64 *g = d.S + (size_t)r0 * NB;
+  if ((NB & 3) == 0) {
+    if (threadIdx.x >= nr) return;
+    u64 *p = g + (size_t)threadIdx.x * NB;
+    u64 v[4], n[4];
+    ld32(v, p);
+    u64 cur = v[0];
+    for (int i = 0; i < NB; i += 4) {
+      u64 o[4];
+      const bool more = i + 4 < NB;
+      if (more) ld32(n, p + i + 4);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const u64 x = (cur ^ v[q + 1]) & __ldg(M + i + q);
+        o[q] = cur ^ x;
+        cur = v[q + 1] ^ x;
+      }
+      o[3] = cur;
+      if (more) {
+        const u64 x = (cur ^ n[0]) & __ldg(M + i + 3);
+        o[3] = cur ^ x;
+        cur = n[0] ^ x;
+      }
+      st32(p + i, o);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = n[q];
+    }
+    return;
+  }
+  // rows sit in SMEM with an odd stride (in words): the threads' scans then
+  // hit distinct banks (an even stride such as NB = 22 is a many-way conflict)
+  const int rs = NB | 1;
   for (int k = threadIdx.x; k < nr * NB; k += blockDim.x) {
     const int row = k / NB;
     rows[row * rs + (k - row * NB)] = g[k];
   }
   __syncthreads();
   if (threadIdx.x < nr) {
-    const long long t = r0 + threadIdx.x;
-    const int r = (int)(t % NR), w = (int)(t / ((long long)NR * d.V));
     u64 *p = rows + (size_t)threadIdx.x * rs;
-    const u64 *M = d.M + ((size_t)w * NR + r) * (NB - 1);
     u64 cur = p[0];
     for (int i = 0; i < NB - 1; ++i) {
       const u64 m = __ldg(M + i);
@@ -595,16 +788,6 @@ __device__ __forceinline__ uint32_t run_mask(const RunShape &r, int ch) {
   return (1u << min(r.H, r.nz - ch * r.H)) - 1u;
 }
 __device__ __forceinline__ uint32_t run_starts(uint32_t m, uint32_t mask) { return ((m ^ (m << 1)) | 1u) & mask; }
-
-// The 8 x 8 bit matrix with byte i, bit j at bit 8 i + j, transposed.
-__device__ __forceinline__ u64 transpose8(u64 x) {
-  u64 t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull;
-  x ^= t ^ (t << 7);
-  t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull;
-  x ^= t ^ (t << 14);
-  t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull;
-  return x ^ t ^ (t << 28);
-}
 
 template <int NS>
 struct RunLab {
@@ -1106,13 +1289,15 @@ __global__ void kb_sp_zero(const __grid_constant__ SpBatchDev b) {
   const long long i = (long long)blk * blockDim.x + threadIdx.x;
   if (i < (long long)d.nw * 64 * d.NR * d.NB) d.U2[i] = 0;
 }
-__global__ void __launch_bounds__(256) kb_sp_energy(const __grid_constant__ SpBatchDev b) {
+__global__ void __launch_bounds__(kEnMaxThreads, 4) kb_sp_energy(const __grid_constant__ SpBatchDev b) {
+  extern __shared__ __align__(16) unsigned char smem[];
   SPB_ITEM(SPB_ENERGY)
-  sp_energy_body(d, (long long)blk * blockDim.x + threadIdx.x);
+  sp_energy_body(d, blk, smem);
 }
-__global__ void __launch_bounds__(64) kb_sp_pt(const __grid_constant__ SpBatchDev b) {
+__global__ void __launch_bounds__(kPtThreads) kb_sp_pt(const __grid_constant__ SpBatchDev b) {
+  extern __shared__ __align__(16) unsigned char smem[];
   SPB_ITEM(SPB_PT)
-  sp_pt_body(d, blk, threadIdx.x);
+  sp_pt_body(d, blk, smem);
 }
 __global__ void __launch_bounds__(kPermRows) kb_sp_permute(const __grid_constant__ SpBatchDev b) {
   extern __shared__ u64 rows[];
@@ -1153,7 +1338,7 @@ void sp_batch_blocks(const SpDev &d, bool cluster, uint32_t out[SPB_COUNT]) {
                                  : (uint32_t)((n + d.kt - 1) / d.kt);
   }
   out[SPB_ZERO] = out[SPB_MEASURE] = (uint32_t)((nw * 64 * G + 255) / 256);
-  out[SPB_ENERGY] = (uint32_t)((nw * ((d.esites + d.echunk - 1) / d.echunk) * G + 255) / 256);
+  out[SPB_ENERGY] = (uint32_t)en_blocks(d);
   out[SPB_PT] = (uint32_t)(nw * d.NR);
   out[SPB_PERMUTE] = (uint32_t)((nw * d.V * d.NR + kPermRows - 1) / kPermRows);
   if (cluster && d.nclust > 0) {
@@ -1178,6 +1363,8 @@ cudaError_t sp_batch_setup() {
   cudaError_t e = max_dynamic_smem(kb_sp_pass);
   if (e == cudaSuccess) e = max_dynamic_smem(kb_sp_cluster);
   if (e == cudaSuccess) e = max_dynamic_smem(kb_sp_permute);
+  if (e == cudaSuccess) e = max_dynamic_smem(kb_sp_energy);
+  if (e == cudaSuccess) e = max_dynamic_smem(kb_sp_pt);
   return e;
 }
 
@@ -1193,12 +1380,12 @@ cudaError_t sp_batch_sweep(const SpBatchDev &b, int ncol_max, cudaStream_t st) {
 
 static void spb_energy(const SpBatchDev &b, cudaStream_t st) {
   kb_sp_zero<<<b.total[SPB_ZERO], 256, 0, st>>>(b);
-  kb_sp_energy<<<b.total[SPB_ENERGY], 256, 0, st>>>(b);
+  kb_sp_energy<<<b.total[SPB_ENERGY], b.energy_threads, b.energy_smem, st>>>(b);
 }
 
 cudaError_t sp_batch_tempering(const SpBatchDev &b, cudaStream_t st) {
   spb_energy(b, st);
-  kb_sp_pt<<<b.total[SPB_PT], 64, 0, st>>>(b);
+  kb_sp_pt<<<b.total[SPB_PT], kPtThreads, b.pt_smem, st>>>(b);
   kb_sp_permute<<<b.total[SPB_PERMUTE], kPermRows, b.perm_smem, st>>>(b);
   return cudaGetLastError();
 }
@@ -1321,7 +1508,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_sp_persist(const __grid_
       if (i < (long long)d.nw * 64 * d.NR * d.NB) d.U2[i] = 0;
     })
     if (!sp_grid_sync(p, epoch)) return false;
-    SPP_SUB(SPB_ENERGY, 256, sp_energy_body(d, (long long)blk * 256 + ltid))
+    SPP_BLOCKS(SPB_ENERGY, sp_energy_body(d, blk, smem))
     return sp_grid_sync(p, epoch);
   };
   for (int it = 0; it < p.itmax; ++it) {
@@ -1341,7 +1528,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_sp_persist(const __grid_
           }
         }
         if (!energy()) return;
-        SPP_SUB(SPB_PT, 64, sp_pt_body(d, blk, ltid))
+        SPP_BLOCKS(SPB_PT, sp_pt_body(d, blk, smem))
         SPP_SYNC();
         SPP_BLOCKS(SPB_PERMUTE, sp_permute_body(d, blk, reinterpret_cast<u64 *>(smem)))
         SPP_SYNC();
@@ -1384,8 +1571,8 @@ int sp_persist_grid(const SpBatchDev &b, size_t smem) {
     return 0;
   uint32_t work = (uint32_t)b.njobs;
   for (int k = 0; k < SPB_COUNT; ++k) {
-    const uint32_t sub = (k == SPB_PT) ? kPersistThreads / 64
-                         : (k >= SPB_PASS0 && k <= SPB_PASS3) || k == SPB_PERMUTE || k == SPB_CL0 || k == SPB_CL1
+    const uint32_t sub = (k >= SPB_PASS0 && k <= SPB_PASS3) || k == SPB_ENERGY || k == SPB_PT || k == SPB_PERMUTE ||
+                                 k == SPB_CL0 || k == SPB_CL1
                              ? 1 : kPersistThreads / 256;
     work = std::max(work, (b.total[k] + sub - 1) / sub);
   }
@@ -1422,10 +1609,14 @@ __global__ void __launch_bounds__(512) k_sp_pass_items(const __grid_constant__ S
   sp_pass_items_body(d, off, n, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)n * d.NR * d.NB,
                      (long long)gridDim.x * blockDim.x, smem);
 }
-__global__ void __launch_bounds__(256) k_sp_energy(const __grid_constant__ SpDev d) {
-  sp_energy_body(d, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(kEnMaxThreads, 4) k_sp_energy(const __grid_constant__ SpDev d) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  sp_energy_body(d, blockIdx.x, smem);
 }
-__global__ void __launch_bounds__(64) k_sp_pt(const __grid_constant__ SpDev d) { sp_pt_body(d, blockIdx.x, threadIdx.x); }
+__global__ void __launch_bounds__(kPtThreads) k_sp_pt(const __grid_constant__ SpDev d) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  sp_pt_body(d, blockIdx.x, smem);
+}
 __global__ void __launch_bounds__(kPermRows) k_sp_permute(const __grid_constant__ SpDev d) {
   extern __shared__ u64 rows[];
   sp_permute_body(d, blockIdx.x, rows);
@@ -1503,6 +1694,8 @@ cudaError_t sp_setup() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, cl);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_sp_permute, cudaFuncAttributeMaxDynamicSharedMemorySize, kPermRows * 65 * 8);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_energy, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_pt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pt_smem(64));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_slab<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_slab<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_slab<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
@@ -1527,19 +1720,19 @@ cudaError_t sp_launch_energy(const SpDev &d, cudaStream_t st) {
   const int G = d.NR * d.NB;
   cudaError_t e = cudaMemsetAsync(d.U2, 0, sizeof(int32_t) * (size_t)d.nw * 64 * G, st);
   if (e != cudaSuccess) return e;
-  const long long n = (long long)d.nw * ((d.esites + d.echunk - 1) / d.echunk) * G;
-  k_sp_energy<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d);
+  const int nth = d.en.threads;
+  k_sp_energy<<<(unsigned)en_blocks(d), nth, en_smem(d, nth), st>>>(d);
   return cudaGetLastError();
 }
 
 cudaError_t sp_launch_pt(const SpDev &d, cudaStream_t st) {
-  k_sp_pt<<<d.nw * d.NR, 64, 0, st>>>(d);
+  k_sp_pt<<<d.nw * d.NR, kPtThreads, pt_smem(d.NB), st>>>(d);
   return cudaGetLastError();
 }
 
 cudaError_t sp_launch_permute(const SpDev &d, cudaStream_t st) {
   const long long n = (long long)d.nw * d.V * d.NR;
-  k_sp_permute<<<(unsigned)((n + kPermRows - 1) / kPermRows), kPermRows, (size_t)kPermRows * (d.NB | 1) * 8, st>>>(d);
+  k_sp_permute<<<(unsigned)((n + kPermRows - 1) / kPermRows), kPermRows, perm_smem(d.NB), st>>>(d);
   return cudaGetLastError();
 }
 
@@ -1754,7 +1947,7 @@ int ea_sp_create(const ea_sp_geom *gp, int32_t device, ea_sp **out) {
   d.cthreads = sp_cluster_threads(d.L, d.Lz);
   d.esites = d.V;
   d.epair = 0;
-  d.echunk = sp_energy_chunk(d);
+  sp_energy_shape(d, sp_energy_chunk(d));
   for (int k = 0; k <= g.ncol && k < 9; ++k) d.col_off[k] = g.col_off[k];
   if (!d.kt) { delete c; return spfail(EA_ERR_ARG, "NB=%d x NR=%d does not fit in shared memory", d.NB, d.NR); }
   c->device = device;
@@ -2017,7 +2210,7 @@ int ea_sp_set_couplings(ea_sp *c, const uint64_t *J) {
   c->pair_energy = sp_pair_energy(c->g, c->d.nw, J);
   c->d.epair = c->pair_energy ? 1 : 0;
   c->d.esites = c->pair_energy ? c->g.col_off[2] - c->g.col_off[1] : c->d.V;
-  c->d.echunk = sp_energy_chunk(c->d);
+  sp_energy_shape(c->d, sp_energy_chunk(c->d));
   return EA_OK;
 }
 
@@ -2115,13 +2308,13 @@ int ea_sp_autotune(ea_sp *c, int32_t *tile, int32_t *echunk, int32_t *cthreads) 
   const int ec0 = d.echunk;
   int best_ec = ec0;
   best = 1e30f;
-  for (int ec : {ec0 / 4, ec0 / 2, ec0, ec0 * 2, ec0 * 4}) {
-    if (ec < 1 || ec > 256) continue;
-    d.echunk = ec;
+  for (int ec : {ec0 / 4, ec0 / 2, ec0, ec0 * 2, kEnSites}) {
+    if (ec < 1 || ec > kEnSites) continue;
+    sp_energy_shape(d, ec);
     const float ms = timed([&] { sp_launch_energy(d, c->st); });
     if (ms < best) { best = ms; best_ec = ec; }
   }
-  d.echunk = best_ec;
+  sp_energy_shape(d, best_ec);
   // block size of the labelling (lattices labelled in SMEM)
   int best_ct = d.cthreads;
   if (d.V <= kSpClusterMaxV) {
@@ -2299,7 +2492,8 @@ static int sp_run_persist(ea_sp *c, const ea_cadence *cad) {
   p.ncol_max = d.ncol;
   p.bar = c->p_bar;
   p.err = c->p_err;
-  size_t smem = std::max(sp_sweep_smem(d.NB, d.NR, d.kt), (size_t)kPermRows * (d.NB | 1) * 8);
+  size_t smem = std::max(sp_sweep_smem(d.NB, d.NR, d.kt), perm_smem(d.NB));
+  smem = std::max(smem, std::max(en_smem(d, kPersistThreads), pt_smem(d.NB)));
   if (p.cluster) smem = std::max(smem, sp_cluster_smem(d.L, d.Lz));
   const int grid = sp_persist_grid(p.b, smem);
   if (grid < 1) return spfail(EA_ERR_CUDA, "persistent bin kernel: no co-resident grid for %zu bytes of shared memory", smem);
@@ -2531,7 +2725,7 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
   const int n = (int)k.jobs.size();
   std::vector<SpDev> hj(n);
   std::vector<uint32_t> hp((size_t)SPB_COUNT * (n + 1), 0);
-  int pass_smem = 0, perm_smem = 0, cl_smem = 0;
+  int pass_smem = 0, prm_smem = 0, cl_smem = 0, e_smem = 0, t_smem = 0, e_threads = 32;
   for (int i = 0; i < n; ++i) {
     hj[i] = k.jobs[i]->d;
     uint32_t cnt[SPB_COUNT];
@@ -2539,7 +2733,10 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
     for (int q = 0; q < SPB_COUNT; ++q) hp[(size_t)q * (n + 1) + i + 1] = hp[(size_t)q * (n + 1) + i] + cnt[q];
     pass_smem = std::max(pass_smem, (int)(hj[i].pgrid ? sp_items_smem(hj[i].NB)
                                                        : sp_sweep_smem(hj[i].NB, hj[i].NR, hj[i].kt)));
-    perm_smem = std::max(perm_smem, kPermRows * (hj[i].NB | 1) * 8);
+    prm_smem = std::max(prm_smem, (int)perm_smem(hj[i].NB));
+    e_threads = std::max(e_threads, hj[i].en.threads);
+    e_smem = std::max(e_smem, (int)en_smem(hj[i], kPersistThreads));  // a persistent launch's blocks are the larger
+    t_smem = std::max(t_smem, (int)pt_smem(hj[i].NB));
     if (cluster) cl_smem = std::max(cl_smem, (int)sp_cluster_smem(hj[i].L, hj[i].Lz));
   }
   if (k.up_jobs.size() != hj.size() || std::memcmp(k.up_jobs.data(), hj.data(), sizeof(SpDev) * n) ||
@@ -2559,7 +2756,10 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
     bd.total[q] = hp[(size_t)q * (n + 1) + n];
   }
   bd.pass_smem = pass_smem;
-  bd.perm_smem = perm_smem;
+  bd.perm_smem = prm_smem;
+  bd.energy_smem = e_smem;
+  bd.energy_threads = e_threads;
+  bd.pt_smem = t_smem;
   bd.cluster_smem = cl_smem;
   bd.cluster_threads = k.cl_threads;
   return EA_OK;
@@ -2705,7 +2905,7 @@ int ea_sp_batch_run(ea_sp_batch *b, const ea_cadence *cad) {
     p.ncol_max = b->all.ncol_max;
     p.bar = b->p_bar;
     p.err = b->p_err;
-    const size_t smem = (size_t)std::max(std::max(p.b.pass_smem, p.b.perm_smem), p.b.cluster_smem);
+    const size_t smem = (size_t)std::max({p.b.pass_smem, p.b.perm_smem, p.b.cluster_smem, p.b.energy_smem, p.b.pt_smem});
     const int grid = sp_persist_grid(p.b, smem);
     if (grid < 1) return spfail(EA_ERR_CUDA, "persistent bin kernel: no co-resident grid for %zu bytes of shared memory", smem);
     SCU(sp_launch_persist(p, grid, smem, b->bs));

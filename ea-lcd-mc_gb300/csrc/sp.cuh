@@ -35,10 +35,19 @@ bool sp_graph(int L, int Lz, int bc, SpGraph &g);
 void sp_couplings(const SpGraph &g, int nwords, uint64_t seed_J, uint64_t *J);
 void sp_spins(const SpGraph &g, int nwords, int NR, int NB, uint64_t seed_u, uint64_t *S);
 
+// Launch shape of the energy count (k_sp_energy).
+struct EnShape {
+  int lanes;    // columns of a block, one lane each
+  int nslice;   // column slices
+  int threads;  // block size
+  int tile, ntile;  // sites of a block, tiles of a word
+};
+
 // Device view of a sample-packed job (kernel parameter).
 struct SpDev {
   int L, Lz, V, bc, NB, NR, nw, ncol, kt;
   int echunk;                        // sites per thread of the energy count
+  EnShape en;
   int esites, epair;                 // sites the count walks: all V, or (epair = 1) the colour-1 sites, counted twice
   int cthreads;                      // block size of the one-job cluster labelling
   int pgrid;                         // > 0: one-job colour passes as the per-item pass on this many CTAs
@@ -117,8 +126,8 @@ struct SpBatchDev {
   int njobs;
   const uint32_t *pre[SPB_COUNT];
   uint32_t total[SPB_COUNT];
-  int pass_smem, perm_smem, cluster_smem;  // dynamic SMEM of the largest job
-  int cluster_threads;                      // block size of the labelling
+  int pass_smem, perm_smem, cluster_smem, energy_smem, pt_smem;  // dynamic SMEM of the largest job
+  int cluster_threads, energy_threads;     // block sizes of the labelling and of the count
 };
 void sp_batch_blocks(const SpDev &d, bool cluster, uint32_t out[SPB_COUNT]);
 
