@@ -170,14 +170,19 @@ __device__ __forceinline__ void gather6(const u64 *oth, const int *nb, int flags
 
 // Bit-sliced local field and Metropolis flip mask (main.cu:1474-1506): flip with
 // probability min(1, p^(3-c)) where c counts satisfied-minus-unsatisfied pairs.
-__device__ __forceinline__ u64 flip_mask(const u64 f[6], u64 b0, u64 b1, u64 b2) {
+// From the random words b0, b1, b2 it takes id2 = b0 & b1 and id1 = (b0 ^ id2)
+// | (id2 & b2).
+__device__ __forceinline__ u64 flip_mask_id(const u64 f[6], u64 id1, u64 id2) {
   u64 k1 = f[0] ^ f[1], k2 = f[0] & f[1];
   const u64 j1 = k1 ^ f[2], j2 = k2 ^ (k1 & f[2]);
   k1 = f[3] ^ f[4]; k2 = f[3] & f[4];
   const u64 j3 = k1 ^ f[5], j4 = k2 ^ (k1 & f[5]);
-  b1 = b0 & b1; b2 = b1 & b2;
-  const u64 id2 = b1, id1 = (b0 ^ b1) | b2, j24 = j2 | j4;
+  const u64 j24 = j2 | j4;
   return (j1 & j3 & id1) | ((j24 | id2) & (j1 | j3 | id1)) | ((j2 & j4) | (j24 & id2));
+}
+__device__ __forceinline__ u64 flip_mask(const u64 f[6], u64 b0, u64 b1, u64 b2) {
+  b1 = b0 & b1; b2 = b1 & b2;
+  return flip_mask_id(f, (b0 ^ b1) | b2, b1);
 }
 
 // ---------------------------------------------------------------------------

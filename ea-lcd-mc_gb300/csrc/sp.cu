@@ -155,57 +155,151 @@ __device__ __forceinline__ void sp_pass_body(const SpDev &d, int off, int n, int
 
 // The per-item form of a colour pass.  A thread takes (site, replica, slot)
 // items of the colour in turn -- consecutive lanes on consecutive slots, so a
-// warp's loads and stores cover consecutive words -- draws the item's three
-// random words and updates the item's word in each sample word.  The block
-// stages the 11-bit pre-search tables once (the thresholds, rarely read past
-// them, come through the read-only cache); no random word goes through SMEM
-// and no barrier separates drawing from updating.  The words are those of the
-// tiles (same random words per (slot, site, replica), same flip mask).  This
-// form suits jobs with few sample words, whose tiles spend their time on
-// barriers and SMEM traffic for random words used once.
+// warp's loads and stores cover consecutive words -- draws the item's random
+// words and updates the item's word in each sample word.  The block stages the
+// 11-bit pre-search tables once (the thresholds, rarely read past them, come
+// through the read-only cache); no barrier separates drawing from updating.
+// The words are those of the tiles (same random words per (slot, site,
+// replica), same flip mask).  This form suits jobs with few sample words,
+// whose tiles spend their time on barriers and SMEM traffic for random words
+// used once.
+//
+// The flip mask uses the three random words as b0, b0 & b1 and b0 & b1 & b2
+// only, and a bit of b0 is set with probability exp(-4 beta): where a 32-bit
+// half of b0 is 0 that half of b1 and b2 does not matter, nor that of b2 where
+// b0 & b1 is 0.  So a warp draws b0 for kItemsRound items a lane, collects the
+// halves that need b1 in a queue, draws those -- a full warp at a time, each
+// lane one half of any lane's item -- and the same for b2: 3.2 to 3.3 of an
+// item's 6 words on T in [0.6, 1.6] and [0.7, 1.6] (the draws are
+// counter-based, so the ones made are the same).  The loops stay rolled: the
+// three copies of a draw are most of the code, and unrolled by item they
+// missed the instruction cache.  The pass is bound by instruction issue (65 % of
+// the slots), mostly of these draws: 24 x 24 x 192, 32 temperatures, 4
+// replicas, one word: 760 -> 559 us a sweep; 12 x 12 x 48, 24 temperatures: 62
+// -> 55.
 // The thread takes items t0, t0 + stride, ... below tend of the colour's
 // n x NR x NB (the block's threads take consecutive t0): one job runs it on
-// a grid of resident CTAs (k_sp_pass_items), a batch on 4 x 512 items a
-// block (sp_pass_any).
+// a grid of resident CTAs (k_sp_pass_items), a batch on kItemsPerThread x 512
+// items a block (sp_pass_any).
+constexpr int kItemsRound = 3;
+constexpr int kItemsThreads = 1024;  // one job: one table copy for an SM's 32 warps
+// A warp's SMEM: the flip mask's two words in the making by (item, half,
+// lane), the items' Philox index and column, and the queue.
+struct ItemsWarp {
+  uint32_t id1[kItemsRound][2][32];  // b0, then (b0 ^ id2) | b0 & b1 & b2
+  uint32_t id2[kItemsRound][2][32];  // b0 & b1
+  uint32_t tp[kItemsRound][32];
+  uint16_t col[kItemsRound][32];
+  uint16_t queue[kItemsRound * 64];
+};
+
 __device__ __forceinline__ void sp_pass_items_body(const SpDev &d, int off, int n, long long t0, long long tend,
                                                    long long stride, unsigned char *smem) {
-  const int NB = d.NB, NR = d.NR, G = NR * NB, V = d.V;
-  uint8_t *s_pre = smem;
+  const int NB = d.NB, NR = d.NR, G = NR * NB, V = d.V, lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const uint8_t *s_pre = smem;
+  ItemsWarp &sw = reinterpret_cast<ItemsWarp *>(smem + (size_t)NB * kPre11Stride)[threadIdx.x >> 5];
   {
     const uint4 *ps = reinterpret_cast<const uint4 *>(d.pre11);
-    uint4 *pd = reinterpret_cast<uint4 *>(s_pre);
+    uint4 *pd = reinterpret_cast<uint4 *>(smem);
     for (int i = threadIdx.x; i < NB * (kPre11Stride / 16); i += blockDim.x) pd[i] = ps[i];
   }
   __syncthreads();
   const long long t1 = min(tend, (long long)n * G);
   const size_t wps = (size_t)V * G;  // words per sample word
-  for (long long t = t0; t < t1; t += stride) {
-    const int b = (int)(t % NB), r = (int)((t / NB) % NR), k = (int)(t / G);
-    const int site = __ldg(d.col_sites + off + k);
-    const uint32_t tp = (uint32_t)(((size_t)b * V + site) * NR + r);
-    const uint4 c = d.ctr[r];
-    const uint32_t key = __ldg(d.keys + r);
-    const u64 *cum = d.cum + b * 256;
-    const uint8_t *pre = s_pre + b * kPre11Stride;
-    uint32_t w[6];
+  // the item's site index k and column g, stepped without divisions
+  int k = (int)(t0 / G), g = (int)(t0 - (long long)k * G);
+  const int sk = (int)(stride / G), sg = (int)(stride - (long long)sk * G);
+  for (long long t = t0; t - lane < t1;) {
+    int site[kItemsRound], col[kItemsRound];
 #pragma unroll
-    for (int q = 0; q < 6; ++q)
-      w[q] = rnd_word_by(c.x + q, c.y, c.z + tp, c.w, key, tp,
-                         [&](uint32_t hi, uint32_t lo) { return lut_byte11(hi, lo, cum, pre); });
-    const u64 r0 = ((u64)w[0] << 32) | w[1], r1 = ((u64)w[2] << 32) | w[3], r2 = ((u64)w[4] << 32) | w[5];
-    int nbr[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) nbr[q] = __ldg(d.nb + (size_t)site * 6 + q);
-    u64 *Sc = d.S + (size_t)r * NB + b;
-    for (int ww = 0; ww < d.nw; ++ww) {
-      u64 *Sw = Sc + (size_t)ww * wps;
-      const u64 *Jp = d.J + ((size_t)ww * V + site) * 6;
-      const u64 sv = Sw[(size_t)site * G];
-      u64 f[6];
-#pragma unroll
-      for (int q = 0; q < 6; ++q) f[q] = sv ^ __ldg(Jp + q) ^ Sw[(size_t)nbr[q] * G];
-      Sw[(size_t)site * G] = sv ^ flip_mask(f, r0, r1, r2);
+    for (int it = 0; it < kItemsRound; ++it, t += stride, k += sk, g += sg) {
+      if (g >= G) { g -= G; ++k; }
+      site[it] = t < t1 ? __ldg(d.col_sites + off + k) : -1;
+      col[it] = g;
+      const int r = (int)d.fd_NB.div((uint32_t)g), b = g - r * NB;
+      sw.tp[it][lane] = (uint32_t)(((size_t)b * V + site[it]) * NR + r);
+      sw.col[it][lane] = t < t1 ? (uint16_t)g : 0xFFFFu;
     }
+    int nq = 0;
+#pragma unroll 1
+    for (int it = 0; it < kItemsRound; ++it) {
+      const uint32_t cg = sw.col[it][lane], tp = sw.tp[it][lane];
+      uint32_t w0 = 0, w1 = 0;
+      if (cg != 0xFFFFu) {
+        const int r = (int)d.fd_NB.div(cg), b = (int)cg - r * NB;
+        const uint4 c = d.ctr[r];
+        const uint32_t key = __ldg(d.keys + r);
+        const u64 *cum = d.cum + b * 256;
+        const uint8_t *pre = s_pre + b * kPre11Stride;
+        auto byte = [&](uint32_t hi, uint32_t lo) { return lut_byte11(hi, lo, cum, pre); };
+        w0 = rnd_word_by(c.x, c.y, c.z + tp, c.w, key, tp, byte);
+        w1 = rnd_word_by(c.x + 1, c.y, c.z + tp, c.w, key, tp, byte);
+      }
+      sw.id1[it][0][lane] = w0;
+      sw.id1[it][1][lane] = w1;
+      sw.id2[it][0][lane] = sw.id2[it][1][lane] = 0;
+      unsigned m = __ballot_sync(0xffffffffu, w0 != 0);
+      if (w0) sw.queue[nq + __popc(m & below)] = (uint16_t)(it << 6 | lane);
+      nq += __popc(m);
+      m = __ballot_sync(0xffffffffu, w1 != 0);
+      if (w1) sw.queue[nq + __popc(m & below)] = (uint16_t)(it << 6 | 32 | lane);
+      nq += __popc(m);
+    }
+#pragma unroll 1
+    for (int q = 2; q < 6 && nq; q += 2) {
+      __syncwarp();
+      int next = 0;  // the next queue, in place: it never runs ahead of the reads
+      for (int i0 = 0; i0 < nq; i0 += 32) {
+        const bool on = i0 + lane < nq;
+        const int e = on ? sw.queue[i0 + lane] : 0, it = e >> 6, h = (e >> 5) & 1, l = e & 31;
+        uint32_t a = 0;
+        if (on) {
+          const uint32_t cg = sw.col[it][l], tp = sw.tp[it][l];
+          const int r = (int)d.fd_NB.div(cg), b = (int)cg - r * NB;
+          const uint4 c = d.ctr[r];
+          const u64 *cum = d.cum + b * 256;
+          const uint8_t *pre = s_pre + b * kPre11Stride;
+          a = rnd_word_by(c.x + q + h, c.y, c.z + tp, c.w, __ldg(d.keys + r), tp,
+                          [&](uint32_t hi, uint32_t lo) { return lut_byte11(hi, lo, cum, pre); });
+          if (q == 2) {
+            const uint32_t b0 = sw.id1[it][h][l];
+            a &= b0;
+            sw.id2[it][h][l] = a;
+            sw.id1[it][h][l] = b0 ^ a;
+          } else {
+            sw.id1[it][h][l] |= a & sw.id2[it][h][l];
+          }
+        }
+        if (q == 2) {
+          const unsigned m = __ballot_sync(0xffffffffu, a != 0);
+          if (a) sw.queue[next + __popc(m & below)] = (uint16_t)e;
+          next += __popc(m);
+        }
+      }
+      nq = next;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int it = 0; it < kItemsRound; ++it) {
+      if (site[it] < 0) continue;
+      const u64 id1 = ((u64)sw.id1[it][0][lane] << 32) | sw.id1[it][1][lane];
+      const u64 id2 = ((u64)sw.id2[it][0][lane] << 32) | sw.id2[it][1][lane];
+      int nbr[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) nbr[q] = __ldg(d.nb + (size_t)site[it] * 6 + q);
+      u64 *Sc = d.S + col[it];
+      for (int ww = 0; ww < d.nw; ++ww) {
+        u64 *Sw = Sc + (size_t)ww * wps;
+        const u64 *Jp = d.J + ((size_t)ww * V + site[it]) * 6;
+        const u64 sv = Sw[(size_t)site[it] * G];
+        u64 f[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) f[q] = sv ^ __ldg(Jp + q) ^ Sw[(size_t)nbr[q] * G];
+        Sw[(size_t)site[it] * G] = sv ^ flip_mask_id(f, id1, id2);
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -349,10 +443,10 @@ __device__ __forceinline__ void sp_energy_body(const SpDev &d, int blk, unsigned
       const uint4 *nb = reinterpret_cast<const uint4 *>(sN + k * 8);
       const ulonglong2 *J = reinterpret_cast<const ulonglong2 *>(sJ + k * 6);
       const uint4 na = nb[0], nc = nb[1];
-      const u64 sv = __ldg(Sc + nc.z);
+      const u64 sv = Sc[nc.z];
       u64 f[6];
-      f[0] = __ldg(Sc + na.x); f[1] = __ldg(Sc + na.y); f[2] = __ldg(Sc + na.z);
-      f[3] = __ldg(Sc + na.w); f[4] = __ldg(Sc + nc.x); f[5] = __ldg(Sc + nc.y);
+      f[0] = Sc[na.x]; f[1] = Sc[na.y]; f[2] = Sc[na.z];
+      f[3] = Sc[na.w]; f[4] = Sc[nc.x]; f[5] = Sc[nc.y];
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const ulonglong2 j = J[q];
@@ -443,8 +537,8 @@ __device__ __forceinline__ void sp_pt_body(const SpDev &d, int wr, unsigned char
   for (int t = threadIdx.x; t < 64 * NB; t += blockDim.x) {
     const int lane = t / NB, b = t - lane * NB;
     const size_t o = row + (size_t)lane * G + b;
-    es[b * 65 + lane] = nt - __ldg(d.U2 + o);
-    ps[b * 64 + lane] = __ldg(d.perm + o);
+    es[b * 65 + lane] = nt - d.U2[o];
+    ps[b * 64 + lane] = d.perm[o];
   }
   for (int i = threadIdx.x; i < NB; i += blockDim.x) {
     eo[i] = __ldg(d.expoff + i);
@@ -526,11 +620,10 @@ constexpr int kPermRows = 128;
 
 __device__ __forceinline__ void ld32(u64 v[4], const u64 *p) {
   asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
-               : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p) : "memory");
+               : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
 }
 __device__ __forceinline__ void st32(u64 *p, const u64 v[4]) {
-  asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v[0]), "l"(v[1]), "l"(v[2]), "l"(v[3])
-               : "memory");
+  asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v[0]), "l"(v[1]), "l"(v[2]), "l"(v[3]));
 }
 
 inline size_t perm_smem(int NB) { return NB & 3 ? (size_t)kPermRows * (NB | 1) * 8 : 0; }
@@ -557,13 +650,13 @@ __device__ __forceinline__ void sp_permute_body(const SpDev &d, int blk, u64 *ro
       if (more) ld32(n, p + i + 4);
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
-        const u64 x = (cur ^ v[q + 1]) & __ldg(M + i + q);
+        const u64 x = (cur ^ v[q + 1]) & M[i + q];
         o[q] = cur ^ x;
         cur = v[q + 1] ^ x;
       }
       o[3] = cur;
       if (more) {
-        const u64 x = (cur ^ n[0]) & __ldg(M + i + 3);
+        const u64 x = (cur ^ n[0]) & M[i + 3];
         o[3] = cur ^ x;
         cur = n[0] ^ x;
       }
@@ -585,7 +678,7 @@ __device__ __forceinline__ void sp_permute_body(const SpDev &d, int blk, u64 *ro
     u64 *p = rows + (size_t)threadIdx.x * rs;
     u64 cur = p[0];
     for (int i = 0; i < NB - 1; ++i) {
-      const u64 m = __ldg(M + i);
+      const u64 m = M[i];
       const u64 nxt = p[i + 1];
       const u64 x = (cur ^ nxt) & m;
       p[i] = cur ^ x;
@@ -1604,7 +1697,7 @@ __global__ void __launch_bounds__(512) k_sp_pass(const __grid_constant__ SpDev d
   sp_pass_body(d, off, n, blockIdx.x, smem);
 }
 
-__global__ void __launch_bounds__(512) k_sp_pass_items(const __grid_constant__ SpDev d, int off, int n) {
+__global__ void __launch_bounds__(kItemsThreads, 1) k_sp_pass_items(const __grid_constant__ SpDev d, int off, int n) {
   extern __shared__ __align__(16) unsigned char smem[];
   sp_pass_items_body(d, off, n, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)n * d.NR * d.NB,
                      (long long)gridDim.x * blockDim.x, smem);
@@ -1660,14 +1753,14 @@ size_t sp_cluster_smem(int L, int Lz);
 size_t sp_sweep_smem(int NB, int NR, int kt) {
   return (size_t)NB * 256 * 10 + (size_t)3 * NB * kt * NR * 8 + (size_t)kt * 7 * 4;
 }
-size_t sp_items_smem(int NB) { return (size_t)NB * kPre11Stride; }
+size_t sp_items_smem(int NB, int threads) { return (size_t)NB * kPre11Stride + threads / 32 * sizeof(ItemsWarp); }
 
 // Grid of the per-item pass: every CTA resident at once (the kernel's
 // registers and the threshold tables' SMEM allowing); 0 if none fits.
 int sp_items_grid(int NB) {
   int dev = 0, nsm = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sp_pass_items, 512, sp_items_smem(NB)) != cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sp_pass_items, kItemsThreads, sp_items_smem(NB, kItemsThreads)) != cudaSuccess)
     return 0;
   return per_sm * nsm;
 }
@@ -1707,8 +1800,9 @@ cudaError_t sp_launch_pass(const SpDev &d, int colour, int off, int n, cudaStrea
   k_sp_fill<<<1, 64, 0, st>>>(d);
   (void)colour;
   if (n > 0 && d.pgrid > 0) {
-    const long long blocks = ((long long)n * d.NR * d.NB + 511) / 512;
-    k_sp_pass_items<<<(unsigned)std::min<long long>(blocks, d.pgrid), 512, sp_items_smem(d.NB), st>>>(d, off, n);
+    const long long blocks = ((long long)n * d.NR * d.NB + kItemsThreads - 1) / kItemsThreads;
+    k_sp_pass_items<<<(unsigned)std::min<long long>(blocks, d.pgrid), kItemsThreads, sp_items_smem(d.NB, kItemsThreads), st>>>(
+        d, off, n);
   } else if (n > 0) {
     const int grid = (n + d.kt - 1) / d.kt;
     k_sp_pass<<<grid, 512, sp_sweep_smem(d.NB, d.NR, d.kt), st>>>(d, off, n);
@@ -1945,6 +2039,7 @@ int ea_sp_create(const ea_sp_geom *gp, int32_t device, ea_sp **out) {
   for (int k = 0; k < g.ncol; ++k) maxc = std::max(maxc, g.col_off[k + 1] - g.col_off[k]);
   d.kt = sp_kt(d.NB, d.NR, maxc);
   d.cthreads = sp_cluster_threads(d.L, d.Lz);
+  d.fd_NB.set((uint32_t)d.NB);
   d.esites = d.V;
   d.epair = 0;
   sp_energy_shape(d, sp_energy_chunk(d));
@@ -2492,7 +2587,7 @@ static int sp_run_persist(ea_sp *c, const ea_cadence *cad) {
   p.ncol_max = d.ncol;
   p.bar = c->p_bar;
   p.err = c->p_err;
-  size_t smem = std::max(sp_sweep_smem(d.NB, d.NR, d.kt), perm_smem(d.NB));
+  size_t smem = std::max(d.pgrid ? sp_items_smem(d.NB, kPersistThreads) : sp_sweep_smem(d.NB, d.NR, d.kt), perm_smem(d.NB));
   smem = std::max(smem, std::max(en_smem(d, kPersistThreads), pt_smem(d.NB)));
   if (p.cluster) smem = std::max(smem, sp_cluster_smem(d.L, d.Lz));
   const int grid = sp_persist_grid(p.b, smem);
@@ -2731,7 +2826,7 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
     uint32_t cnt[SPB_COUNT];
     sp_batch_blocks(hj[i], cluster, cnt);
     for (int q = 0; q < SPB_COUNT; ++q) hp[(size_t)q * (n + 1) + i + 1] = hp[(size_t)q * (n + 1) + i] + cnt[q];
-    pass_smem = std::max(pass_smem, (int)(hj[i].pgrid ? sp_items_smem(hj[i].NB)
+    pass_smem = std::max(pass_smem, (int)(hj[i].pgrid ? sp_items_smem(hj[i].NB, kPersistThreads)  // the batched launch has as many threads
                                                        : sp_sweep_smem(hj[i].NB, hj[i].NR, hj[i].kt)));
     prm_smem = std::max(prm_smem, (int)perm_smem(hj[i].NB));
     e_threads = std::max(e_threads, hj[i].en.threads);

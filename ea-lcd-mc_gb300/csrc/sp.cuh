@@ -19,6 +19,7 @@
 #include <vector>
 #include <cuda_runtime.h>
 #include "eagb.h"
+#include "kernels.cuh"
 
 namespace eagb {
 
@@ -46,6 +47,7 @@ struct EnShape {
 // Device view of a sample-packed job (kernel parameter).
 struct SpDev {
   int L, Lz, V, bc, NB, NR, nw, ncol, kt;
+  FastDiv fd_NB;
   int echunk;                        // sites per thread of the energy count
   EnShape en;
   int esites, epair;                 // sites the count walks: all V, or (epair = 1) the colour-1 sites, counted twice
@@ -100,7 +102,7 @@ int sp_kt(int NB, int NR, int nsites_colour);
 int sp_slab_planes(int L, int Lz, int nw, int nclust, int *samples);
 int sp_energy_chunk(const SpDev &d);
 size_t sp_sweep_smem(int NB, int NR, int kt);
-size_t sp_items_smem(int NB);
+size_t sp_items_smem(int NB, int threads);
 int sp_items_grid(int NB);
 cudaError_t sp_setup();
 cudaError_t sp_launch_pass(const SpDev &d, int colour, int off, int n, cudaStream_t st);
