@@ -40,7 +40,8 @@ __device__ __forceinline__ void sp_fill_body(const SpDev &d) {
 // consecutive lanes touch consecutive words of a site.  The Philox thread
 // index of (slot b, site i, replica r) is (b*V + i)*NR + r.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void sp_pass_body(const SpDev &d, int off, int n, int tile, unsigned char *smem) {
+__device__ __forceinline__ void sp_pass_body(const SpDev &d, const uint4 *ctr, int off, int n, int tile,
+                                             unsigned char *smem) {
   const int NB = d.NB, NR = d.NR, kt = d.kt, V = d.V;
   u64 *s_cum = reinterpret_cast<u64 *>(smem);
   uint16_t *s_pre = reinterpret_cast<uint16_t *>(s_cum + NB * 256);
@@ -74,7 +75,7 @@ __device__ __forceinline__ void sp_pass_body(const SpDev &d, int off, int n, int
     if (k0 + kk >= n) continue;
     const int site = s_nb[kk * 7];
     const uint32_t tp = (uint32_t)(((size_t)b * V + site) * NR + r);
-    const uint4 c = d.ctr[r];
+    const uint4 c = ctr[r];
     const uint32_t key = d.keys[r];
     const u64 *cum = s_cum + b * 256;
     const uint16_t *pre = s_pre + b * 256;
@@ -193,8 +194,8 @@ struct ItemsWarp {
   uint16_t queue[kItemsRound * 64];
 };
 
-__device__ __forceinline__ void sp_pass_items_body(const SpDev &d, int off, int n, long long t0, long long tend,
-                                                   long long stride, unsigned char *smem) {
+__device__ __forceinline__ void sp_pass_items_body(const SpDev &d, const uint4 *ctr, int off, int n, long long t0,
+                                                   long long tend, long long stride, unsigned char *smem) {
   const int NB = d.NB, NR = d.NR, G = NR * NB, V = d.V, lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const uint8_t *s_pre = smem;
@@ -228,7 +229,7 @@ __device__ __forceinline__ void sp_pass_items_body(const SpDev &d, int off, int 
       uint32_t w0 = 0, w1 = 0;
       if (cg != 0xFFFFu) {
         const int r = (int)d.fd_NB.div(cg), b = (int)cg - r * NB;
-        const uint4 c = d.ctr[r];
+        const uint4 c = ctr[r];
         const uint32_t key = __ldg(d.keys + r);
         const u64 *cum = d.cum + b * 256;
         const uint8_t *pre = s_pre + b * kPre11Stride;
@@ -257,7 +258,7 @@ __device__ __forceinline__ void sp_pass_items_body(const SpDev &d, int off, int 
         if (on) {
           const uint32_t cg = sw.col[it][l], tp = sw.tp[it][l];
           const int r = (int)d.fd_NB.div(cg), b = (int)cg - r * NB;
-          const uint4 c = d.ctr[r];
+          const uint4 c = ctr[r];
           const u64 *cum = d.cum + b * 256;
           const uint8_t *pre = s_pre + b * kPre11Stride;
           a = rnd_word_by(c.x + q + h, c.y, c.z + tp, c.w, __ldg(d.keys + r), tp,
@@ -305,14 +306,18 @@ __device__ __forceinline__ void sp_pass_items_body(const SpDev &d, int off, int 
 
 // A job's colour pass by its form; blk counts the job's blocks of the pass
 // (tiles, or kItemsPerThread x blockDim.x items of the per-item form).
-constexpr int kItemsPerThread = 4;
-__device__ __forceinline__ void sp_pass_any(const SpDev &d, int colour, int blk, unsigned char *smem) {
+// One round: a second one with an item or two a lane costs a batch of small
+// jobs 3 to 10 %; two full rounds suit 24 tubes of L 8..12 (9.2 against 9.6 ms a
+// bin) but not 16 of L 6 and 9 (7.7 against 6.3).
+constexpr int kItemsPerThread = kItemsRound;
+__device__ __forceinline__ void sp_pass_any(const SpDev &d, const uint4 *ctr, int colour, int blk, unsigned char *smem) {
   const int off = d.col_off[colour], n = d.col_off[colour + 1] - off;
   if (d.pgrid) {
     const long long t0 = (long long)blk * blockDim.x * kItemsPerThread;
-    sp_pass_items_body(d, off, n, t0 + threadIdx.x, t0 + (long long)blockDim.x * kItemsPerThread, blockDim.x, smem);
+    sp_pass_items_body(d, ctr, off, n, t0 + threadIdx.x, t0 + (long long)blockDim.x * kItemsPerThread, blockDim.x,
+                       smem);
   } else {
-    sp_pass_body(d, off, n, blk, smem);
+    sp_pass_body(d, ctr, off, n, blk, smem);
   }
 }
 
@@ -1366,16 +1371,10 @@ __device__ __forceinline__ int spb_job(const uint32_t *pre, int n, uint32_t v) {
   const SpDev &d = s_job;                                     \
   const int blk = (int)(blockIdx.x - __ldg(pre_ + jb));
 
-__global__ void kb_sp_fill(const __grid_constant__ SpBatchDev b, int colour) {
-  __shared__ SpDev d;
-  if (threadIdx.x == 0) d = b.jobs[blockIdx.x];
-  __syncthreads();
-  if (colour < d.ncol) sp_fill_body(d);
-}
-__global__ void __launch_bounds__(512) kb_sp_pass(const __grid_constant__ SpBatchDev b, int colour) {
+__global__ void __launch_bounds__(512, 2) kb_sp_pass(const __grid_constant__ SpBatchDev b, int sweep, int colour) {
   extern __shared__ __align__(16) unsigned char smem[];
   SPB_ITEM(SPB_PASS0 + colour)
-  sp_pass_any(d, colour, blk, smem);
+  sp_pass_any(d, d.ctrs + (size_t)(sweep * d.ncol + colour) * d.NR, colour, blk, smem);
 }
 __global__ void kb_sp_zero(const __grid_constant__ SpBatchDev b) {
   SPB_ITEM(SPB_ZERO)
@@ -1456,18 +1455,16 @@ cudaError_t sp_batch_setup() {
   cudaError_t e = max_dynamic_smem(kb_sp_pass);
   if (e == cudaSuccess) e = max_dynamic_smem(kb_sp_cluster);
   if (e == cudaSuccess) e = max_dynamic_smem(kb_sp_permute);
+  if (e == cudaSuccess) e = sp_batch_ctr_setup();
   if (e == cudaSuccess) e = max_dynamic_smem(kb_sp_energy);
   if (e == cudaSuccess) e = max_dynamic_smem(kb_sp_pt);
   return e;
 }
 
-// One sweep of every job: colour by colour, each job's counters advanced only
-// for the colours it has.
-cudaError_t sp_batch_sweep(const SpBatchDev &b, int ncol_max, cudaStream_t st) {
-  for (int c = 0; c < ncol_max; ++c) {
-    kb_sp_fill<<<b.njobs, 64, 0, st>>>(b, c);
-    if (b.total[SPB_PASS0 + c]) kb_sp_pass<<<b.total[SPB_PASS0 + c], 512, b.pass_smem, st>>>(b, c);
-  }
+// Sweep `sweep` of the counters drawn last (sp_batch_ctr_chain), colour by colour.
+cudaError_t sp_batch_sweep(const SpBatchDev &b, int ncol_max, int sweep, cudaStream_t st) {
+  for (int c = 0; c < ncol_max; ++c)
+    if (b.total[SPB_PASS0 + c]) kb_sp_pass<<<b.total[SPB_PASS0 + c], 512, b.pass_smem, st>>>(b, sweep, c);
   return cudaGetLastError();
 }
 
@@ -1616,7 +1613,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_sp_persist(const __grid_
               if (c < s_job[0].ncol) sp_fill_body(s_job[0]);
             }
             SPP_SYNC();
-            SPP_BLOCKS(SPB_PASS0 + c, sp_pass_any(d, c, blk, smem))
+            SPP_BLOCKS(SPB_PASS0 + c, sp_pass_any(d, d.ctr, c, blk, smem))
             SPP_SYNC();
           }
         }
@@ -1682,7 +1679,6 @@ cudaError_t sp_launch_persist(const SpPersistDev &p, int grid, size_t smem, cuda
 // ---------------------------------------------------------------------------
 // One-job kernels: the bodies above, one block per item
 // ---------------------------------------------------------------------------
-__global__ void k_sp_fill(const __grid_constant__ SpDev d) { sp_fill_body(d); }
 // Pseudo-random overlap words (a 64-bit mix of the index) for timing the
 // labelling on clusters of a random overlap; only the autotuner uses it.
 __global__ void k_sp_noise(unsigned long long *Q, long long n) {
@@ -1692,15 +1688,16 @@ __global__ void k_sp_noise(unsigned long long *Q, long long n) {
   x ^= x >> 31; x *= 0xBF58476D1CE4E5B9ull; x ^= x >> 29; x *= 0x94D049BB133111EBull; x ^= x >> 32;
   Q[i] = x;
 }
-__global__ void __launch_bounds__(512) k_sp_pass(const __grid_constant__ SpDev d, int off, int n) {
+__global__ void __launch_bounds__(512, 2) k_sp_pass(const __grid_constant__ SpDev d, int pass, int off, int n) {
   extern __shared__ __align__(16) unsigned char smem[];
-  sp_pass_body(d, off, n, blockIdx.x, smem);
+  sp_pass_body(d, d.ctrs + (size_t)pass * d.NR, off, n, blockIdx.x, smem);
 }
 
-__global__ void __launch_bounds__(kItemsThreads, 1) k_sp_pass_items(const __grid_constant__ SpDev d, int off, int n) {
+__global__ void __launch_bounds__(kItemsThreads, 1) k_sp_pass_items(const __grid_constant__ SpDev d, int pass, int off,
+                                                                     int n) {
   extern __shared__ __align__(16) unsigned char smem[];
-  sp_pass_items_body(d, off, n, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)n * d.NR * d.NB,
-                     (long long)gridDim.x * blockDim.x, smem);
+  sp_pass_items_body(d, d.ctrs + (size_t)pass * d.NR, off, n, (long long)blockIdx.x * blockDim.x + threadIdx.x,
+                     (long long)n * d.NR * d.NB, (long long)gridDim.x * blockDim.x, smem);
 }
 __global__ void __launch_bounds__(kEnMaxThreads, 4) k_sp_energy(const __grid_constant__ SpDev d) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1796,16 +1793,15 @@ cudaError_t sp_setup() {
   return e;
 }
 
-cudaError_t sp_launch_pass(const SpDev &d, int colour, int off, int n, cudaStream_t st) {
-  k_sp_fill<<<1, 64, 0, st>>>(d);
-  (void)colour;
+// Colour pass `pass` of the counters drawn last (sp_launch_ctr_chain).
+cudaError_t sp_launch_pass(const SpDev &d, int pass, int off, int n, cudaStream_t st) {
   if (n > 0 && d.pgrid > 0) {
     const long long blocks = ((long long)n * d.NR * d.NB + kItemsThreads - 1) / kItemsThreads;
     k_sp_pass_items<<<(unsigned)std::min<long long>(blocks, d.pgrid), kItemsThreads, sp_items_smem(d.NB, kItemsThreads), st>>>(
-        d, off, n);
+        d, pass, off, n);
   } else if (n > 0) {
     const int grid = (n + d.kt - 1) / d.kt;
-    k_sp_pass<<<grid, 512, sp_sweep_smem(d.NB, d.NR, d.kt), st>>>(d, off, n);
+    k_sp_pass<<<grid, 512, sp_sweep_smem(d.NB, d.NR, d.kt), st>>>(d, pass, off, n);
   }
   return cudaGetLastError();
 }
@@ -2062,6 +2058,7 @@ int ea_sp_create(const ea_sp_geom *gp, int32_t device, ea_sp **out) {
   { uint16_t *p; SOWN(p, (size_t)d.NB * 256); d.pre = p; }
   { uint8_t *p; SOWN(p, (size_t)d.NB * kPre11Stride); d.pre11 = p; }
   SOWN(d.ctr, (size_t)d.NR);
+  SOWN(d.ctrs, (size_t)kCtrPasses * d.NR);
   { uint32_t *p; SOWN(p, (size_t)d.NR); d.keys = p; }
   SOWN(d.prc, (size_t)d.NR);
   SOWN(d.xo, (size_t)d.NR);
@@ -2443,11 +2440,23 @@ int ea_sp_autotune(ea_sp *c, int32_t *tile, int32_t *echunk, int32_t *cthreads) 
   return EA_OK;
 }
 
-static int sp_sweeps(ea_sp *c, int n) {
+// The passes of n sweeps from pass `pass` of the counters drawn last.
+static int sp_passes(ea_sp *c, int n, int pass) {
   const SpGraph &g = c->g;
   for (int s = 0; s < n; ++s)
     for (int k = 0; k < g.ncol; ++k)
-      SCU(sp_launch_pass(c->d, k, g.col_off[k], g.col_off[k + 1] - g.col_off[k], c->st));
+      SCU(sp_launch_pass(c->d, pass++, g.col_off[k], g.col_off[k + 1] - g.col_off[k], c->st));
+  return EA_OK;
+}
+
+static int sp_sweeps(ea_sp *c, int n) {
+  while (n > 0) {
+    const int m = std::min(n, kCtrPasses / c->g.ncol);
+    SCU(sp_launch_ctr_chain(c->d, m * c->g.ncol, c->d.ctrs, c->st));
+    const int rc = sp_passes(c, m, 0);
+    if (rc) return rc;
+    n -= m;
+  }
   return EA_OK;
 }
 
@@ -2716,9 +2725,13 @@ int ea_sp_run(ea_sp *c, const ea_cadence *cad, double *avgE) {
   // one iteration: every launch reads its counters (pass, tempering step,
   // move) from the device, so the captured graph replays each iteration
   auto iteration = [&]() -> int {
+    // the counters of every sweep up to the move at once, when they fit
+    const long long per = (long long)cad->ptfr * c->g.ncol;
+    const bool ahead = per * cad->houfr <= kCtrPasses;
     for (int im = 0; im < cad->mesfr; ++im) {
+      if (ahead) SCU(sp_launch_ctr_chain(c->d, (int)per * cad->houfr, c->d.ctrs, c->st));
       for (int ih = 0; ih < cad->houfr; ++ih) {
-        int r = sp_sweeps(c, cad->ptfr);
+        int r = ahead ? sp_passes(c, cad->ptfr, (int)per * ih) : sp_sweeps(c, cad->ptfr);
         if (!r) r = sp_pt(c);
         if (r) return r;
       }
@@ -2820,7 +2833,7 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
   const int n = (int)k.jobs.size();
   std::vector<SpDev> hj(n);
   std::vector<uint32_t> hp((size_t)SPB_COUNT * (n + 1), 0);
-  int pass_smem = 0, prm_smem = 0, cl_smem = 0, e_smem = 0, t_smem = 0, e_threads = 32;
+  int pass_smem = 0, prm_smem = 0, cl_smem = 0, e_smem = 0, t_smem = 0, e_threads = 32, nrep = 1;
   for (int i = 0; i < n; ++i) {
     hj[i] = k.jobs[i]->d;
     uint32_t cnt[SPB_COUNT];
@@ -2829,6 +2842,7 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
     pass_smem = std::max(pass_smem, (int)(hj[i].pgrid ? sp_items_smem(hj[i].NB, kPersistThreads)  // the batched launch has as many threads
                                                        : sp_sweep_smem(hj[i].NB, hj[i].NR, hj[i].kt)));
     prm_smem = std::max(prm_smem, (int)perm_smem(hj[i].NB));
+    nrep = std::max(nrep, hj[i].NR);
     e_threads = std::max(e_threads, hj[i].en.threads);
     e_smem = std::max(e_smem, (int)en_smem(hj[i], kPersistThreads));  // a persistent launch's blocks are the larger
     t_smem = std::max(t_smem, (int)pt_smem(hj[i].NB));
@@ -2854,6 +2868,7 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
   bd.perm_smem = prm_smem;
   bd.energy_smem = e_smem;
   bd.energy_threads = e_threads;
+  bd.nrep = nrep;
   bd.pt_smem = t_smem;
   bd.cluster_smem = cl_smem;
   bd.cluster_threads = k.cl_threads;
@@ -2862,9 +2877,21 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
 
 static cudaError_t spb_iteration(const SpClass &k, const ea_cadence *cad, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
+  const int fit = kCtrPasses / k.ncol_max;  // sweeps whose counters are drawn at once
   for (int im = 0; im < cad->mesfr && e == cudaSuccess; ++im) {
+    long long left = (long long)cad->houfr * cad->ptfr;  // sweeps up to the move
+    int drawn = 0, next = 0;
     for (int ih = 0; ih < cad->houfr && e == cudaSuccess; ++ih) {
-      for (int sw = 0; sw < cad->ptfr && e == cudaSuccess; ++sw) e = sp_batch_sweep(k.bd, k.ncol_max, st);
+      for (int sw = 0; sw < cad->ptfr && e == cudaSuccess; ++sw) {
+        if (next == drawn) {
+          drawn = (int)std::min<long long>(left, fit);
+          next = 0;
+          e = sp_batch_ctr_chain(k.bd, drawn, st);
+          if (e != cudaSuccess) break;
+        }
+        e = sp_batch_sweep(k.bd, k.ncol_max, next++, st);
+        --left;
+      }
       if (e == cudaSuccess) e = sp_batch_tempering(k.bd, st);
     }
     if (e == cudaSuccess && cad->cluster) e = sp_batch_houdayer(k.bd, st);
@@ -3058,7 +3085,7 @@ int ea_sp_job_bytes(const ea_sp_geom *gp, const ea_cadence *cad, const double *b
   add(V * 24); add(V * 4);                                   // neighbour table, colour lists
   add(nw * V * G * 8); add(nw * V * 48);                     // spins, couplings
   add(NB * 256 * 8); add(NB * 256 * 2); add(NB * kPre11Stride);  // thresholds, pre-searches
-  add(NR * 16); add(NR * 4); add(NR * sizeof(ea_hq)); add(NR * sizeof(ea_xoshiro)); add(8);
+  add(NR * 16); add(NR * 16 * kCtrPasses); add(NR * 4); add(NR * sizeof(ea_hq)); add(NR * sizeof(ea_xoshiro)); add(8);
   add(nw * 64 * G * 4); add(nw * 64 * G * 4); add(nw * 64 * G);   // U2, E, slot permutations
   add(nw * 64 * NR * (NB - 1) * 4); add(nw * NR * (NB - 1) * 8); // accepted swaps, lane masks
   add(NB * 8); add(NB * 4); add(8); add(nw * 64 * G * 8);   // betas, exp offsets, step, averages

@@ -36,6 +36,9 @@ bool sp_graph(int L, int Lz, int bc, SpGraph &g);
 void sp_couplings(const SpGraph &g, int nwords, uint64_t seed_J, uint64_t *J);
 void sp_spins(const SpGraph &g, int nwords, int NR, int NB, uint64_t seed_u, uint64_t *S);
 
+// Colour passes whose counters are drawn by one launch.
+constexpr int kCtrPasses = 512;
+
 // Launch shape of the energy count (k_sp_energy).
 struct EnShape {
   int lanes;    // columns of a block, one lane each
@@ -61,7 +64,8 @@ struct SpDev {
   const unsigned long long *cum;     // [NB][256] thresholds
   const uint16_t *pre;               // [NB][256] 8-bit pre-search
   const uint8_t *pre11;              // [NB][2064] 11-bit pre-search (the per-item pass)
-  uint4 *ctr;                        // [NR] Philox counters of the current pass
+  uint4 *ctr;                        // [NR] Philox counters of the last pass
+  uint4 *ctrs;                       // [kCtrPasses][NR] those of the passes drawn ahead
   const uint32_t *keys;              // [NR]
   ea_hq *prc;                        // [NR]
   ea_xoshiro *xo;                    // [NR]
@@ -105,7 +109,8 @@ size_t sp_sweep_smem(int NB, int NR, int kt);
 size_t sp_items_smem(int NB, int threads);
 int sp_items_grid(int NB);
 cudaError_t sp_setup();
-cudaError_t sp_launch_pass(const SpDev &d, int colour, int off, int n, cudaStream_t st);
+cudaError_t sp_launch_ctr_chain(const SpDev &d, int npass, uint4 *ctrs, cudaStream_t st);
+cudaError_t sp_launch_pass(const SpDev &d, int pass, int off, int n, cudaStream_t st);
 cudaError_t sp_launch_energy(const SpDev &d, cudaStream_t st);
 cudaError_t sp_launch_pt(const SpDev &d, cudaStream_t st);
 cudaError_t sp_launch_permute(const SpDev &d, cudaStream_t st);
@@ -130,6 +135,7 @@ struct SpBatchDev {
   uint32_t total[SPB_COUNT];
   int pass_smem, perm_smem, cluster_smem, energy_smem, pt_smem;  // dynamic SMEM of the largest job
   int cluster_threads, energy_threads;     // block sizes of the labelling and of the count
+  int nrep;                                 // the most replicas of a job
 };
 void sp_batch_blocks(const SpDev &d, bool cluster, uint32_t out[SPB_COUNT]);
 
@@ -184,7 +190,9 @@ cudaError_t sp_res_setup();
 // words, then the resident kernel over p.nit iterations.
 cudaError_t sp_res_chunk(const SpResDev &p, const SpResPlan &pl, int npass, uint4 *ctrs, cudaStream_t st);
 cudaError_t sp_batch_setup();
-cudaError_t sp_batch_sweep(const SpBatchDev &b, int ncol_max, cudaStream_t st);
+cudaError_t sp_batch_ctr_setup();
+cudaError_t sp_batch_ctr_chain(const SpBatchDev &b, int nsweep, cudaStream_t st);
+cudaError_t sp_batch_sweep(const SpBatchDev &b, int ncol_max, int sweep, cudaStream_t st);
 cudaError_t sp_batch_tempering(const SpBatchDev &b, cudaStream_t st);
 cudaError_t sp_batch_houdayer(const SpBatchDev &b, cudaStream_t st);
 cudaError_t sp_batch_measure(const SpBatchDev &b, bool from_e, cudaStream_t st);

@@ -42,11 +42,12 @@ constexpr int kResPlanes = 15;
 constexpr int kResMaxSites = ((1 << kResPlanes) - 1) / 6;
 
 // ---------------------------------------------------------------------------
-// Counters of npass consecutive colour passes (the fill step of sp.cu's
-// k_sp_fill, repeated): pass p uses time counter iter0 + p and its parity.
+// Counters of npass consecutive colour passes (fill_bits_body's step,
+// repeated): pass p uses time counter iter0 + p and its parity.  Every path
+// but the persistent kernel's draws its passes' counters this way: a launch of
+// the step alone is a 4 us link in a small job's chain, 0.5 us here.
 // ---------------------------------------------------------------------------
-__global__ void k_sp_ctr_chain(const __grid_constant__ SpDev d, int npass, uint4 *ctrs) {
-  extern __shared__ __align__(16) unsigned char sm[];
+__device__ __forceinline__ void sp_ctr_chain_body(const SpDev &d, int npass, uint4 *ctrs, unsigned char *sm) {
   ea_hq *hs = reinterpret_cast<ea_hq *>(sm);
   ea_xoshiro *xs = reinterpret_cast<ea_xoshiro *>(hs + d.NR);
   const int NR = d.NR;
@@ -72,6 +73,36 @@ __global__ void k_sp_ctr_chain(const __grid_constant__ SpDev d, int npass, uint4
   for (int i = threadIdx.x; i < nh; i += blockDim.x) hw[i] = h64[i];
   for (int i = threadIdx.x; i < nx; i += blockDim.x) xw[i] = x64[i];
   if (threadIdx.x == 0) *d.iter = iter0 + npass;
+}
+
+__global__ void k_sp_ctr_chain(const __grid_constant__ SpDev d, int npass, uint4 *ctrs) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  sp_ctr_chain_body(d, npass, ctrs, sm);
+}
+// A block per job of a batch, nsweep sweeps of its colours.
+__global__ void kb_sp_ctr_chain(const __grid_constant__ SpBatchDev b, int nsweep) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ SpDev d;
+  if (threadIdx.x == 0) d = b.jobs[blockIdx.x];
+  __syncthreads();
+  sp_ctr_chain_body(d, nsweep * d.ncol, d.ctrs, sm);
+}
+
+static size_t ctr_smem(int NR) { return (size_t)NR * (sizeof(ea_hq) + sizeof(ea_xoshiro)); }
+static int ctr_threads(int NR) { return NR <= 32 ? 32 : 64; }
+
+cudaError_t sp_launch_ctr_chain(const SpDev &d, int npass, uint4 *ctrs, cudaStream_t st) {
+  k_sp_ctr_chain<<<1, ctr_threads(d.NR), ctr_smem(d.NR), st>>>(d, npass, ctrs);
+  return cudaGetLastError();
+}
+
+cudaError_t sp_batch_ctr_setup() {
+  return cudaFuncSetAttribute(kb_sp_ctr_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctr_smem(64));
+}
+
+cudaError_t sp_batch_ctr_chain(const SpBatchDev &b, int nsweep, cudaStream_t st) {
+  kb_sp_ctr_chain<<<b.njobs, ctr_threads(b.nrep), ctr_smem(b.nrep), st>>>(b, nsweep);
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -729,14 +760,15 @@ size_t sp_res_launch_sweeps(size_t V, size_t G, const ea_cadence *cad) {
 
 cudaError_t sp_res_chunk(const SpResDev &p, const SpResPlan &pl, int npass, uint4 *ctrs, cudaStream_t st) {
   const SpDev &d = p.d;
-  k_sp_ctr_chain<<<1, d.NR <= 32 ? 32 : 64, (size_t)d.NR * (sizeof(ea_hq) + sizeof(ea_xoshiro)), st>>>(d, npass, ctrs);
+  cudaError_t e = sp_launch_ctr_chain(d, npass, ctrs, st);
+  if (e != cudaSuccess) return e;
   const int nsweep = npass / d.ncol;
   const long long n = (long long)nsweep * d.V * d.NR * d.NB;
   k_sp_draw<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, nsweep, ctrs, const_cast<u64 *>(p.R));
   const int npt = p.nit * p.mesfr * p.houfr;
   const long long nx = (long long)npt * d.nw * d.NR * (d.NB - 1) * 64;
   if (nx > 0) k_sp_pt_uniforms<<<(unsigned)((nx + 255) / 256), 256, 0, st>>>(d, npt, const_cast<u64 *>(p.X));
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute at;
   const cudaLaunchConfig_t cfg = res_config(pl.ncta, pl.smem, st, &at);
