@@ -121,6 +121,13 @@ int choose_kt(const Geometry &g) {
   return 0;
 }
 
+// CTAs that share a tile: as many as fit the GPU beside each other (2 an SM),
+// while each has an item for every lane group.
+int choose_split(const Geometry &g, int kt) {
+  const int tiles = (g.half + kt - 1) / kt, groups = 512 / (kt * g.NR), items = g.ns * g.NB;
+  return std::max(1, std::min(2 * 152 / tiles, (items + groups - 1) / groups));
+}
+
 int check(ea_ctx *c) {
   if (!c) return fail(EA_ERR_ARG, "null context");
   return EA_OK;
@@ -281,6 +288,7 @@ int ea_create(const ea_geom *gp, int32_t device, ea_ctx **out) {
   j.NB = g.NB; j.NR = g.NR; j.ns = g.ns; j.half = g.half; j.msc_l = g.msc_l; j.msc_s = g.msc_s;
   j.msc_lz = g.msc_lz; j.L = g.L; j.Lz = g.Lz; j.V = g.V; j.bc = g.bc; j.kt = kt;
   j.ntiles = (g.half + kt - 1) / kt;
+  j.nsplit = choose_split(g, kt);
   j.cc_xq = (int)(((1ULL << 32) - 1 + (uint64_t)g.L) % (uint64_t)g.L);
   set_dividers(j);
   const size_t nsr = (size_t)g.ns * g.NR;
@@ -294,12 +302,14 @@ int ea_create(const ea_geom *gp, int32_t device, ea_ctx **out) {
   OWN(j.wctb, nsr * g.NB);
   OWN(j.wbtc, nsr * g.NB);
   OWN(j.ctr, (size_t)g.NR);
+  OWN(j.ctrs, (size_t)kCtrPasses * g.NR);
   { uint32_t *p; OWN(p, (size_t)g.NR); j.keys = p; }
   OWN(j.prc, (size_t)g.NR);
   OWN(j.xo, (size_t)g.NR);
   OWN(j.iter, 1);
-  OWN(j.epart, (size_t)j.ntiles * nsr * g.NB);
   OWN(j.E, nsr * g.NB);
+  j.e_r = 1;
+  j.e_c = g.NR;
   OWN(j.pt, nsr);
   { double *p; OWN(p, (size_t)g.NB); j.betas = p; }
   { int32_t *p; OWN(p, (size_t)g.NB); j.expoff = p; }
@@ -617,18 +627,28 @@ static void prof_end(ea_ctx *c, int kind, cudaEvent_t b) {
   c->prof_ev[kind].push_back({b, e});
 }
 
-static int mc(ea_ctx *c, int n) {
+// Counters of the half-sweeps to come, drawn kCtrPasses at a time (they depend
+// on nothing else).
+struct CtrAhead {
+  long long left;  // half-sweeps whose counters are not drawn yet
+  int drawn = 0, next = 0;
+};
+
+// n sweeps, energies with the last one.
+static int mc(ea_ctx *c, int n, CtrAhead &a) {
   for (int sw = 0; sw < n; ++sw)
     for (int p = 0; p < 2; ++p) {
-      CU(launch_fill_bits(c->j, p, c->st));
+      if (a.next == a.drawn) {
+        a.drawn = (int)std::min<long long>(a.left, kCtrPasses);
+        a.left -= a.drawn;
+        a.next = 0;
+        CU(launch_ctr_chain(c->j, a.drawn, c->st));
+      }
       cudaEvent_t b = prof_begin(c);
-      CU(launch_sweep(c->j, p, sw == n - 1 && p == 1, c->st));
+      CU(launch_sweep(c->j, a.next++, p, sw < n - 1 ? kEnergyNone : p ? kEnergyAdd : kEnergyZero, c->st));
       prof_end(c, EA_K_SWEEP, b);
     }
-  if (n > 0) {
-    CU(launch_energy_reduce(c->j, c->st));
-    c->energies_fresh = true;
-  }
+  if (n > 0) c->energies_fresh = true;
   return EA_OK;
 }
 
@@ -636,13 +656,13 @@ int ea_monte_carlo(ea_ctx *c, int32_t nsweeps) {
   if (check(c) || nsweeps < 0) return fail(EA_ERR_ARG, "bad arguments");
   if (!c->have_temps) return fail(EA_ERR_STATE, "temperatures not set");
   if (set_device(c)) return EA_ERR_CUDA;
-  return mc(c, nsweeps);
+  CtrAhead a{2LL * nsweeps};
+  return mc(c, nsweeps, a);
 }
 
 static int measure(ea_ctx *c) {
   cudaEvent_t b = prof_begin(c);
   CU(launch_energy(c->j, c->st));
-  CU(launch_energy_reduce(c->j, c->st));
   prof_end(c, EA_K_ENERGY, b);
   c->energies_fresh = true;
   return EA_OK;
@@ -654,8 +674,13 @@ int ea_measure_energy(ea_ctx *c, int32_t *out) {
   int rc = measure(c);
   if (rc) return rc;
   if (out) {
-    CU(cudaMemcpyAsync(out, c->j.E, sizeof(int32_t) * c->g.ns * c->g.NR * c->g.NB, cudaMemcpyDeviceToHost, c->st));
+    const int NR = c->g.NR, NB = c->g.NB;
+    std::vector<int32_t> e((size_t)c->g.ns * NR * NB);  // [sample][clone][replica]
+    CU(cudaMemcpyAsync(e.data(), c->j.E, sizeof(int32_t) * e.size(), cudaMemcpyDeviceToHost, c->st));
     CU(cudaStreamSynchronize(c->st));
+    for (int s = 0; s < c->g.ns; ++s)
+      for (int k = 0; k < NB; ++k)
+        for (int r = 0; r < NR; ++r) out[((size_t)s * NR + r) * NB + k] = e[((size_t)s * NB + k) * NR + r];
   }
   return EA_OK;
 }
@@ -781,6 +806,9 @@ int ea_run_bin(ea_ctx *c, const ea_cadence *cad, double *avgE, uint8_t *hist, in
   if (!c->have_temps) return fail(EA_ERR_STATE, "temperatures not set");
   if (set_device(c)) return EA_ERR_CUDA;
   const Geometry &g = c->g;
+  int rc;
+  // everything a move needs, so that a refusal leaves the job as it is
+  if (cad->cluster && (rc = houdayer_prepare(c, cad->nclust, c->st))) return rc;
   int frec, maxit;
   trw(cad->itmax, &frec, &maxit);
   const size_t nsr = (size_t)g.ns * g.NR;
@@ -794,11 +822,11 @@ int ea_run_bin(ea_ctx *c, const ea_cadence *cad, double *avgE, uint8_t *hist, in
   c->j.maxit_trw = maxit;
   CU(cudaMemsetAsync(c->avgE, 0, nsr * g.NB * 8, c->st));
   CU(cudaMemsetAsync(c->hist, 0, nsr * maxit * g.NB, c->st));
-  int rc;
+  CtrAhead ahead{2LL * cad->itmax * cad->mesfr * cad->houfr * cad->ptfr};
   for (int it = 0; it < cad->itmax; ++it) {
     for (int im = 0; im < cad->mesfr; ++im) {
       for (int ih = 0; ih < cad->houfr; ++ih) {
-        if ((rc = mc(c, cad->ptfr))) return rc;
+        if ((rc = mc(c, cad->ptfr, ahead))) return rc;
         if (!c->energies_fresh && (rc = measure(c))) return rc;
         if ((rc = pt(c))) return rc;
       }
@@ -890,7 +918,7 @@ struct ea_batch {
   int up_slot = 0;
   BatchDev bd{};
   cudaGraphExec_t cycle = nullptr;
-  int cycle_ptfr = -1;
+  int cycle_ptfr = -1, cycle_n = -1;
   float tuned_ms = 0.f;  // autotuner: two sweeps of the chosen tile width
 };
 
@@ -904,14 +932,9 @@ static int set_tile(ea_ctx *c, int kt) {
   const size_t smem = sweep_smem_for(g.NB, g.NR, kt);
   if (smem > 227 * 1024) return fail(EA_ERR_ARG, "tile width %d needs %zu bytes of shared memory", kt, smem);
   const int nt = (g.half + kt - 1) / kt;
-  if (nt > j.ntiles) {
-    int32_t *p = nullptr;
-    int rc = own(c, p, (size_t)nt * g.ns * g.NR * g.NB);
-    if (rc) return rc;
-    j.epart = p;
-  }
   j.kt = kt;
   j.ntiles = nt;
+  j.nsplit = choose_split(g, kt);
   return EA_OK;
 }
 
@@ -943,6 +966,7 @@ static int batch_upload(ea_batch *b) {
   int slab_threads = 32, flip_smem = 0;
   for (int i = 0; i < n; ++i) {
     hj[i] = b->jobs[i]->j;
+    hj[i].nsplit = 1;  // a batch fills the GPU with the tiles of its jobs
     uint32_t cnt[KB_COUNT];
     batch_blocks(hj[i], cnt);
     for (int k = 0; k < KB_COUNT; ++k) hp[(size_t)k * (n + 1) + i + 1] = hp[(size_t)k * (n + 1) + i] + cnt[k];
@@ -996,7 +1020,7 @@ static int batch_upload(ea_batch *b) {
 // Autotuner: times the batched half-sweeps of every tile width that fits, on
 // the batch's own jobs, and keeps the fastest.  What the timing sweeps change
 // (spin words, half-sweep counter, Philox counters, the two generators that
-// feed them) is copied aside on the device first and put back after, so the
+// feed them, the energies) is copied aside on the device first and put back after, so the
 // jobs are left exactly as they were.
 static int batch_autotune(ea_batch *b, float *best_ms) {
   const int c8[3] = {4, 2, 1}, c4[3] = {8, 4, 2}, c2[3] = {16, 8, 4};
@@ -1017,6 +1041,7 @@ static int batch_autotune(ea_batch *b, float *best_ms) {
     parts.push_back({x->j.ctr, sizeof(uint4) * g.NR});
     parts.push_back({x->j.prc, sizeof(ea_hq) * g.NR});
     parts.push_back({x->j.xo, sizeof(ea_xoshiro) * g.NR});
+    parts.push_back({x->j.E, sizeof(int32_t) * g.ns * g.NR * g.NB});
   }
   for (const Part &q : parts) total += (q.n + 255) & ~(size_t)255;
   char *save = nullptr;
@@ -1040,11 +1065,9 @@ static int batch_autotune(ea_batch *b, float *best_ms) {
     float ms = 0.f;
     for (int rep = 0; rep < 2; ++rep) {  // the first pass warms up
       cudaEventRecord(e0, b->bs);
-      for (int cyc = 0; cyc < 2; ++cyc)
-        for (int p = 0; p < 2; ++p) {
-          batch_fill_bits(b->bd, p, b->bs);
-          batch_sweep(b->bd, b->NR, kt, b->NBmax, p, p == 1, true, b->bs);
-        }
+      batch_ctr_chain(b->bd, b->NR, 4, b->bs);
+      for (int p = 0; p < 4; ++p)
+        batch_sweep(b->bd, b->NR, kt, b->NBmax, p, p & 1, p & 1 ? kEnergyAdd : kEnergyZero, true, b->bs);
       cudaEventRecord(e1, b->bs);
       cudaEventSynchronize(e1);
       cudaEventElapsedTime(&ms, e0, e1);
@@ -1178,26 +1201,45 @@ int ea_batch_set_jobs(ea_batch *b, ea_ctx *const *jobs, int32_t njobs) {
   return batch_upload(b);
 }
 
-// One tempering cycle for every job: ptfr sweeps (energy fused into the last
-// odd half-sweep), or an energy pass when ptfr is 0, then the swaps.
-static int batch_cycle_launch(ea_batch *b, int ptfr) {
-  for (int sw = 0; sw < ptfr; ++sw)
-    for (int p = 0; p < 2; ++p) {
-      CU(batch_fill_bits(b->bd, p, b->bs));
-      CU(batch_sweep(b->bd, b->NR, b->KT, b->NBmax, p, sw == ptfr - 1 && p == 1, true, b->bs));
-    }
-  if (ptfr == 0) CU(batch_sweep(b->bd, b->NR, b->KT, b->NBmax, 0, true, false, b->bs));
-  CU(batch_energy_reduce(b->bd, b->bs));
-  CU(batch_pt(b->bd, b->bs));
+static int batch_energy(ea_batch *b) {
+  CU(batch_zero_energy(b->bd, b->bs));
+  CU(batch_sweep(b->bd, b->NR, b->KT, b->NBmax, 0, 0, kEnergyAdd, false, b->bs));
   return EA_OK;
 }
 
-static int batch_cycle(ea_batch *b, int ptfr) {
-  if (!b->cycle || b->cycle_ptfr != ptfr) {
+// `n` tempering cycles for every job: ptfr sweeps each (energy fused into the
+// last odd half-sweep), or an energy pass when ptfr is 0, then the swaps.
+static int batch_cycle_launch(ea_batch *b, int n, int ptfr) {
+  const long long all = 2LL * n * ptfr;
+  int drawn = 0, next = 0, rc;  // half-sweeps whose counters are drawn, used
+  long long done = 0;
+  for (int ih = 0; ih < n; ++ih) {
+    for (int sw = 0; sw < ptfr; ++sw)
+      for (int p = 0; p < 2; ++p) {
+        if (next == drawn) {
+          drawn = (int)std::min<long long>(all - done, kCtrPasses);
+          next = 0;
+          CU(batch_ctr_chain(b->bd, b->NR, drawn, b->bs));
+        }
+        CU(batch_sweep(b->bd, b->NR, b->KT, b->NBmax, next++, p, sw < ptfr - 1 ? kEnergyNone : p ? kEnergyAdd : kEnergyZero,
+                       true, b->bs));
+        ++done;
+      }
+    if (ptfr == 0 && (rc = batch_energy(b))) return rc;
+    CU(batch_pt(b->bd, b->bs));
+  }
+  return EA_OK;
+}
+
+// Cycles of one graph launch: long runs between moves go in pieces.
+constexpr int kGraphCycles = 32;
+
+static int batch_cycle(ea_batch *b, int n, int ptfr) {
+  if (!b->cycle || b->cycle_ptfr != ptfr || b->cycle_n != n) {
     if (b->cycle) { cudaGraphExecDestroy(b->cycle); b->cycle = nullptr; }
     cudaGraph_t graph = nullptr;
     CU(cudaStreamBeginCapture(b->bs, cudaStreamCaptureModeThreadLocal));
-    const int rc = batch_cycle_launch(b, ptfr);
+    const int rc = batch_cycle_launch(b, n, ptfr);
     const cudaError_t e = cudaStreamEndCapture(b->bs, &graph);
     if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
     CU(e);
@@ -1205,6 +1247,7 @@ static int batch_cycle(ea_batch *b, int ptfr) {
     cudaGraphDestroy(graph);
     CU(ei);
     b->cycle_ptfr = ptfr;
+    b->cycle_n = n;
   }
   CU(cudaGraphLaunch(b->cycle, b->bs));
   return EA_OK;
@@ -1272,15 +1315,13 @@ int ea_batch_run_bin(ea_batch *b, const ea_cadence *cad) {
   if (rc) return rc;
   for (int it = 0; it < cad->itmax; ++it) {
     for (int im = 0; im < cad->mesfr; ++im) {
-      for (int ih = 0; ih < cad->houfr; ++ih) {
-        // with ptfr = 0 the cycle measures the energies before the swaps
-        // (measuring energies that are still fresh leaves them unchanged)
-        if ((rc = batch_cycle(b, cad->ptfr))) return rc;
-      }
+      // with ptfr = 0 the cycle measures the energies before the swaps
+      // (measuring energies that are still fresh leaves them unchanged)
+      for (int ih = 0; ih < cad->houfr; ih += kGraphCycles)
+        if ((rc = batch_cycle(b, std::min(kGraphCycles, cad->houfr - ih), cad->ptfr))) return rc;
       if (cad->cluster && (rc = batch_houdayer(b, cad->nclust))) return rc;
     }
-    CU(batch_sweep(b->bd, b->NR, b->KT, b->NBmax, 0, true, false, b->bs));
-    CU(batch_energy_reduce(b->bd, b->bs));
+    if ((rc = batch_energy(b))) return rc;
     CU(batch_measure(b->bd, (it % frec == frec - 1) ? it / frec : -1, b->bs));
   }
   // later work of each job comes after the batch
@@ -1357,14 +1398,12 @@ int ea_job_bytes(const ea_geom *gp, const ea_cadence *cad, const double *betas, 
     tot += n >= (1ull << 20) ? (n + (2ull << 20) - 1) & ~((2ull << 20) - 1) : (n + 511) & ~(uint64_t)511;
   };
   const uint64_t nsr = (uint64_t)g.ns * g.NR, NB = g.NB, half = g.half, V = g.V;
-  const int ktmin = g.NR == 8 ? 1 : g.NR == 4 ? 2 : 4;
   add((uint64_t)g.ns * g.words_per_sample() * 8);            // spins
   add((uint64_t)g.ns * 12 * half * 8);                       // couplings
   add(12 * half * 4); add(2 * half);                         // neighbour table, flags
   add(NB * 256 * 8); add(NB * 256 * 2);                      // thresholds, pre-search
   add(nsr * NB); add(nsr * NB);                              // permutations
-  add(g.NR * 16); add(g.NR * 4); add(g.NR * sizeof(ea_hq)); add(g.NR * sizeof(ea_xoshiro)); add(8);
-  add(2 * ((half + ktmin - 1) / ktmin) * nsr * NB * 4);      // energy partials (two tile widths at most)
+  add(g.NR * 16); add(g.NR * 16 * kCtrPasses); add(g.NR * 4); add(g.NR * sizeof(ea_hq)); add(g.NR * sizeof(ea_xoshiro)); add(8);
   add(nsr * NB * 4); add(nsr * sizeof(ea_hq)); add(NB * 8); add(NB * 4);
   for (int k = 0; k < 3; ++k) add(nsr * (NB - 1) * 8);       // tempering statistics
   add(8); add(sizeof(ea_hq)); add(16); add(nsr * NB * 8);    // inexact, random_c, pairs, averages

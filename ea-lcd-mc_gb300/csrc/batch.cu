@@ -8,7 +8,7 @@ void batch_blocks(const JobDev &j, uint32_t out[KB_COUNT]) {
   const uint32_t nsrb = (uint32_t)(j.ns * j.NR * j.NB);
   const uint32_t nlat = (uint32_t)(j.ns * j.nclust);
   out[KB_SWEEP] = (uint32_t)j.ntiles;
-  out[KB_REDUCE] = (nsrb + 255) / 256;
+  out[KB_ZERO] = (nsrb + 255) / 256;
   out[KB_PT] = (uint32_t)(j.ns * ((j.NR + 7) / 8));
   out[KB_MEASURE] = (nsrb + 255) / 256;
   out[KB_START] = j.nclust > 0 ? 1 + (uint32_t)(j.xw_seg * (kXwStreams / 256)) : 0;
@@ -63,40 +63,44 @@ __device__ __forceinline__ uint32_t fetch_chunk(uint32_t *ctr, uint32_t nchunks,
     const uint32_t vend = min(total, (c + 1) * chunk);                                     \
     for (uint32_t v = c * chunk; v < vend; ++v)
 
-__global__ void kb_fill_bits(const __grid_constant__ BatchDev b, int parity) {
-  fill_bits_body(b.jobs[blockIdx.x], parity);
+__global__ void kb_ctr_chain(const __grid_constant__ BatchDev b, int npass) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const JobDev j = b.jobs[blockIdx.x];
+  ctr_chain_body(j.prc, j.xo, j.iter, j.jobid, j.NR, npass, j.ctrs, j.ctr, smem, [](int p, long long) { return p & 1; });
 }
 
 template <int NR, int KT, bool UPDATE>
-__global__ void __launch_bounds__(512, 2) kb_sweep(const __grid_constant__ BatchDev b, int parity, int energy) {
+__global__ void __launch_bounds__(512, 2) kb_sweep(const __grid_constant__ BatchDev b, int pass, int parity, int energy) {
   extern __shared__ __align__(16) unsigned char smem[];
   int staged = -1;  // job whose thresholds are in SMEM
   BATCH_LOOP(KB_SWEEP) {
     const int jb = item_job(pre, b.njobs, v);
     const JobDev jd = b.jobs[jb];  // a copy: no aliasing with the job's arrays
-    sweep_body<NR, KT, UPDATE>(jd, (int)(v - __ldg(pre + jb)), parity, energy, smem, jb != staged);
+    sweep_body<NR, KT, UPDATE>(jd, jd.ctrs + (size_t)pass * NR, (int)(v - __ldg(pre + jb)), parity, energy, smem,
+                               jb != staged);
     staged = jb;
     __syncthreads();
   }
   }
 }
 
-__global__ void kb_energy_reduce(const __grid_constant__ BatchDev b) {
-  BATCH_LOOP(KB_REDUCE) {
+__global__ void kb_zero_energy(const __grid_constant__ BatchDev b) {
+  BATCH_LOOP(KB_ZERO) {
     const int jb = item_job(pre, b.njobs, v);
-    energy_reduce_body(b.jobs[jb], (int)(v - __ldg(pre + jb)) * blockDim.x + threadIdx.x);
+    const JobDev &j = b.jobs[jb];
+    const int i = (int)(v - __ldg(pre + jb)) * blockDim.x + threadIdx.x;
+    if (i < j.ns * j.NB * j.NR) j.E[i] = 0;
   }
   }
 }
 
 __global__ void __launch_bounds__(256) kb_pt(const __grid_constant__ BatchDev b) {
-  __shared__ u64 s_ira[8][256];
-  __shared__ uint8_t s_wc[8][256];
+  __shared__ PtShared sh;
   BATCH_LOOP(KB_PT) {
     const int jb = item_job(pre, b.njobs, v);
     const JobDev j = b.jobs[jb];
     const int l = (int)(v - __ldg(pre + jb));
-    pt_body(j, l % j.ns, l / j.ns, s_ira, s_wc);
+    pt_body(j, l % j.ns, l / j.ns, sh);
     __syncthreads();
   }
   }
@@ -227,43 +231,43 @@ cudaError_t batch_setup(int NR, int KT) {
 
 int batch_sweep_smem(int NR, int KT, int NBmax) { return (int)sweep_smem_for(NBmax, NR, KT); }
 
-cudaError_t batch_fill_bits(const BatchDev &b, int parity, cudaStream_t st) {
-  kb_fill_bits<<<b.njobs, 64, 0, st>>>(b, parity);
+cudaError_t batch_ctr_chain(const BatchDev &b, int NR, int npass, cudaStream_t st) {
+  kb_ctr_chain<<<b.njobs, kCtrThreads, ctr_smem(NR), st>>>(b, npass);
   return cudaGetLastError();
 }
 
 template <int NR, int KT>
-static cudaError_t batch_sweep_t(const BatchDev &b, int NBmax, int parity, bool energy, bool update, cudaStream_t st) {
+static cudaError_t batch_sweep_t(const BatchDev &b, int NBmax, int pass, int parity, int energy, bool update, cudaStream_t st) {
   if (!b.total[KB_SWEEP]) return cudaSuccess;
   if (update) {
     const int sm = batch_sweep_smem(NR, KT, NBmax);
     const int per_sm = sm > 0 ? (int)((228 * 1024) / (sm + 1024)) : 4;
     kb_sweep<NR, KT, true><<<grid_for(chunks(b, KB_SWEEP), per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm)), 512, sm, st>>>(
-        b, parity, energy ? 1 : 0);
+        b, pass, parity, energy);
   } else {
-    kb_sweep<NR, KT, false><<<grid_for(chunks(b, KB_SWEEP), 4), 512, KT * 8 * 4, st>>>(b, parity, 1);
+    kb_sweep<NR, KT, false><<<grid_for(chunks(b, KB_SWEEP), 4), 512, KT * 8 * 4, st>>>(b, pass, parity, energy);
   }
   return cudaGetLastError();
 }
 
-cudaError_t batch_sweep(const BatchDev &b, int NR, int KT, int NBmax, int parity, bool energy, bool update,
+cudaError_t batch_sweep(const BatchDev &b, int NR, int KT, int NBmax, int pass, int parity, int energy, bool update,
                         cudaStream_t st) {
   switch (NR * 100 + KT) {
-    case 801: return batch_sweep_t<8, 1>(b, NBmax, parity, energy, update, st);
-    case 802: return batch_sweep_t<8, 2>(b, NBmax, parity, energy, update, st);
-    case 804: return batch_sweep_t<8, 4>(b, NBmax, parity, energy, update, st);
-    case 402: return batch_sweep_t<4, 2>(b, NBmax, parity, energy, update, st);
-    case 404: return batch_sweep_t<4, 4>(b, NBmax, parity, energy, update, st);
-    case 408: return batch_sweep_t<4, 8>(b, NBmax, parity, energy, update, st);
-    case 204: return batch_sweep_t<2, 4>(b, NBmax, parity, energy, update, st);
-    case 208: return batch_sweep_t<2, 8>(b, NBmax, parity, energy, update, st);
-    case 216: return batch_sweep_t<2, 16>(b, NBmax, parity, energy, update, st);
+    case 801: return batch_sweep_t<8, 1>(b, NBmax, pass, parity, energy, update, st);
+    case 802: return batch_sweep_t<8, 2>(b, NBmax, pass, parity, energy, update, st);
+    case 804: return batch_sweep_t<8, 4>(b, NBmax, pass, parity, energy, update, st);
+    case 402: return batch_sweep_t<4, 2>(b, NBmax, pass, parity, energy, update, st);
+    case 404: return batch_sweep_t<4, 4>(b, NBmax, pass, parity, energy, update, st);
+    case 408: return batch_sweep_t<4, 8>(b, NBmax, pass, parity, energy, update, st);
+    case 204: return batch_sweep_t<2, 4>(b, NBmax, pass, parity, energy, update, st);
+    case 208: return batch_sweep_t<2, 8>(b, NBmax, pass, parity, energy, update, st);
+    case 216: return batch_sweep_t<2, 16>(b, NBmax, pass, parity, energy, update, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
-cudaError_t batch_energy_reduce(const BatchDev &b, cudaStream_t st) {
-  if (b.total[KB_REDUCE]) kb_energy_reduce<<<grid_for(chunks(b, KB_REDUCE), 8), 256, 0, st>>>(b);
+cudaError_t batch_zero_energy(const BatchDev &b, cudaStream_t st) {
+  if (b.total[KB_ZERO]) kb_zero_energy<<<grid_for(chunks(b, KB_ZERO), 8), 256, 0, st>>>(b);
   return cudaGetLastError();
 }
 

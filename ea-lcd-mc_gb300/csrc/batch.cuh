@@ -9,7 +9,7 @@
 namespace eagb {
 
 // Work-list kinds: the blocks of one job for each one-job kernel.
-enum { KB_SWEEP = 0, KB_REDUCE, KB_PT, KB_MEASURE, KB_OVERLAP, KB_SLAB, KB_MERGE, KB_COMPRESS, KB_FLIP, KB_START, KB_COUNT };
+enum { KB_SWEEP = 0, KB_ZERO, KB_PT, KB_MEASURE, KB_OVERLAP, KB_SLAB, KB_MERGE, KB_COMPRESS, KB_FLIP, KB_START, KB_COUNT };
 
 constexpr int kBatchMaxJobs = 1024;
 
@@ -36,10 +36,10 @@ int batch_sweep_smem(int NR, int KT, int NBmax);
 // Kernel attributes and device figures the launchers use; called before any
 // launch (and so before a stream capture).
 cudaError_t batch_setup(int NR, int KT);
-cudaError_t batch_fill_bits(const BatchDev &b, int parity, cudaStream_t st);
-cudaError_t batch_sweep(const BatchDev &b, int NR, int KT, int NBmax, int parity, bool energy, bool update,
+cudaError_t batch_ctr_chain(const BatchDev &b, int NR, int npass, cudaStream_t st);
+cudaError_t batch_sweep(const BatchDev &b, int NR, int KT, int NBmax, int pass, int parity, int energy, bool update,
                         cudaStream_t st);
-cudaError_t batch_energy_reduce(const BatchDev &b, cudaStream_t st);
+cudaError_t batch_zero_energy(const BatchDev &b, cudaStream_t st);
 cudaError_t batch_pt(const BatchDev &b, cudaStream_t st);
 cudaError_t batch_measure(const BatchDev &b, int itm, cudaStream_t st);
 cudaError_t batch_move_start(const BatchDev &b, cudaStream_t st);

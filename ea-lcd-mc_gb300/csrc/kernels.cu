@@ -23,22 +23,20 @@ void set_dividers(JobDev &j) {
   j.fd_hl.set(j.msc_l / 2); j.fd_nclust.set(j.nclust > 0 ? j.nclust : 1);
 }
 
-__global__ void k_fill_bits(const __grid_constant__ JobDev j, int parity) { fill_bits_body(j, parity); }
-
-template <int NR, int KT, bool UPDATE>
-__global__ void __launch_bounds__(512, 2) k_sweep(const __grid_constant__ JobDev j, int parity, int energy) {
+__global__ void k_ctr_chain(const __grid_constant__ JobDev j, int npass) {
   extern __shared__ __align__(16) unsigned char smem[];
-  sweep_body<NR, KT, UPDATE>(j, blockIdx.x, parity, energy, smem);
+  ctr_chain_body(j.prc, j.xo, j.iter, j.jobid, j.NR, npass, j.ctrs, j.ctr, smem, [](int p, long long) { return p & 1; });
 }
 
-__global__ void k_energy_reduce(const __grid_constant__ JobDev j) {
-  energy_reduce_body(j, blockIdx.x * blockDim.x + threadIdx.x);
+template <int NR, int KT, bool UPDATE>
+__global__ void __launch_bounds__(512, 2) k_sweep(const __grid_constant__ JobDev j, int pass, int parity, int energy) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  sweep_body<NR, KT, UPDATE>(j, j.ctrs + (size_t)pass * NR, blockIdx.x, parity, energy, smem);
 }
 
 __global__ void __launch_bounds__(256) k_pt(const __grid_constant__ JobDev j) {
-  __shared__ u64 s_ira[8][256];
-  __shared__ uint8_t s_wc[8][256];
-  pt_body(j, blockIdx.x, blockIdx.y, s_ira, s_wc);
+  __shared__ PtShared sh;
+  pt_body(j, blockIdx.x, blockIdx.y, sh);
 }
 
 __global__ void k_measure(const __grid_constant__ JobDev j, int itm) {
@@ -170,7 +168,7 @@ int sweep_kt(const JobDev &j) { return j.kt; }
 size_t sweep_smem_bytes(const JobDev &j) { return sweep_smem_for(j.NB, j.NR, j.kt); }
 
 template <int NR, int KT>
-static cudaError_t launch_sweep_t(const JobDev &j, int parity, bool energy, bool update, cudaStream_t st) {
+static cudaError_t launch_sweep_t(const JobDev &j, int pass, int parity, int energy, bool update, cudaStream_t st) {
   if (update) {
     const size_t sm = sweep_smem_bytes(j);
     static bool attr = false;
@@ -178,45 +176,40 @@ static cudaError_t launch_sweep_t(const JobDev &j, int parity, bool energy, bool
       cudaFuncSetAttribute(k_sweep<NR, KT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
       attr = true;
     }
-    k_sweep<NR, KT, true><<<j.ntiles, 512, sm, st>>>(j, parity, energy ? 1 : 0);
+    k_sweep<NR, KT, true><<<j.ntiles * j.nsplit, 512, sm, st>>>(j, pass, parity, energy);
   } else {
-    k_sweep<NR, KT, false><<<j.ntiles, 512, (size_t)KT * 8 * 4, st>>>(j, parity, 1);
+    k_sweep<NR, KT, false><<<j.ntiles * j.nsplit, 512, (size_t)KT * 8 * 4, st>>>(j, pass, parity, energy);
   }
   return cudaGetLastError();
 }
 
-static cudaError_t dispatch_sweep(const JobDev &j, int parity, bool energy, bool update, cudaStream_t st) {
+static cudaError_t dispatch_sweep(const JobDev &j, int pass, int parity, int energy, bool update, cudaStream_t st) {
   switch (j.NR * 100 + j.kt) {
-    case 801: return launch_sweep_t<8, 1>(j, parity, energy, update, st);
-    case 802: return launch_sweep_t<8, 2>(j, parity, energy, update, st);
-    case 804: return launch_sweep_t<8, 4>(j, parity, energy, update, st);
-    case 402: return launch_sweep_t<4, 2>(j, parity, energy, update, st);
-    case 404: return launch_sweep_t<4, 4>(j, parity, energy, update, st);
-    case 408: return launch_sweep_t<4, 8>(j, parity, energy, update, st);
-    case 204: return launch_sweep_t<2, 4>(j, parity, energy, update, st);
-    case 208: return launch_sweep_t<2, 8>(j, parity, energy, update, st);
-    case 216: return launch_sweep_t<2, 16>(j, parity, energy, update, st);
+    case 801: return launch_sweep_t<8, 1>(j, pass, parity, energy, update, st);
+    case 802: return launch_sweep_t<8, 2>(j, pass, parity, energy, update, st);
+    case 804: return launch_sweep_t<8, 4>(j, pass, parity, energy, update, st);
+    case 402: return launch_sweep_t<4, 2>(j, pass, parity, energy, update, st);
+    case 404: return launch_sweep_t<4, 4>(j, pass, parity, energy, update, st);
+    case 408: return launch_sweep_t<4, 8>(j, pass, parity, energy, update, st);
+    case 204: return launch_sweep_t<2, 4>(j, pass, parity, energy, update, st);
+    case 208: return launch_sweep_t<2, 8>(j, pass, parity, energy, update, st);
+    case 216: return launch_sweep_t<2, 16>(j, pass, parity, energy, update, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
-cudaError_t launch_fill_bits(const JobDev &j, int parity, cudaStream_t st) {
-  k_fill_bits<<<1, 64, 0, st>>>(j, parity);
+cudaError_t launch_ctr_chain(const JobDev &j, int npass, cudaStream_t st) {
+  k_ctr_chain<<<1, kCtrThreads, ctr_smem(j.NR), st>>>(j, npass);
   return cudaGetLastError();
 }
 
-cudaError_t launch_sweep(const JobDev &j, int parity, bool energy, cudaStream_t st) {
-  return dispatch_sweep(j, parity, energy, true, st);
+cudaError_t launch_sweep(const JobDev &j, int pass, int parity, int energy, cudaStream_t st) {
+  return dispatch_sweep(j, pass, parity, energy, true, st);
 }
 
 cudaError_t launch_energy(const JobDev &j, cudaStream_t st) {
-  return dispatch_sweep(j, 0, true, false, st);
-}
-
-cudaError_t launch_energy_reduce(const JobDev &j, cudaStream_t st) {
-  const int n = j.ns * j.NB * j.NR;
-  k_energy_reduce<<<(n + 255) / 256, 256, 0, st>>>(j);
-  return cudaGetLastError();
+  const cudaError_t e = cudaMemsetAsync(j.E, 0, sizeof(int32_t) * (size_t)j.ns * j.NB * j.NR, st);
+  return e != cudaSuccess ? e : dispatch_sweep(j, 0, 0, kEnergyAdd, false, st);
 }
 
 cudaError_t launch_pt(const JobDev &j, cudaStream_t st) {

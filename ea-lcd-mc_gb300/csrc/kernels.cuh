@@ -39,15 +39,17 @@ struct JobDev {
   const unsigned long long *cum;    // [NB][256] thresholds
   const uint16_t *pre;              // [NB][256] 8-bit pre-search
   uint8_t *wctb, *wbtc;             // [s][rep][NB]
-  uint4 *ctr;                       // [NR] Philox counters of the current half-sweep
+  uint4 *ctr;                       // [NR] Philox counters of the last half-sweep
+  uint4 *ctrs;                      // [kCtrPasses][NR] those of the half-sweeps drawn ahead
   const uint32_t *keys;             // [NR]
   ea_hq *prc;                       // [NR]
   ea_xoshiro *xo;                   // [NR]
   long long *iter;                  // half-sweep counter (device scalar)
   uint32_t jobid;
-  int32_t *epart;                   // [ntiles][s][clone][rep] energy partial sums
   int ntiles, kt;
-  int32_t *E;                       // [s][rep][clone]
+  int nsplit;                       // CTAs that share a tile of the half-sweep
+  int32_t *E;                       // energies: s NR NB + rep e_r + clone e_c
+  int e_r, e_c;                     // (1, NR): a tile's sums of the replicas of a clone are neighbours
   // parallel tempering
   ea_hq *pt;                        // [s][rep]
   const double *betas;              // [NB]
@@ -82,6 +84,8 @@ struct JobDev {
   FastDiv fd_L, fd_S, fd_ml, fd_mlz, fd_hl, fd_nclust;
 };
 
+// Half-sweeps (colour passes) whose counters are drawn by one launch.
+constexpr int kCtrPasses = 512;
 constexpr int kSlabSites = 8192;        // sites of a slab held in SMEM
 constexpr int kSlabMaxPerThread = 16;   // sites a thread of the slab labelling owns
 
@@ -108,10 +112,13 @@ inline size_t sweep_smem_for(int NB, int NR, int KT) {
   return (size_t)3 * NB * KT * NR * 8 + (size_t)NB * 256 * 2 + (size_t)KT * 8 * 4;
 }
 
-cudaError_t launch_fill_bits(const JobDev &j, int parity, cudaStream_t st);
-cudaError_t launch_sweep(const JobDev &j, int parity, bool energy, cudaStream_t st);
+// Counters of npass half-sweeps (even, odd, even, ...) into j.ctrs.
+cudaError_t launch_ctr_chain(const JobDev &j, int npass, cudaStream_t st);
+// Half-sweep `pass` of the counters drawn last.  energy: kEnergyZero clears the
+// energies (before the odd half-sweep that adds them up), kEnergyAdd adds.
+enum { kEnergyNone = 0, kEnergyAdd = 1, kEnergyZero = 2 };
+cudaError_t launch_sweep(const JobDev &j, int pass, int parity, int energy, cudaStream_t st);
 cudaError_t launch_energy(const JobDev &j, cudaStream_t st);
-cudaError_t launch_energy_reduce(const JobDev &j, cudaStream_t st);
 cudaError_t launch_pt(const JobDev &j, cudaStream_t st);
 cudaError_t launch_measure(const JobDev &j, int itm, cudaStream_t st);
 cudaError_t launch_houdayer_group(const JobDev &j, int group, cudaStream_t st);

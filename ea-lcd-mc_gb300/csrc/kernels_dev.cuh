@@ -53,6 +53,42 @@ __device__ __forceinline__ uint4 next_counter(ea_xoshiro *x, ea_hq *h, long long
   return c;
 }
 
+// Counters of npass consecutive half-sweeps (colour passes), one thread per
+// replica with the states staged in SMEM: a launch of one step alone is a 4 us
+// link in a small job's chain of kernels, a step here takes half a
+// microsecond (a block of 256 threads: 32 took 30 us to stage 8 replicas).
+// parity(pass, time counter) is the counter's parity bit.
+// sm: NR x (sizeof(ea_hq) + sizeof(ea_xoshiro)) bytes.
+template <class Parity>
+__device__ __forceinline__ void ctr_chain_body(ea_hq *prc, ea_xoshiro *xo, long long *iter, uint32_t jobid, int NR,
+                                               int npass, uint4 *ctrs, uint4 *last, unsigned char *sm, Parity parity) {
+  ea_hq *hs = reinterpret_cast<ea_hq *>(sm);
+  ea_xoshiro *xs = reinterpret_cast<ea_xoshiro *>(hs + NR);
+  const int nh = NR * (int)(sizeof(ea_hq) / 8), nx = NR * (int)(sizeof(ea_xoshiro) / 8);
+  u64 *h64 = reinterpret_cast<u64 *>(hs), *x64 = reinterpret_cast<u64 *>(xs);
+  u64 *hg = reinterpret_cast<u64 *>(prc), *xg = reinterpret_cast<u64 *>(xo);
+#pragma unroll 8
+  for (int i = threadIdx.x; i < nh; i += blockDim.x) h64[i] = hg[i];
+  for (int i = threadIdx.x; i < nx; i += blockDim.x) x64[i] = xg[i];
+  const long long iter0 = *iter;
+  __syncthreads();
+  const int r = threadIdx.x;
+  if (r < NR) {
+    uint4 c = make_uint4(0u, 0u, 0u, 0u);
+    for (int p = 0; p < npass; ++p) {
+      c = next_counter(xs + r, hs + r, iter0 + p, parity(p, iter0 + p), jobid);
+      ctrs[(size_t)p * NR + r] = c;
+    }
+    if (npass > 0) last[r] = c;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nh; i += blockDim.x) hg[i] = h64[i];
+  for (int i = threadIdx.x; i < nx; i += blockDim.x) xg[i] = x64[i];
+  if (threadIdx.x == 0) *iter = iter0 + npass;
+}
+inline size_t ctr_smem(int NR) { return (size_t)NR * (sizeof(ea_hq) + sizeof(ea_xoshiro)); }
+constexpr int kCtrThreads = 256;
+
 __device__ __forceinline__ void fill_bits_body(const JobDev &j, int parity) {
   const int r = threadIdx.x;
   const long long iter = *j.iter;
@@ -195,14 +231,22 @@ __device__ __forceinline__ u64 flip_mask(const u64 f[6], u64 b0, u64 b1, u64 b2)
 // updates every (sample, clone, half-site, replica) word of its tile, picking
 // the words of the clone's current temperature.  The random word indices
 // depend only on (beta, half-site, replica, counter), never on the launch
-// shape.  With ENERGY it also adds up, per (sample, clone, replica), the
-// energy of the updated words (each bond has exactly one end on each parity).
+// shape.  A tile of a job too small to fill the GPU is shared by nsplit CTAs,
+// each drawing the words and updating its share of the (sample, clone) pairs
+// (`part` of nsplit), and its draws are spread over all the CTA's threads.
+// With energy = kEnergyAdd it also adds, per (sample, clone, replica),
+// the energy of the updated words (each bond has exactly one end on each
+// parity) to E, one atomic addition per tile (integers: the order does not
+// matter); kEnergyZero clears E, which the half-sweep before that one does.
+// Per-tile partial sums and a reduction kernel took 34 us a sweep on the large
+// tube and a link of 3 to 10 us in a small job's chain.
 // ---------------------------------------------------------------------------
 template <int NR, int KT, bool UPDATE>
 // stage = false: the thresholds of this job are already in SMEM (the block's
 // previous tile was of the same job).
-__device__ __forceinline__ void sweep_body(const JobDev &j, int tile, int parity, int energy, unsigned char *smem,
-                                           bool stage = true) {
+__device__ __forceinline__ void sweep_body(const JobDev &j, const uint4 *ctr, int blk, int parity, int energy,
+                                           unsigned char *smem, bool stage = true) {
+  const int tile = blk / j.nsplit, part = blk - tile * j.nsplit;
   const int NB = j.NB, half = j.half;
   u64 *s_rnd = reinterpret_cast<u64 *>(smem);
   uint16_t *s_pre = reinterpret_cast<uint16_t *>(s_rnd + (UPDATE ? 3 * NB * KT * NR : 0));
@@ -210,6 +254,8 @@ __device__ __forceinline__ void sweep_body(const JobDev &j, int tile, int parity
   const int k0 = tile * KT;
   const int tid = threadIdx.x, nth = blockDim.x;
 
+  if (energy == kEnergyZero)
+    for (int i = blk * nth + tid; i < j.ns * NB * NR; i += j.ntiles * j.nsplit * nth) j.E[i] = 0;
   if (UPDATE && stage) {
     const uint4 *ps = reinterpret_cast<const uint4 *>(j.pre);
     uint4 *pd = reinterpret_cast<uint4 *>(s_pre);
@@ -224,22 +270,33 @@ __device__ __forceinline__ void sweep_body(const JobDev &j, int tile, int parity
   __syncthreads();
 
   if (UPDATE) {
-    const int ntrip = NB * KT * NR;
-    for (int t = tid; t < ntrip; t += nth) {
+    const int ntrip = NB * KT * NR, plane = ntrip;
+    // words 2 q0 .. 2 q1 - 1 of triple t
+    auto draw = [&](int t, int q0, int q1) {
       const int r = t % NR, kk = (t / NR) % KT, b = t / (NR * KT), k = k0 + kk;
-      if (k >= half) continue;
+      if (k >= half) return;
       const uint32_t tp = (uint32_t)((b * half + k) * NR + r);
-      const uint4 c = j.ctr[r];
+      const uint4 c = ctr[r];
       const uint32_t key = j.keys[r];
       const u64 *cum = j.cum + b * 256;
       const uint16_t *pre = s_pre + b * 256;
-      uint32_t w[6];
+      const int o = (b * KT + kk) * NR + r;
 #pragma unroll
-      for (int q = 0; q < 6; ++q) w[q] = rnd_word<true>(c.x + q, c.y, c.z + tp, c.w, key, tp, cum, pre);
-      const int o = (b * KT + kk) * NR + r, plane = NB * KT * NR;
-      s_rnd[o] = ((u64)w[0] << 32) | w[1];
-      s_rnd[plane + o] = ((u64)w[2] << 32) | w[3];
-      s_rnd[2 * plane + o] = ((u64)w[4] << 32) | w[5];
+      for (int q = 0; q < 3; ++q) {
+        if (q < q0 || q >= q1) continue;
+        const uint32_t hi = rnd_word<true>(c.x + 2 * q, c.y, c.z + tp, c.w, key, tp, cum, pre);
+        const uint32_t lo = rnd_word<true>(c.x + 2 * q + 1, c.y, c.z + tp, c.w, key, tp, cum, pre);
+        s_rnd[q * plane + o] = ((u64)hi << 32) | lo;
+      }
+    };
+    if (ntrip * 2 <= nth) {
+      // fewer triples than half the threads: a thread draws one 64-bit word
+      for (int t = tid; t < ntrip * 3; t += nth) {
+        const int q = t / ntrip;
+        draw(t - q * ntrip, q, q + 1);
+      }
+    } else {
+      for (int t = tid; t < ntrip; t += nth) draw(t, 0, 3);
     }
     __syncthreads();
   }
@@ -260,8 +317,9 @@ __device__ __forceinline__ void sweep_body(const JobDev &j, int tile, int parity
 #pragma unroll
   for (int d = 0; d < 6; ++d) nb[d] = s_nb[kk * 8 + d];
   const int nflags = s_nb[kk * 8 + 6];
-  const int nsc = j.ns * NB, iters = (nsc + ngrp - 1) / ngrp;
-  const int sc0 = grp * iters;
+  const int all = j.ns * NB, share = (all + j.nsplit - 1) / j.nsplit;
+  const int nsc = min(all, (part + 1) * share), iters = (share + ngrp - 1) / ngrp;
+  const int sc0 = part * share + grp * iters;
   int s = sc0 / NB, c = sc0 - s * NB, js = -1;
   u64 jw[6];
   for (int it = 0, sc = sc0; it < iters; ++it, ++sc) {
@@ -290,94 +348,162 @@ __device__ __forceinline__ void sweep_body(const JobDev &j, int tile, int parity
         fl = flip_mask(f, s_rnd[o], s_rnd[plane + o], s_rnd[2 * plane + o]);
         *tgt = sv ^ fl;
       }
-      if (energy) {
+      if (energy == kEnergyAdd) {
         int le = 0;
 #pragma unroll
         for (int d = 0; d < 6; ++d) le += __popcll(f[d] ^ fl);
         e = 6 * 64 - 2 * le;
       }
     }
-    if (energy) {
+    if (energy == kEnergyAdd) {
 #pragma unroll
       for (int m = NR; m < G; m <<= 1) e += __shfl_xor_sync(0xffffffffu, e, m);
-      if (valid && kk == 0) j.epart[(((size_t)tile * j.ns + s) * NB + c) * NR + r] = e;
+      if (valid && kk == 0) atomicAdd(j.E + (size_t)s * NR * NB + r * j.e_r + c * j.e_c, e);
     }
     if (++c == NB) { c = 0; ++s; }
   }
 }
 
-// E[s][rep][clone] = sum over tiles (thread per (s, clone, rep)).
-__device__ __forceinline__ void energy_reduce_body(const JobDev &j, int i) {
-  const int n = j.ns * j.NB * j.NR;
-  if (i >= n) return;
-  int e = 0;
-  for (int t = 0; t < j.ntiles; ++t) e += j.epart[(size_t)t * n + i];
-  const int r = i % j.NR, c = (i / j.NR) % j.NB, s = i / (j.NR * j.NB);
-  j.E[((size_t)s * j.NR + r) * j.NB + c] = e;
-}
+// ---------------------------------------------------------------------------
+// Parallel tempering (upd.c:3-48), one warp per (sample, replica) chain.
+//
+// The decisions are a serial chain over the pairs; all else is done by the
+// warp's lanes side by side.  The chain's draws do not depend on the
+// decisions: the Parisi-Rapuano generator adds words at least 24 places back,
+// so 24 draws at a time are made by 24 lanes (the LCG part jumps by its powers,
+// composed over the lanes).  Energies and draws wait in SMEM; the walk takes
+// each decision by a single-precision exp(pt) when the draw is not within
+// 1e-4 of it (its error is below 2e-5, see sp_pt_body) and by the host-libm
+// table otherwise, so it is exact.  The acceptance sums, which take the
+// table's value or exp(pt) of every pair, follow in parallel, one addition
+// per pair and step in FP64 as on the host.  One lane walking everything took
+// 34 us at 32 temperatures and 41 us at 40; this takes 12 and 14.
+// ---------------------------------------------------------------------------
+struct PtWarp {
+  u64 ira[256];
+  u64 x[256];       // FNORM * draw, as bits
+  int es[256];      // energies in beta order, then each pair's dE
+  uint8_t wc[256];
+};
+struct PtShared {
+  PtWarp w[8];
+  float db[256];    // b[i] - b[i+1]
+  int eo[256];      // exp table offsets
+};
 
-// ---------------------------------------------------------------------------
-// Parallel tempering (upd.c:3-48), one warp per (sample, replica) chain: the
-// warp stages the PT generator's lag table in SMEM, lane 0 walks the NB-1
-// pairs in order with FP64 arithmetic rounded as on the host, and exp(pt) comes
-// from the host's libm through the table built at set-up.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void pt_body(const JobDev &j, int s, int ry, u64 (*s_ira)[256], uint8_t (*s_wc)[256]) {
+__device__ __forceinline__ void pt_body(const JobDev &j, int s, int ry, PtShared &sh) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = ry * 8 + w;
+  const int r = ry * 8 + w, NB = j.NB, NP = NB - 1;
+  for (int i = threadIdx.x; i < NB; i += blockDim.x) {
+    sh.eo[i] = j.expoff[i];
+    // betas descend; a difference too small for single precision stays positive
+    const double f = i < NP ? -__dsub_rn(j.betas[i + 1], j.betas[i]) : 0.0;
+    sh.db[i] = f > 0.0 ? fmaxf((float)f, 1e-30f) : (float)f;
+  }
+  __syncthreads();
   if (r >= j.NR) return;
-  const int NB = j.NB;
+  PtWarp &q = sh.w[w];
   const size_t o = (size_t)s * j.NR + r;
   ea_hq *h = j.pt + o;
-  for (int i = lane; i < 256; i += 32) s_ira[w][i] = h->ira[i];
-  for (int i = lane; i < NB; i += 32) s_wc[w][i] = j.wctb[o * NB + i];
+  const int32_t *E = j.E + (size_t)s * j.NR * NB + (size_t)r * j.e_r;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q.ira[i * 32 + lane] = h->ira[i * 32 + lane];
+  for (int i = lane; i < NB; i += 32) {
+    const uint8_t c = j.wctb[o * NB + i];
+    q.wc[i] = c;
+    q.es[i] = E[c * j.e_c];
+  }
+  const uint8_t ip = h->ip, ip1 = h->ip1, ip2 = h->ip2, ip3 = h->ip3;
+  u64 zseed = h->zseed, PR = h->PR, fin = h->final;
+  // draws a batch can make at once: no word of it may be read by a later one
+  auto lag = [](uint8_t d) { return d ? (int)d : 256; };
+  const int most = min(min(32, lag((uint8_t)(ip - ip1))), min(lag((uint8_t)(ip - ip2)), lag((uint8_t)(ip - ip3))));
+  // lane k: k + 1 steps of z -> a z + 1
+  u64 A = 3202034522624059733ULL, C = 1;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const u64 pa = __shfl_up_sync(0xffffffffu, A, d), pc = __shfl_up_sync(0xffffffffu, C, d);
+    if (lane >= d) { C += A * pc; A *= pa; }
+  }
+  const double FNORM = 5.4210108624275218e-20;
   __syncwarp();
-  if (lane == 0) {
-    u64 *ira = s_ira[w];
-    uint8_t *wc = s_wc[w];
-    uint8_t ip = h->ip, ip1 = h->ip1, ip2 = h->ip2, ip3 = h->ip3;
-    u64 zseed = h->zseed, PR = h->PR, fin = h->final;
-    const int32_t *E = j.E + o * NB;
-    double *acc = j.acc + o * (NB - 1), *att = j.att + o * (NB - 1), *accraw = j.accraw + o * (NB - 1);
-    const double FNORM = 5.4210108624275218e-20;
-    for (int i = 0; i < NB - 1; ++i) {
-      att[i] += 1.0;
-      const int dE = E[wc[i + 1]] - E[wc[i]];
-      const double pt = __dmul_rn(-__dsub_rn(j.betas[i + 1], j.betas[i]), (double)dE);
-      const u64 a = ira[ip1] + ira[ip2];
-      ira[ip] = a;
-      PR = a ^ ira[ip3];
-      zseed = zseed * 3202034522624059733ULL + 1;
-      fin = zseed + PR;
-      ++ip; ++ip1; ++ip2; ++ip3;
-      bool change;
-      if (pt >= 0.0) {
-        acc[i] += 1.0;
-        change = true;
+  for (int i0 = 0; i0 < NP; i0 += most) {
+    const int n = min(most, NP - i0);
+    const bool on = lane < n;
+    const u64 a = on ? q.ira[(uint8_t)(ip1 + i0 + lane)] + q.ira[(uint8_t)(ip2 + i0 + lane)] : 0;
+    __syncwarp();
+    if (on) q.ira[(uint8_t)(ip + i0 + lane)] = a;
+    __syncwarp();
+    u64 z = 0, p = 0;
+    if (on) {
+      p = a ^ q.ira[(uint8_t)(ip3 + i0 + lane)];
+      z = A * zseed + C;
+      q.x[i0 + lane] = (u64)__double_as_longlong(__dmul_rn(FNORM, __ull2double_rn(z + p)));
+    }
+    zseed = __shfl_sync(0xffffffffu, z, n - 1);
+    PR = __shfl_sync(0xffffffffu, p, n - 1);
+    fin = zseed + PR;
+    __syncwarp();
+  }
+  // the walk, every lane alike (slot i + 1 still holds its own clone when pair
+  // i is decided, slot i the one carried up from below)
+  const u64 *tab = reinterpret_cast<const u64 *>(j.exptab);
+  uint32_t chg = 0;  // pairs i = lane mod 32 that changed, bit i / 32
+  int ce = q.es[0];
+  uint8_t cc = q.wc[0];
+#pragma unroll 2
+  for (int i = 0; i < NP; ++i) {
+    const int e1 = q.es[i + 1];
+    const uint8_t c1 = q.wc[i + 1];
+    const u64 x = q.x[i];
+    const int base = sh.eo[i], nx = sh.eo[i + 1] - base;
+    const int dE = e1 - ce, m = (-dE) >> 1;
+    const float pt = sh.db[i] * (float)dE, ex = __expf(pt), xf = (float)__longlong_as_double((long long)x);
+    bool change = pt >= 0.f;
+    if (!change) {
+      change = xf < ex;
+      if ((dE & 1) || m < 1 || m > nx)  // outside the table: exp(pt) < 2^-72 (or an odd dE, never seen)
+        change = __longlong_as_double((long long)x) <
+                 exp(__dmul_rn(-__dsub_rn(j.betas[i + 1], j.betas[i]), (double)dE));
+      else if (fabsf(xf - ex) <= 1e-4f * ex)
+        change = x < __ldg(tab + base + m - 1);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      q.es[i] = dE;
+      q.wc[i] = change ? c1 : cc;
+    }
+    if ((i & 31) == lane && change) chg |= 1u << (i >> 5);
+    ce = change ? ce : e1;
+    cc = change ? cc : c1;
+  }
+  if (lane == 0) q.wc[NP] = cc;
+  __syncwarp();
+  double *acc = j.acc + o * NP, *att = j.att + o * NP, *accraw = j.accraw + o * NP;
+  for (int i = lane; i < NP; i += 32) {
+    att[i] += 1.0;
+    const int dE = q.es[i];
+    const double pt = __dmul_rn(-__dsub_rn(j.betas[i + 1], j.betas[i]), (double)dE);
+    double a = 1.0;
+    if (!(pt >= 0.0)) {
+      const int base = sh.eo[i], n = sh.eo[i + 1] - base, m = (-dE) >> 1;
+      if (!(dE & 1) && m >= 1 && m <= n) {
+        a = j.exptab[base + m - 1];
       } else {
-        const int base = j.expoff[i], n = j.expoff[i + 1] - base, m = (-dE) >> 1;
-        double ex;
-        if (!(dE & 1) && m >= 1 && m <= n) {
-          ex = j.exptab[base + m - 1];
-        } else {
-          ex = exp(pt);  // exp(pt) < 2^-72 here: decides only when the draw is 0
-          if (fin == 0 || (dE & 1)) atomicAdd(j.inexact, 1ULL);
-        }
-        acc[i] += ex;
-        change = __dmul_rn(FNORM, __ull2double_rn(fin)) < ex;
-      }
-      if (change) {
-        const uint8_t t = wc[i]; wc[i] = wc[i + 1]; wc[i + 1] = t;
-        accraw[i] += 1.0;
+        a = exp(pt);
+        if (q.x[i] == 0 || (dE & 1)) atomicAdd(j.inexact, 1ULL);  // decided by a draw of 0
       }
     }
-    h->ip = ip; h->ip1 = ip1; h->ip2 = ip2; h->ip3 = ip3;
+    acc[i] += a;
+    if ((chg >> (i >> 5)) & 1u) accraw[i] += 1.0;
+    h->ira[(uint8_t)(ip + i)] = q.ira[(uint8_t)(ip + i)];
+  }
+  if (lane == 0) {
+    h->ip = (uint8_t)(ip + NP); h->ip1 = (uint8_t)(ip1 + NP); h->ip2 = (uint8_t)(ip2 + NP); h->ip3 = (uint8_t)(ip3 + NP);
     h->zseed = zseed; h->PR = PR; h->final = fin;
   }
-  __syncwarp();
-  for (int i = lane; i < 256; i += 32) h->ira[i] = s_ira[w][i];
   for (int i = lane; i < NB; i += 32) {
-    const uint8_t c = s_wc[w][i];
+    const uint8_t c = q.wc[i];
     j.wctb[o * NB + i] = c;
     j.wbtc[o * NB + c] = (uint8_t)i;
   }
@@ -388,8 +514,8 @@ __device__ __forceinline__ void measure_body(const JobDev &j, int i, int itm) {
   const int n = j.ns * j.NR * j.NB;
   if (i >= n) return;
   const size_t o = i / j.NB;
-  const int b = i % j.NB;
-  j.avgE[i] += (double)j.E[o * j.NB + j.wctb[o * j.NB + b]];
+  const int b = i % j.NB, s = (int)o / j.NR, r = (int)o - s * j.NR;
+  j.avgE[i] += (double)j.E[(size_t)s * j.NR * j.NB + r * j.e_r + j.wctb[o * j.NB + b] * j.e_c];
   if (itm >= 0) j.hist[(o * j.maxit_trw + itm) * j.NB + b] = j.wbtc[o * j.NB + b];
 }
 

@@ -7,8 +7,8 @@
 // an allocation may imply.  ea_measure_energy_noalloc serves them: it
 // computes the same energies as ea_measure_energy for spins and couplings that
 // the caller already keeps in device memory, and writes them to a caller
-// buffer.  Its scratch space -- the per-tile partial sums of the energy kernel
-// and the neighbour tables of the geometry -- is the file-scope array below,
+// buffer.  Its scratch space -- the neighbour tables of the geometry; the
+// energies are added up in the caller's buffer -- is the file-scope array below,
 // which every GPU that loads libeagb.so holds until the process exits.
 #include <cuda.h>
 
@@ -23,14 +23,14 @@
 namespace eagb {
 namespace {
 
-// Scratch limits: at most kMaxPartials per-tile energy sums and kMaxHalf
-// half-sites per parity (e.g. L = 32, Lz = 256).
-constexpr size_t kMaxPartials = (size_t)1 << 20;  // 4 MiB of int32
+// Limits: at most kMaxHalf half-sites per parity (e.g. L = 32, Lz = 256: the
+// scratch tables) and kMaxPartials tile energies (the entry point's bound on the
+// job, from when they were kept).
+constexpr size_t kMaxPartials = (size_t)1 << 20;
 constexpr int kMaxHalf = 8192;
-constexpr size_t kPartBytes = kMaxPartials * 4;
 constexpr size_t kIdxBytes = (size_t)12 * kMaxHalf * 4;
 constexpr size_t kFlagBytes = (size_t)2 * kMaxHalf;
-constexpr size_t kScratchBytes = kPartBytes + kIdxBytes + kFlagBytes;  // 4.4 MiB
+constexpr size_t kScratchBytes = kIdxBytes + kFlagBytes;  // 400 KiB
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
@@ -64,8 +64,8 @@ CUcontext current_context() {
 // scratch tables (same tables as the context builds on the host: wrap-around
 // rotation bits 0-5, top plane bit 6, bottom plane bit 7).
 __global__ void k_noalloc_tables(int msc_l, int msc_lz, int half) {
-  int32_t *idx = reinterpret_cast<int32_t *>(g_scratch + kPartBytes);
-  uint8_t *flags = g_scratch + kPartBytes + kIdxBytes;
+  int32_t *idx = reinterpret_cast<int32_t *>(g_scratch);
+  uint8_t *flags = g_scratch + kIdxBytes;
   const int msc_s = msc_l * msc_l, msc_v = msc_s * msc_lz;
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= msc_v) return;
@@ -148,21 +148,21 @@ extern "C" int ea_measure_energy_noalloc(const ea_geom *gp, const uint64_t *d_sp
   JobDev j{};
   j.NB = g.NB; j.NR = g.NR; j.ns = g.ns; j.half = g.half; j.msc_l = g.msc_l; j.msc_s = g.msc_s;
   j.msc_lz = g.msc_lz; j.L = g.L; j.Lz = g.Lz; j.V = g.V; j.bc = g.bc;
-  j.kt = kt; j.ntiles = ntiles;
+  j.kt = kt; j.ntiles = ntiles; j.nsplit = 1;
   set_dividers(j);
   j.spins = const_cast<unsigned long long *>(reinterpret_cast<const unsigned long long *>(d_spins));
   j.J = reinterpret_cast<const unsigned long long *>(d_couplings);
-  j.epart = reinterpret_cast<int32_t *>(base);
-  j.nbidx = reinterpret_cast<const int32_t *>(base + kPartBytes);
-  j.nbflag = base + kPartBytes + kIdxBytes;
-  j.E = d_energies;
+  j.nbidx = reinterpret_cast<const int32_t *>(base);
+  j.nbflag = base + kIdxBytes;
+  j.E = d_energies;  // [sample][replica][clone]
+  j.e_r = g.NB;
+  j.e_c = 1;
   // each launch checked right after it is made
   const char *failed = nullptr;
   cudaError_t e;
   k_noalloc_tables<<<(g.msc_v + 255) / 256, 256, 0, st>>>(g.msc_l, g.msc_lz, g.half);
   if ((e = cudaGetLastError()) != cudaSuccess) failed = "neighbour tables";
-  else if ((e = launch_energy(j, st)) != cudaSuccess) failed = "energy partial sums";
-  else if ((e = launch_energy_reduce(j, st)) != cudaSuccess) failed = "energy reduction";
+  else if ((e = launch_energy(j, st)) != cudaSuccess) failed = "energy";
   if (failed) {
     char msg[256];
     std::snprintf(msg, sizeof(msg), "ea_measure_energy_noalloc: launch of the %s kernel failed: %s", failed,

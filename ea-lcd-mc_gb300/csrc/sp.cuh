@@ -36,9 +36,6 @@ bool sp_graph(int L, int Lz, int bc, SpGraph &g);
 void sp_couplings(const SpGraph &g, int nwords, uint64_t seed_J, uint64_t *J);
 void sp_spins(const SpGraph &g, int nwords, int NR, int NB, uint64_t seed_u, uint64_t *S);
 
-// Colour passes whose counters are drawn by one launch.
-constexpr int kCtrPasses = 512;
-
 // Launch shape of the energy count (k_sp_energy).
 struct EnShape {
   int lanes;    // columns of a block, one lane each

@@ -42,37 +42,13 @@ constexpr int kResPlanes = 15;
 constexpr int kResMaxSites = ((1 << kResPlanes) - 1) / 6;
 
 // ---------------------------------------------------------------------------
-// Counters of npass consecutive colour passes (fill_bits_body's step,
-// repeated): pass p uses time counter iter0 + p and its parity.  Every path
-// but the persistent kernel's draws its passes' counters this way: a launch of
-// the step alone is a 4 us link in a small job's chain, 0.5 us here.
+// Counters of npass consecutive colour passes (ctr_chain_body): pass p uses
+// time counter iter0 + p and its parity.  Every path but the persistent
+// kernel's draws its passes' counters this way.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void sp_ctr_chain_body(const SpDev &d, int npass, uint4 *ctrs, unsigned char *sm) {
-  ea_hq *hs = reinterpret_cast<ea_hq *>(sm);
-  ea_xoshiro *xs = reinterpret_cast<ea_xoshiro *>(hs + d.NR);
-  const int NR = d.NR;
-  const int nh = NR * (int)(sizeof(ea_hq) / 8), nx = NR * (int)(sizeof(ea_xoshiro) / 8);
-  u64 *h64 = reinterpret_cast<u64 *>(hs), *x64 = reinterpret_cast<u64 *>(xs);
-  const u64 *hg = reinterpret_cast<const u64 *>(d.prc), *xg = reinterpret_cast<const u64 *>(d.xo);
-  for (int i = threadIdx.x; i < nh; i += blockDim.x) h64[i] = hg[i];
-  for (int i = threadIdx.x; i < nx; i += blockDim.x) x64[i] = xg[i];
-  const long long iter0 = *d.iter;
-  __syncthreads();
-  const int r = threadIdx.x;
-  if (r < NR) {
-    uint4 c = make_uint4(0u, 0u, 0u, 0u);
-    for (int p = 0; p < npass; ++p) {
-      const long long it = iter0 + p;
-      c = next_counter(xs + r, hs + r, it, (int)(it & 1), d.jobid);
-      ctrs[(size_t)p * NR + r] = c;
-    }
-    if (npass > 0) d.ctr[r] = c;
-  }
-  __syncthreads();
-  u64 *hw = reinterpret_cast<u64 *>(d.prc), *xw = reinterpret_cast<u64 *>(d.xo);
-  for (int i = threadIdx.x; i < nh; i += blockDim.x) hw[i] = h64[i];
-  for (int i = threadIdx.x; i < nx; i += blockDim.x) xw[i] = x64[i];
-  if (threadIdx.x == 0) *d.iter = iter0 + npass;
+  ctr_chain_body(d.prc, d.xo, d.iter, d.jobid, d.NR, npass, ctrs, d.ctr, sm,
+                 [](int, long long it) { return (int)(it & 1); });
 }
 
 __global__ void k_sp_ctr_chain(const __grid_constant__ SpDev d, int npass, uint4 *ctrs) {
@@ -88,11 +64,8 @@ __global__ void kb_sp_ctr_chain(const __grid_constant__ SpBatchDev b, int nsweep
   sp_ctr_chain_body(d, nsweep * d.ncol, d.ctrs, sm);
 }
 
-static size_t ctr_smem(int NR) { return (size_t)NR * (sizeof(ea_hq) + sizeof(ea_xoshiro)); }
-static int ctr_threads(int NR) { return NR <= 32 ? 32 : 64; }
-
 cudaError_t sp_launch_ctr_chain(const SpDev &d, int npass, uint4 *ctrs, cudaStream_t st) {
-  k_sp_ctr_chain<<<1, ctr_threads(d.NR), ctr_smem(d.NR), st>>>(d, npass, ctrs);
+  k_sp_ctr_chain<<<1, kCtrThreads, ctr_smem(d.NR), st>>>(d, npass, ctrs);
   return cudaGetLastError();
 }
 
@@ -101,7 +74,7 @@ cudaError_t sp_batch_ctr_setup() {
 }
 
 cudaError_t sp_batch_ctr_chain(const SpBatchDev &b, int nsweep, cudaStream_t st) {
-  kb_sp_ctr_chain<<<b.njobs, ctr_threads(b.nrep), ctr_smem(b.nrep), st>>>(b, nsweep);
+  kb_sp_ctr_chain<<<b.njobs, kCtrThreads, ctr_smem(b.nrep), st>>>(b, nsweep);
   return cudaGetLastError();
 }
 

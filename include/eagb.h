@@ -181,16 +181,17 @@ int ea_measure_energy(ea_ctx *ctx, int32_t *out);
  * d_energies on `stream` (a cudaStream_t, NULL = legacy default stream), on
  * the calling thread's current device.  NR must be 2, 4 or 8 (the tile
  * widths KT = 16, 8, 4 of the energy kernel); other replica counts get
- * EA_ERR_ARG.  Its scratch is a fixed 4.4 MiB device array inside the
+ * EA_ERR_ARG.  Its scratch is a fixed 400 KiB device array inside the
  * library (held by every GPU that loads it until exit), so it rejects, with
  * EA_ERR_ARG and a message, jobs beyond
  * (L/4)^2 (Lz/4) / 2 <= 8192 half-sites and
- * ceil(half/KT) * nsamples * NB * NR <= 2^20 partial sums (KT = 32/NR).
+ * ceil(half/KT) * nsamples * NB * NR <= 2^20 tile sums (KT = 32/NR).
  * The first call on each device (and the first after that device's context
  * is recreated, e.g. by cudaDeviceReset) looks up the array's device address;
  * make that first call before any stream capture.  All calls share the array,
  * so calls whose kernels overlap on the GPU race; serialise them (one stream,
- * or events).  Nothing in the array needs to start at zero.  A CUDA error
+ * or events).  Nothing in the array or in d_energies
+ * needs to start at zero.  A CUDA error
  * already pending on the calling thread when it is called is reported (and
  * left pending) instead of being taken for a failure of this call. */
 int ea_measure_energy_noalloc(const ea_geom *g, const uint64_t *d_spins, const uint64_t *d_couplings,
