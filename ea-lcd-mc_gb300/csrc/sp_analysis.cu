@@ -16,8 +16,9 @@
 //                   z + d < Lz under open boundaries).
 //
 // Two kernels: bit-sliced counts of the differing spins of each (word, pair,
-// slot, plane) for the 64 samples of a word, then one thread per (sample,
-// slot, distance) summing the nine products in a fixed order (FP64).
+// slot, plane) for the 64 samples of a word, and from them the basis values x
+// and x^3; then the nine products summed in a fixed order (FP64) by one lane
+// per (sample, slot, distance).
 #include <cstdint>
 
 #include "kernels_dev.cuh"
@@ -29,77 +30,122 @@ void set_last_error(const char *msg);  // api.cu
 
 constexpr int kPlanePlanes = 12;  // bit planes of a plane's count: L^2 < 4096
 
-// diff[w][sample][pair][slot][z] = spins that differ between the pair's two
-// replicas on plane z.  One thread per (word, pair, slot, plane).
-__global__ void __launch_bounds__(128) k_sp_plane_diff(const __grid_constant__ SpDev d, int npairs, int32_t *diff) {
+constexpr int kDiffThreads = 256;
+
+// Spins that differ between the pair's two replicas on plane z, for every slot
+// and sample: one block per (word, pair, plane), lane groups of one lane per
+// slot over the plane's sites, the groups' bit planes added through SMEM (one
+// thread a plane and slot was a chain of L^2 loads on few SMs: 63 us on 12 x 12
+// x 48, 24 slots, 2 pairs, now 14).  Writes the counts to diff [w][sample]
+// [pair][slot][z] or, when xs is given, x = 1 - 2 diff / L^2 and x^3 to
+// xs [2][w][pair][slot][z][sample].
+__global__ void __launch_bounds__(kDiffThreads) k_sp_plane_diff(const __grid_constant__ SpDev d, int npairs,
+                                                                int32_t *diff, double *xs) {
+  extern __shared__ u64 pl[];  // [group][bit plane][slot]
   const int NB = d.NB, NR = d.NR, G = NR * NB, Lz = d.Lz, L2 = d.L * d.L;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)d.nw * npairs * NB * Lz) return;
-  const int z = (int)(t % Lz), b = (int)((t / Lz) % NB), k = (int)((t / ((long long)Lz * NB)) % npairs);
-  const int w = (int)(t / ((long long)Lz * NB * npairs));
-  const u64 *Sa = d.S + ((size_t)w * d.V + (size_t)z * L2) * G + (size_t)(2 * k) * NB + b;
-  u64 P[kPlanePlanes];
+  const int z = blockIdx.x % Lz, k = (blockIdx.x / Lz) % npairs, w = blockIdx.x / (Lz * npairs);
+  const int groups = kDiffThreads / NB, g = threadIdx.x / NB, b = threadIdx.x - g * NB;
+  if (g < groups) {
+    const u64 *Sa = d.S + ((size_t)w * d.V + (size_t)z * L2) * G + (size_t)(2 * k) * NB + b;
+    u64 P[kPlanePlanes];
 #pragma unroll
-  for (int q = 0; q < kPlanePlanes; ++q) P[q] = 0;
-  for (int i = 0; i < L2; ++i) {
-    u64 c = __ldg(Sa + (size_t)i * G) ^ __ldg(Sa + (size_t)i * G + NB);
+    for (int q = 0; q < kPlanePlanes; ++q) P[q] = 0;
+#pragma unroll 4
+    for (int i = g; i < L2; i += groups) {
+      u64 c = __ldg(Sa + (size_t)i * G) ^ __ldg(Sa + (size_t)i * G + NB);
 #pragma unroll
-    for (int q = 0; q < kPlanePlanes; ++q) {
-      const u64 h = P[q] & c;
-      P[q] ^= c;
-      c = h;
+      for (int q = 0; q < kPlanePlanes; ++q) {
+        const u64 h = P[q] & c;
+        P[q] ^= c;
+        c = h;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kPlanePlanes; ++q) pl[(g * kPlanePlanes + q) * NB + b] = P[q];
+  }
+  __syncthreads();
+  const double inv = 1.0 / (double)L2;
+  const size_t tab = (size_t)d.nw * npairs * NB * Lz * 64;
+  // a task: samples s, s + 16, s + 32, s + 48 of a slot as 16-bit fields
+  for (int t = threadIdx.x; t < NB * 16; t += kDiffThreads) {
+    const int slot = t >> 4, s = t & 15;
+    u64 acc = 0;
+    for (int q = 0; q < groups; ++q)
+#pragma unroll
+      for (int p = 0; p < kPlanePlanes; ++p)
+        acc += ((pl[(q * kPlanePlanes + p) * NB + slot] >> s) & 0x0001000100010001ull) << p;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int n = (int)((acc >> (16 * q)) & 0xFFFFu), smp = s + 16 * q;
+      if (xs) {
+        const double x = __dsub_rn(1.0, __dmul_rn(2.0 * inv, (double)n));
+        const size_t o = ((((size_t)w * npairs + k) * NB + slot) * Lz + z) * 64 + smp;
+        xs[o] = x;
+        xs[tab + o] = __dmul_rn(__dmul_rn(x, x), x);
+      } else {
+        diff[((((size_t)w * 64 + smp) * npairs + k) * NB + slot) * Lz + z] = n;
+      }
     }
   }
-  int32_t *o = diff + ((((size_t)w * 64) * npairs + k) * NB + b) * Lz + z;
-  const size_t lane_stride = (size_t)npairs * NB * Lz;
-  for (int lane = 0; lane < 64; ++lane) {
-    int n = 0;
-#pragma unroll
-    for (int q = 0; q < kPlanePlanes; ++q) n |= (int)((P[q] >> lane) & 1ull) << q;
-    o[lane * lane_stride] = n;
-  }
-}
-
-__device__ __forceinline__ void basis3(double x, double f[3]) {
-  f[0] = x;
-  f[1] = __dmul_rn(__dmul_rn(x, x), x);
-  f[2] = x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : 0.0);
 }
 
 // C[w*64 + sample][slot][d][3][3] = the correlation matrix at distance d
 // (sums over pairs and planes in a fixed order, then divided by their count).
-__global__ void __launch_bounds__(128) k_sp_plane_corr(const __grid_constant__ SpDev d, int npairs, int dmax,
-                                                       const int32_t *diff, double *C) {
-  const int NB = d.NB, Lz = d.Lz, L2 = d.L * d.L;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)d.nw * 64 * NB * (dmax + 1)) return;
-  const int dd = (int)(t % (dmax + 1)), b = (int)((t / (dmax + 1)) % NB);
-  const long long smp = t / ((long long)(dmax + 1) * NB);  // w * 64 + sample
+// A warp takes one distance of (word, slot) and 32 samples, so its lanes make
+// equally many steps and read neighbouring words.  Bound by the FP64 pipe: a
+// step takes 4 products and 8 sums; products with a sign are sign flips, the
+// signs' own product is counted in integers (both exact).  Thread per
+// (sample, slot, distance), the basis made from the counts at every step:
+// 457 us on 12 x 12 x 48, 24 slots, 2 pairs, 48 distances; now 134 (of which the pipe needs some 75).
+__global__ void __launch_bounds__(256) k_sp_plane_corr(const __grid_constant__ SpDev d, int npairs, int dmax,
+                                                       const double *xs, double *C) {
+  const int NB = d.NB, Lz = d.Lz, nd = dmax + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int ngrp = (nd + nwarp - 1) / nwarp;
+  const int dg = blockIdx.x % ngrp, half = (blockIdx.x / ngrp) & 1, wb = blockIdx.x / (2 * ngrp);
+  const int dd = dg + warp * ngrp, b = wb % NB, w = wb / NB, smp = half * 32 + lane;
+  if (dd >= nd) return;
   const bool pbc = d.bc == EA_PBC;
-  double acc[9];
+  const size_t tab = (size_t)d.nw * npairs * NB * Lz * 64;
+  const int zmax = pbc ? Lz : Lz - dd;
+  double acc[8];
 #pragma unroll
-  for (int q = 0; q < 9; ++q) acc[q] = 0.0;
-  const double inv = 1.0 / (double)L2;
-  long long n = 0;
+  for (int q = 0; q < 8; ++q) acc[q] = 0.0;
+  long long ss = 0;
+  // the value times sign(x): v with its sign flipped, or 0; sign(x) itself.
+  // In integers: FP64 comparisons would take the same pipe as the sums.
+  auto times = [](double v, double x) {
+    const long long xb = __double_as_longlong(x);
+    return __longlong_as_double((xb << 1) == 0 ? 0ll : __double_as_longlong(v) ^ (xb & (1ll << 63)));
+  };
+  auto sgn = [](double x) {
+    const long long xb = __double_as_longlong(x);
+    return (xb << 1) == 0 ? 0 : (xb < 0 ? -1 : 1);
+  };
   for (int k = 0; k < npairs; ++k) {
-    const int32_t *row = diff + (((size_t)smp * npairs + k) * NB + b) * Lz;
-    const int zmax = pbc ? Lz : Lz - dd;
+    const double *X = xs + (((size_t)w * npairs + k) * NB + b) * Lz * 64 + smp;
+#pragma unroll 2
     for (int z = 0; z < zmax; ++z) {
-      const int z2 = pbc ? (z + dd) % Lz : z + dd;
-      const double x1 = __dsub_rn(1.0, __dmul_rn(2.0 * inv, (double)row[z]));
-      const double x2 = __dsub_rn(1.0, __dmul_rn(2.0 * inv, (double)row[z2]));
-      double f[3], g[3];
-      basis3(x1, f);
-      basis3(x2, g);
-#pragma unroll
-      for (int p = 0; p < 3; ++p)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) acc[p * 3 + q] = __dadd_rn(acc[p * 3 + q], __dmul_rn(f[p], g[q]));
-      ++n;
+      int z2 = z + dd;
+      if (z2 >= Lz) z2 -= Lz;
+      const double f0 = __ldg(X + (size_t)z * 64), f1 = __ldg(X + tab + (size_t)z * 64);
+      const double g0 = __ldg(X + (size_t)z2 * 64), g1 = __ldg(X + tab + (size_t)z2 * 64);
+      acc[0] = __dadd_rn(acc[0], __dmul_rn(f0, g0));
+      acc[1] = __dadd_rn(acc[1], __dmul_rn(f0, g1));
+      acc[2] = __dadd_rn(acc[2], times(f0, g0));
+      acc[3] = __dadd_rn(acc[3], __dmul_rn(f1, g0));
+      acc[4] = __dadd_rn(acc[4], __dmul_rn(f1, g1));
+      acc[5] = __dadd_rn(acc[5], times(f1, g0));
+      acc[6] = __dadd_rn(acc[6], times(g0, f0));
+      acc[7] = __dadd_rn(acc[7], times(g1, f0));
+      ss += sgn(f0) * sgn(g0);
     }
   }
-  double *o = C + (size_t)t * 9;
-  for (int q = 0; q < 9; ++q) o[q] = n ? acc[q] / (double)n : 0.0;
+  const long long n = (long long)npairs * zmax;
+  double *o = C + (((size_t)w * 64 + smp) * NB + b) * nd * 9 + (size_t)dd * 9;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) o[q] = n ? acc[q] / (double)n : 0.0;
+  o[8] = n ? (double)ss / (double)n : 0.0;
 }
 
 }  // namespace eagb
@@ -110,6 +156,11 @@ extern "C" {
 
 // Defined in sp.cu: the job's device view and stream.
 int ea_sp_device_view(ea_sp *job, SpDev *d, cudaStream_t *st);
+
+static void launch_plane_diff(const SpDev &d, int npairs, int32_t *diff, double *xs, cudaStream_t st) {
+  const size_t sm = (size_t)(kDiffThreads / d.NB) * d.NB * kPlanePlanes * 8;
+  k_sp_plane_diff<<<(unsigned)((size_t)d.nw * npairs * d.Lz), kDiffThreads, sm, st>>>(d, npairs, diff, xs);
+}
 
 static int an_fail(const char *m) {
   set_last_error(m);
@@ -127,9 +178,8 @@ int ea_sp_plane_overlaps(ea_sp *job, int32_t nrep, int32_t *diff) {
   const size_t n = (size_t)d.nw * 64 * npairs * d.NB * d.Lz;
   int32_t *dd = nullptr;
   cudaError_t e = cudaMalloc((void **)&dd, n * 4);
-  const long long nt = (long long)d.nw * npairs * d.NB * d.Lz;
   if (e == cudaSuccess) {
-    k_sp_plane_diff<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(d, npairs, dd);
+    launch_plane_diff(d, npairs, dd, nullptr, st);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(diff, dd, n * 4, cudaMemcpyDeviceToHost, st);
@@ -151,21 +201,19 @@ int ea_sp_plane_correlations(ea_sp *job, int32_t nrep, int32_t dmax, double *C) 
   if (dmax < 0 || dmax >= d.Lz) return an_fail("dmax: 0..Lz-1");
   if (d.L * d.L >= (1 << kPlanePlanes)) return an_fail("planes of at most 4095 sites");
   const int npairs = nrep / 2;
-  const size_t nd = (size_t)d.nw * 64 * npairs * d.NB * d.Lz, nc = (size_t)d.nw * 64 * d.NB * (dmax + 1) * 9;
-  int32_t *dd = nullptr;
-  double *dc = nullptr;
-  cudaError_t e = cudaMalloc((void **)&dd, nd * 4);
+  const size_t nx = 2 * (size_t)d.nw * 64 * npairs * d.NB * d.Lz, nc = (size_t)d.nw * 64 * d.NB * (dmax + 1) * 9;
+  double *dx = nullptr, *dc = nullptr;
+  cudaError_t e = cudaMalloc((void **)&dx, nx * 8);
   if (e == cudaSuccess) e = cudaMalloc((void **)&dc, nc * 8);
   if (e == cudaSuccess) {
-    const long long nt = (long long)d.nw * npairs * d.NB * d.Lz;
-    k_sp_plane_diff<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(d, npairs, dd);
-    const long long nt2 = (long long)d.nw * 64 * d.NB * (dmax + 1);
-    k_sp_plane_corr<<<(unsigned)((nt2 + 127) / 128), 128, 0, st>>>(d, npairs, dmax, dd, dc);
+    launch_plane_diff(d, npairs, nullptr, dx, st);
+    const int ngrp = (dmax + 1 + 7) / 8;
+    k_sp_plane_corr<<<(unsigned)((size_t)d.nw * d.NB * 2 * ngrp), 256, 0, st>>>(d, npairs, dmax, dx, dc);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(C, dc, nc * 8, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (dd) cudaFree(dd);
+  if (dx) cudaFree(dx);
   if (dc) cudaFree(dc);
   if (e != cudaSuccess) {
     set_last_error(cudaGetErrorString(e));
