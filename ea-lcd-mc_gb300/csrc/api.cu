@@ -283,7 +283,8 @@ int ea_create(const ea_geom *gp, int32_t device, ea_ctx **out) {
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) { delete c; return fail(EA_ERR_CUDA, "cudaSetDevice(%d): %s", device, cudaGetErrorString(e)); }
   e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
-  if (e != cudaSuccess) { delete c; return fail(EA_ERR_CUDA, "stream: %s", cudaGetErrorString(e)); }
+  if (e == cudaSuccess) e = houdayer_setup();
+  if (e != cudaSuccess) { ea_destroy(c); return fail(EA_ERR_CUDA, "set-up: %s", cudaGetErrorString(e)); }
   JobDev &j = c->j;
   j.NB = g.NB; j.NR = g.NR; j.ns = g.ns; j.half = g.half; j.msc_l = g.msc_l; j.msc_s = g.msc_s;
   j.msc_lz = g.msc_lz; j.L = g.L; j.Lz = g.Lz; j.V = g.V; j.bc = g.bc; j.kt = kt;
@@ -711,7 +712,7 @@ static int ensure_cluster(ea_ctx *c, int nclust, cudaStream_t st) {
     j.xw_w = xw_rows(j.xw_n, j.xw_seg);
     CU(dalloc(j.xw_bits, xw_words(j.xw_n)));
     CU(dalloc(j.xw_state, (size_t)j.xw_seg * 6 * kXwStreams));
-    CU(dalloc(j.xw_pos, 2));
+    CU(dalloc(j.xw_pos, 3));
     CU(dalloc(c->xw_mat, 2 * (size_t)kXwMat));
     j.xw_jump = c->xw_mat;
     if (j.xw_seg > 1) {
@@ -772,11 +773,9 @@ static int houdayer(ea_ctx *c, int nclust) {
   cudaEvent_t b = prof_begin(c);
   CU(launch_move_start(c->j, c->st));
   prof_end(c, EA_K_RNG, b);
-  for (int grp = 0; grp < 2; ++grp) {
-    b = prof_begin(c);
-    CU(launch_houdayer_group(c->j, grp, c->st));
-    prof_end(c, EA_K_CLUSTER, b);
-  }
+  b = prof_begin(c);
+  CU(launch_houdayer(c->j, c->st));
+  prof_end(c, EA_K_CLUSTER, b);
   houdayer_finish(c);
   return EA_OK;
 }
@@ -963,19 +962,22 @@ static int batch_upload(ea_batch *b) {
   const int n = (int)b->jobs.size();
   std::vector<JobDev> hj(n);
   std::vector<uint32_t> hp((size_t)KB_COUNT * (n + 1), 0);
-  int slab_threads = 32, flip_smem = 0;
+  int slab_threads = 32, slab_smem = 0, move_threads = 32, move_smem = 0, flip_smem = 0;
   for (int i = 0; i < n; ++i) {
     hj[i] = b->jobs[i]->j;
     hj[i].nsplit = 1;  // a batch fills the GPU with the tiles of its jobs
     uint32_t cnt[KB_COUNT];
     batch_blocks(hj[i], cnt);
     for (int k = 0; k < KB_COUNT; ++k) hp[(size_t)k * (n + 1) + i + 1] = hp[(size_t)k * (n + 1) + i] + cnt[k];
+    const CcShape cc = cnt[KB_SLAB] || cnt[KB_MOVE] ? cc_shape(hj[i]) : CcShape{};
     if (cnt[KB_SLAB]) {
-      int D, P, ns;
-      slab_shape(hj[i], &D, &P, &ns);
-      const int t = hj[i].L * hj[i].L * P;
-      if (t > slab_threads) slab_threads = t;
-      if ((int)flip_smem_bytes(hj[i]) > flip_smem) flip_smem = (int)flip_smem_bytes(hj[i]);
+      slab_threads = std::max(slab_threads, cc.threads);
+      slab_smem = std::max(slab_smem, (int)cc.smem);
+      flip_smem = std::max(flip_smem, (int)flip_smem_bytes(hj[i]));
+    }
+    if (cnt[KB_MOVE]) {
+      move_threads = std::max(move_threads, cc.threads);
+      move_smem = std::max(move_smem, (int)cc.smem);
     }
   }
   const bool same = b->up_jobs.size() == hj.size() &&
@@ -1002,11 +1004,14 @@ static int batch_upload(ea_batch *b) {
     b->bd.total[k] = hp[(size_t)k * (n + 1) + n];
   }
   b->bd.slab_threads = slab_threads;
+  b->bd.slab_smem = slab_smem;
+  b->bd.move_threads = move_threads;
+  b->bd.move_smem = move_smem;
   b->bd.flip_smem = flip_smem;
   b->bd.ctr = b->d_ctr;
   // chunks of work items a block takes at a time: one heavy item, or several
   // light ones so that the job lookup and the fetch are amortised
-  const uint32_t chunk[KB_COUNT] = {1, 4, 1, 4, 4, 1, 4, 4, 1, 1};
+  const uint32_t chunk[KB_COUNT] = {1, 4, 1, 4, 4, 1, 4, 4, 1, 1, 1};
   for (int k = 0; k < KB_COUNT; ++k) b->bd.chunk[k] = chunk[k];
   if (b->bd.total[KB_SWEEP] >= 8u * 304u) b->bd.chunk[KB_SWEEP] = 2;
   // the cycle graph holds the descriptor by value
@@ -1260,12 +1265,14 @@ static int batch_houdayer(ea_batch *b, int nclust) {
     if ((rc = houdayer_prepare(c, nclust, b->bs))) return rc;
   if ((rc = batch_upload(b))) return rc;
   CU(batch_move_start(b->bd, b->bs));
+  CU(batch_move(b->bd, b->bs));
   for (int grp = 0; grp < 2; ++grp) {
     CU(batch_houdayer_group(b->bd, grp, b->bs));
     // jobs whose planes exceed the slab labelling take the one-job path
     for (int i = 0; i < n; ++i) {
       const uint32_t *pre = b->up_pre.data() + (size_t)KB_SLAB * (n + 1);
-      if (pre[i + 1] != pre[i]) continue;
+      const uint32_t *whole = b->up_pre.data() + (size_t)KB_MOVE * (n + 1);
+      if (pre[i + 1] != pre[i] || whole[i + 1] != whole[i]) continue;
       CU(launch_houdayer_group(b->jobs[i]->j, grp, b->bs));
     }
   }

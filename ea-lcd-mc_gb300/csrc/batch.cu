@@ -1,5 +1,8 @@
 // batch.cu -- persistent batched kernels over a packed (job, block) work list.
 #include "batch.cuh"
+
+#include <algorithm>
+
 #include "kernels_dev.cuh"
 
 namespace eagb {
@@ -12,11 +15,12 @@ void batch_blocks(const JobDev &j, uint32_t out[KB_COUNT]) {
   out[KB_PT] = (uint32_t)(j.ns * ((j.NR + 7) / 8));
   out[KB_MEASURE] = (nsrb + 255) / 256;
   out[KB_START] = j.nclust > 0 ? 1 + (uint32_t)(j.xw_seg * (kXwStreams / 256)) : 0;
-  int D, P, nslab;
-  if (j.nclust > 0 && slab_shape(j, &D, &P, &nslab) && flip_smem_bytes(j) <= kFlipMaxSmem) {
+  const CcShape cc = j.nclust > 0 ? cc_shape(j) : CcShape{};
+  out[KB_MOVE] = cc.whole ? 2 * nlat : 0;
+  if (!cc.whole && cc.planes > 0 && flip_smem_bytes(j) <= kFlipMaxSmem) {
     out[KB_OVERLAP] = (uint32_t)((2 * j.half + 255) / 256) * nlat;
-    out[KB_SLAB] = (uint32_t)nslab * nlat;
-    out[KB_MERGE] = (uint32_t)((nslab * j.L * j.L + 255) / 256) * nlat;
+    out[KB_SLAB] = (uint32_t)cc.nslab * nlat;
+    out[KB_MERGE] = (uint32_t)((cc.nslab * j.L * j.L + 255) / 256) * nlat;
     out[KB_COMPRESS] = out[KB_MERGE];
     out[KB_FLIP] = nlat;
   } else {
@@ -32,13 +36,6 @@ __device__ __forceinline__ int item_job(const uint32_t *pre, int n, uint32_t v) 
     if (__ldg(pre + mid) <= v) lo = mid; else hi = mid - 1;
   }
   return lo;
-}
-
-__device__ __forceinline__ void dev_slab_shape(const JobDev &j, int &D, int &P, int &nslab) {
-  const int S = j.L * j.L;
-  D = min(j.Lz, kSlabSites / S);
-  P = max(1, min(D, 512 / S));
-  nslab = (j.Lz + D - 1) / D;
 }
 
 // Next chunk of work for this block.  Every block fetches until it draws a
@@ -124,16 +121,26 @@ __global__ void kb_overlap(const __grid_constant__ BatchDev b, int g) {
   }
 }
 
-__global__ void __launch_bounds__(1024, 2) kb_cc_slab(const __grid_constant__ BatchDev b) {
-  __shared__ uint32_t lab[kSlabSites];
-  __shared__ uint8_t qs[kSlabSites];
+__global__ void __launch_bounds__(1024) kb_cc_slab(const __grid_constant__ BatchDev b) {
+  extern __shared__ __align__(16) unsigned char smem[];
   BATCH_LOOP(KB_SLAB) {
     const int jb = item_job(pre, b.njobs, v);
     const JobDev j = b.jobs[jb];
-    int D, P, nslab;
-    dev_slab_shape(j, D, P, nslab);
     const int l = (int)(v - __ldg(pre + jb));
-    cc_slab_body(j, D, P, l % nslab, (size_t)(l / nslab), lab, qs);
+    cc_slab_body(j, j.cc_D, l % j.cc_nslab, (size_t)(l / j.cc_nslab), smem);
+    __syncthreads();
+  }
+  }
+}
+
+// The whole move of jobs whose lattices fit SMEM, both groups.
+__global__ void __launch_bounds__(1024) kb_move(const __grid_constant__ BatchDev b) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  BATCH_LOOP(KB_MOVE) {
+    const int jb = item_job(pre, b.njobs, v);
+    const JobDev j = b.jobs[jb];
+    const int l = (int)(v - __ldg(pre + jb));
+    move_body(j, l & 1, (size_t)(l >> 1), smem);
     __syncthreads();
   }
   }
@@ -143,10 +150,8 @@ __global__ void kb_cc_merge(const __grid_constant__ BatchDev b) {
   BATCH_LOOP(KB_MERGE) {
     const int jb = item_job(pre, b.njobs, v);
     const JobDev j = b.jobs[jb];
-    int D, P, nslab;
-    dev_slab_shape(j, D, P, nslab);
-    const int gx = (nslab * j.L * j.L + 255) / 256, l = (int)(v - __ldg(pre + jb));
-    cc_merge_body(j, D, nslab, (l % gx) * 256 + threadIdx.x, (size_t)(l / gx));
+    const int gx = (j.cc_nslab * j.L * j.L + 255) / 256, l = (int)(v - __ldg(pre + jb));
+    cc_merge_body(j, j.cc_D, j.cc_nslab, (l % gx) * 256 + threadIdx.x, (size_t)(l / gx));
   }
   }
 }
@@ -155,10 +160,8 @@ __global__ void kb_cc_compress(const __grid_constant__ BatchDev b) {
   BATCH_LOOP(KB_COMPRESS) {
     const int jb = item_job(pre, b.njobs, v);
     const JobDev j = b.jobs[jb];
-    int D, P, nslab;
-    dev_slab_shape(j, D, P, nslab);
-    const int gx = (nslab * j.L * j.L + 255) / 256, l = (int)(v - __ldg(pre + jb));
-    cc_compress_body(j, D, nslab, (l % gx) * 256 + threadIdx.x, (size_t)(l / gx));
+    const int gx = (j.cc_nslab * j.L * j.L + 255) / 256, l = (int)(v - __ldg(pre + jb));
+    cc_compress_body(j, j.cc_D, j.cc_nslab, (l % gx) * 256 + threadIdx.x, (size_t)(l / gx));
   }
   }
 }
@@ -171,6 +174,7 @@ __global__ void __launch_bounds__(256) kb_move_start(const __grid_constant__ Bat
     const int blk = (int)(v - __ldg(pre + jb));
     if (blk > 0) xw_body(jd, blk - 1, s_m);
     else if (threadIdx.x == 0) pairs_body(jd);
+    xw_done(jd);
   }
   }
 }
@@ -214,6 +218,8 @@ cudaError_t batch_setup(int NR, int KT) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kb_flip, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlipMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kb_cc_slab, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kb_move, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
   if (e != cudaSuccess) return e;
   switch (NR * 100 + KT) {
     case 801: return sweep_setup<8, 1>();
@@ -286,11 +292,22 @@ cudaError_t batch_move_start(const BatchDev &b, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Blocks an SM holds of a labelling launch (at most 56 registers a thread).
+static int per_sm(int threads, int smem) {
+  const int t = std::max(1, std::min(65536 / (std::max(threads, 32) * 56), 2048 / std::max(threads, 32)));
+  return std::max(1, std::min(t, (227 * 1024) / (smem + 1024)));
+}
+
+cudaError_t batch_move(const BatchDev &b, cudaStream_t st) {
+  if (b.total[KB_MOVE])
+    kb_move<<<grid_for(chunks(b, KB_MOVE), per_sm(b.move_threads, b.move_smem)), b.move_threads, b.move_smem, st>>>(b);
+  return cudaGetLastError();
+}
+
 cudaError_t batch_houdayer_group(const BatchDev &b, int g, cudaStream_t st) {
   if (!b.total[KB_SLAB]) return cudaSuccess;
   kb_overlap<<<grid_for(chunks(b, KB_OVERLAP), 8), 256, 0, st>>>(b, g);
-  const int per_sm = b.slab_threads > 0 ? 2048 / b.slab_threads : 1;
-  kb_cc_slab<<<grid_for(chunks(b, KB_SLAB), per_sm < 1 ? 1 : per_sm), b.slab_threads, 0, st>>>(b);
+  kb_cc_slab<<<grid_for(chunks(b, KB_SLAB), per_sm(b.slab_threads, b.slab_smem)), b.slab_threads, b.slab_smem, st>>>(b);
   kb_cc_merge<<<grid_for(chunks(b, KB_MERGE), 8), 256, 0, st>>>(b);
   kb_cc_compress<<<grid_for(chunks(b, KB_COMPRESS), 8), 256, 0, st>>>(b);
   kb_flip<<<grid_for(chunks(b, KB_FLIP), 4), 512, b.flip_smem, st>>>(b, g);

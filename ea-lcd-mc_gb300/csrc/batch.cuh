@@ -9,7 +9,7 @@
 namespace eagb {
 
 // Work-list kinds: the blocks of one job for each one-job kernel.
-enum { KB_SWEEP = 0, KB_ZERO, KB_PT, KB_MEASURE, KB_OVERLAP, KB_SLAB, KB_MERGE, KB_COMPRESS, KB_FLIP, KB_START, KB_COUNT };
+enum { KB_SWEEP = 0, KB_ZERO, KB_PT, KB_MEASURE, KB_OVERLAP, KB_SLAB, KB_MERGE, KB_COMPRESS, KB_FLIP, KB_START, KB_MOVE, KB_COUNT };
 
 constexpr int kBatchMaxJobs = 1024;
 
@@ -25,7 +25,8 @@ struct BatchDev {
   uint32_t total[KB_COUNT];
   uint32_t chunk[KB_COUNT];
   uint32_t *ctr;     // [KB_COUNT] work counters
-  int slab_threads;  // block size of the slab labelling (largest L^2 * P)
+  int slab_threads, slab_smem;  // launch of the slab labelling (largest of the jobs)
+  int move_threads, move_smem;  // launch of the whole-lattice move
   int flip_smem;     // dynamic SMEM of the flip (largest lattice)
 };
 
@@ -43,6 +44,7 @@ cudaError_t batch_zero_energy(const BatchDev &b, cudaStream_t st);
 cudaError_t batch_pt(const BatchDev &b, cudaStream_t st);
 cudaError_t batch_measure(const BatchDev &b, int itm, cudaStream_t st);
 cudaError_t batch_move_start(const BatchDev &b, cudaStream_t st);
+cudaError_t batch_move(const BatchDev &b, cudaStream_t st);
 cudaError_t batch_houdayer_group(const BatchDev &b, int g, cudaStream_t st);
 
 }  // namespace eagb

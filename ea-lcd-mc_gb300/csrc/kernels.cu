@@ -2,25 +2,60 @@
 // kernels_dev.cuh) and their launchers.
 #include "kernels_dev.cuh"
 
+#include <algorithm>
 #include <cstdio>
 
 namespace eagb {
 
-bool slab_shape(const JobDev &j, int *D, int *P, int *nslab) {
+// SMEM of a slab's labelling: three CTAs an SM when slabs of a fair number of
+// planes still fit (fewer planes leave more faces to the union across slabs).
+constexpr size_t kSlabSmem = 74 * 1024;
+constexpr size_t kRunMax = 224 * 1024;
+
+static int cc_threads(const RunShape &r) {
+  const int passes = (r.nseg + 1023) / 1024;
+  return std::min(1024, ((r.nseg + passes - 1) / passes + 31) / 32 * 32);
+}
+
+CcShape cc_shape(const JobDev &j) {
+  CcShape c{};
   const int S = j.L * j.L;
-  if (S > 1024) return false;
-  const int d = j.Lz < kSlabSites / S ? j.Lz : kSlabSites / S;
-  int p = 512 / S;
-  if (p > d) p = d;
-  if (p < 1) p = 1;
-  if ((d + p - 1) / p > kSlabMaxPerThread) return false;
-  *D = d; *P = p; *nslab = (j.Lz + d - 1) / d;
-  return true;
+  const size_t q = (size_t)j.V / 8;
+  // whole: label indices in 16 bits, the overlap words beside the labels
+  if (j.V <= 65536 && run_label_smem(run_shape(j.L, j.Lz)) + q <= kRunMax) {
+    const RunShape r = run_shape(j.L, j.Lz);
+    c.whole = true;
+    c.planes = j.Lz;
+    c.nslab = 1;
+    c.threads = cc_threads(r);
+    c.smem = run_label_smem(r) + q;
+    return c;
+  }
+  if (S > kSlabPlane) return c;
+  size_t lim = kSlabSmem;
+  auto most = [&](size_t smem) {
+    int D = 0;
+    while (D < j.Lz && S * (D + 1) <= 65536 && run_label_smem(run_shape(j.L, D + 1)) <= smem) ++D;
+    return D;
+  };
+  int D = most(lim);
+  if (D < 8) D = most(lim = kRunMax);
+  if (D < 1) return c;
+  c.nslab = (j.Lz + D - 1) / D;
+  c.planes = (j.Lz + c.nslab - 1) / c.nslab;  // slabs of equal height
+  c.nslab = (j.Lz + c.planes - 1) / c.planes;
+  const RunShape r = run_shape(j.L, c.planes);
+  c.threads = cc_threads(r);
+  c.smem = run_label_smem(r);
+  return c;
 }
 
 void set_dividers(JobDev &j) {
   j.fd_L.set(j.L); j.fd_S.set(j.L * j.L); j.fd_ml.set(j.msc_l); j.fd_mlz.set(j.msc_lz);
   j.fd_hl.set(j.msc_l / 2); j.fd_nclust.set(j.nclust > 0 ? j.nclust : 1);
+  const CcShape c = cc_shape(j);
+  j.cc_D = c.planes;
+  j.cc_nslab = c.nslab;
 }
 
 __global__ void k_ctr_chain(const __grid_constant__ JobDev j, int npass) {
@@ -47,10 +82,14 @@ __global__ void k_hou_overlap(const __grid_constant__ JobDev j, int g) {
   overlap_body(j, g, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
 }
 
-__global__ void __launch_bounds__(1024, 2) k_cc_slab(const __grid_constant__ JobDev j, int D, int P) {
-  __shared__ uint32_t lab[kSlabSites];
-  __shared__ uint8_t qs[kSlabSites];
-  cc_slab_body(j, D, P, blockIdx.x, blockIdx.y, lab, qs);
+__global__ void __launch_bounds__(1024) k_cc_slab(const __grid_constant__ JobDev j) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  cc_slab_body(j, j.cc_D, blockIdx.x, blockIdx.y, smem);
+}
+
+__global__ void __launch_bounds__(1024) k_hou_move(const __grid_constant__ JobDev j) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  move_body(j, blockIdx.y, blockIdx.x, smem);
 }
 
 __global__ void k_cc_merge(const __grid_constant__ JobDev j, int D, int nslab) {
@@ -98,35 +137,6 @@ __global__ void k_cc_init(JobDev j) {
     if (q_bit(j, Q, x, y, zm) == q) m = min(m, (uint32_t)(x + L * y + S * zm));
   }
   j.label[t] = m;
-}
-
-// Planes of 1025..8192 sites: a CTA-wide loop over the slab's sites.
-__global__ void __launch_bounds__(512) k_cc_local(JobDev j, int D) {
-  __shared__ uint32_t lab[kSlabSites];
-  __shared__ uint8_t qs[kSlabSites];
-  const int L = j.L, S = L * L, tid = threadIdx.x, nth = blockDim.x;
-  const size_t lat = blockIdx.y;
-  const int z0 = blockIdx.x * D, nz = min(D, j.Lz - z0), n = S * nz;
-  const u64 *Q = j.Q + lat * 2 * j.half;
-  for (int i = tid; i < n; i += nth) {
-    const int zl = j.fd_S.div(i), xy = i - zl * S, y = j.fd_L.div(xy), x = xy - y * L;
-    qs[i] = (uint8_t)q_bit(j, Q, x, y, z0 + zl);
-    lab[i] = (uint32_t)i;
-  }
-  __syncthreads();
-  for (int i = tid; i < n; i += nth) {
-    const int zl = j.fd_S.div(i), xy = i - zl * S, y = j.fd_L.div(xy), x = xy - y * L, q = qs[i];
-    const int xm = x == 0 ? L - 1 : x - 1, ym = y == 0 ? L - 1 : y - 1;
-    // site 0 tests its x-wrap bond against x = cc_xq (see JobDev::cc_xq)
-    const int xt = (z0 == 0 && i == 0) ? j.cc_xq : xm;
-    if (qs[xt + L * y + S * zl] == q) cc_unite(lab, (uint32_t)i, (uint32_t)(xm + L * y + S * zl));
-    if (qs[x + L * ym + S * zl] == q) cc_unite(lab, (uint32_t)i, (uint32_t)(x + L * ym + S * zl));
-    if (zl > 0 && qs[i - S] == q) cc_unite(lab, (uint32_t)i, (uint32_t)(i - S));
-  }
-  __syncthreads();
-  uint32_t *glab = j.label + lat * j.V + (size_t)z0 * S;
-  const uint32_t off = (uint32_t)z0 * S;
-  for (int i = tid; i < n; i += nth) glab[i] = off + cc_find(lab, (uint32_t)i);
 }
 
 // Label reduction of Komura (HoudayerXEA.cu:254-331): every bond that is not
@@ -224,39 +234,45 @@ cudaError_t launch_measure(const JobDev &j, int itm, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+cudaError_t houdayer_setup() {
+  cudaError_t e = cudaFuncSetAttribute(k_cc_slab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunMax);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hou_move, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunMax);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hou_flip, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlipMaxSmem);
+  return e;
+}
+
+cudaError_t launch_houdayer(const JobDev &j, cudaStream_t st) {
+  const CcShape cc = cc_shape(j);
+  if (cc.whole) {
+    k_hou_move<<<dim3((unsigned)(j.ns * j.nclust), 2), cc.threads, cc.smem, st>>>(j);
+    return cudaGetLastError();
+  }
+  cudaError_t e = cudaSuccess;
+  for (int g = 0; g < 2 && e == cudaSuccess; ++g) e = launch_houdayer_group(j, g, st);
+  return e;
+}
+
 cudaError_t launch_houdayer_group(const JobDev &j, int g, cudaStream_t st) {
   const size_t ns = (size_t)j.ns * j.nclust * j.V;
   const unsigned bs = (unsigned)((ns + 255) / 256);
   const unsigned nlat = (unsigned)(j.ns * j.nclust);
   k_hou_overlap<<<dim3((2 * j.half + 255) / 256, nlat), 256, 0, st>>>(j, g);
-  int D, P, nslab;
-  if (slab_shape(j, &D, &P, &nslab)) {
-    k_cc_slab<<<dim3(nslab, nlat), j.L * j.L * P, 0, st>>>(j, D, P);
+  const CcShape cc = cc_shape(j);
+  if (cc.planes > 0) {
+    const int D = cc.planes, nslab = cc.nslab;
+    k_cc_slab<<<dim3(nslab, nlat), cc.threads, cc.smem, st>>>(j);
     k_cc_merge<<<dim3((nslab * j.L * j.L + 255) / 256, nlat), 256, 0, st>>>(j, D, nslab);
     k_cc_compress<<<dim3((nslab * j.L * j.L + 255) / 256, nlat), 256, 0, st>>>(j, D, nslab);
     const size_t sm = flip_smem_bytes(j);
     if (sm <= kFlipMaxSmem) {
-      static bool attr = false;
-      if (!attr) {
-        cudaFuncSetAttribute(k_hou_flip, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlipMaxSmem);
-        attr = true;
-      }
       k_hou_flip<<<nlat, 512, sm, st>>>(j, g);
       return cudaGetLastError();
     }
   } else {
-    const int S = j.L * j.L;
-    if (S <= kSlabSites) {
-      D = min(j.Lz, kSlabSites / S);
-      nslab = (j.Lz + D - 1) / D;
-      k_cc_local<<<dim3(nslab, nlat), 512, 0, st>>>(j, D);
-      k_cc_merge<<<dim3((nslab * S + 255) / 256, nlat), 256, 0, st>>>(j, D, nslab);
-    } else {
-      // planes too large for SMEM: Komura's passes on global labels
-      k_cc_init<<<bs, 256, 0, st>>>(j);
-      k_cc_flatten<<<bs, 256, 0, st>>>(j);
-      k_cc_union<<<bs, 256, 0, st>>>(j);
-    }
+    // planes too large for SMEM: Komura's passes on global labels
+    k_cc_init<<<bs, 256, 0, st>>>(j);
+    k_cc_flatten<<<bs, 256, 0, st>>>(j);
+    k_cc_union<<<bs, 256, 0, st>>>(j);
   }
   k_hou_select<<<dim3((j.V + 255) / 256, nlat), 256, 0, st>>>(j, g);
   k_hou_apply<<<dim3((2 * j.half + 3) / 4, nlat), 256, 0, st>>>(j, g);

@@ -72,7 +72,7 @@ struct JobDev {
   uint32_t *xw_bits;                // bit (xw_pos[0] mod 32) + i: coin i of the move
   uint32_t *xw_state;               // [segment][d, v0..v4][4096] generator states at the next move's rows
   const uint32_t *xw_jump;          // advances a state from its segment's end to the next move's segment
-  unsigned long long *xw_pos;       // first position of this move, of the next
+  unsigned long long *xw_pos;       // first position of this move, of the next; blocks of its start that are done
   unsigned long long xw_n;          // coins of a move: 2 groups x [s][NB][V]
   int xw_seg, xw_w;                 // segments, rows of a segment
   // x coordinate against which site 0 tests its periodic -x bond.  The
@@ -82,12 +82,13 @@ struct JobDev {
   int cc_xq;
   // dividers of the site <-> multispin-word maps
   FastDiv fd_L, fd_S, fd_ml, fd_mlz, fd_hl, fd_nclust;
+  int cc_D, cc_nslab;               // planes of a slab, slabs (see CcShape)
 };
 
 // Half-sweeps (colour passes) whose counters are drawn by one launch.
 constexpr int kCtrPasses = 512;
-constexpr int kSlabSites = 8192;        // sites of a slab held in SMEM
-constexpr int kSlabMaxPerThread = 16;   // sites a thread of the slab labelling owns
+// Planes of up to this many sites are labelled in SMEM.
+constexpr int kSlabPlane = 8192;
 
 // Shared memory of the one-CTA-per-lattice selection and flip (V/8 bytes of
 // selection bits + the 64 bit offsets); larger lattices take the two-kernel
@@ -95,9 +96,15 @@ constexpr int kSlabMaxPerThread = 16;   // sites a thread of the slab labelling 
 constexpr size_t kFlipMaxSmem = 200 * 1024;
 size_t flip_smem_bytes(const JobDev &j);
 
-// Slab labelling shape of a job: planes per slab D, planes per pass P and the
-// number of slabs; false when its planes need the generic labelling.
-bool slab_shape(const JobDev &j, int *D, int *P, int *nslab);
+// How a move labels a job's lattices: whole (a CTA a lattice does the whole
+// move), in slabs of `planes` z planes, or (planes = 0) in global memory.
+struct CcShape {
+  bool whole;
+  int planes, nslab;
+  int threads;
+  size_t smem;
+};
+CcShape cc_shape(const JobDev &j);
 
 // Fills the dividers of j from its sizes (nclust included).
 void set_dividers(JobDev &j);
@@ -121,6 +128,10 @@ cudaError_t launch_sweep(const JobDev &j, int pass, int parity, int energy, cuda
 cudaError_t launch_energy(const JobDev &j, cudaStream_t st);
 cudaError_t launch_pt(const JobDev &j, cudaStream_t st);
 cudaError_t launch_measure(const JobDev &j, int itm, cudaStream_t st);
+// The move's kernels of both groups, after launch_move_start.
+cudaError_t launch_houdayer(const JobDev &j, cudaStream_t st);
+// Those of one group of a job that is not labelled whole.
 cudaError_t launch_houdayer_group(const JobDev &j, int group, cudaStream_t st);
+cudaError_t houdayer_setup();
 
 }  // namespace eagb

@@ -9,6 +9,7 @@
 // relative to the reference project).
 #pragma once
 #include "kernels.cuh"
+#include "runs.cuh"
 #include "xorwow.cuh"
 
 namespace eagb {
@@ -541,11 +542,6 @@ __device__ __forceinline__ void pairs_body(const JobDev &j) {
 // q = s_r1 ^ s_r2 per (sample, beta < nclust, parity, half) (main.cu:889-936).
 __device__ __forceinline__ void overlap_body(const JobDev &j, int g, int w, size_t lat) {
   if (w >= 2 * j.half) return;
-  if (g == 0 && lat == 0 && w == 0) {  // the coins are drawn: the next move's continue where they ended
-    const u64 pos = j.xw_pos[1];
-    j.xw_pos[0] = pos;
-    j.xw_pos[1] = pos + j.xw_n;
-  }
   const size_t i = lat * 2 * j.half + w;
   const int p = w >= j.half, k = w - p * j.half;
   const int s = j.fd_nclust.div((uint32_t)lat), b = (int)lat - s * j.nclust;
@@ -587,96 +583,115 @@ __device__ __forceinline__ void cc_unite(uint32_t *lab, uint32_t a, uint32_t b) 
   }
 }
 
-// Slab labelling.  A CTA labels the equal-overlap clusters of D consecutive z
-// planes of one (sample, beta) lattice in SMEM.  Local index order is natural
-// order shifted by z0 L^2, so a slab root is the smallest global index of its
-// slab piece; only bonds between slabs are left for k_cc_merge.
+// Labelling by runs (runs.cuh) of one lattice in SMEM, whole or D consecutive z
+// planes of it.  Local index order is natural order shifted by z0 L^2, so a
+// root is the smallest global index of its (piece of a) cluster.  The bonds are
+// those of the union-find of the reference (HoudayerXEA.cu:77-121): x and y
+// periodic, z inside the planes, the z wrap under PBC when the lattice is
+// whole; site 0 tests its x-wrap bond against x = cc_xq (see JobDev::cc_xq).
+// A thread takes a column of a chunk of planes: neighbouring lanes take
+// neighbouring columns, whose label slots lie in distinct banks but for pairs.
 
-// Planes of up to 1024 sites: one thread per (x, y) column and P planes
-// (at most 16 sites a thread), in lock-step rounds so that no lane walks a
-// long chain while the others wait:
-//   hook:  every bond whose two labels differ hangs the larger label below
-//          the smaller (atomicMin);
-//   jump:  lab[i] = lab[lab[i]] until every label is a root;
-// until a hook round finds nothing to do.  Labels only decrease and always
-// name a site of the same cluster, so at the end every site holds the
-// smallest index of its slab cluster.  The bonds are those of the union-find
-// of the reference (HoudayerXEA.cu:77-121): -x and -y periodic, -z inside the
-// slab.
+// Planes bonded along x of a column, with site 0's test put right: the contact
+// of column L - 1 (y = 0) with column 0 on the first plane.
+__device__ __forceinline__ uint32_t cc_bonds(const JobDev &j, const RunLab<1> &rl, int z0, int ch, int col, uint32_t eq) {
+  if (z0 == 0 && ch == 0 && col == j.L - 1)
+    eq = (eq & ~1u) | (uint32_t)(((rl.qm[0] ^ rl.qm[j.cc_xq]) & 1u) == 0);
+  return eq;
+}
 
-// Threads from S*P on (a batched launch sized for a larger plane) own no
-// sites and only take part in the barriers.
-__device__ __forceinline__ void cc_slab_body(const JobDev &j, int D, int P, int slab, size_t lat, uint32_t *lab, uint8_t *qs) {
-  const int L = j.L, S = L * L, t = threadIdx.x;
-  const int z0 = slab * D, nz = t < S * P ? min(D, j.Lz - z0) : 0;
-  const u64 *Q = j.Q + lat * 2 * j.half;
-  const int zp = j.fd_S.div(t), xy = t - zp * S, y = j.fd_L.div(xy), x = xy - y * L;
-  {
-    const int bx = j.fd_ml.div(x), by = j.fd_ml.div(y);
+// The q words of the planes [z0, z0 + nz) from the lattice's overlap words
+// (word(index): the 64 bits of a (parity, half) word).
+template <class Word>
+__device__ __forceinline__ void cc_columns(const JobDev &j, const RunLab<1> &rl, int z0, Word &&word) {
+  const RunShape &r = rl.r;
+  rl.columns();
+  rl.items([&](int it, int ch, int col) {
+    const int y = j.fd_L.div(col), x = col - y * j.L, bx = j.fd_ml.div(x), by = j.fd_ml.div(y);
     const int mxy = (x - bx * j.msc_l) + j.msc_l * (y - by * j.msc_l), sxy = bx + 4 * by;
-    int z = z0 + zp, bz = j.fd_mlz.div(z), gz = z - bz * j.msc_lz;
-    for (int zl = zp; zl < nz; zl += P) {
-      const int i = xy + S * zl, m = mxy + j.msc_s * gz, p = (x ^ y ^ z) & 1;
-      qs[i] = (uint8_t)((Q[(size_t)p * j.half + (m >> 1)] >> (sxy + 16 * bz)) & 1);
-      lab[i] = (uint32_t)i;
-      z += P;
-      gz += P;
-      while (gz >= j.msc_lz) { gz -= j.msc_lz; ++bz; }
+    int z = z0 + ch * r.H, bz = j.fd_mlz.div(z), gz = z - bz * j.msc_lz, p = (x ^ y ^ z) & 1;
+    const int hc = min(r.H, r.nz - ch * r.H);
+    uint32_t m = 0;
+    for (int k = 0; k < hc; ++k) {
+      m |= (uint32_t)((word(p * j.half + ((mxy + j.msc_s * gz) >> 1)) >> (sxy + 16 * bz)) & 1ull) << k;
+      p ^= 1;
+      if (++gz == j.msc_lz) { gz = 0; ++bz; }
     }
+    rl.qm[it] = m;
+  });
+}
+
+// Planes [slab D, ...) of lattice lat, labels written as global indices.
+// Threads: any number; SMEM: slab_smem.
+__device__ __forceinline__ void cc_slab_body(const JobDev &j, int D, int slab, size_t lat, unsigned char *sm) {
+  const int z0 = slab * D, nz = min(D, j.Lz - z0);
+  const u64 *Q = j.Q + lat * 2 * j.half;
+  const RunLab<1> rl(sm, j.L, nz);
+  const RunShape &r = rl.r;
+  cc_columns(j, rl, z0, [&](int i) { return __ldg(Q + i); });
+  rl.label(false, false, [&](int ch, int col, uint32_t eq) { return cc_bonds(j, rl, z0, ch, col, eq); });
+  rl.jump([](uint16_t *, int, uint32_t) {});
+  __syncthreads();
+  const uint32_t off = (uint32_t)z0 * r.S;
+  uint32_t *glab = j.label + lat * j.V + off;
+  for (int i = threadIdx.x; i < nz * r.S; i += blockDim.x) {
+    const int z = j.fd_S.div(i), col = i - z * r.S, ch = z / r.H;
+    const uint32_t st = run_starts(rl.qm[ch * r.S + col], (2u << (z - ch * r.H)) - 1u);
+    glab[i] = off + rl.lab[(ch * r.H + 31 - __clz(st)) * r.S + col];
+  }
+}
+
+// The whole move of group g on lattice lat in one CTA, for lattices that fit
+// SMEM (whole_smem): overlap words, labels, selection and the flip of both
+// replicas (main.cu:776-991; HoudayerXEA.cu:54-374).
+__device__ __forceinline__ void move_body(const JobDev &j, int g, size_t lat, unsigned char *sm) {
+  const RunLab<1> rl(sm, j.L, j.Lz);
+  const RunShape &r = rl.r;
+  u64 *Q = reinterpret_cast<u64 *>(sm + run_label_smem(r));
+  const int s = j.fd_nclust.div((uint32_t)lat), b = (int)lat - s * j.nclust;
+  const int r1 = j.pairs[2 * g], r2 = j.pairs[2 * g + 1];
+  const int c1 = j.wctb[((size_t)s * j.NR + r1) * j.NB + b], c2 = j.wctb[((size_t)s * j.NR + r2) * j.NB + b];
+  const size_t wpc = (size_t)j.half * j.NR, wpp = wpc * j.NB;
+  u64 *S1 = j.spins + (size_t)s * 2 * wpp + (size_t)c1 * wpc + r1;
+  u64 *S2 = j.spins + (size_t)s * 2 * wpp + (size_t)c2 * wpc + r2;
+  for (int w = threadIdx.x; w < 2 * j.half; w += blockDim.x) {
+    const size_t o = (w >= j.half ? wpp : 0) + (size_t)(w >= j.half ? w - j.half : w) * j.NR;
+    Q[w] = S1[o] ^ S2[o];
   }
   __syncthreads();
-  const int xm = x == 0 ? L - 1 : x - 1, ym = y == 0 ? L - 1 : y - 1;
-  const int ixm = xm + L * y, iym = x + L * ym;
-  // bond bits of this thread's sites: 3 per site (-x, -y, -z)
-  u64 bonds = 0;
-  {
-    int k = 0;
-    for (int zl = zp; zl < nz; zl += P, ++k) {
-      const int i = xy + S * zl, q = qs[i], pl = S * zl;
-      // site 0 tests its x-wrap bond against x = cc_xq (see JobDev::cc_xq)
-      const int xt = (z0 == 0 && i == 0) ? j.cc_xq : xm;
-      const u64 b = (u64)(qs[xt + L * y + pl] == q) | ((u64)(qs[iym + pl] == q) << 1) |
-                    ((u64)(zl > 0 && qs[i - S] == q) << 2);
-      bonds |= b << (3 * k);
+  cc_columns(j, rl, 0, [&](int i) { return Q[i]; });
+  rl.label(j.bc == EA_PBC, false, [&](int ch, int col, uint32_t eq) { return cc_bonds(j, rl, 0, ch, col, eq); });
+  __syncthreads();
+  const u64 ub = xw_base(j, g) + ((u64)s * j.NB + b) * (u64)j.V;
+  const uint32_t *u = j.xw_bits + (ub >> 5), us = (uint32_t)ub & 31u;
+  uint32_t *Q32 = reinterpret_cast<uint32_t *>(Q);
+  rl.items([&](int it, int ch, int col) {
+    const uint16_t *l = rl.slot(ch, col);
+    const uint32_t mask = run_mask(r, ch);
+    // coins at the run starts as changes from run to run, then summed upwards
+    uint32_t f = 0, prev = 0;
+    for (uint32_t st = run_starts(rl.qm[it], mask); st; st &= st - 1u) {
+      const uint32_t bit = st & (0u - st);
+      const uint32_t c = xw_coin(u, us + (uint32_t)rl.root(l[(31 - __clz(bit)) * r.S]));
+      if (c != prev) f |= bit;
+      prev = c;
     }
+    f ^= f << 1; f ^= f << 2; f ^= f << 4; f ^= f << 8; f ^= f << 16;
+    const int y = j.fd_L.div(col), x = col - y * j.L, bx = j.fd_ml.div(x), by = j.fd_ml.div(y);
+    const int mxy = (x - bx * j.msc_l) + j.msc_l * (y - by * j.msc_l), sxy = bx + 4 * by;
+    for (f &= mask; f; f &= f - 1u) {
+      const int z = ch * r.H + 31 - __clz(f & (0u - f)), bz = j.fd_mlz.div(z), gz = z - bz * j.msc_lz;
+      const int w = ((x ^ y ^ z) & 1) * j.half + ((mxy + j.msc_s * gz) >> 1), bit = sxy + 16 * bz;
+      atomicXor(Q32 + 2 * w + (bit >> 5), 1u << (bit & 31));  // q' = q xor [selected]
+    }
+  });
+  __syncthreads();
+  for (int w = threadIdx.x; w < 2 * j.half; w += blockDim.x) {
+    const size_t o = (w >= j.half ? wpp : 0) + (size_t)(w >= j.half ? w - j.half : w) * j.NR;
+    const u64 q = Q[w];
+    S1[o] ^= q;
+    S2[o] ^= q;
   }
-  for (;;) {
-    int hooked = 0;
-    {
-      int k = 0;
-      for (int zl = zp; zl < nz; zl += P, ++k) {
-        const unsigned b = (unsigned)(bonds >> (3 * k)) & 7u;
-        if (!b) continue;
-        const int i = xy + S * zl, pl = S * zl;
-        const uint32_t li = lab[i];
-        if (b & 1) {
-          const uint32_t lj = lab[ixm + pl];
-          if (lj != li) { atomicMin(&lab[max(li, lj)], min(li, lj)); hooked = 1; }
-        }
-        if (b & 2) {
-          const uint32_t lj = lab[iym + pl];
-          if (lj != li) { atomicMin(&lab[max(li, lj)], min(li, lj)); hooked = 1; }
-        }
-        if (b & 4) {
-          const uint32_t lj = lab[i - S];
-          if (lj != li) { atomicMin(&lab[max(li, lj)], min(li, lj)); hooked = 1; }
-        }
-      }
-    }
-    if (!__syncthreads_or(hooked)) break;
-    for (;;) {
-      int moved = 0;
-      for (int zl = zp; zl < nz; zl += P) {
-        const int i = xy + S * zl;
-        const uint32_t l = lab[i], ll = lab[l];
-        if (ll != l) { lab[i] = ll; moved = 1; }
-      }
-      if (!__syncthreads_or(moved)) break;
-    }
-  }
-  uint32_t *glab = j.label + lat * j.V + (size_t)z0 * S;
-  const uint32_t off = (uint32_t)z0 * S;
-  for (int zl = zp; zl < nz; zl += P) glab[xy + S * zl] = off + lab[xy + S * zl];
 }
 
 // Bonds across slab faces (z = f D with z - 1), and the z wrap under PBC,

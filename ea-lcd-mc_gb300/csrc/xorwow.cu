@@ -100,18 +100,19 @@ __global__ void __launch_bounds__(64) k_xw_init(const __grid_constant__ JobDev j
 #pragma unroll
     for (int i = 0; i < 5; ++i) st[(i + 1) * kXwStreams] = v[i];
   }
-  if (t == 0) j.xw_pos[0] = j.xw_pos[1] = offset % kXwStreams;
+  if (t == 0) {
+    j.xw_pos[0] = j.xw_pos[1] = offset % kXwStreams;
+    j.xw_pos[2] = 0;
+  }
 }
 
 // The replica pairs ride in block 0 (one thread, a chain of a few generator
 // steps): one launch less in a small job's chain.
 __global__ void __launch_bounds__(256) k_move_start(const __grid_constant__ JobDev j) {
   __shared__ __align__(16) uint32_t s_m[kXwMat];
-  if (blockIdx.x == 0) {
-    if (threadIdx.x == 0) pairs_body(j);
-    return;
-  }
-  xw_body(j, blockIdx.x - 1, s_m);
+  if (blockIdx.x > 0) xw_body(j, blockIdx.x - 1, s_m);
+  else if (threadIdx.x == 0) pairs_body(j);
+  xw_done(j);
 }
 
 cudaError_t launch_xw_init(const JobDev &j, unsigned long long seed, unsigned long long offset, const uint32_t *jump_w,

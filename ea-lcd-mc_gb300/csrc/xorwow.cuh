@@ -39,7 +39,7 @@ void xw_jump(uint64_t rows, uint32_t m[kXwMat]);
 cudaError_t launch_xw_init(const JobDev &j, unsigned long long seed, unsigned long long offset, const uint32_t *jump_w,
                            cudaStream_t st);
 // The start of a move: its replica pairs and its coins (from position
-// xw_pos[1]; the overlap step of group 0 then moves the positions on).
+// xw_pos[1], which then becomes xw_pos[0]).
 cudaError_t launch_move_start(const JobDev &j, cudaStream_t st);
 
 #ifdef __CUDACC__
@@ -131,6 +131,20 @@ __device__ __forceinline__ void xw_body(const JobDev &j, int blk, uint32_t *s_m)
 #pragma unroll
   for (int q = 0; q < 5; ++q) st[(q + 1) * kXwStreams] = v[q];
   if (j.xw_seg == 1 && nrows > adv) edge_row(adv);
+}
+
+// A block of a move's start is done: the last one moves the positions on.
+__device__ __forceinline__ void xw_done(const JobDev &j) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(j.xw_pos + 2, 1ull) + 1 == (unsigned long long)j.xw_seg * (kXwStreams / 256) + 1) {
+      const unsigned long long p = j.xw_pos[1];
+      j.xw_pos[0] = p;
+      j.xw_pos[1] = p + j.xw_n;
+      j.xw_pos[2] = 0;
+    }
+  }
 }
 
 // [U < 0.5] of (group g, index i of its call): bit base + i of j.xw_bits.
