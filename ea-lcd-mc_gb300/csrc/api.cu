@@ -109,20 +109,23 @@ int choose_kt(const Geometry &g) {
   if (env) {
     int kt = atoi(env);
     for (int i = 0; i < 3; ++i)
-      if (c[i] == kt && smem(kt) <= 227 * 1024) return kt;
+      if (c[i] == kt && smem(kt) <= kSweepMax) return kt;
   }
   for (int i = 0; i < 3; ++i) {
     const int kt = c[i];
     const int tiles = (g.half + kt - 1) / kt;
-    if (smem(kt) <= 227 * 1024 && tiles >= 2 * 152) return kt;
+    if (smem(kt) <= kSweepMax && tiles >= 2 * 152) return kt;
   }
   for (int i = 2; i >= 0; --i)
-    if (smem(c[i]) <= 227 * 1024) return c[i];
+    if (smem(c[i]) <= kSweepMax) return c[i];
   return 0;
 }
 
 // CTAs that share a tile: as many as fit the GPU beside each other (2 an SM),
-// while each has an item for every lane group.
+// while each has an item for every lane group.  (16^2 x 64, 24 temperatures, 4
+// replicas, 8 samples: 14.1 us a half-sweep with one CTA a tile, 12.7 with 2,
+// 13.0 with 4, 18.8 with 6; the 24^2 x 192 tube's 432 tiles: 93 with one, 107
+// with 2.)
 int choose_split(const Geometry &g, int kt) {
   const int tiles = (g.half + kt - 1) / kt, groups = 512 / (kt * g.NR), items = g.ns * g.NB;
   return std::max(1, std::min(2 * 152 / tiles, (items + groups - 1) / groups));
@@ -299,7 +302,8 @@ int ea_create(const ea_geom *gp, int32_t device, ea_ctx **out) {
   { int32_t *p; OWN(p, (size_t)12 * g.half); j.nbidx = p; }
   { uint8_t *p; OWN(p, (size_t)2 * g.half); j.nbflag = p; }
   { unsigned long long *p; OWN(p, (size_t)g.NB * 256); j.cum = p; }
-  { uint16_t *p; OWN(p, (size_t)g.NB * 256); j.pre = p; }
+  j.pre_bits = sweep_pre_bits(g.NB);
+  { uint8_t *p; OWN(p, (size_t)g.NB * pre_stride(j.pre_bits)); j.pre = p; }
   OWN(j.wctb, nsr * g.NB);
   OWN(j.wbtc, nsr * g.NB);
   OWN(j.ctr, (size_t)g.NR);
@@ -408,18 +412,19 @@ int ea_set_temperatures(ea_ctx *c, const double *betas, const uint64_t *cum) {
   const Geometry &g = c->g;
   for (int i = 0; i + 1 < g.NB; ++i)
     if (betas[i] < betas[i + 1]) return fail(EA_ERR_ARG, "betas must be sorted from largest to smallest");
-  std::vector<uint16_t> pre((size_t)g.NB * 256);
+  const int stride = pre_stride(c->j.pre_bits);
+  std::vector<uint8_t> pre((size_t)g.NB * stride);
   for (int b = 0; b < g.NB; ++b) {
     if (cum[(size_t)b * 256 + 255] != ~0ULL) return fail(EA_ERR_ARG, "threshold 255 of beta %d is not 2^64-1", b);
     for (int n = 1; n < 256; ++n)
       if (cum[(size_t)b * 256 + n] < cum[(size_t)b * 256 + n - 1]) return fail(EA_ERR_ARG, "thresholds of beta %d decrease", b);
-    presearch8(cum + (size_t)b * 256, pre.data() + (size_t)b * 256);
+    presearch(cum + (size_t)b * 256, c->j.pre_bits, pre.data() + (size_t)b * stride);
   }
   std::vector<double> tab;
   pt_exp_table(betas, g.NB, tab, c->expoff);
   if (set_device(c)) return EA_ERR_CUDA;
   CU(cudaMemcpyAsync((void *)c->j.cum, cum, sizeof(uint64_t) * 256 * g.NB, cudaMemcpyHostToDevice, c->st));
-  CU(cudaMemcpyAsync((void *)c->j.pre, pre.data(), pre.size() * 2, cudaMemcpyHostToDevice, c->st));
+  CU(cudaMemcpyAsync((void *)c->j.pre, pre.data(), pre.size(), cudaMemcpyHostToDevice, c->st));
   CU(cudaMemcpyAsync((void *)c->j.betas, betas, sizeof(double) * g.NB, cudaMemcpyHostToDevice, c->st));
   CU(cudaMemcpyAsync((void *)c->j.expoff, c->expoff.data(), sizeof(int32_t) * g.NB, cudaMemcpyHostToDevice, c->st));
   CU(cudaStreamSynchronize(c->st));
@@ -929,7 +934,7 @@ static int set_tile(ea_ctx *c, int kt) {
   if (kt == j.kt) return EA_OK;
   const Geometry &g = c->g;
   const size_t smem = sweep_smem_for(g.NB, g.NR, kt);
-  if (smem > 227 * 1024) return fail(EA_ERR_ARG, "tile width %d needs %zu bytes of shared memory", kt, smem);
+  if (smem > kSweepMax) return fail(EA_ERR_ARG, "tile width %d needs %zu bytes of shared memory", kt, smem);
   const int nt = (g.half + kt - 1) / kt;
   j.kt = kt;
   j.ntiles = nt;
@@ -940,7 +945,7 @@ static int set_tile(ea_ctx *c, int kt) {
 static int batch_kt(const ea_batch *b, int forced) {
   const int c8[3] = {4, 2, 1}, c4[3] = {8, 4, 2}, c2[3] = {16, 8, 4};
   const int *c = b->NR == 8 ? c8 : b->NR == 4 ? c4 : c2;
-  auto fits = [&](int kt) { return batch_sweep_smem(b->NR, kt, b->NBmax) <= 227 * 1024 - 256; };
+  auto fits = [&](int kt) { return batch_sweep_smem(b->NR, kt, b->NBmax) <= kBatchSweepMax; };
   if (forced) {
     for (int i = 0; i < 3; ++i)
       if (c[i] == forced && fits(forced)) return forced;
@@ -1032,7 +1037,7 @@ static int batch_autotune(ea_batch *b, float *best_ms) {
   const int *c = b->NR == 8 ? c8 : b->NR == 4 ? c4 : c2;
   std::vector<int> cand;
   for (int i = 0; i < 3; ++i)
-    if (batch_sweep_smem(b->NR, c[i], b->NBmax) <= 227 * 1024 - 256) cand.push_back(c[i]);
+    if (batch_sweep_smem(b->NR, c[i], b->NBmax) <= kBatchSweepMax) cand.push_back(c[i]);
   if (cand.empty()) return fail(EA_ERR_ARG, "no tile width fits NB=%d in shared memory", b->NBmax);
   b->KT = cand[0];
   if (cand.size() == 1) return EA_OK;
@@ -1191,7 +1196,7 @@ int ea_batch_set_jobs(ea_batch *b, ea_ctx *const *jobs, int32_t njobs) {
     if (c->g.NB > nbmax) nbmax = c->g.NB;
     nj.push_back(c);
   }
-  if (batch_sweep_smem(b->NR, b->KT, nbmax) > 227 * 1024 - 256)
+  if (batch_sweep_smem(b->NR, b->KT, nbmax) > kBatchSweepMax)
     return fail(EA_ERR_ARG, "NB=%d does not fit the batch's tile width %d", nbmax, b->KT);
   CU(cudaSetDevice(b->device));
   for (ea_ctx *c : nj) {
@@ -1408,7 +1413,7 @@ int ea_job_bytes(const ea_geom *gp, const ea_cadence *cad, const double *betas, 
   add((uint64_t)g.ns * g.words_per_sample() * 8);            // spins
   add((uint64_t)g.ns * 12 * half * 8);                       // couplings
   add(12 * half * 4); add(2 * half);                         // neighbour table, flags
-  add(NB * 256 * 8); add(NB * 256 * 2);                      // thresholds, pre-search
+  add(NB * 256 * 8); add(NB * pre_stride(sweep_pre_bits(g.NB)));           // thresholds, pre-search
   add(nsr * NB); add(nsr * NB);                              // permutations
   add(g.NR * 16); add(g.NR * 16 * kCtrPasses); add(g.NR * 4); add(g.NR * sizeof(ea_hq)); add(g.NR * sizeof(ea_xoshiro)); add(8);
   add(nsr * NB * 4); add(nsr * sizeof(ea_hq)); add(NB * 8); add(NB * 4);

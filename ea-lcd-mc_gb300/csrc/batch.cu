@@ -235,7 +235,13 @@ cudaError_t batch_setup(int NR, int KT) {
   }
 }
 
-int batch_sweep_smem(int NR, int KT, int NBmax) { return (int)sweep_smem_for(NBmax, NR, KT); }
+// The largest of any job with at most NBmax temperatures (the tables shrink
+// where their bits do).
+int batch_sweep_smem(int NR, int KT, int NBmax) {
+  size_t m = 0;
+  for (int nb = 2; nb <= NBmax; ++nb) m = std::max(m, sweep_smem_for(nb, NR, KT));
+  return (int)m;
+}
 
 cudaError_t batch_ctr_chain(const BatchDev &b, int NR, int npass, cudaStream_t st) {
   kb_ctr_chain<<<b.njobs, kCtrThreads, ctr_smem(NR), st>>>(b, npass);

@@ -12,6 +12,7 @@ namespace eagb {
 enum { KB_SWEEP = 0, KB_ZERO, KB_PT, KB_MEASURE, KB_OVERLAP, KB_SLAB, KB_MERGE, KB_COMPRESS, KB_FLIP, KB_START, KB_MOVE, KB_COUNT };
 
 constexpr int kBatchMaxJobs = 1024;
+constexpr int kBatchSweepMax = 227 * 1024 - 256;
 
 // Device view of a batch (kernel parameter).  pre[k] is the exclusive prefix
 // sum over jobs of their block counts for kind k ([njobs + 1] entries).

@@ -304,19 +304,19 @@ void presearch8(const uint64_t *cum, uint16_t *pre) {
   }
 }
 
-// The 11-bit pre-search: pre[t] = the first byte n with (t << 53) < cum[n]
-// for t < 2048 and 255 from entry 2048 on (kPre11Stride entries a
-// temperature).  A key R in bucket t = R >> 53 has its byte in
-// [pre[t], pre[t+1]]: the search is monotone in R, so the first byte of the
+// The pre-search with 2^bits buckets: pre[t] = the first byte n with
+// (t << (64 - bits)) < cum[n] for t < 2^bits and 255 from entry 2^bits on
+// (pre_stride(bits) entries a temperature).  A key R in bucket t has its byte
+// in [pre[t], pre[t+1]]: the search is monotone in R, so the first byte of the
 // next bucket bounds every byte of this one.
-void presearch11(const uint64_t *cum, uint8_t *pre) {
+void presearch(const uint64_t *cum, int bits, uint8_t *pre) {
   int n = 0;
-  for (int t = 0; t < 2048; ++t) {
-    const uint64_t lo = (uint64_t)t << 53;
+  for (int t = 0; t < (1 << bits); ++t) {
+    const uint64_t lo = (uint64_t)t << (64 - bits);
     while (n < 255 && !(lo < cum[n])) ++n;
     pre[t] = (uint8_t)n;
   }
-  for (int t = 2048; t < kPre11Stride; ++t) pre[t] = 255;
+  for (int t = 1 << bits; t < pre_stride(bits); ++t) pre[t] = 255;
 }
 
 // pt = -(beta[i+1]-beta[i]) * dE in double, exactly as upd.c:16-17 forms it,

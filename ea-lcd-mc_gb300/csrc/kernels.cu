@@ -183,7 +183,7 @@ static cudaError_t launch_sweep_t(const JobDev &j, int pass, int parity, int ene
     const size_t sm = sweep_smem_bytes(j);
     static bool attr = false;
     if (!attr) {
-      cudaFuncSetAttribute(k_sweep<NR, KT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      cudaFuncSetAttribute(k_sweep<NR, KT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepMax);
       attr = true;
     }
     k_sweep<NR, KT, true><<<j.ntiles * j.nsplit, 512, sm, st>>>(j, pass, parity, energy);

@@ -37,7 +37,8 @@ struct JobDev {
   const int32_t *nbidx;             // [parity][dir][half]
   const uint8_t *nbflag;            // [parity][half]
   const unsigned long long *cum;    // [NB][256] thresholds
-  const uint16_t *pre;              // [NB][256] 8-bit pre-search
+  const uint8_t *pre;               // [NB][pre_stride(pre_bits)] pre-search
+  int pre_bits;
   uint8_t *wctb, *wbtc;             // [s][rep][NB]
   uint4 *ctr;                       // [NR] Philox counters of the last half-sweep
   uint4 *ctrs;                      // [kCtrPasses][NR] those of the half-sweeps drawn ahead
@@ -112,11 +113,18 @@ void set_dividers(JobDev &j);
 // Tile width (half-sites per CTA) of the fused sweep kernel.
 int sweep_kt(const JobDev &j);
 size_t sweep_smem_bytes(const JobDev &j);
-// Dynamic SMEM of a fused half-sweep CTA: the random triples of the tile
-// (3 x NB x KT x NR words), the pre-search tables (NB x 256 x 2 B) and the
-// tile's neighbour records (KT x 8 ints).
+constexpr size_t kSweepMax = 227 * 1024 - 64;  // less the kernel's static SMEM
+// Bits of the pre-search tables, so that two CTAs of a half-sweep fit an SM:
+// the more, the fewer threshold searches (0.22 steps a byte with 8 bits, 0.04
+// with 11, on a ladder of 32 temperatures from 0.7 to 1.6: a half-sweep of the
+// 24^2 x 192 tube takes 104, 100, 96, 93 us with 8, 9, 10, 11 bits, of 8^3
+// 12.5, 11.1, 10.4, 9.5).
+inline int sweep_pre_bits(int NB) { return NB <= 40 ? 11 : NB <= 72 ? 10 : NB <= 128 ? 9 : 8; }
+// Dynamic SMEM of a fused half-sweep CTA: the flip mask's two words of every
+// triple of the tile and the queues of their halves, the pre-search tables
+// and the tile's neighbour records (KT x 8 ints).
 inline size_t sweep_smem_for(int NB, int NR, int KT) {
-  return (size_t)3 * NB * KT * NR * 8 + (size_t)NB * 256 * 2 + (size_t)KT * 8 * 4;
+  return (size_t)NB * KT * NR * (16 + 8) + (size_t)NB * (((1 << sweep_pre_bits(NB)) + 16) & ~15) + (size_t)KT * 8 * 4;
 }
 
 // Counters of npass half-sweeps (even, odd, even, ...) into j.ctrs.

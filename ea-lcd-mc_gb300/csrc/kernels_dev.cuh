@@ -133,20 +133,23 @@ __device__ __forceinline__ uint32_t lut_byte(uint32_t hi, uint32_t lo, const u64
   return a;
 }
 
-// The same search with the 11-bit pre-search of presearch11 (host.cpp): a
-// key in bucket t = hi >> 21 has its byte in [pre[t], pre[t+1]]; thresholds
-// through the read-only cache.  Narrower buckets leave a bisection to fewer
+// The same search with the pre-search of presearch (host.cpp): a key in bucket
+// t = hi >> shift (shift = 32 - bits) has its byte in [pre[t], pre[t+1]];
+// thresholds through the read-only cache.  Narrower buckets leave a bisection to fewer
 // keys: 0.04 steps per byte on the benchmark sets against 0.18-0.21 with the
 // 8-bit pre-search, and a warp waits for its slowest lane at each search.
-__device__ __forceinline__ uint32_t lut_byte11(uint32_t hi, uint32_t lo, const u64 *cum, const uint8_t *pre) {
+__device__ __forceinline__ uint32_t lut_byte_pre(uint32_t hi, uint32_t lo, const u64 *cum, const uint8_t *pre, int shift) {
   const u64 R = ((u64)hi << 32) | lo;
-  const uint32_t t = hi >> 21;
+  const uint32_t t = hi >> shift;
   uint32_t a = pre[t], b = pre[t + 1];
   while (a < b) {
     const uint32_t m = (a + b) >> 1;
     if (R < __ldg(cum + m)) b = m; else a = m + 1;
   }
   return a;
+}
+__device__ __forceinline__ uint32_t lut_byte11(uint32_t hi, uint32_t lo, const u64 *cum, const uint8_t *pre) {
+  return lut_byte_pre(hi, lo, cum, pre, 21);
 }
 
 // One random word from a Philox counter: the four keys' bytes by `byte`
@@ -223,18 +226,94 @@ __device__ __forceinline__ u64 flip_mask(const u64 f[6], u64 b0, u64 b1, u64 b2)
 }
 
 // ---------------------------------------------------------------------------
+// The flip mask's two words (flip_mask_id) of ntrip random triples, drawn by a
+// CTA: id1 = (b0 ^ id2) | (id2 & b2), id2 = b0 & b1.  Where a 32-bit half of b0
+// is 0 that half of b1 and b2 does not matter, nor that of b2 where b0 & b1 is
+// 0, and b0's bits are rare on a tempering ladder (exp(-4 beta)): the halves
+// that need a draw are queued and drawn by whichever threads are free, 3.2 to
+// 3.3 draws a triple instead of 6 (counter-based: the ones made are the same).
+// item(t, c, key, tp, b): the Philox counter, key and index of triple t and its
+// temperature, false if it has none; byte(b, hi, lo): the threshold search.
+// queue: 4 ntrip entries, ntrip <= 2^14; cnt: 2.  All in SMEM; ends with a
+// barrier.
+template <class Item, class Byte>
+__device__ __forceinline__ void draw_ids(int ntrip, Item &&item, Byte &&byte, u64 *id1, u64 *id2, uint16_t *queue, int *cnt) {
+  uint32_t *i1 = reinterpret_cast<uint32_t *>(id1), *i2 = reinterpret_cast<uint32_t *>(id2);
+  uint16_t *qa = queue, *qb = queue + 2 * ntrip;
+  const int lane = threadIdx.x & 31, i00 = threadIdx.x - lane;
+  const unsigned below = (1u << lane) - 1u;
+  if (threadIdx.x == 0) cnt[0] = cnt[1] = 0;
+  __syncthreads();
+  auto word = [&](int q, int t) -> uint32_t {
+    uint4 c;
+    uint32_t key, tp;
+    int b;
+    if (!item(t, c, key, tp, b)) return 0u;
+    return rnd_word_by(c.x + q, c.y, c.z + tp, c.w, key, tp, [&](uint32_t hi, uint32_t lo) { return byte(b, hi, lo); });
+  };
+  auto push = [&](uint16_t *qu, int *n, bool on, int i) {
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    int base = 0;
+    if (lane == 0 && m) base = atomicAdd(n, __popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (on) qu[base + __popc(m & below)] = (uint16_t)i;
+  };
+  // i = 2 t + h: half h (0: the high one) of triple t
+#pragma unroll 1
+  for (int i0 = i00; i0 < 2 * ntrip; i0 += blockDim.x) {
+    const int i = i0 + lane;
+    uint32_t w = 0;
+    if (i < 2 * ntrip) {
+      w = word(i & 1, i >> 1);
+      i1[i ^ 1] = w;
+      i2[i ^ 1] = 0;
+    }
+    push(qa, cnt, w != 0, i);
+  }
+  __syncthreads();
+  const int n1 = cnt[0];
+#pragma unroll 1
+  for (int i0 = i00; i0 < n1; i0 += blockDim.x) {
+    const bool on = i0 + lane < n1;
+    const int i = on ? qa[i0 + lane] : 0;
+    uint32_t a = 0;
+    if (on) {
+      const uint32_t b0 = i1[i ^ 1];
+      a = b0 & word(2 + (i & 1), i >> 1);
+      i2[i ^ 1] = a;
+      i1[i ^ 1] = b0 ^ a;
+    }
+    push(qb, cnt + 1, a != 0, i);
+  }
+  __syncthreads();
+  const int n2 = cnt[1];
+#pragma unroll 1
+  for (int q = threadIdx.x; q < n2; q += blockDim.x) {
+    const int i = qb[q];
+    i1[i ^ 1] |= i2[i ^ 1] & word(4 + (i & 1), i >> 1);
+  }
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
 // Fused half-sweep.  A CTA owns KT half-sites of one parity.  It stages every
-// temperature's 8-bit pre-search (NB x 512 B) in SMEM -- the thresholds
+// temperature's pre-search in SMEM -- the thresholds
 // themselves, rarely needed past the pre-search, are read through the
-// read-only cache, which keeps a CTA's SMEM small -- generates the 3 random words
+// read-only cache, which keeps a CTA's SMEM small -- draws the random words
 // of each (beta, half-site, replica) once -- they are shared by all samples, as
 // the reference's random buffer has no sample axis (main.cu:1430) -- and then
 // updates every (sample, clone, half-site, replica) word of its tile, picking
-// the words of the clone's current temperature.  The random word indices
+// the words of the clone's current temperature.  What bounds it is the draws,
+// about half of a CTA's time.  Six words a thread one after another through an
+// 8-bit pre-search, a chain of threshold reads behind most of them, took 104 us
+// a half-sweep of the 24^2 x 192 tube (32 temperatures, 8 replicas, 31
+// samples), draw_ids and 11 bits take 93; 16^2 x 48 with 40 temperatures
+// 27 -> 21 us, 16^2 x 64 with 24 17.4 -> 13.1, 8^3 11.9 -> 9.6.
+// The random word indices
 // depend only on (beta, half-site, replica, counter), never on the launch
 // shape.  A tile of a job too small to fill the GPU is shared by nsplit CTAs,
 // each drawing the words and updating its share of the (sample, clone) pairs
-// (`part` of nsplit), and its draws are spread over all the CTA's threads.
+// (`part` of nsplit).
 // With energy = kEnergyAdd it also adds, per (sample, clone, replica),
 // the energy of the updated words (each bond has exactly one end on each
 // parity) to E, one atomic addition per tile (integers: the order does not
@@ -249,9 +328,12 @@ __device__ __forceinline__ void sweep_body(const JobDev &j, const uint4 *ctr, in
                                            unsigned char *smem, bool stage = true) {
   const int tile = blk / j.nsplit, part = blk - tile * j.nsplit;
   const int NB = j.NB, half = j.half;
-  u64 *s_rnd = reinterpret_cast<u64 *>(smem);
-  uint16_t *s_pre = reinterpret_cast<uint16_t *>(s_rnd + (UPDATE ? 3 * NB * KT * NR : 0));
-  int *s_nb = reinterpret_cast<int *>(s_pre + (UPDATE ? NB * 256 : 0));
+  const int ntrip = UPDATE ? NB * KT * NR : 0, stride = UPDATE ? (((1 << j.pre_bits) + 16) & ~15) : 0;
+  u64 *s_id1 = reinterpret_cast<u64 *>(smem), *s_id2 = s_id1 + ntrip;
+  uint16_t *s_queue = reinterpret_cast<uint16_t *>(s_id2 + ntrip);
+  uint8_t *s_pre = reinterpret_cast<uint8_t *>(s_queue + 4 * ntrip);
+  int *s_nb = reinterpret_cast<int *>(s_pre + (size_t)NB * stride);
+  __shared__ int s_cnt[2];
   const int k0 = tile * KT;
   const int tid = threadIdx.x, nth = blockDim.x;
 
@@ -260,7 +342,7 @@ __device__ __forceinline__ void sweep_body(const JobDev &j, const uint4 *ctr, in
   if (UPDATE && stage) {
     const uint4 *ps = reinterpret_cast<const uint4 *>(j.pre);
     uint4 *pd = reinterpret_cast<uint4 *>(s_pre);
-    for (int i = tid; i < NB * 32; i += nth) pd[i] = ps[i];
+    for (int i = tid; i < NB * (stride / 16); i += nth) pd[i] = ps[i];
   }
   if (tid < KT * 8) {
     const int kk = tid >> 3, f = tid & 7, k = k0 + kk;
@@ -271,35 +353,20 @@ __device__ __forceinline__ void sweep_body(const JobDev &j, const uint4 *ctr, in
   __syncthreads();
 
   if (UPDATE) {
-    const int ntrip = NB * KT * NR, plane = ntrip;
-    // words 2 q0 .. 2 q1 - 1 of triple t
-    auto draw = [&](int t, int q0, int q1) {
-      const int r = t % NR, kk = (t / NR) % KT, b = t / (NR * KT), k = k0 + kk;
-      if (k >= half) return;
-      const uint32_t tp = (uint32_t)((b * half + k) * NR + r);
-      const uint4 c = ctr[r];
-      const uint32_t key = j.keys[r];
-      const u64 *cum = j.cum + b * 256;
-      const uint16_t *pre = s_pre + b * 256;
-      const int o = (b * KT + kk) * NR + r;
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        if (q < q0 || q >= q1) continue;
-        const uint32_t hi = rnd_word<true>(c.x + 2 * q, c.y, c.z + tp, c.w, key, tp, cum, pre);
-        const uint32_t lo = rnd_word<true>(c.x + 2 * q + 1, c.y, c.z + tp, c.w, key, tp, cum, pre);
-        s_rnd[q * plane + o] = ((u64)hi << 32) | lo;
-      }
-    };
-    if (ntrip * 2 <= nth) {
-      // fewer triples than half the threads: a thread draws one 64-bit word
-      for (int t = tid; t < ntrip * 3; t += nth) {
-        const int q = t / ntrip;
-        draw(t - q * ntrip, q, q + 1);
-      }
-    } else {
-      for (int t = tid; t < ntrip; t += nth) draw(t, 0, 3);
-    }
-    __syncthreads();
+    draw_ids(
+        ntrip,
+        [&](int t, uint4 &c, uint32_t &key, uint32_t &tp, int &b) {
+          const int r = t % NR, kk = (t / NR) % KT, k = k0 + kk;
+          b = t / (NR * KT);
+          tp = (uint32_t)((b * half + k) * NR + r);
+          c = ctr[r];
+          key = j.keys[r];
+          return k < half;
+        },
+        [&](int b, uint32_t hi, uint32_t lo) {
+          return lut_byte_pre(hi, lo, j.cum + b * 256, s_pre + b * stride, 32 - j.pre_bits);
+        },
+        s_id1, s_id2, s_queue, s_cnt);
   }
 
   // Update phase.  Lanes form groups of G = KT*NR; a lane keeps its
@@ -345,8 +412,8 @@ __device__ __forceinline__ void sweep_body(const JobDev &j, const uint4 *ctr, in
       u64 fl = 0;
       if (UPDATE) {
         const int beta = j.wbtc[(s * NR + r) * NB + c];
-        const int o = (beta * KT + kk) * NR + r, plane = NB * KT * NR;
-        fl = flip_mask(f, s_rnd[o], s_rnd[plane + o], s_rnd[2 * plane + o]);
+        const int o = (beta * KT + kk) * NR + r;
+        fl = flip_mask_id(f, s_id1[o], s_id2[o]);
         *tgt = sv ^ fl;
       }
       if (energy == kEnergyAdd) {

@@ -1763,7 +1763,7 @@ int ea_sp_host_init(const ea_sp_geom *gp, uint64_t seed_J, uint64_t seed_u, uint
 int ea_sp_presearch11(const uint64_t *cum, uint8_t *pre) {
   if (!cum || !pre) return spfail(EA_ERR_ARG, "null argument");
   if (cum[255] != ~0ULL) return spfail(EA_ERR_ARG, "threshold 255 is not 2^64-1");
-  presearch11(cum, pre);
+  presearch(cum, 11, pre);
   return EA_OK;
 }
 
@@ -1940,7 +1940,7 @@ int ea_sp_set_temperatures(ea_sp *c, const double *betas, const uint64_t *cum) {
   for (int b = 0; b < NB; ++b) {
     if (cum[(size_t)b * 256 + 255] != ~0ULL) return spfail(EA_ERR_ARG, "threshold 255 of beta %d is not 2^64-1", b);
     presearch8(cum + (size_t)b * 256, pre.data() + (size_t)b * 256);
-    presearch11(cum + (size_t)b * 256, pre11.data() + (size_t)b * kPre11Stride);
+    presearch(cum + (size_t)b * 256, 11, pre11.data() + (size_t)b * kPre11Stride);
   }
   std::vector<double> tab;
   pt_exp_table(betas, NB, tab, c->expoff);
