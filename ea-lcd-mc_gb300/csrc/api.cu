@@ -491,6 +491,8 @@ int ea_get_spins(ea_ctx *c, int32_t s, uint64_t *even, uint64_t *odd) {
   const size_t n = c->g.words_per_parity();
   if (set_device(c)) return EA_ERR_CUDA;
   const unsigned long long *base = c->j.spins + (size_t)s * 2 * n;
+  prefault(even, n * 8);
+  prefault(odd, n * 8);
   CU(cudaMemcpyAsync(even, base, n * 8, cudaMemcpyDeviceToHost, c->st));
   CU(cudaMemcpyAsync(odd, base + n, n * 8, cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
@@ -841,6 +843,8 @@ int ea_run_bin(ea_ctx *c, const ea_cadence *cad, double *avgE, uint8_t *hist, in
   }
   if (maxit_trw) *maxit_trw = maxit;
   if (!avgE && !hist) return EA_OK;  // nothing to hand back: stay asynchronous
+  if (avgE) prefault(avgE, nsr * g.NB * 8);  // beside the bin's last cycles
+  if (hist) prefault(hist, nsr * maxit * g.NB);
   if (avgE) CU(cudaMemcpyAsync(avgE, c->avgE, nsr * g.NB * 8, cudaMemcpyDeviceToHost, c->st));
   if (hist) CU(cudaMemcpyAsync(hist, c->hist, nsr * maxit * g.NB, cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
@@ -1454,6 +1458,8 @@ int ea_bin_results(ea_ctx *c, double *avgE, uint8_t *hist, int32_t *maxit_trw) {
   const size_t nsr = (size_t)g.ns * g.NR;
   CU(cudaStreamSynchronize(c->st));
   const int maxit = c->j.maxit_trw;
+  if (avgE) prefault(avgE, nsr * g.NB * 8);
+  if (hist && c->hist) prefault(hist, nsr * maxit * g.NB);
   if (avgE) CU(cudaMemcpy(avgE, c->avgE, nsr * g.NB * 8, cudaMemcpyDeviceToHost));
   if (hist && c->hist) CU(cudaMemcpy(hist, c->hist, nsr * maxit * g.NB, cudaMemcpyDeviceToHost));
   if (maxit_trw) *maxit_trw = maxit;

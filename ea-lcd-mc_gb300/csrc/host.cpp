@@ -6,6 +6,10 @@
 // PROGRAM/src/med.c, PROGRAM/src/upd.c.
 #include "host.hpp"
 
+#include <sys/mman.h>
+#include <unistd.h>
+
+#include <cerrno>
 #include <cmath>
 #include <cstring>
 
@@ -302,6 +306,18 @@ void presearch8(const uint64_t *cum, uint16_t *pre) {
     const uint64_t lo = (uint64_t)b << 56, hi = lo | ((1ULL << 56) - 1);
     pre[b] = (uint16_t)(first_above(lo) | (first_above(hi) << 8));
   }
+}
+
+void prefault(void *p, size_t n) {
+#ifdef MADV_POPULATE_WRITE
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p & ~(page - 1);
+  if (!p || n < page) return;  // small results lie among the caller's other data
+  const int err = errno;
+  (void)madvise((void *)a, (uintptr_t)p + n - a, MADV_POPULATE_WRITE);
+  errno = err;
+#else
+  (void)p, (void)n;
+#endif
 }
 
 // The pre-search with 2^bits buckets: pre[t] = the first byte n with

@@ -2023,6 +2023,7 @@ int ea_sp_set_spins(ea_sp *c, const uint64_t *S) {
 int ea_sp_get_spins(ea_sp *c, uint64_t *S) {
   if (!c || !S) return spfail(EA_ERR_ARG, "null argument");
   SCU(cudaSetDevice(c->device));
+  prefault(S, (size_t)c->d.nw * c->d.V * c->d.NR * c->d.NB * 8);
   SCU(cudaMemcpyAsync(S, c->d.S, (size_t)c->d.nw * c->d.V * c->d.NR * c->d.NB * 8, cudaMemcpyDeviceToHost, c->st));
   SCU(cudaStreamSynchronize(c->st));
   return EA_OK;
@@ -2221,6 +2222,7 @@ int ea_sp_energy(ea_sp *c, int32_t *U2) {
   SCU(cudaSetDevice(c->device));
   SCU(sp_launch_energy(c->d, c->st));
   if (U2) {
+    prefault(U2, sizeof(int32_t) * (size_t)c->d.nw * 64 * c->d.NR * c->d.NB);
     SCU(cudaMemcpyAsync(U2, c->d.U2, sizeof(int32_t) * (size_t)c->d.nw * 64 * c->d.NR * c->d.NB,
                         cudaMemcpyDeviceToHost, c->st));
     SCU(cudaStreamSynchronize(c->st));
@@ -2247,6 +2249,10 @@ int ea_sp_get_tempering(ea_sp *c, int32_t *E, uint8_t *perm, uint32_t *acc, uint
   const SpDev &d = c->d;
   const size_t n = (size_t)d.nw * 64 * d.NR * d.NB;
   SCU(cudaSetDevice(c->device));
+  prefault(E, n * 4);
+  prefault(perm, n);
+  prefault(acc, (size_t)d.nw * 64 * d.NR * (d.NB - 1) * 4);
+  prefault(masks, (size_t)d.nw * d.NR * (d.NB - 1) * 8);
   if (E) SCU(cudaMemcpyAsync(E, d.E, n * 4, cudaMemcpyDeviceToHost, c->st));
   if (perm) SCU(cudaMemcpyAsync(perm, d.perm, n, cudaMemcpyDeviceToHost, c->st));
   if (acc) SCU(cudaMemcpyAsync(acc, d.acc, (size_t)d.nw * 64 * d.NR * (d.NB - 1) * 4, cudaMemcpyDeviceToHost, c->st));

@@ -21,6 +21,7 @@
 // per (sample, slot, distance).
 #include <cstdint>
 
+#include "host.hpp"
 #include "kernels_dev.cuh"
 #include "sp.cuh"
 
@@ -182,6 +183,7 @@ int ea_sp_plane_overlaps(ea_sp *job, int32_t nrep, int32_t *diff) {
     launch_plane_diff(d, npairs, dd, nullptr, st);
     e = cudaGetLastError();
   }
+  prefault(diff, n * 4);
   if (e == cudaSuccess) e = cudaMemcpyAsync(diff, dd, n * 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (dd) cudaFree(dd);
@@ -211,6 +213,7 @@ int ea_sp_plane_correlations(ea_sp *job, int32_t nrep, int32_t dmax, double *C) 
     k_sp_plane_corr<<<(unsigned)((size_t)d.nw * d.NB * 2 * ngrp), 256, 0, st>>>(d, npairs, dmax, dx, dc);
     e = cudaGetLastError();
   }
+  prefault(C, nc * 8);
   if (e == cudaSuccess) e = cudaMemcpyAsync(C, dc, nc * 8, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (dx) cudaFree(dx);
