@@ -1697,6 +1697,7 @@ struct ea_sp {
   SpDev d{};
   std::vector<void *> owned;
   std::vector<int32_t> expoff;
+  bool exp_falls = false;             // no pair's table rises
   double *exptab = nullptr;
   bool have_temps = false;
   // one iteration of the bin cadence, replayed as a CUDA graph
@@ -1719,7 +1720,8 @@ struct ea_sp {
   SpDev r_dev{};
   int r_state = 0;                    // 0: not planned, 1: eligible, 2: not eligible
   uint4 *r_ctrs = nullptr;
-  unsigned long long *r_R = nullptr, *r_X = nullptr;
+  unsigned long long *r_R = nullptr;
+  int32_t *r_X = nullptr;
   size_t r_cap_pass = 0, r_cap_sweep = 0, r_cap_pt = 0;
   bool pair_energy = false;           // see sp_pair_energy
 };
@@ -1958,7 +1960,12 @@ int ea_sp_set_temperatures(ea_sp *c, const double *betas, const uint64_t *cum) {
   SCU(cudaStreamSynchronize(c->st));
   c->d.exptab = c->exptab;
   c->have_temps = true;
-  c->r_state = 0;  // the resident plan stages the exp table: plan again
+  // the resident kernel's draws take the table's values to fall along each
+  // pair's energies, as exp does
+  c->exp_falls = true;
+  for (int i = 0; i + 1 < NB; ++i)
+    for (int k = c->expoff[i] + 1; k < c->expoff[i + 1]; ++k) c->exp_falls = c->exp_falls && tab[k] <= tab[k - 1];
+  c->r_state = 0;
   return EA_OK;
 }
 
@@ -2362,7 +2369,7 @@ static int sp_run_persist(ea_sp *c, const ea_cadence *cad) {
 
 static bool sp_res_ok(ea_sp *c) {
   if (c->r_state == 0 || std::memcmp(&c->r_dev, &c->d, sizeof(SpDev))) {
-    c->r_state = sp_res_plan(c->d, c->g.col_sites.data(), c->expoff.empty() ? 0 : c->expoff.back(), c->r_plan) ? 1 : 2;
+    c->r_state = c->exp_falls && sp_res_plan(c->d, c->g.col_sites.data(), c->r_plan) ? 1 : 2;
     c->r_dev = c->d;
   }
   return c->r_state == 1;
@@ -2379,7 +2386,7 @@ static int sp_run_resident(ea_sp *c, const ea_cadence *cad) {
   const SpDev &d = c->d;
   const SpResPlan &pl = c->r_plan;
   const int spi = cad->mesfr * cad->houfr * cad->ptfr;  // sweeps per iteration
-  const size_t words_sweep = (size_t)3 * d.V * d.NR * d.NB;
+  const size_t words_sweep = (size_t)2 * d.V * d.NR * d.NB;
   const size_t nsweep = sp_res_launch_sweeps(d.V, (size_t)d.NR * d.NB, cad), npass = nsweep * d.ncol;
   const int ipl = cad->cluster ? 1 : (int)(nsweep / spi);  // iterations per launch
   const size_t npt = nsweep / cad->ptfr;                    // tempering steps per launch
@@ -2389,11 +2396,12 @@ static int sp_run_resident(ea_sp *c, const ea_cadence *cad) {
     if (c->r_R) cudaFree(c->r_R);
     if (c->r_X) cudaFree(c->r_X);
     c->r_ctrs = nullptr;
-    c->r_R = c->r_X = nullptr;
+    c->r_R = nullptr;
+    c->r_X = nullptr;
     c->r_cap_pass = c->r_cap_sweep = c->r_cap_pt = 0;
     SCU(cudaMalloc((void **)&c->r_ctrs, sizeof(uint4) * npass * d.NR));
     SCU(cudaMalloc((void **)&c->r_R, 8 * words_sweep * nsweep));
-    SCU(cudaMalloc((void **)&c->r_X, 8 * npt * d.nw * d.NR * (d.NB - 1) * 64));
+    SCU(cudaMalloc((void **)&c->r_X, 4 * npt * d.nw * d.NR * (d.NB - 1) * 64));
     c->r_cap_pass = npass;
     c->r_cap_sweep = nsweep;
     c->r_cap_pt = npt;
@@ -2408,10 +2416,7 @@ static int sp_run_resident(ea_sp *c, const ea_cadence *cad) {
   p.ptfr = cad->ptfr;
   p.ncta = pl.ncta;
   p.nslm = pl.nslm;
-  p.upc = pl.upc;
-  p.ntab = pl.ntab;
-  p.lpc_count = pl.lpc_count;
-  p.lpc_energy = pl.lpc_energy;
+  p.parts = pl.parts;
   std::memcpy(p.kr, pl.kr, sizeof(p.kr));
   if (cad->cluster) {
     // per houfr block: one resident launch (sweeps and tempering steps, no
@@ -2863,11 +2868,11 @@ int ea_sp_job_bytes(const ea_sp_geom *gp, const ea_cadence *cad, const double *b
     }
   }
   if (cad && sp_res_fits(gp->L, gp->Lz, (int)nw, (int)NR, (int)NB)) {
-    // the resident kernel's counters, random words and tempering uniforms
+    // the resident kernel's counters, random words and tempering draws
     const uint64_t ns = sp_res_launch_sweeps(V, G, cad);
     add(ns * g.ncol * NR * 16);
-    add(ns * 24 * V * G);
-    if (cad->ptfr > 0) add(ns / cad->ptfr * nw * NR * (NB - 1) * 64 * 8);
+    add(ns * 16 * V * G);
+    if (cad->ptfr > 0) add(ns / cad->ptfr * nw * NR * (NB - 1) * 64 * 4);
   }
   *bytes = tot + (2ull << 20);                               // stream, graph, small-allocation pages
   return EA_OK;

@@ -147,34 +147,32 @@ struct SpPersistDev {
 int sp_persist_grid(const SpBatchDev &b, size_t smem);
 cudaError_t sp_launch_persist(const SpPersistDev &p, int grid, size_t smem, cudaStream_t st);
 
-// Resident bin kernel (sp_resident.cu): bins without cluster moves of a job
-// whose words fit in the shared memory of one thread-block cluster.  CTA c
-// of the cluster owns the sites [c*nslm, (c+1)*nslm); the random words of
-// the launch's sweeps are drawn beforehand by k_sp_draw.
+// Resident bin kernel (sp_resident.cu): bins of a job whose words would fit in
+// the shared memory of one thread-block cluster, a cluster for every unit
+// (word, replica).  CTA c of a cluster owns the sites [c*nslm, (c+1)*nslm); the
+// random words of the launch's sweeps are drawn beforehand by k_sp_draw.
 constexpr int kResMaxCta = 16;
 constexpr int kResMinBlock = 4;  // fewest sweeps between cluster moves for a resident launch to pay
 constexpr int kResMaxColours = 8;
 struct SpResDev {
   SpDev d;
-  const unsigned long long *R;  // [sweep][colour blocks: 3 planes x NR x NB x sites of the colour]
-  const unsigned long long *X;  // [tempering step][word x replica][pair][sample] FNORM * u as bits
+  const unsigned long long *R;  // [sweep][colour blocks: 2 planes x NR x NB x sites of the colour]
+  const int32_t *X;              // [tempering step][word x replica][pair][sample] draws (k_sp_pt_draw)
   int nit, nsweep, houfr, mesfr, ptfr;  // iterations and sweeps of this launch, the cadence
   int pair_energy;               // count the energy in the last colour pass (see ea_sp::pair_energy)
   int measure;                   // add the energies to the bin's sums after each iteration (no cluster moves)
-  int ncta, nslm, upc;           // CTAs, sites per CTA, tempering chains (word, replica) per CTA
-  int ntab;                      // exp table entries staged in SMEM (0: read from global memory)
-  int lpc_count, lpc_energy;     // lanes per column of the counts in the last pass / the energy phase (8, 16, 32)
+  int ncta, nslm;                // CTAs of a unit (word, replica), sites per CTA
+  int parts;                     // CTAs whose counts are kept apart (ncta, or 0: added up by atomics)
   int kr[kResMaxCta + 1][kResMaxColours];  // first index into colour k's site list of CTA c's sites
 };
 struct SpResPlan {
-  int ncta = 0, nslm = 0, upc = 0, ntab = 0, npl = 0, lpc_count = 32, lpc_energy = 32;
+  int ncta = 0, nslm = 0, parts = 0, npl = 0;
   size_t smem = 0;
   int kr[kResMaxCta + 1][kResMaxColours] = {};
 };
 // Fills `pl` and returns true when the job can run resident (colours, SMEM,
-// a co-resident cluster); col_sites: the host's colour-ordered site list,
-// ntab: entries of the job's exp table.
-bool sp_res_plan(const SpDev &d, const int32_t *col_sites, int ntab, SpResPlan &pl);
+// a co-resident cluster); col_sites: the host's colour-ordered site list.
+bool sp_res_plan(const SpDev &d, const int32_t *col_sites, SpResPlan &pl);
 bool sp_res_fits(int L, int Lz, int nw, int NR, int NB);  // the size test of sp_res_plan alone
 // Sweeps of random words one resident launch holds: whole iterations of the
 // cadence, up to 16 MB, at least one iteration; with cluster moves one block

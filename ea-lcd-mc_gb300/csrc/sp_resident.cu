@@ -2,23 +2,37 @@
 //
 // A job too small to fill the GPU spends a per-phase launch on every colour
 // pass, energy count, tempering step and permute, and each of those phases
-// is a short latency-bound chain.  For bins without cluster moves, a job
-// whose words fit in the shared memory of one thread-block cluster runs
-// instead as three launches per chunk of sweeps:
+// is a short latency-bound chain.  A job whose words fit in the shared memory
+// of one thread-block cluster runs instead as four launches per chunk of
+// sweeps (with cluster moves, per block of sweeps between two):
 //
 //   k_sp_ctr_chain  the Philox counters of every colour pass of the chunk: one
 //                   thread per replica steps its xoshiro256++ and
 //                   Parisi-Rapuano generators (the counters never depend on
 //                   the spins), the states staged in SMEM;
-//   k_sp_draw       the three random words of every (pass, site, replica,
-//                   slot) at once on the whole GPU -- the integer-heavy part
-//                   of a sweep, now fully parallel;
-//   k_sp_resident   one cluster of up to 16 CTAs holds the spin and coupling
-//                   words in distributed shared memory (CTA c owns a run of
-//                   sites) and runs every sweep, energy count, tempering
-//                   step, permute and measurement of the chunk, phases
-//                   separated by cluster barriers; neighbour words on other
-//                   CTAs are read through DSMEM.
+//   k_sp_draw       the random words of every (pass, site, replica, slot) at
+//                   once on the whole GPU -- the integer-heavy part of a
+//                   sweep, now fully parallel;
+//   k_sp_pt_draw    the tempering draws of every (step, pair, chain);
+//   k_sp_resident   a cluster of up to 16 CTAs for each unit -- a (word,
+//                   replica), whose chain of temperatures meets no other
+//                   between two moves -- holds its spin and coupling words in
+//                   distributed shared memory (CTA c owns a run of sites) and
+//                   runs every sweep, energy count, tempering step, permute
+//                   and measurement of the chunk, phases separated by cluster
+//                   barriers; neighbour words on other CTAs are read through
+//                   DSMEM.
+//
+// What bounds the resident kernel is latency.  A step (a sweep, a count, a
+// tempering step) of the 6^2 x 24 tube with 12 temperatures, 2 replicas and 64
+// samples takes 7 us: 3 cluster barriers of 1600 cycles, most of it the fence
+// of cluster scope, two colour passes of 1600, the count's sum and the stores
+// to the other CTAs 2700, the tempering walk 2800.  One cluster for the whole
+// job (three in four of its neighbour words on other CTAs), four barriers, a
+// tempering step in one CTA with a table look-up a pair and two items' code
+// unrolled side by side took 13.8 us (a bin of 64 steps with its draws 1011 us,
+// now 687); a bin of 32 sweeps and 4 moves of a 7^2 x 21 tube with 13
+// temperatures, 3 words and 3 replicas, 9 units, took 1952 us, now 955.
 //
 // Every phase computes what the per-phase kernels of sp.cu compute (same
 // random words, update rule, bit-sliced counts, FP64 tempering rule and
@@ -28,6 +42,7 @@
 
 #include <algorithm>
 
+#include "host.hpp"
 #include "kernels_dev.cuh"
 #include "sp.cuh"
 
@@ -36,6 +51,7 @@ namespace cg = cooperative_groups;
 namespace eagb {
 
 constexpr int kResThreads = 512;
+constexpr size_t kResSmem = 227 * 1024 - 256;  // dynamic, less the static part
 // bit planes of the per-sample counts summed over a warp: a CTA holds at most
 // (2^15 - 1) / 6 sites
 constexpr int kResPlanes = 15;
@@ -79,49 +95,71 @@ cudaError_t sp_batch_ctr_chain(const SpBatchDev &b, int nsweep, cudaStream_t st)
 }
 
 // ---------------------------------------------------------------------------
-// Random words of nsweep sweeps: one thread per (sweep, colour, site of the
-// colour, replica, slot), the words sp_pass_body draws for it (thresholds
-// through the read-only cache).  Per sweep the colours follow each other;
-// colour k's block holds 3 planes of NR * NB * n_k words, item (r, b, kk) at
-// (r * NB + b) * n_k + kk of each plane (the site fastest, as the resident
-// kernel's lanes read them).
+// Random words of nsweep sweeps: every (sweep, colour, site of the colour,
+// replica, slot) as the two words of its flip mask (draw_ids of the words
+// sp_pass_body draws; thresholds and pre-search through the read-only cache).
+// Per sweep the colours follow each other; colour k's block holds 2 planes of
+// NR * NB * n_k words, item (r, b, kk) at (r * NB + b) * n_k + kk of each plane
+// (the site fastest, as the resident kernel's lanes read them).  A CTA draws
+// kDrawItems of them.  (All six words of every item, an 8-bit pre-search and
+// three planes: 13 thousand items a us of the 6^2 x 24 tube, now 24.)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_sp_draw(const __grid_constant__ SpDev d, int nsweep, const uint4 *ctrs,
-                                                 u64 *R) {
-  const int NB = d.NB, NR = d.NR, G = NR * NB, V = d.V, ncol = d.ncol;
-  const long long per = (long long)V * G;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= per * nsweep) return;
-  const int s = (int)(t / per);
-  const int rem = (int)(t - (long long)s * per);
-  int k = 0;
-  while (k + 1 < ncol && rem >= d.col_off[k + 1] * G) ++k;
-  const int nk = d.col_off[k + 1] - d.col_off[k];
-  const int e = rem - d.col_off[k] * G;
-  const int col = e / nk, kk = e - col * nk, r = col / NB, b = col - r * NB;
-  const int site = __ldg(d.col_sites + d.col_off[k] + kk);
-  const uint4 c = ctrs[((size_t)s * ncol + k) * NR + r];
-  const uint32_t tp = (uint32_t)(((size_t)b * V + site) * NR + r);
-  const uint32_t key = __ldg(d.keys + r);
-  const u64 *cum = d.cum + b * 256;
-  const uint16_t *pre = d.pre + b * 256;
-  uint32_t w[6];
-#pragma unroll
-  for (int q = 0; q < 6; ++q) w[q] = rnd_word<true>(c.x + q, c.y, c.z + tp, c.w, key, tp, cum, pre);
-  u64 *Rs = R + (size_t)s * 3 * per + (size_t)3 * d.col_off[k] * G;
-  const size_t pl = (size_t)nk * G;
-  Rs[e] = ((u64)w[0] << 32) | w[1];
-  Rs[pl + e] = ((u64)w[2] << 32) | w[3];
-  Rs[2 * pl + e] = ((u64)w[4] << 32) | w[5];
+constexpr int kDrawItems = 768, kDrawThreads = 256;
+__global__ void __launch_bounds__(kDrawThreads) k_sp_draw(const __grid_constant__ SpDev d, int nsweep, const uint4 *ctrs,
+                                                          u64 *R) {
+  __shared__ u64 id1[kDrawItems], id2[kDrawItems];
+  __shared__ uint16_t queue[4 * kDrawItems];
+  __shared__ int cnt[2];
+  const int NB = d.NB, NR = d.NR, G = NR * NB, V = d.V, ncol = d.ncol, per = V * G;
+  const long long t0 = (long long)blockIdx.x * kDrawItems, left = (long long)per * nsweep - t0;
+  const int n = left < kDrawItems ? (int)left : kDrawItems, s0 = (int)(t0 / per), e0 = (int)(t0 - (long long)s0 * per);
+  // item t of the CTA: its sweep, colour and place e in the colour's block
+  auto place = [&](int t, int &s, int &k, int &nk, int &e) {
+    e = e0 + t;
+    s = s0;
+    while (e >= per) e -= per, ++s;
+    k = 0;
+    while (k + 1 < ncol && e >= d.col_off[k + 1] * G) ++k;
+    nk = d.col_off[k + 1] - d.col_off[k];
+    e -= d.col_off[k] * G;
+  };
+  draw_ids(
+      n,
+      [&](int t, uint4 &c, uint32_t &key, uint32_t &tp, int &b) {
+        int s, k, nk, e;
+        place(t, s, k, nk, e);
+        const int col = e / nk, r = col / NB, site = __ldg(d.col_sites + d.col_off[k] + e - col * nk);
+        b = col - r * NB;
+        c = ctrs[((size_t)s * ncol + k) * NR + r];
+        key = __ldg(d.keys + r);
+        tp = (uint32_t)(((size_t)b * V + site) * NR + r);
+        return true;
+      },
+      [&](int b, uint32_t hi, uint32_t lo) {
+        return lut_byte11(hi, lo, d.cum + b * 256, d.pre11 + (size_t)b * kPre11Stride);
+      },
+      id1, id2, queue, cnt);
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    int s, k, nk, e;
+    place(t, s, k, nk, e);
+    u64 *o = R + (size_t)s * 2 * per + (size_t)2 * d.col_off[k] * G + e;
+    o[0] = id1[t];
+    o[(size_t)nk * G] = id2[t];
+  }
 }
 
 // ---------------------------------------------------------------------------
-// Tempering uniforms of npt steps (sp_pt_body's draw): Philox4x32-10 of
-// (step, pair, chain) keyed by the tempering seed, as FNORM * u in FP64 (an
-// exact scaling of u rounded to 53 bits), stored as the double's bits.
+// Tempering draws of npt steps (sp_pt_body's): u of Philox4x32-10 of (step,
+// pair, chain) keyed by the tempering seed, x = FNORM * u in FP64 (an exact
+// scaling of u rounded to 53 bits), and from it the largest m = -dE / 2 the
+// pair's exchange is still accepted at: the table's exp(pt(m)), m = 1, 2, ...,
+// decrease (sp_res_ok), so x < exp(pt(m)) holds up to some m.  INT_MAX: at
+// every m (x = 0, or betas that are equal); INT_MIN: at none (betas the other
+// way round).  Off the resident kernel's serial chain, where a look-up of the
+// table a pair took 510 cycles with all around it.
 // X: [step][word x replica][pair][sample].
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_sp_pt_uniforms(const __grid_constant__ SpDev d, int npt, u64 *X) {
+__global__ void __launch_bounds__(256) k_sp_pt_draw(const __grid_constant__ SpDev d, int npt, int32_t *X) {
   const int NR = d.NR, NP = d.NB - 1, nunits = d.nw * NR;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)npt * nunits * NP * 64) return;
@@ -136,128 +174,210 @@ __global__ void __launch_bounds__(256) k_sp_pt_uniforms(const __grid_constant__ 
   uint32_t v0 = (uint32_t)step, v1 = (uint32_t)(step >> 32), v2 = (uint32_t)pi, v3 = chain;
   philox10(v0, v1, v2, v3, (uint32_t)d.pt_seed, (uint32_t)(d.pt_seed >> 32));
   const double FNORM = 5.4210108624275218e-20;
-  X[t] = (u64)__double_as_longlong(__dmul_rn(FNORM, __ull2double_rn(((u64)v0 << 32) | v1)));
+  const double x = __dmul_rn(FNORM, __ull2double_rn(((u64)v0 << 32) | v1));
+  const double f = -__dsub_rn(d.betas[pi + 1], d.betas[pi]);
+  int m = 0x7FFFFFFF;
+  if (x != 0.0 && f != 0.0) {
+    if (f < 0.0) m = (int)0x80000000;
+    else {
+      const double *tab = d.exptab + d.expoff[pi];
+      int lo = 0, hi = d.expoff[pi + 1] - d.expoff[pi];
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (x < __ldg(tab + mid)) lo = mid + 1; else hi = mid;
+      }
+      m = lo;
+    }
+  }
+  X[t] = m;
 }
 
 // ---------------------------------------------------------------------------
-// The resident kernel's phases.  Site i of the lattice lives in CTA i / nslm
-// at local index i % nslm.  SMEM arrays keep the site (or the sample) as the
-// fastest index, so that the lanes of a warp -- consecutive sites of one
-// (replica, slot) column, or consecutive samples of one chain -- touch
-// consecutive words:
-//   S   [nw][NR*NB][nslm]  spin words         J    [nw][6][nslm] coupling words
-//   nbl [6][nslm]          neighbour of each bond slot as (CTA << 16 | local index)
-//   lst [nsl]              the CTA's sites, colour by colour
-// and per chain (unit u = (word, replica) = lu * ncta + rank, 64 samples):
-//   U2s, Es, Av, Ps [upc][NB][64]    As [upc][NB-1][64]    Ms [upc][NB-1]
+// The resident kernel's phases, of one chain of temperatures (unit = (word,
+// replica)) in a cluster.  Site i of the lattice lives in CTA i / nslm at local
+// index i % nslm.  SMEM arrays keep the site (or the sample) as the fastest
+// index, so that the lanes of a warp -- consecutive sites of one slot, or
+// consecutive samples -- touch consecutive words:
+//   S   [NB][nslm]  spin words                J    [6][nslm] coupling words
+//   nbl [6][nslm]   SMEM address of each bond slot's neighbour in slot 0, mapped
+//                   into its CTA, bit 0 set if that is another one
+//   lst [nsl]       the CTA's sites, colour by colour
+//   Pt  [ncta][NB][64]  every CTA's counts of its sites
+// and the unit's tempering state, the same in every CTA:
+//   U2s, Es, Av, Ps [NB][64]    As, Xs [NB-1][64]    Ms [NB-1]
 // ---------------------------------------------------------------------------
 struct ResCta {
-  int rank, site_lo, nsl;
+  int rank, unit, w, r, site_lo, nsl;
 };
 
 struct ResShared {
+  int32_t *Xs;   // the step's draws (k_sp_pt_draw)
+  uint16_t *Pt;
   u64 *S, *J;
   u64 *Ms;       // lanes that swapped, per pair
-  u64 *Mall;     // [nunits][NB-1] every chain's masks, gathered for the permute
   long long *Av; // the bin's energy sums (integers: exactly the double sums, all below 2^53)
-  u64 *Tab;      // [ntab] host-libm exp table as bits (when staged)
-  int32_t *U2s;  // counts of the whole lattice (DSMEM atomics of every CTA)
+  int32_t *U2s;  // counts of the whole lattice
   int32_t *Es;
   uint32_t *As;
   uint32_t *nbl;
-  int32_t *EO;   // [NB] exp table offsets
   int32_t *SG;   // [NB-1] sign of -(beta[i+1] - beta[i])
   uint16_t *lst;
   uint8_t *Ps;
-  u64 *Xs;       // [upc][NB-1][64] tempering uniforms of the step
 };
 
-__host__ __device__ inline size_t res_smem_bytes(int nw, int nslm, int NR, int NB, int upc, int ntab) {
-  const size_t G = (size_t)NR * NB, NP = NB - 1, nunits = (size_t)nw * NR, U = (size_t)upc * 64;
-  const size_t b = 8 * ((size_t)nw * nslm * G + (size_t)nw * nslm * 6 + upc * NP + nunits * NP + U * NB + (size_t)ntab +
-                        U * NP) +
-                   4 * (2 * U * NB + U * NP + (size_t)nslm * 6 + NB + NP) + 2 * (size_t)nslm + U * NB;
+// parts: CTAs that leave their counts in Pt (0: added to U2s by atomics, for
+// ladders whose Pt would not fit)
+__host__ __device__ inline size_t res_smem_bytes(int nslm, int NB, int parts) {
+  const size_t NP = NB - 1;
+  const size_t b = 8 * ((size_t)nslm * NB + (size_t)nslm * 6 + NP + 64 * NB) +
+                   4 * (2 * 64 * NB + 2 * 64 * NP + (size_t)nslm * 6 + NP) + 2 * ((size_t)nslm + parts * 64 * NB) + 64 * NB;
   return (b + 15) & ~(size_t)15;
 }
 
 __device__ __forceinline__ ResShared res_carve(unsigned char *smem, const SpResDev &p) {
-  const SpDev &d = p.d;
-  const size_t G = (size_t)d.NR * d.NB, NP = d.NB - 1, nunits = (size_t)d.nw * d.NR, U = (size_t)p.upc * 64;
+  const size_t NB = p.d.NB, NP = NB - 1;
   ResShared s;
-  s.S = reinterpret_cast<u64 *>(smem);
-  s.J = s.S + (size_t)d.nw * p.nslm * G;
-  s.Ms = s.J + (size_t)d.nw * p.nslm * 6;
-  s.Mall = s.Ms + (size_t)p.upc * NP;
-  s.Xs = s.Mall + nunits * NP;
-  s.Av = reinterpret_cast<long long *>(s.Xs + U * NP);
-  s.Tab = reinterpret_cast<u64 *>(s.Av + U * d.NB);
-  s.U2s = reinterpret_cast<int32_t *>(s.Tab + p.ntab);
-  s.Es = s.U2s + U * d.NB;
-  s.As = reinterpret_cast<uint32_t *>(s.Es + U * d.NB);
-  s.nbl = s.As + U * NP;
-  s.EO = reinterpret_cast<int32_t *>(s.nbl + (size_t)p.nslm * 6);
-  s.SG = s.EO + d.NB;
+  s.Xs = reinterpret_cast<int32_t *>(smem);
+  s.Pt = reinterpret_cast<uint16_t *>(s.Xs + 64 * NP);
+  s.S = reinterpret_cast<u64 *>(s.Pt + p.parts * 64 * NB);
+  s.J = s.S + p.nslm * NB;
+  s.Ms = s.J + (size_t)p.nslm * 6;
+  s.Av = reinterpret_cast<long long *>(s.Ms + NP);
+  s.U2s = reinterpret_cast<int32_t *>(s.Av + 64 * NB);
+  s.Es = s.U2s + 64 * NB;
+  s.As = reinterpret_cast<uint32_t *>(s.Es + 64 * NB);
+  s.nbl = s.As + 64 * NP;
+  s.SG = reinterpret_cast<int32_t *>(s.nbl + (size_t)p.nslm * 6);
   s.lst = reinterpret_cast<uint16_t *>(s.SG + NP);
   s.Ps = reinterpret_cast<uint8_t *>(s.lst + p.nslm);
   return s;
 }
 
-// The word of column Sc (this CTA's copy of a (word, column) row of S) at the
-// site packed in nb, from this CTA or another one of the cluster.
-__device__ __forceinline__ u64 res_word(const cg::cluster_group &cl, const ResCta &me, u64 *Sc, uint32_t nb) {
-  const int own = (int)(nb >> 16), nl = (int)(nb & 0xFFFFu);
-  return own == me.rank ? Sc[nl] : cl.map_shared_rank(Sc, own)[nl];
+// Cluster barrier in two halves.  The release is one warp's, behind a barrier
+// of the CTA that orders the other warps' writes before it: a fence of cluster
+// scope by each of 16 warps took 1750 cycles, by one 1600, and the others are
+// free meanwhile.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncthreads();
+  if (threadIdx.x < 32) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Addresses in the cluster's shared memory.
+__device__ __forceinline__ uint32_t smem_addr(const void *q) { return (uint32_t)__cvta_generic_to_shared(q); }
+__device__ __forceinline__ uint32_t mapa(uint32_t a, int rank) {
+  uint32_t o;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(rank));
+  return o;
+}
+// The neighbour word a (an nbl entry) of the column `off` bytes behind column
+// 0: one of two predicated loads, so that a site's six are in flight together
+// (branches between them took one round trip after another).
+__device__ __forceinline__ u64 res_word(uint32_t a, uint32_t off) {
+  u64 v;
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p ld.shared::cluster.u64 %0, [%1];\n@!p ld.shared.u64 %0, [%1];\n}"
+      : "=l"(v)
+      : "r"((a & ~7u) + off), "r"(a & 1u)
+      : "memory");
+  return v;
 }
 
-// One colour pass over the CTA's sites of colour k (sp_pass_body's update):
-// a group of lpc lanes per (word, column), lanes over the colour's sites.
-__device__ __forceinline__ void res_pass(const SpResDev &p, const cg::cluster_group &cl, const ResCta &me,
-                                         const ResShared &s, int sweep, int k) {
-  const SpDev &d = p.d;
-  const int G = d.NR * d.NB, nslm = p.nslm;
-  const int off = d.col_off[k], nk = d.col_off[k + 1] - off;
-  const int kb = p.kr[me.rank][k], nkc = p.kr[me.rank + 1][k] - kb;
-  if (nkc <= 0) return;
-  int loff = 0;
-  for (int c = 0; c < k; ++c) loff += p.kr[me.rank + 1][c] - p.kr[me.rank][c];
-  const u64 *Rk = p.R + (size_t)sweep * 3 * d.V * G + (size_t)3 * off * G + kb;
-  const size_t pl = (size_t)nk * G;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int lpc = p.lpc_count, cpw = 32 / lpc, gl = lane & (lpc - 1), ncols = d.nw * G;
-  for (int c = warp * cpw + lane / lpc; c < ncols; c += nwarp * cpw) {
-    const int w = c / G, col = c - w * G;
-    u64 *Sc = s.S + (size_t)c * nslm;
-    const u64 *Jw = s.J + (size_t)w * 6 * nslm;
-    const u64 *Rc = Rk + (size_t)col * nk;
-    for (int kl = gl; kl < nkc; kl += lpc) {
-      const int local = s.lst[loff + kl];
-      const u64 r0 = __ldg(Rc + kl), r1 = __ldg(Rc + pl + kl), r2 = __ldg(Rc + 2 * pl + kl);
-      const u64 sv = Sc[local];
-      u64 f[6];
+// A colour's share of the CTA: the colour's sites, the CTA's of them, the
+// first of those in the colour's list and in lst.
+struct ResColour {
+  int nk, nkc, kb, loff;
+  uint32_t mul;  // ceil(2^32 / nkc): i / nkc = umulhi(i, mul) for the items' i, i nkc < 2^32 (SMEM bounds i)
+};
+__device__ __forceinline__ int res_slot(const ResColour &q, int i) {
+  return q.nkc == 1 ? i : (int)__umulhi((uint32_t)i, q.mul);
+}
+// The random words of item (slot b, site kl) of a colour pass: planes pl apart.
+struct ResPass {
+  const u64 *R;
+  size_t pl;
+};
+__device__ __forceinline__ ResPass res_pass_at(const SpResDev &p, const ResCta &me, const ResColour &q, int sweep, int k) {
+  const size_t G = (size_t)p.d.NR * p.d.NB;
+  return {p.R + ((size_t)sweep * p.d.V + p.d.col_off[k]) * 2 * G + (size_t)me.r * p.d.NB * q.nk + q.kb, q.nk * G};
+}
+__device__ __forceinline__ void res_fetch(const ResPass &a, const ResColour &q, int b, int kl, bool on, u64 r[2]) {
+  if (!on) return;
+  const u64 *g = a.R + b * q.nk + kl;
+  r[0] = __ldg(g);
+  r[1] = __ldg(g + a.pl);
+}
+// Whether the energy is counted in pass k of sweep sw of a tempering step.
+__device__ __forceinline__ bool res_counts(const SpResDev &p, int sw, int k) {
+  return p.pair_energy && k == p.d.ncol - 1 && sw == p.ptfr - 1;
+}
+// The random words of a thread's first item of a pass, read while the barrier
+// before it is waited for (the read from L2 is about as long as the rest of a
+// pass of a small job).  A pass that counts has a warp per slot, lanes over the
+// colour's sites, the others their (slot, site) items over all threads.
+__device__ __forceinline__ void res_prefetch(const SpResDev &p, const ResCta &me, const ResColour *col, int sweep, int k,
+                                             bool counts, u64 r[2]) {
+  if (sweep >= p.nsweep) return;
+  const ResColour q = col[k];
+  if (q.nkc <= 0) return;
+  const int b = counts ? (int)threadIdx.x >> 5 : res_slot(q, threadIdx.x);
+  const int kl = counts ? (int)threadIdx.x & 31 : (int)threadIdx.x - b * q.nkc;
+  res_fetch(res_pass_at(p, me, q, sweep, k), q, b, kl, b < p.d.NB && kl < q.nkc, r);
+}
+
+// sv ^ J ^ neighbour of the six bond slots of a site (sp_pass_body's f).
+__device__ __forceinline__ void res_bonds(const SpResDev &p, const ResShared &s, int b, int local, u64 sv, u64 f[6]) {
+  const int nslm = p.nslm;
+  const u64 *J = s.J + local;
+  const uint32_t off = (uint32_t)(b * nslm) * 8u;
 #pragma unroll
-      for (int q = 0; q < 6; ++q) f[q] = sv ^ Jw[(size_t)q * nslm + local] ^ res_word(cl, me, Sc, s.nbl[q * nslm + local]);
-      Sc[local] = sv ^ flip_mask(f, r0, r1, r2);
-    }
+  for (int q = 0; q < 6; ++q) f[q] = res_word(s.nbl[q * nslm + local], off);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) f[q] ^= sv ^ J[q * nslm];
+}
+
+// One colour pass over the CTA's sites of colour k (sp_pass_body's update), the
+// random words of a thread's first item in r, the next one's read before an
+// item is worked on.
+__device__ __forceinline__ void res_pass(const SpResDev &p, const ResCta &me, const ResShared &s, const ResColour &q,
+                                         int sweep, int k, u64 r[2]) {
+  if (q.nkc <= 0) return;
+  const ResPass a = res_pass_at(p, me, q, sweep, k);
+  const int n = p.d.NB * q.nkc, nth = blockDim.x;
+  int i = threadIdx.x, b = res_slot(q, i), kl = i - b * q.nkc;
+#pragma unroll 1
+  while (i < n) {
+    const int ni = i + nth, nb = res_slot(q, ni), nkl = ni - nb * q.nkc;
+    u64 x[2] = {0, 0}, f[6];
+    res_fetch(a, q, nb, nkl, ni < n, x);
+    const int local = s.lst[q.loff + kl];
+    u64 *S = s.S + b * p.nslm + local;
+    const u64 sv = *S;
+    res_bonds(p, s, b, local, sv, f);
+    *S = sv ^ flip_mask_id(f, r[0], r[1]);
+    i = ni;
+    b = nb;
+    kl = nkl;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) r[j] = x[j];
   }
 }
 
-// Asynchronous 8-byte global-to-SMEM copies (cp.async); a thread waits for
+// Asynchronous 16-byte global-to-SMEM copies (cp.async); a thread waits for
 // all of its copies with cp_async_wait_all (a hardware wait) before the
 // barrier that publishes them.
-__device__ __forceinline__ void cp_async8(void *smem, const void *g) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sa), "l"(g) : "memory");
+__device__ __forceinline__ void cp_async16(void *smem, const void *g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(smem)), "l"(g) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Tempering uniforms of this CTA's chains for step ptj into Xs.
+// Draws of the unit for tempering step ptj into Xs.
 __device__ __forceinline__ void res_stage_x(const SpResDev &p, const ResCta &me, const ResShared &s, int ptj) {
-  const int NP = p.d.NB - 1, nunits = p.d.nw * p.d.NR, per = NP * 64;
-  for (int t = threadIdx.x; t < p.upc * per; t += blockDim.x) {
-    const int lu = t / per, e = t - lu * per, u = lu * p.ncta + me.rank;
-    if (u < nunits) cp_async8(s.Xs + t, p.X + ((size_t)ptj * nunits + u) * per + e);
-  }
+  const int NP = p.d.NB - 1;
+  const int32_t *g = p.X + ((size_t)ptj * p.d.nw * p.d.NR + me.unit) * NP * 64;
+  for (int t = threadIdx.x; t < NP * 16; t += blockDim.x) cp_async16(s.Xs + 4 * t, g + 4 * t);
   cp_async_commit();
 }
 
@@ -282,36 +402,55 @@ __device__ __forceinline__ void res_count_add(u64 *P, int npl, const u64 f[6]) {
   }
 }
 
-// A group of lpc lanes (8, 16 or 32; one (word, column) per group, lpc | 32)
-// sums its bit-sliced counters (a butterfly of bit-sliced additions inside
-// the group); then lane l of the group holds samples l, l + lpc, ... of the
-// sum and adds them, times `scale`, to the counts of the chain (word,
-// replica r) at slot b in the CTA that owns the chain (DSMEM atomics).
-// Every lane of the warp takes part in the shuffles; `valid` lanes add.
+// A warp (one slot) sums its bit-sliced counters: in each round a lane keeps
+// half of its samples and gives the other half's planes to its partner, so that
+// lane l ends with samples 2 l and 2 l + 1.  Their counts go into this CTA's
+// part of every CTA's Pt, or are added to its U2s.  (Loops kept rolled: the kernel runs through all its
+// code once a step, and what is unrolled comes from the instruction cache
+// again each time.)
 template <int NPL>
-__device__ __forceinline__ void res_count_flush(const SpResDev &p, const cg::cluster_group &cl, const ResCta &me,
-                                                const ResShared &s, u64 *P, int lpc, bool valid, int w, int r, int b,
-                                                int scale) {
-  const int gl = threadIdx.x & (lpc - 1), NB = p.d.NB;
-  for (int m = lpc >> 1; m >= 1; m >>= 1) {
-    u64 cy = 0;
+__device__ __forceinline__ void res_count_flush(const SpResDev &p, const ResCta &me, const ResShared &s, const u64 *P,
+                                                int b, int scale) {
+  const int lane = threadIdx.x & 31;
+  uint32_t H[NPL];
+  {
+    const bool up = lane & 16;
+    uint32_t cy = 0;
 #pragma unroll
     for (int q = 0; q < NPL; ++q) {
-      const u64 o = __shfl_xor_sync(0xffffffffu, P[q], m);
-      const u64 t = P[q] ^ o ^ cy;
-      cy = (P[q] & o) | (cy & (P[q] ^ o));
-      P[q] = t;
+      const uint32_t lo = (uint32_t)P[q], hi = (uint32_t)(P[q] >> 32), a = up ? hi : lo;
+      const uint32_t o = __shfl_xor_sync(0xffffffffu, up ? lo : hi, 16);
+      H[q] = a ^ o ^ cy;
+      cy = (a & o) | (cy & (a ^ o));
     }
   }
-  if (!valid) return;
-  const int u = w * p.d.NR + r, own = u % p.ncta, lu = u / p.ncta;
-  int32_t *dst = (own == me.rank ? s.U2s : cl.map_shared_rank(s.U2s, own)) + ((size_t)lu * NB + b) * 64;
-  for (int smp = gl; smp < 64; smp += lpc) {
-    int c = 0;
+#pragma unroll 1
+  for (int m = 8; m >= 1; m >>= 1) {  // 2 m samples kept; the bits above them are no longer used
+    const int keep = lane & m ? 2 * m : 0, give = 2 * m - keep;
+    uint32_t cy = 0;
 #pragma unroll
-    for (int q = 0; q < NPL; ++q) c |= (int)((P[q] >> smp) & 1ull) << q;
-    atomicAdd(dst + smp, scale * c);
+    for (int q = 0; q < NPL; ++q) {
+      const uint32_t a = H[q] >> keep, o = __shfl_xor_sync(0xffffffffu, H[q] >> give, m);
+      H[q] = a ^ o ^ cy;
+      cy = (a & o) | (cy & (a ^ o));
+    }
   }
+  uint32_t v = 0;
+#pragma unroll
+  for (int q = 0; q < NPL; ++q) v |= ((H[q] & 1u) | (H[q] & 2u) << 15) << q;
+  if (!p.parts) {
+    const uint32_t to = smem_addr(s.U2s + b * 64 + 2 * lane);
+    for (int c = 0; c < p.ncta; ++c)
+      for (int j = 0; j < 2; ++j)
+        asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(mapa(to + 4 * j, c)),
+                     "r"(scale * (j ? v >> 16 : v & 0xFFFFu))
+                     : "memory");
+    return;
+  }
+  const uint32_t own = smem_addr(s.Pt + ((size_t)me.rank * p.d.NB + b) * 64 + 2 * lane);
+#pragma unroll 2
+  for (int c = 0; c < p.ncta; ++c)
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa(own, c)), "r"(v) : "memory");
 }
 
 // The last colour pass of a sweep on a two-colour lattice with the energy
@@ -321,184 +460,171 @@ __device__ __forceinline__ void res_count_flush(const SpResDev &p, const cg::clu
 // once their pass has flipped them (f ^= flip).  A warp per (word, column),
 // lanes over the colour's sites.
 template <int NPL>
-__device__ __forceinline__ void res_pass_count(const SpResDev &p, const cg::cluster_group &cl, const ResCta &me,
-                                               const ResShared &s, int sweep, int k) {
-  const SpDev &d = p.d;
-  const int NB = d.NB, G = d.NR * NB, nslm = p.nslm;
-  const int off = d.col_off[k], nk = d.col_off[k + 1] - off;
-  const int kb = p.kr[me.rank][k], nkc = p.kr[me.rank + 1][k] - kb;
-  int loff = 0;
-  for (int c = 0; c < k; ++c) loff += p.kr[me.rank + 1][c] - p.kr[me.rank][c];
-  const u64 *Rk = p.R + (size_t)sweep * 3 * d.V * G + (size_t)3 * off * G + kb;
-  const size_t pl = (size_t)nk * G;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int lpc = p.lpc_count, cpw = 32 / lpc, gl = lane & (lpc - 1), ncols = d.nw * G;
-  for (int base = warp * cpw; base < ncols; base += nwarp * cpw) {
-    const int c = base + lane / lpc;
-    const bool valid = c < ncols;
-    const int cc = valid ? c : 0, w = cc / G, col = cc - w * G, r = col / NB, b = col - r * NB;
-    u64 *Sc = s.S + (size_t)cc * nslm;
-    const u64 *Jw = s.J + (size_t)w * 6 * nslm;
-    const u64 *Rc = Rk + (size_t)col * nk;
+__device__ __forceinline__ void res_pass_count(const SpResDev &p, const ResCta &me, const ResShared &s,
+                                               const ResColour &q, int sweep, int k, u64 r[2]) {
+  const ResPass a = res_pass_at(p, me, q, sweep, k);
+  const int NB = p.d.NB, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+#pragma unroll 1
+  for (int b = threadIdx.x >> 5; b < NB; b += nwarp) {
     u64 P[NPL];
 #pragma unroll
-    for (int q = 0; q < NPL; ++q) P[q] = 0;
-    for (int kl = gl; valid && kl < nkc; kl += lpc) {
-      const int local = s.lst[loff + kl];
-      const u64 r0 = __ldg(Rc + kl), r1 = __ldg(Rc + pl + kl), r2 = __ldg(Rc + 2 * pl + kl);
-      const u64 sv = Sc[local];
-      u64 f[6];
+    for (int j = 0; j < NPL; ++j) P[j] = 0;
+#pragma unroll 1
+    for (int kl = lane; kl < q.nkc; kl += 32) {
+      u64 x[2] = {0, 0}, f[6];
+      res_fetch(a, q, b, kl + 32, kl + 32 < q.nkc, x);
+      const int local = s.lst[q.loff + kl];
+      u64 *S = s.S + b * p.nslm + local;
+      const u64 sv = *S;
+      res_bonds(p, s, b, local, sv, f);
+      const u64 m = flip_mask_id(f, r[0], r[1]);
+      *S = sv ^ m;
 #pragma unroll
-      for (int q = 0; q < 6; ++q) f[q] = sv ^ Jw[(size_t)q * nslm + local] ^ res_word(cl, me, Sc, s.nbl[q * nslm + local]);
-      const u64 m = flip_mask(f, r0, r1, r2);
-      Sc[local] = sv ^ m;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) f[q] ^= m;
+      for (int e = 0; e < 6; ++e) f[e] ^= m;
       res_count_add(P, NPL, f);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) r[j] = x[j];
     }
-    res_count_flush<NPL>(p, cl, me, s, P, lpc, valid, w, r, b, 2);
+    res_fetch(a, q, b + nwarp, lane, b + nwarp < NB && lane < q.nkc, r);
+    res_count_flush<NPL>(p, me, s, P, b, 2);
   }
 }
 
-// Unsatisfied half-edges per (word, sample, replica, slot) (sp_energy_body's
-// count): a warp per (word, column) of the CTA, lanes over its sites,
-// bit-sliced counters summed over the warp by a butterfly of bit-sliced
-// additions; lane l then holds samples l and l + 32 and adds them to the
-// chain's counts in the CTA that owns the chain (DSMEM atomics).
+// Unsatisfied half-edges per (sample, slot) of the CTA's sites
+// (sp_energy_body's count).
 template <int NPL>
-__device__ __forceinline__ void res_energy(const SpResDev &p, const cg::cluster_group &cl, const ResCta &me,
-                                           const ResShared &s) {
-  const SpDev &d = p.d;
-  const int NB = d.NB, G = d.NR * NB, nslm = p.nslm;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int lpc = p.lpc_energy, cpw = 32 / lpc, gl = lane & (lpc - 1), ncols = d.nw * G;
-  for (int base = warp * cpw; base < ncols; base += nwarp * cpw) {
-    const int c = base + lane / lpc;
-    const bool valid = c < ncols;
-    const int cc = valid ? c : 0, w = cc / G, col = cc - w * G, r = col / NB, b = col - r * NB;
-    u64 *Sc = s.S + (size_t)cc * nslm;
-    const u64 *Jw = s.J + (size_t)w * 6 * nslm;
+__device__ __forceinline__ void res_energy(const SpResDev &p, const ResCta &me, const ResShared &s) {
+  const int NB = p.d.NB, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+#pragma unroll 1
+  for (int b = threadIdx.x >> 5; b < NB; b += nwarp) {
     u64 P[NPL];
 #pragma unroll
     for (int q = 0; q < NPL; ++q) P[q] = 0;
-    for (int i = gl; valid && i < me.nsl; i += lpc) {
-      const u64 sv = Sc[i];
+#pragma unroll 1
+    for (int i = lane; i < me.nsl; i += 32) {
       u64 f[6];
-#pragma unroll
-      for (int q = 0; q < 6; ++q) f[q] = sv ^ Jw[(size_t)q * nslm + i] ^ res_word(cl, me, Sc, s.nbl[q * nslm + i]);
+      res_bonds(p, s, b, i, s.S[b * p.nslm + i], f);
       res_count_add(P, NPL, f);
     }
-    res_count_flush<NPL>(p, cl, me, s, P, lpc, valid, w, r, b, 1);
+    res_count_flush<NPL>(p, me, s, P, b, 1);
   }
 }
 
-// One tempering step of the CTA's chains (sp_pt_body's rule and uniforms).
-// pt = -(beta[i+1] - beta[i]) * dE is >= 0 exactly when dE has the sign of
-// -(beta[i+1] - beta[i]) (or that factor is zero), so the walk needs no FP64:
-// FNORM * u is formed beforehand for every pair, and both it and the table's
-// exp values are non-negative doubles, which order as their bit patterns.
-// With `measure`, the slots' energies are added to the bin's sums
-// (sp_measure_u2_body after a tempering step).  The chains' counts are then
-// cleared for the next energy phase.
-__device__ __forceinline__ void res_tempering(const SpResDev &p, const ResCta &me, const ResShared &s, int ptj,
-                                              bool measure, bool last) {
+// One tempering step of the unit (sp_pt_body's rule and draws), by every CTA
+// for itself: what it costs is one chain of NB - 1 decisions, and another
+// CTA's would be a barrier away.  The counts are first summed from the CTAs'
+// parts.  pt = -(beta[i+1] - beta[i]) * dE is >= 0 exactly when dE has the
+// sign of -(beta[i+1] - beta[i]) (or that factor is zero); below, the exchange
+// is accepted up to the m = -dE / 2 that k_sp_pt_draw found.  The walk finds the
+// lanes that swap and nothing more; res_permute applies them.  `last`: the
+// counts are handed back.
+__device__ __forceinline__ void res_tempering(const SpResDev &p, const ResCta &me, const ResShared &s, bool last) {
   const SpDev &d = p.d;
-  const int NB = d.NB, NR = d.NR, G = NR * NB, NP = NB - 1, nunits = d.nw * NR, upc = p.upc, ncta = p.ncta;
-  const int nt = 3 * d.V;
-  for (int lu = threadIdx.x >> 6; lu < upc; lu += blockDim.x >> 6) {
-    const int u = lu * ncta + me.rank;
-    if (u >= nunits) continue;  // the same for the unit's 64 threads
-    const int lane = threadIdx.x & 63;
-    int32_t *Eo = s.Es + (size_t)lu * NB * 64 + lane;
-    uint8_t *Po = s.Ps + (size_t)lu * NB * 64 + lane;
-    const int32_t *Uo = s.U2s + (size_t)lu * NB * 64 + lane;
-    const u64 *xo = s.Xs + (size_t)lu * NP * 64 + lane;
-    uint32_t *ao = s.As + (size_t)lu * NP * 64 + lane;
-    uint32_t *Mh = reinterpret_cast<uint32_t *>(s.Ms + (size_t)lu * NP);
-    // the pairs in chunks of 4: every input that does not depend on the
-    // carried configuration is read first, then the 4 decisions are taken
-    // in order (the table entry is read whether or not it decides: index 0
-    // when m is out of range; the table has at least one entry)
-    int carry_e = nt - Uo[0];
-    uint32_t carry_p = Po[0];
-    for (int i0 = 0; i0 < NP; i0 += 4) {
-      int e1[4], sg[4], eb[4], nx[4];
-      uint32_t p1[4];
-      u64 x[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int i = min(i0 + j, NP - 1);
-        e1[j] = nt - Uo[(i + 1) * 64];
-        p1[j] = Po[(i + 1) * 64];
-        x[j] = xo[(size_t)i * 64];
-        sg[j] = s.SG[i];
-        eb[j] = s.EO[i];
-        nx[j] = s.EO[i + 1] - eb[j];
+  const int NB = d.NB, NP = NB - 1, ncta = p.ncta;
+  const int n2 = NB * 32, scale = p.pair_energy ? 2 : 1;
+  const uint32_t *Pw = reinterpret_cast<const uint32_t *>(s.Pt);
+  for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+    int2 &U2 = reinterpret_cast<int2 *>(s.U2s)[i];
+    if (p.parts) {
+      int lo = 0, hi = 0;
+#pragma unroll 4
+      for (int c = 0; c < ncta; ++c) {
+        const uint32_t v = Pw[c * n2 + i];
+        lo += (int)(v & 0xFFFFu);
+        hi += (int)(v >> 16);
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int i = i0 + j;
-        if (i >= NP) break;
-        const int dE = e1[j] - carry_e, m = (-dE) >> 1;
-        const bool up = sg[j] == 0 || (sg[j] > 0 ? dE >= 0 : dE <= 0);
-        const bool inr = m >= 1 && m <= nx[j];
-        const int ti = inr ? eb[j] + m - 1 : 0;
-        const u64 tv = p.ntab ? s.Tab[ti] : (u64)__double_as_longlong(__ldg(d.exptab + ti));
-        const bool change = up || (inr ? x[j] < tv : x[j] == 0);
-        Eo[i * 64] = change ? e1[j] : carry_e;
-        Po[i * 64] = (uint8_t)(change ? p1[j] : carry_p);
-        ao[i * 64] += change ? 1u : 0u;
-        carry_e = change ? carry_e : e1[j];
-        carry_p = change ? carry_p : p1[j];
-        Mh[2 * i + (lane >> 5)] = __ballot_sync(0xffffffffu, change);
-      }
+      U2 = make_int2(scale * lo, scale * hi);
     }
-    Eo[NP * 64] = carry_e;
-    Po[NP * 64] = (uint8_t)carry_p;
-    if (measure) {
-      long long *av = s.Av + (size_t)lu * NB * 64 + lane;
-      for (int b = 0; b < NB; ++b) av[b * 64] += Eo[b * 64];
+    if (last && me.rank == 0) {
+      const int smp = 2 * (i & 31), b = i >> 5;
+      int32_t *U = d.U2 + ((size_t)me.w * 64 + smp) * d.NR * NB + (size_t)me.r * NB + b;
+      U[0] = U2.x;
+      U[(size_t)d.NR * NB] = U2.y;
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < upc * 64 * NB; i += blockDim.x) {
-    if (last) {
-      const int lane = i & 63, rest = i >> 6, lu = rest / NB, b = rest - lu * NB;
-      const int u = lu * ncta + me.rank;
-      if (u < nunits) {
-        const int w = u / NR, r = u - w * NR;
-        d.U2[((size_t)w * 64 + lane) * G + (size_t)r * NB + b] = s.U2s[i];
-      }
+  if (threadIdx.x < 64) {
+    const int lane = threadIdx.x;
+    const int32_t *Uo = s.U2s + lane, *xo = s.Xs + lane;
+    uint32_t *Mh = reinterpret_cast<uint32_t *>(s.Ms) + (lane >> 5);
+    // what does not depend on the carried configuration is read a pair ahead
+    int carry = Uo[0], u1 = Uo[64], x = xo[0], sg = s.SG[0];
+#pragma unroll 1
+    for (int i = 0; i < NP; ++i) {
+      const int n = min(i + 1, NP - 1), u1n = Uo[(n + 1) * 64], xn = xo[n * 64], sgn = s.SG[n];
+      const int dE = carry - u1, m = (-dE) >> 1;  // energies are 3 V - U2
+      const bool change = (sg < 0 ? dE <= 0 : dE >= 0) || (m <= x && (m != 0 || x == 0x7FFFFFFF));
+      const uint32_t lanes = __ballot_sync(0xffffffffu, change);
+      if ((lane & 31) == 0) Mh[2 * i] = lanes;
+      carry = change ? carry : u1;
+      u1 = u1n;
+      x = xn;
+      sg = sgn;
     }
-    s.U2s[i] = 0;
   }
+  __syncthreads();
 }
 
-// The accepted swaps applied to the CTA's rows (sp_permute_body), the masks
-// of every chain gathered from their CTAs first; rows (word, replica, site)
-// with the site fastest.
-__device__ __forceinline__ void res_permute(const SpResDev &p, const cg::cluster_group &cl, const ResCta &me,
-                                            const ResShared &s) {
-  const SpDev &d = p.d;
-  const int NB = d.NB, NR = d.NR, NP = NB - 1, nunits = d.nw * NR, ncta = p.ncta, nslm = p.nslm;
-  for (int i = threadIdx.x; i < nunits * NP; i += blockDim.x) {
-    const int u = i / NP, pi = i - u * NP, own = u % ncta;
-    const size_t o = (size_t)(u / ncta) * NP + pi;
-    s.Mall[i] = own == me.rank ? s.Ms[o] : cl.map_shared_rank(s.Ms, own)[o];
+// The swaps applied to the unit's acceptances, and by the last two warps, a lane
+// a sample, to its energies and slot ids; with `measure`, the slots' energies
+// are added to the bin's sums (sp_measure_u2_body after a tempering step).
+// Needed by the next tempering step only, so it runs while the barrier behind
+// the permute is waited for.
+__device__ __forceinline__ void res_state(const SpResDev &p, const ResShared &s, bool measure) {
+  const int NP = p.d.NB - 1, nth = blockDim.x, nt = 3 * p.d.V;
+  if (threadIdx.x < nth - 64) {
+    for (int i = threadIdx.x; i < NP * 64; i += nth - 64) s.As[i] += (uint32_t)(s.Ms[i >> 6] >> (i & 63)) & 1u;
+    return;
   }
-  __syncthreads();
-  const int rows = nunits * me.nsl;
-  for (int t = threadIdx.x; t < rows; t += blockDim.x) {
-    const int u = t / me.nsl, i = t - u * me.nsl;  // u = w * NR + r
-    u64 *row = s.S + (size_t)u * NB * nslm + i;    // column r * NB + b of word w
-    const u64 *M = s.Mall + (size_t)u * NP;
+  const int lane = threadIdx.x & 63;
+  int carry_e = nt - s.U2s[lane], e1 = nt - s.U2s[64 + lane];
+  uint32_t carry_p = s.Ps[lane], p1 = s.Ps[64 + lane];
+#pragma unroll 1
+  for (int i = 0; i < NP; ++i) {
+    const int o = i * 64 + lane, n = min(i + 2, NP) * 64 + lane, e1n = nt - s.U2s[n];
+    const uint32_t p1n = s.Ps[n];
+    const bool change = (s.Ms[i] >> lane) & 1ull;
+    const int e = change ? e1 : carry_e;
+    s.Es[o] = e;
+    s.Ps[o] = (uint8_t)(change ? p1 : carry_p);
+    if (measure) s.Av[o] += e;
+    carry_e = change ? carry_e : e1;
+    carry_p = change ? carry_p : p1;
+    e1 = e1n;
+    p1 = p1n;
+  }
+  s.Es[NP * 64 + lane] = carry_e;
+  s.Ps[NP * 64 + lane] = (uint8_t)carry_p;
+  if (measure) s.Av[NP * 64 + lane] += carry_e;
+  if (!p.parts)  // the next counts come after another barrier (two colours, or the energy's own phase)
+    for (int i = 0; i <= NP; ++i) s.U2s[i * 64 + lane] = 0;
+}
+
+// The accepted swaps applied to the CTA's sites (sp_permute_body), four slots
+// read ahead of the chain through them.
+__device__ __forceinline__ void res_permute(const SpResDev &p, const ResCta &me, const ResShared &s) {
+  const int NP = p.d.NB - 1, nslm = p.nslm, nth = blockDim.x;
+  for (int t = threadIdx.x; t < me.nsl; t += nth) {
+    u64 *row = s.S + t;
     u64 cur = row[0];
-    for (int b = 0; b < NP; ++b) {
-      const u64 m = M[b], nxt = row[(size_t)(b + 1) * nslm], x = (cur ^ nxt) & m;
-      row[(size_t)b * nslm] = cur ^ x;
-      cur = nxt ^ x;
+#pragma unroll 1
+    for (int b0 = 0; b0 < NP; b0 += 4) {
+      u64 m[4], nxt[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int b = min(b0 + j, NP - 1);
+        m[j] = s.Ms[b];
+        nxt[j] = row[(b + 1) * nslm];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (b0 + j >= NP) break;
+        const u64 x = (cur ^ nxt[j]) & m[j];
+        row[(b0 + j) * nslm] = cur ^ x;
+        cur = nxt[j] ^ x;
+      }
     }
-    row[(size_t)NP * nslm] = cur;
+    row[NP * nslm] = cur;
   }
 }
 
@@ -507,128 +633,125 @@ template <int NPL>
 __global__ void __launch_bounds__(kResThreads, 1) k_sp_resident(const __grid_constant__ SpResDev p) {
   const cg::cluster_group cl = cg::this_cluster();
   const SpDev &d = p.d;
-  const int NB = d.NB, NR = d.NR, G = NR * NB, NP = NB - 1, V = d.V, nw = d.nw, ncol = d.ncol;
-  const int nslm = p.nslm, ncta = p.ncta, upc = p.upc, nunits = nw * NR;
+  const int NB = d.NB, NR = d.NR, G = NR * NB, NP = NB - 1, V = d.V, ncol = d.ncol;
+  const int nslm = p.nslm;
   ResCta me;
   me.rank = (int)cl.block_rank();
+  me.unit = (int)(blockIdx.x / (unsigned)p.ncta);
+  me.w = me.unit / NR;
+  me.r = me.unit - me.w * NR;
   me.site_lo = me.rank * nslm;
   me.nsl = min(nslm, V - me.site_lo);
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ ResColour col[kResMaxColours];
   const ResShared s = res_carve(smem, p);
   const int tid = threadIdx.x, nth = blockDim.x;
 
-  // the CTA's words and neighbour table, its sites by colour, the tempering
-  // tables, and the energies, slot ids, acceptances and sums of its chains
-  // (global memory reads in global order, SMEM writes transposed)
-  const int nS = nw * me.nsl * G, nJ = nw * me.nsl * 6;
+  // the CTA's words and neighbour table, its sites by colour, and the unit's
+  // signs, energies, slot ids, acceptances and sums
+  if (tid < ncol) {
+    ResColour q;
+    q.nk = d.col_off[tid + 1] - d.col_off[tid];
+    q.kb = p.kr[me.rank][tid];
+    q.nkc = p.kr[me.rank + 1][tid] - q.kb;
+    q.loff = 0;
+    for (int c = 0; c < tid; ++c) q.loff += p.kr[me.rank + 1][c] - p.kr[me.rank][c];
+    q.mul = q.nkc > 1 ? (uint32_t)(0xFFFFFFFFu / (uint32_t)q.nkc) + 1u : 0u;
+    col[tid] = q;
+  }
+  const int nS = me.nsl * NB, nJ = me.nsl * 6;
+  u64 *gS = d.S + ((size_t)me.w * V + me.site_lo) * G + (size_t)me.r * NB;
   for (int i = tid; i < nS; i += nth) {
-    const int col = i % G, rest = i / G, si = rest % me.nsl, w = rest / me.nsl;
-    s.S[((size_t)w * G + col) * nslm + si] = d.S[((size_t)w * V + me.site_lo + si) * G + col];
+    const int si = i / NB, b = i - si * NB;
+    s.S[b * nslm + si] = gS[(size_t)si * G + b];
   }
   for (int i = tid; i < nJ; i += nth) {
-    const int q = i % 6, rest = i / 6, si = rest % me.nsl, w = rest / me.nsl;
-    s.J[((size_t)w * 6 + q) * nslm + si] = d.J[((size_t)w * V + me.site_lo + si) * 6 + q];
-  }
-  for (int i = tid; i < me.nsl * 6; i += nth) {
-    const int nbs = __ldg(d.nb + (size_t)me.site_lo * 6 + i), own = nbs / nslm, q = i % 6, si = i / 6;
-    s.nbl[q * nslm + si] = ((uint32_t)own << 16) | (uint32_t)(nbs - own * nslm);
+    const int q = i % 6, si = i / 6;
+    s.J[q * nslm + si] = d.J[((size_t)me.w * V + me.site_lo) * 6 + i];
+    const int nbs = __ldg(d.nb + (size_t)me.site_lo * 6 + i), own = nbs / nslm;
+    const uint32_t a = smem_addr(s.S + (nbs - own * nslm));
+    s.nbl[q * nslm + si] = own == me.rank ? a : mapa(a, own) | 1u;
   }
   for (int k = 0, loff = 0; k < ncol; ++k) {
     const int kb = p.kr[me.rank][k], nkc = p.kr[me.rank + 1][k] - kb, off = d.col_off[k];
     for (int j = tid; j < nkc; j += nth) s.lst[loff + j] = (uint16_t)(__ldg(d.col_sites + off + kb + j) - me.site_lo);
     loff += nkc;
   }
-  for (int i = tid; i < NB; i += nth) s.EO[i] = d.expoff[i];
   for (int i = tid; i < NP; i += nth) {
     const double f = -__dsub_rn(d.betas[i + 1], d.betas[i]);
     s.SG[i] = f > 0.0 ? 1 : (f < 0.0 ? -1 : 0);
   }
-  for (int i = tid; i < p.ntab; i += nth) s.Tab[i] = (u64)__double_as_longlong(d.exptab[i]);
-  for (int i = tid; i < upc * 64 * NB; i += nth) {
-    s.U2s[i] = 0;
-    const int lane = i & 63, rest = i >> 6, lu = rest / NB, b = rest - lu * NB;
-    const int u = lu * ncta + me.rank;
-    if (u >= nunits) continue;
-    const int w = u / NR, r = u - w * NR;
-    const size_t o = ((size_t)w * 64 + lane) * G + (size_t)r * NB + b;
+  const size_t row0 = (size_t)me.w * 64 * NR + me.r;  // of sample 0; samples NR rows apart
+  for (int i = tid; i < 64 * NB; i += nth) {
+    const size_t o = (row0 + (size_t)(i & 63) * NR) * NB + (i >> 6);
     s.Es[i] = d.E[o];
     s.Ps[i] = d.perm[o];
     s.Av[i] = (long long)d.avgE[o];
   }
-  for (int i = tid; i < upc * 64 * NP; i += nth) {
-    const int lane = i & 63, rest = i >> 6, lu = rest / NP, pi = rest - lu * NP;
-    const int u = lu * ncta + me.rank;
-    if (u >= nunits) continue;
-    const int w = u / NR, r = u - w * NR;
-    s.As[i] = d.acc[(((size_t)w * 64 + lane) * NR + r) * NP + pi];
-  }
-  const unsigned long long step0 = *d.ptstep;
+  for (int i = tid; i < 64 * NB; i += nth) s.U2s[i] = 0;
+  for (int i = tid; i < 64 * NP; i += nth) s.As[i] = d.acc[(row0 + (size_t)(i & 63) * NR) * NP + (i >> 6)];
   cl.sync();
 
   int sweep = 0, ptj = 0;
+  u64 words[2] = {};
+  res_prefetch(p, me, col, 0, 0, res_counts(p, 0, 0), words);
   for (int it = 0; it < p.nit; ++it)
     for (int im = 0; im < p.mesfr; ++im)
       for (int ih = 0; ih < p.houfr; ++ih) {
         res_stage_x(p, me, s, ptj);
         for (int sw = 0; sw < p.ptfr; ++sw, ++sweep)
           for (int k = 0; k < ncol; ++k) {
-            if (p.pair_energy && k == ncol - 1 && sw == p.ptfr - 1) res_pass_count<NPL>(p, cl, me, s, sweep, k);
-            else res_pass(p, cl, me, s, sweep, k);
-            cp_async_wait_all();  // this step's uniforms (staged before the first pass)
-            cl.sync();
+            if (res_counts(p, sw, k)) res_pass_count<NPL>(p, me, s, col[k], sweep, k, words);
+            else res_pass(p, me, s, col[k], sweep, k, words);
+            const bool wrap = k == ncol - 1;
+            if (wrap && sw == p.ptfr - 1) cp_async_wait_all();  // the step's draws
+            cluster_arrive();  // before the reads: its fence would wait for them
+            const int sw1 = wrap ? (sw + 1 == p.ptfr ? 0 : sw + 1) : sw, k1 = wrap ? 0 : k + 1;
+            res_prefetch(p, me, col, sweep + wrap, k1, res_counts(p, sw1, k1), words);
+            cluster_wait();
           }
         if (!p.pair_energy) {
-          res_energy<NPL>(p, cl, me, s);
-          cl.sync();
+          res_energy<NPL>(p, me, s);
+          cluster_arrive();
+          cluster_wait();
         }
         const bool lastpt = im == p.mesfr - 1 && ih == p.houfr - 1;
-        res_tempering(p, me, s, ptj, p.measure && lastpt, lastpt && it == p.nit - 1);
-        cl.sync();
-        res_permute(p, cl, me, s);
-        cl.sync();
+        res_tempering(p, me, s, lastpt && it == p.nit - 1);
+        res_permute(p, me, s);
+        cluster_arrive();
+        res_state(p, s, p.measure && lastpt);
+        cluster_wait();
         ++ptj;
       }
 
+  __syncthreads();  // res_state's writes
+
   // back to global memory
   for (int i = tid; i < nS; i += nth) {
-    const int col = i % G, rest = i / G, si = rest % me.nsl, w = rest / me.nsl;
-    d.S[((size_t)w * V + me.site_lo + si) * G + col] = s.S[((size_t)w * G + col) * nslm + si];
+    const int si = i / NB, b = i - si * NB;
+    gS[(size_t)si * G + b] = s.S[b * nslm + si];
   }
-  for (int i = tid; i < upc * 64 * NB; i += nth) {
-    const int lane = i & 63, rest = i >> 6, lu = rest / NB, b = rest - lu * NB;
-    const int u = lu * ncta + me.rank;
-    if (u >= nunits) continue;
-    const int w = u / NR, r = u - w * NR;
-    const size_t o = ((size_t)w * 64 + lane) * G + (size_t)r * NB + b;
+  if (me.rank != 0) return;
+  for (int i = tid; i < 64 * NB; i += nth) {
+    const size_t o = (row0 + (size_t)(i & 63) * NR) * NB + (i >> 6);
     d.E[o] = s.Es[i];
     d.perm[o] = s.Ps[i];
     d.avgE[o] = (double)s.Av[i];
   }
-  for (int i = tid; i < upc * 64 * NP; i += nth) {
-    const int lane = i & 63, rest = i >> 6, lu = rest / NP, pi = rest - lu * NP;
-    const int u = lu * ncta + me.rank;
-    if (u >= nunits) continue;
-    const int w = u / NR, r = u - w * NR;
-    d.acc[(((size_t)w * 64 + lane) * NR + r) * NP + pi] = s.As[i];
-  }
-  for (int i = tid; i < upc * NP; i += nth) {
-    const int lu = i / NP, pi = i - lu * NP, u = lu * ncta + me.rank;
-    if (u < nunits) d.M[(size_t)u * NP + pi] = s.Ms[i];
-  }
-  if (me.rank == 0 && tid == 0) *d.ptstep = step0 + (unsigned long long)ptj;
+  for (int i = tid; i < 64 * NP; i += nth) d.acc[(row0 + (size_t)(i & 63) * NR) * NP + (i >> 6)] = s.As[i];
+  for (int i = tid; i < NP; i += nth) d.M[(size_t)me.unit * NP + i] = s.Ms[i];
+  if (blockIdx.x == 0 && tid == 0) *d.ptstep += (unsigned long long)ptj;
 }
 
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
-static int res_lanes(int sites) { return sites <= 32 ? 8 : sites <= 96 ? 16 : 32; }
-
 // Counter planes of the energy phase's warp sums: 6 * nslm < 2^NPL.
 static int res_npl(int nslm) { return 6 * nslm < (1 << 10) ? 10 : kResPlanes; }
 
 template <int NPL>
 static cudaError_t res_attrs() {
-  cudaError_t e = cudaFuncSetAttribute(k_sp_resident<NPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  cudaError_t e = cudaFuncSetAttribute(k_sp_resident<NPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_resident<NPL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   return e;
 }
@@ -642,9 +765,9 @@ cudaError_t sp_res_setup() {
   return e;
 }
 
-static cudaLaunchConfig_t res_config(int ncta, size_t smem, cudaStream_t st, cudaLaunchAttribute *at) {
+static cudaLaunchConfig_t res_config(int ncta, int units, size_t smem, cudaStream_t st, cudaLaunchAttribute *at) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)ncta);
+  cfg.gridDim = dim3((unsigned)(ncta * units));
   cfg.blockDim = dim3(kResThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -657,38 +780,36 @@ static cudaLaunchConfig_t res_config(int ncta, size_t smem, cudaStream_t st, cud
   return cfg;
 }
 
-// Whether the job's share of the widest split (sites split evenly over 16
-// CTAs) fits one CTA's shared memory (the exp table left in global memory).
+// Whether a unit's share of the widest split (sites split evenly over 16 CTAs)
+// fits one CTA's shared memory, and the job's words those of kResMaxCta.
 bool sp_res_fits(int L, int Lz, int nw, int NR, int NB) {
   if (NB < 2 || L < 1 || Lz < 1) return false;
   const long long V = (long long)L * L * Lz, nslm = (V + kResMaxCta - 1) / kResMaxCta;
-  const int ncta = (int)((V + nslm - 1) / nslm);
-  if (nslm > kResMaxSites) return false;
-  const int upc = (nw * NR + ncta - 1) / ncta;
-  return res_smem_bytes(nw, (int)nslm, NR, NB, upc, 0) <= 227 * 1024;
+  if (nslm > kResMaxSites || 8 * V * nw * NR * NB > (long long)kResMaxCta * 227 * 1024) return false;
+  return res_smem_bytes((int)nslm, NB, 0) <= kResSmem;
 }
 
-// The most CTAs (sites split into equal runs, at most 16) whose cluster the
-// GPU can hold with the job's shared memory; none when a CTA's share does
-// not fit.  The exp table is staged in SMEM when it fits beside the words.
-bool sp_res_plan(const SpDev &d, const int32_t *col_sites, int ntab, SpResPlan &pl) {
-  if (d.ncol < 1 || d.ncol > kResMaxColours || d.NB < 2) return false;
-  const int nunits = d.nw * d.NR;
-  const size_t lim = 227 * 1024;
+// The CTAs of a unit's cluster (sites split into equal runs, at most 16): the
+// most whose clusters the GPU can hold at once for all units, else the fewest
+// whose share fits; none when no share does.  (Steps of the 6^2 x 24 tube, two
+// units: 16, 12, 8 CTAs a unit 701, 729, 759 us a bin of 64, 6 and 4 856 and
+// 977 before the last changes to the kernel.)
+bool sp_res_plan(const SpDev &d, const int32_t *col_sites, SpResPlan &pl) {
+  if (d.ncol < 1 || d.ncol > kResMaxColours || !sp_res_fits(d.L, d.Lz, d.nw, d.NR, d.NB)) return false;
+  const int units = d.nw * d.NR;
   int last = 0;
+  bool found = false;
   for (int want = std::min(kResMaxCta, d.V); want >= 1; --want) {
     const int nslm = (d.V + want - 1) / want, ncta = (d.V + nslm - 1) / nslm;
     if (ncta == last) continue;
     last = ncta;
-    if (nslm > kResMaxSites) return false;
-    const int upc = (nunits + ncta - 1) / ncta;
-    int nt = ntab;
-    size_t smem = res_smem_bytes(d.nw, nslm, d.NR, d.NB, upc, nt);
-    if (smem > lim) smem = res_smem_bytes(d.nw, nslm, d.NR, d.NB, upc, nt = 0);
-    if (smem > lim) return false;
+    int parts = ncta;
+    size_t smem = res_smem_bytes(nslm, d.NB, parts);
+    if (smem > kResSmem) smem = res_smem_bytes(nslm, d.NB, parts = 0);
+    if (nslm > kResMaxSites || smem > kResSmem) break;
     const int npl = res_npl(nslm);
     cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = res_config(ncta, smem, nullptr, &at);
+    const cudaLaunchConfig_t cfg = res_config(ncta, units, smem, nullptr, &at);
     int nclusters = 0;
     const cudaError_t e = npl == 10 ? cudaOccupancyMaxActiveClusters(&nclusters, k_sp_resident<10>, &cfg)
                                     : cudaOccupancyMaxActiveClusters(&nclusters, k_sp_resident<kResPlanes>, &cfg);
@@ -697,6 +818,7 @@ bool sp_res_plan(const SpDev &d, const int32_t *col_sites, int ntab, SpResPlan &
       continue;
     }
     if (nclusters < 1) continue;
+    found = true;
     for (int c = 0; c <= ncta; ++c)
       for (int k = 0; k < d.ncol; ++k) {
         const int32_t *b = col_sites + d.col_off[k], *e2 = col_sites + d.col_off[k + 1];
@@ -704,23 +826,16 @@ bool sp_res_plan(const SpDev &d, const int32_t *col_sites, int ntab, SpResPlan &
       }
     pl.ncta = ncta;
     pl.nslm = nslm;
-    pl.upc = upc;
-    // lanes per counted column: about 2-4 sites a lane (a butterfly level
-    // costs the same whatever the number of sites behind it)
-    int most = 0;
-    for (int c = 0; c < ncta; ++c) most = std::max(most, pl.kr[c + 1][d.ncol - 1] - pl.kr[c][d.ncol - 1]);
-    pl.lpc_count = res_lanes(most);
-    pl.lpc_energy = res_lanes(nslm);
-    pl.ntab = nt;
+    pl.parts = parts;
     pl.npl = npl;
     pl.smem = smem;
-    return true;
+    if (nclusters >= units) break;
   }
-  return false;
+  return found;
 }
 
 size_t sp_res_launch_sweeps(size_t V, size_t G, const ea_cadence *cad) {
-  const size_t spi = (size_t)cad->mesfr * cad->houfr * cad->ptfr, bytes_sweep = 24 * V * G;
+  const size_t spi = (size_t)cad->mesfr * cad->houfr * cad->ptfr, bytes_sweep = 16 * V * G;
   if (cad->cluster) {
     // one launch per block of houfr x ptfr sweeps between two cluster moves
     const size_t blk = (size_t)cad->houfr * cad->ptfr;
@@ -737,14 +852,14 @@ cudaError_t sp_res_chunk(const SpResDev &p, const SpResPlan &pl, int npass, uint
   if (e != cudaSuccess) return e;
   const int nsweep = npass / d.ncol;
   const long long n = (long long)nsweep * d.V * d.NR * d.NB;
-  k_sp_draw<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, nsweep, ctrs, const_cast<u64 *>(p.R));
+  k_sp_draw<<<(unsigned)((n + kDrawItems - 1) / kDrawItems), kDrawThreads, 0, st>>>(d, nsweep, ctrs, const_cast<u64 *>(p.R));
   const int npt = p.nit * p.mesfr * p.houfr;
   const long long nx = (long long)npt * d.nw * d.NR * (d.NB - 1) * 64;
-  if (nx > 0) k_sp_pt_uniforms<<<(unsigned)((nx + 255) / 256), 256, 0, st>>>(d, npt, const_cast<u64 *>(p.X));
+  if (nx > 0) k_sp_pt_draw<<<(unsigned)((nx + 255) / 256), 256, 0, st>>>(d, npt, const_cast<int32_t *>(p.X));
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute at;
-  const cudaLaunchConfig_t cfg = res_config(pl.ncta, pl.smem, st, &at);
+  const cudaLaunchConfig_t cfg = res_config(pl.ncta, d.nw * d.NR, pl.smem, st, &at);
   return pl.npl == 10 ? cudaLaunchKernelEx(&cfg, k_sp_resident<10>, p)
                       : cudaLaunchKernelEx(&cfg, k_sp_resident<kResPlanes>, p);
 }
