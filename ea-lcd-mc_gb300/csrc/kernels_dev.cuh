@@ -821,7 +821,10 @@ __device__ __forceinline__ int word_site0(const JobDev &j, int p, int k) {
 // main.cu:776-832,938-991): bit i of s_bits is [U(root(i)) < 0.5], built in
 // natural order (coalesced label reads, one ballot per 32 sites); then each
 // word gathers its 64 bits from SMEM, q' = q xor sel, and s_r1 ^= q',
-// s_r2 ^= q'.  s_bits holds V/32 words, s_off 64.
+// s_r2 ^= q'.  s_bits holds V/32 words, s_off 64.  What bounds it is the chain
+// of reads behind a site's label, two to three of 64 (24^2 x 192 sites, 496
+// lattices: 185 us with a site a thread at a time, 131 with 4, 126 with 8 or 12).
+constexpr int kFlipSites = 8;
 __device__ __forceinline__ void flip_body(const JobDev &j, int g, size_t lat, uint32_t *s_bits,
                                           int *s_off) {
   const int t = threadIdx.x, nth = blockDim.x;
@@ -831,12 +834,31 @@ __device__ __forceinline__ void flip_body(const JobDev &j, int g, size_t lat, ui
   const uint32_t *u = j.xw_bits + (ub >> 5);
   const uint32_t us = (uint32_t)ub & 31u;
   if (t < 64) s_off[t] = word_bit_offset(j, t);
-  for (int base = 0; base < j.V; base += nth) {
-    const int site = base + t;
-    bool sel = false;
-    if (site < j.V) sel = xw_coin(u, us + cc_find(lab, (uint32_t)site));
-    const unsigned ball = __ballot_sync(0xffffffffu, sel);
-    if ((t & 31) == 0 && site < j.V) s_bits[site >> 5] = ball;
+  for (int base = t; base - t < j.V; base += kFlipSites * nth) {
+    uint32_t l[kFlipSites];
+#pragma unroll
+    for (int i = 0; i < kFlipSites; ++i) l[i] = base + i * nth < j.V ? lab[base + i * nth] : 0u;
+    bool more;
+    do {  // cc_find of all of them
+      uint32_t n[kFlipSites];
+      more = false;
+#pragma unroll
+      for (int i = 0; i < kFlipSites; ++i) n[i] = lab[l[i]];
+#pragma unroll
+      for (int i = 0; i < kFlipSites; ++i) {
+        more = more || n[i] != l[i];
+        l[i] = n[i];
+      }
+    } while (more);
+    bool sel[kFlipSites];
+#pragma unroll
+    for (int i = 0; i < kFlipSites; ++i) sel[i] = xw_coin(u, us + l[i]);
+#pragma unroll
+    for (int i = 0; i < kFlipSites; ++i) {
+      const int site = base + i * nth;
+      const unsigned ball = __ballot_sync(0xffffffffu, sel[i]);
+      if ((t & 31) == 0 && site < j.V) s_bits[site >> 5] = ball;
+    }
   }
   __syncthreads();
   const int r1 = j.pairs[2 * g], r2 = j.pairs[2 * g + 1];
