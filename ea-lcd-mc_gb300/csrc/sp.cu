@@ -1523,7 +1523,19 @@ int sp_kt(int NB, int NR, int nsites_colour) {
   if (sp_sweep_smem(NB, NR, kt) > lim) return 0;
   while (kt < 64 && sp_sweep_smem(NB, NR, 2 * kt) <= lim && (nsites_colour + 2 * kt - 1) / (2 * kt) >= 2 * 152)
     kt <<= 1;
-  return kt;
+  // In between, where whole rounds of the GPU (two CTAs an SM where their SMEM
+  // allows) make a colour shorter: 12^2 x 48 with
+  // 24 temperatures and 4 replicas takes 370 us a sweep of 4096 samples with 8
+  // sites a tile (1.4 rounds), 313 with 12 (0.95), of 256 samples 94 and 82;
+  // 24^2 x 96 with 32 temperatures and 256 samples 930 and 901.
+  auto rounds = [&](int k) {
+    const int slots = 152 * (2 * (sp_sweep_smem(NB, NR, k) + 1536) <= 228 * 1024 ? 2 : 1), tiles = (nsites_colour + k - 1) / k;
+    return (tiles + slots - 1) / slots;
+  };
+  int best = kt;
+  for (int k = kt + 1; k < 2 * kt && k < 64 && sp_sweep_smem(NB, NR, k) <= lim; ++k)
+    if (rounds(k) * k < rounds(best) * best) best = k;
+  return best;
 }
 
 cudaError_t sp_setup() {
