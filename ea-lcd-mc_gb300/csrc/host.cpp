@@ -296,18 +296,6 @@ int scalar_energy(const Geometry &g, const uint8_t *u, const uint8_t *J6) {
   return 3 * V - 2 * e;
 }
 
-void presearch8(const uint64_t *cum, uint16_t *pre) {
-  auto first_above = [&](uint64_t R) {
-    int n = 0;
-    while (n < 255 && !(R < cum[n])) ++n;
-    return n;
-  };
-  for (int b = 0; b < 256; ++b) {
-    const uint64_t lo = (uint64_t)b << 56, hi = lo | ((1ULL << 56) - 1);
-    pre[b] = (uint16_t)(first_above(lo) | (first_above(hi) << 8));
-  }
-}
-
 void prefault(void *p, size_t n) {
 #ifdef MADV_POPULATE_WRITE
   const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p & ~(page - 1);

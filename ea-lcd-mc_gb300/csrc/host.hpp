@@ -68,10 +68,7 @@ int scalar_energy(const Geometry &g, const uint8_t *u, const uint8_t *J6);
 // range that is not the host's is left to the copy to refuse.
 void prefault(void *p, size_t n);
 
-// 8-bit pre-search of the cumulative thresholds: entry b = (lo, hi) bounds of the
-// byte drawn for any R whose top 8 bits are b.
-void presearch8(const uint64_t *cum, uint16_t *pre);
-// The same with 2^bits buckets and one byte a bucket (see host.cpp).
+// Pre-search of the cumulative thresholds with 2^bits buckets (see host.cpp).
 constexpr int pre_stride(int bits) { return ((1 << bits) + 16) & ~15; }  // 2^bits + 1 entries, padded to 16 bytes
 void presearch(const uint64_t *cum, int bits, uint8_t *pre);
 constexpr int kPre11Stride = pre_stride(11);

@@ -118,26 +118,12 @@ __device__ __forceinline__ void philox10(uint32_t &v0, uint32_t &v1, uint32_t &v
   }
 }
 
-// GCUM: the thresholds are read from global memory through the read-only
-// cache instead of SMEM (the pre-search pins the byte without reading them
-// for most R: 0.05-0.35 bisection steps per byte on the benchmark sets).
-template <bool GCUM = false>
-__device__ __forceinline__ uint32_t lut_byte(uint32_t hi, uint32_t lo, const u64 *cum, const uint16_t *pre) {
-  const u64 R = ((u64)hi << 32) | lo;
-  const uint32_t e = pre[hi >> 24];
-  uint32_t a = e & 255u, b = e >> 8;
-  while (a < b) {
-    const uint32_t m = (a + b) >> 1;
-    if (R < (GCUM ? __ldg(cum + m) : cum[m])) b = m; else a = m + 1;
-  }
-  return a;
-}
-
-// The same search with the pre-search of presearch (host.cpp): a key in bucket
-// t = hi >> shift (shift = 32 - bits) has its byte in [pre[t], pre[t+1]];
-// thresholds through the read-only cache.  Narrower buckets leave a bisection to fewer
-// keys: 0.04 steps per byte on the benchmark sets against 0.18-0.21 with the
-// 8-bit pre-search, and a warp waits for its slowest lane at each search.
+// Threshold search of a random byte with the pre-search of presearch
+// (host.cpp): a key in bucket t = hi >> shift (shift = 32 - bits) has its byte
+// in [pre[t], pre[t+1]]; thresholds through the read-only cache.  Narrower
+// buckets leave a bisection to fewer keys: 0.04 steps a byte on the benchmark
+// sets with 11 bits against 0.22 with 8, and a warp waits for its slowest lane
+// at each search.
 __device__ __forceinline__ uint32_t lut_byte_pre(uint32_t hi, uint32_t lo, const u64 *cum, const uint8_t *pre, int shift) {
   const u64 R = ((u64)hi << 32) | lo;
   const uint32_t t = hi >> shift;
@@ -167,13 +153,6 @@ __device__ __forceinline__ uint32_t rnd_word_by(uint32_t cx, uint32_t cy, uint32
   const uint32_t rot = (s0 + v1 + s2 + v3) >> 27;
   const uint32_t bb = byte(v0, s0) | (byte(v1, s1) << 8) | (byte(v2, s2) << 16) | (byte(v3, s3) << 24);
   return __funnelshift_l(bb, bb, rot);  // rotate left; rot 0 leaves the word as it is
-}
-
-template <bool GCUM = false>
-__device__ __forceinline__ uint32_t rnd_word(uint32_t cx, uint32_t cy, uint32_t cz, uint32_t cw, uint32_t key,
-                                             uint32_t tid, const u64 *cum, const uint16_t *pre) {
-  return rnd_word_by(cx, cy, cz, cw, key, tid,
-                     [&](uint32_t hi, uint32_t lo) { return lut_byte<GCUM>(hi, lo, cum, pre); });
 }
 
 // ---------------------------------------------------------------------------
@@ -220,11 +199,6 @@ __device__ __forceinline__ u64 flip_mask_id(const u64 f[6], u64 id1, u64 id2) {
   const u64 j24 = j2 | j4;
   return (j1 & j3 & id1) | ((j24 | id2) & (j1 | j3 | id1)) | ((j2 & j4) | (j24 & id2));
 }
-__device__ __forceinline__ u64 flip_mask(const u64 f[6], u64 b0, u64 b1, u64 b2) {
-  b1 = b0 & b1; b2 = b1 & b2;
-  return flip_mask_id(f, (b0 ^ b1) | b2, b1);
-}
-
 // ---------------------------------------------------------------------------
 // The flip mask's two words (flip_mask_id) of ntrip random triples, drawn by a
 // CTA: id1 = (b0 ^ id2) | (id2 & b2), id2 = b0 & b1.  Where a 32-bit half of b0

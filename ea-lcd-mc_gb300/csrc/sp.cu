@@ -34,29 +34,34 @@ __device__ __forceinline__ void sp_fill_body(const SpDev &d) {
 
 // ---------------------------------------------------------------------------
 // One colour pass.  A CTA owns kt sites of the colour: it stages every
-// temperature's thresholds in SMEM, draws the three random words of each
-// (slot, site, replica) once -- shared by the nw sample words, as the
-// reference shares them across samples (main.cu:1430) -- and updates all
-// (word, site, replica, slot) words of its tile in memory order, so that
-// consecutive lanes touch consecutive words of a site.  The Philox thread
-// index of (slot b, site i, replica r) is (b*V + i)*NR + r.
+// temperature's pre-search in SMEM (the thresholds, rarely read past it, come
+// through the read-only cache), draws the random words of each (slot, site,
+// replica) once -- shared by the nw sample words, as the reference shares them
+// across samples (main.cu:1430) -- and updates all (word, site, replica, slot)
+// words of its tile in memory order, so that consecutive lanes touch
+// consecutive words of a site.  The Philox thread index of (slot b, site i,
+// replica r) is (b*V + i)*NR + r.  The draws (draw_ids) are most of a pass of
+// few sample words: six words a thread, an 8-bit pre-search and the thresholds
+// in SMEM took 77 us a
+// sweep of the 12^2 x 48 tube (24 temperatures, 4 replicas) with 128 samples,
+// 55 now, with 4096 313 and 258.  (A CTA that kept the tables for its next tile
+// spilled registers: 4 % slower.)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void sp_pass_body(const SpDev &d, const uint4 *ctr, int off, int n, int tile,
                                              unsigned char *smem) {
   const int NB = d.NB, NR = d.NR, kt = d.kt, V = d.V;
-  u64 *s_cum = reinterpret_cast<u64 *>(smem);
-  uint16_t *s_pre = reinterpret_cast<uint16_t *>(s_cum + NB * 256);
-  u64 *s_rnd = reinterpret_cast<u64 *>(s_pre + NB * 256);
-  int *s_nb = reinterpret_cast<int *>(s_rnd + 3 * NB * kt * NR);  // [kt][7]: site, 6 neighbours
+  const int plane = NB * kt * NR;
+  uint8_t *s_pre = smem;
+  u64 *s_id1 = reinterpret_cast<u64 *>(s_pre + (size_t)NB * kPre11Stride), *s_id2 = s_id1 + plane;
+  uint16_t *s_queue = reinterpret_cast<uint16_t *>(s_id2 + plane);
+  int *s_nb = reinterpret_cast<int *>(s_queue + 4 * plane);  // [kt][7]: site, 6 neighbours
+  __shared__ int s_cnt[2];
   const int tid = threadIdx.x, nth = blockDim.x;
   const int k0 = tile * kt;
   {
-    const uint4 *cs = reinterpret_cast<const uint4 *>(d.cum);
-    uint4 *cd = reinterpret_cast<uint4 *>(s_cum);
-    for (int i = tid; i < NB * 128; i += nth) cd[i] = cs[i];
-    const uint4 *ps = reinterpret_cast<const uint4 *>(d.pre);
+    const uint4 *ps = reinterpret_cast<const uint4 *>(d.pre11);
     uint4 *pd = reinterpret_cast<uint4 *>(s_pre);
-    for (int i = tid; i < NB * 32; i += nth) pd[i] = ps[i];
+    for (int i = tid; i < NB * (kPre11Stride / 16); i += nth) pd[i] = ps[i];
   }
   for (int i = tid; i < kt * 7; i += nth) {
     const int kk = i / 7, f = i % 7, k = k0 + kk;
@@ -70,26 +75,22 @@ __device__ __forceinline__ void sp_pass_body(const SpDev &d, const uint4 *ctr, i
   __syncthreads();
   // random words at [site of the tile][replica][slot]: the update phase's
   // consecutive lanes (consecutive slots) then read consecutive words
-  const int plane = NB * kt * NR;
-  for (int t = tid; t < plane; t += nth) {
-    const int b = t % NB, r = (t / NB) % NR, kk = t / (NB * NR);
-    if (k0 + kk >= n) continue;
-    const int site = s_nb[kk * 7];
-    const uint32_t tp = (uint32_t)(((size_t)b * V + site) * NR + r);
-    const uint4 c = ctr[r];
-    const uint32_t key = d.keys[r];
-    const u64 *cum = s_cum + b * 256;
-    const uint16_t *pre = s_pre + b * 256;
-    uint32_t w[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) w[q] = rnd_word(c.x + q, c.y, c.z + tp, c.w, key, tp, cum, pre);
-    s_rnd[t] = ((u64)w[0] << 32) | w[1];
-    s_rnd[plane + t] = ((u64)w[2] << 32) | w[3];
-    s_rnd[2 * plane + t] = ((u64)w[4] << 32) | w[5];
-  }
-  __syncthreads();
+  const uint32_t mB = 0xFFFFFFFFu / (uint32_t)NB + 1u, mR = NR > 1 ? 0xFFFFFFFFu / (uint32_t)NR + 1u : 0u;
+  draw_ids(
+      plane,
+      [&](int t, uint4 &c, uint32_t &key, uint32_t &tp, int &b) {
+        const int q = (int)__umulhi((uint32_t)t, mB);  // t / NB, exact: t NB < 2^32
+        const int kk = NR > 1 ? (int)__umulhi((uint32_t)q, mR) : q, r = q - kk * NR;
+        b = t - q * NB;
+        tp = (uint32_t)(((size_t)b * V + s_nb[kk * 7]) * NR + r);
+        c = ctr[r];
+        key = d.keys[r];
+        return k0 + kk < n;
+      },
+      [&](int b, uint32_t hi, uint32_t lo) { return lut_byte11(hi, lo, d.cum + b * 256, s_pre + b * kPre11Stride); },
+      s_id1, s_id2, s_queue, s_cnt);
   // Update phase.  A thread keeps one (replica, slot) column (lg) for the
-  // whole loop -- its three random words stay in registers per site -- and
+  // whole loop -- its random words stay in registers per site -- and
   // walks (site of the tile, sample word) with a stride of nth/G groups, so
   // the G lanes of a group touch the G consecutive words of one site.
   const int G = NR * NB;
@@ -121,12 +122,11 @@ __device__ __forceinline__ void sp_pass_body(const SpDev &d, const uint4 *ctr, i
           f1[q] = sv.y ^ jq ^ nq.y;
         }
         const int o = (kk * NR + r) * NB + b;
-        const ulonglong2 r0 = *reinterpret_cast<const ulonglong2 *>(s_rnd + o);
-        const ulonglong2 r1 = *reinterpret_cast<const ulonglong2 *>(s_rnd + plane + o);
-        const ulonglong2 r2 = *reinterpret_cast<const ulonglong2 *>(s_rnd + 2 * plane + o);
+        const ulonglong2 i1 = *reinterpret_cast<const ulonglong2 *>(s_id1 + o);
+        const ulonglong2 i2 = *reinterpret_cast<const ulonglong2 *>(s_id2 + o);
         ulonglong2 out;
-        out.x = sv.x ^ flip_mask(f0, r0.x, r1.x, r2.x);
-        out.y = sv.y ^ flip_mask(f1, r0.y, r1.y, r2.y);
+        out.x = sv.x ^ flip_mask_id(f0, i1.x, i2.x);
+        out.y = sv.y ^ flip_mask_id(f1, i1.y, i2.y);
         Sw[(size_t)site * G2] = out;
         for (kk += step; kk >= nk; kk -= nk) ++w;
       }
@@ -149,7 +149,7 @@ __device__ __forceinline__ void sp_pass_body(const SpDev &d, const uint4 *ctr, i
 #pragma unroll
       for (int q = 0; q < 6; ++q) f[q] = sv ^ __ldg(Jp + q) ^ Sw[(size_t)sn[q + 1] * G];
       const int o = (kk * NR + r) * NB + b;
-      Sw[(size_t)site * G] = sv ^ flip_mask(f, s_rnd[o], s_rnd[plane + o], s_rnd[2 * plane + o]);
+      Sw[(size_t)site * G] = sv ^ flip_mask_id(f, s_id1[o], s_id2[o]);
       for (kk += step; kk >= nk; kk -= nk) ++w;
     }
   }
@@ -1497,7 +1497,7 @@ __global__ void k_sp_measure_u2(const __grid_constant__ SpDev d, int from_e) {
 size_t sp_cluster_smem(int L, int Lz);
 
 size_t sp_sweep_smem(int NB, int NR, int kt) {
-  return (size_t)NB * 256 * 10 + (size_t)3 * NB * kt * NR * 8 + (size_t)kt * 7 * 4;
+  return (size_t)NB * kPre11Stride + (size_t)NB * kt * NR * (16 + 8) + (size_t)kt * 7 * 4;
 }
 size_t sp_items_smem(int NB, int threads) { return (size_t)NB * kPre11Stride + threads / 32 * sizeof(ItemsWarp); }
 
@@ -1518,28 +1518,30 @@ int sp_items_grid(int NB) {
 int sp_kt(int NB, int NR, int nsites_colour) {
   int kt = 1;
   while (kt < 64 && NB * kt * NR < 256) kt <<= 1;
-  const size_t lim = 227 * 1024 - 512;  // room for the batched kernels' static SMEM
+  const size_t lim = 227 * 1024 - 512;  // room for the kernels' static SMEM
   while (kt > 1 && sp_sweep_smem(NB, NR, kt) > lim) kt >>= 1;
   if (sp_sweep_smem(NB, NR, kt) > lim) return 0;
-  while (kt < 64 && sp_sweep_smem(NB, NR, 2 * kt) <= lim && (nsites_colour + 2 * kt - 1) / (2 * kt) >= 2 * 152)
+  auto two = [&](int k) { return 2 * (sp_sweep_smem(NB, NR, k) + 1536) <= 228 * 1024; };  // CTAs an SM
+  while (kt < 32 && sp_sweep_smem(NB, NR, 2 * kt) <= lim && (two(2 * kt) || !two(kt)) &&
+         (nsites_colour + 2 * kt - 1) / (2 * kt) >= 2 * 152)
     kt <<= 1;
-  // In between, where whole rounds of the GPU (two CTAs an SM where their SMEM
-  // allows) make a colour shorter: 12^2 x 48 with
-  // 24 temperatures and 4 replicas takes 370 us a sweep of 4096 samples with 8
-  // sites a tile (1.4 rounds), 313 with 12 (0.95), of 256 samples 94 and 82;
-  // 24^2 x 96 with 32 temperatures and 256 samples 930 and 901.
+  // In between, where whole rounds of the GPU make a colour shorter: 12^2 x 48
+  // with 24 temperatures and 4 replicas takes 370 us a sweep of 4096 samples
+  // with 8 sites a tile (1.4 rounds), 313 with 12 (0.95), of 256 samples 94 and
+  // 82.  Never so wide that one CTA an SM is left: 24^2 x 96, 32 temperatures,
+  // 128 samples takes 444 us with 16 sites, 571 with 24.
   auto rounds = [&](int k) {
-    const int slots = 152 * (2 * (sp_sweep_smem(NB, NR, k) + 1536) <= 228 * 1024 ? 2 : 1), tiles = (nsites_colour + k - 1) / k;
+    const int slots = two(k) ? 2 * 152 : 152, tiles = (nsites_colour + k - 1) / k;
     return (tiles + slots - 1) / slots;
   };
   int best = kt;
-  for (int k = kt + 1; k < 2 * kt && k < 64 && sp_sweep_smem(NB, NR, k) <= lim; ++k)
+  for (int k = kt + 1; k < 2 * kt && k < 64 && sp_sweep_smem(NB, NR, k) <= lim && two(k) == two(kt); ++k)
     if (rounds(k) * k < rounds(best) * best) best = k;
   return best;
 }
 
 cudaError_t sp_setup() {
-  cudaError_t e = cudaFuncSetAttribute(k_sp_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  cudaError_t e = cudaFuncSetAttribute(k_sp_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 512);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_pass_items, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   const int cl = (int)std::max(kRunSmem, (size_t)kSpClusterMaxV * 7);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, cl);
@@ -1818,7 +1820,6 @@ int ea_sp_create(const ea_sp_geom *gp, int32_t device, ea_sp **out) {
   SOWN(d.S, nw * V * G);
   { unsigned long long *p; SOWN(p, nw * V * 6); d.J = p; }
   { unsigned long long *p; SOWN(p, (size_t)d.NB * 256); d.cum = p; }
-  { uint16_t *p; SOWN(p, (size_t)d.NB * 256); d.pre = p; }
   { uint8_t *p; SOWN(p, (size_t)d.NB * kPre11Stride); d.pre11 = p; }
   SOWN(d.ctr, (size_t)d.NR);
   SOWN(d.ctrs, (size_t)kCtrPasses * d.NR);
@@ -1949,11 +1950,9 @@ int ea_sp_set_temperatures(ea_sp *c, const double *betas, const uint64_t *cum) {
   const int NB = c->d.NB;
   for (int i = 0; i + 1 < NB; ++i)
     if (betas[i] < betas[i + 1]) return spfail(EA_ERR_ARG, "betas must be sorted from largest to smallest");
-  std::vector<uint16_t> pre((size_t)NB * 256);
   std::vector<uint8_t> pre11((size_t)NB * kPre11Stride);
   for (int b = 0; b < NB; ++b) {
     if (cum[(size_t)b * 256 + 255] != ~0ULL) return spfail(EA_ERR_ARG, "threshold 255 of beta %d is not 2^64-1", b);
-    presearch8(cum + (size_t)b * 256, pre.data() + (size_t)b * 256);
     presearch(cum + (size_t)b * 256, 11, pre11.data() + (size_t)b * kPre11Stride);
   }
   std::vector<double> tab;
@@ -1965,7 +1964,6 @@ int ea_sp_set_temperatures(ea_sp *c, const double *betas, const uint64_t *cum) {
   SCU(cudaMalloc((void **)&c->exptab, sizeof(double) * std::max<size_t>(1, tab.size())));
   SCU(cudaMemcpyAsync(c->exptab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c->st));
   SCU(cudaMemcpyAsync((void *)c->d.cum, cum, sizeof(uint64_t) * 256 * NB, cudaMemcpyHostToDevice, c->st));
-  SCU(cudaMemcpyAsync((void *)c->d.pre, pre.data(), pre.size() * 2, cudaMemcpyHostToDevice, c->st));
   SCU(cudaMemcpyAsync((void *)c->d.pre11, pre11.data(), pre11.size(), cudaMemcpyHostToDevice, c->st));
   SCU(cudaMemcpyAsync((void *)c->d.betas, betas, sizeof(double) * NB, cudaMemcpyHostToDevice, c->st));
   SCU(cudaMemcpyAsync((void *)c->d.expoff, c->expoff.data(), sizeof(int32_t) * NB, cudaMemcpyHostToDevice, c->st));
@@ -2856,7 +2854,7 @@ int ea_sp_job_bytes(const ea_sp_geom *gp, const ea_cadence *cad, const double *b
   const uint64_t V = g.V, NB = gp->nbetas, NR = gp->nrep, nw = gp->nwords, G = NR * NB;
   add(V * 24); add(V * 4);                                   // neighbour table, colour lists
   add(nw * V * G * 8); add(nw * V * 48);                     // spins, couplings
-  add(NB * 256 * 8); add(NB * 256 * 2); add(NB * kPre11Stride);  // thresholds, pre-searches
+  add(NB * 256 * 8); add(NB * kPre11Stride);  // thresholds, pre-search
   add(NR * 16); add(NR * 16 * kCtrPasses); add(NR * 4); add(NR * sizeof(ea_hq)); add(NR * sizeof(ea_xoshiro)); add(8);
   add(nw * 64 * G * 4); add(nw * 64 * G * 4); add(nw * 64 * G);   // U2, E, slot permutations
   add(nw * 64 * NR * (NB - 1) * 4); add(nw * NR * (NB - 1) * 8); // accepted swaps, lane masks

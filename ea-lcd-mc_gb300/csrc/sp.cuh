@@ -59,8 +59,7 @@ struct SpDev {
   unsigned long long *S;             // [nw][V][NR][NB] spin words
   const unsigned long long *J;       // [nw][V][6] coupling words
   const unsigned long long *cum;     // [NB][256] thresholds
-  const uint16_t *pre;               // [NB][256] 8-bit pre-search
-  const uint8_t *pre11;              // [NB][2064] 11-bit pre-search (the per-item pass)
+  const uint8_t *pre11;              // [NB][2064] 11-bit pre-search
   uint4 *ctr;                        // [NR] Philox counters of the last pass
   uint4 *ctrs;                       // [kCtrPasses][NR] those of the passes drawn ahead
   const uint32_t *keys;              // [NR]
