@@ -34,12 +34,12 @@ WORKLOAD = "L24_Lz192_OBC_NB32_NR8_ns31_ptfr1_houfr5"
 # DRAM bytes (read + write) of one k_sweep launch of this workload, from the
 # ncu capture of one k_sweep launch of the bench (its full-set capture)
 KSWEEP_DRAM_BYTES = 140.6e6
-# The integer-op model of the fused sweep (the Philox4x32-10 rounds, the
-# post-mix and rotation of a random word, the threshold search per byte, the
-# bit-sliced update per word), in 32-bit operations: 6 Philox calls of
-# 78 + 18 + 4 ops and 24 searches of 6 + 6 x (iterations) ops per random
-# triple, 60 ops per updated word.
-OPS_TRIPLE_BASE, OPS_PER_ITER, OPS_WORD = 6 * (78 + 18 + 4) + 24 * 6, 24 * 6, 60
+# The integer-op model of a pass (the Philox4x32-10 rounds, the post-mix and
+# rotation of a random word, the threshold search per byte, the bit-sliced
+# update per word), in 32-bit operations: a 32-bit random word is a Philox call
+# of 78 + 18 + 4 ops and 4 searches of 6 + 6 x (iterations) ops, a random triple
+# draws 2 to 6 of them (draws_per_triple), 60 ops per updated word.
+OPS_DRAW_BASE, OPS_PER_ITER, OPS_WORD = (78 + 18 + 4) + 4 * 6, 4 * 6, 60
 # mixed-geometry workload of the batched vs plain comparison: every
 # L x (Lz/L) x boundary x NT combination is one job class
 # (36 geometry classes; either 36 jobs of 32 samples or 288 jobs of 4)
@@ -63,44 +63,12 @@ def peaks():
         return 6800.0, "fallback"
 
 
-def lut_search_iters(cum):
-    """Expected iterations of the threshold search of one byte for a uniform
-    64-bit R: the bisection between the bounds of the 8-bit pre-search
-    (lut_byte in kernels_dev.cuh), weighted by the exact probability of each
-    result byte within each of the 256 pre-search buckets."""
-    c = [int(x) for x in np.asarray(cum, np.uint64)]
-
-    def first_above(R):
-        n = 0
-        while n < 255 and not R < c[n]:
-            n += 1
-        return n
-
-    tot = 0
-    for t in range(256):
-        lo_r, hi_r = t << 56, ((t + 1) << 56) - 1
-        a0, b0 = first_above(lo_r), first_above(hi_r)
-        for n in range(a0, b0 + 1):
-            lo = max(c[n - 1] if n > 0 else 0, lo_r)
-            hi = hi_r if n == 255 else min(c[n] - 1, hi_r)
-            if hi < lo:
-                continue
-            a, b, d = a0, b0, 0
-            while a < b:
-                m = (a + b) >> 1
-                d += 1
-                if n <= m:
-                    b = m
-                else:
-                    a = m + 1
-            tot += (hi - lo + 1) * d
-    return tot / float(1 << 64)
-
-
 def lut_search_iters11(cum):
-    """The same expectation for the 11-bit pre-search of the per-item pass
-    (lut_byte11): bucket t = R >> 53 searches [pre[t], pre[t+1]], pre[t] the
-    first byte whose threshold is above t << 53."""
+    """Expected iterations of the threshold search of one byte for a uniform
+    64-bit R: the bisection left by the 11-bit pre-search (lut_byte11), weighted
+    by the exact probability of each result byte within each bucket: bucket
+    t = R >> 53 searches [pre[t], pre[t+1]], pre[t] the first byte whose
+    threshold is above t << 53."""
     c = [int(x) for x in np.asarray(cum, np.uint64)]
 
     def first_above(R):
@@ -137,12 +105,24 @@ def lut_search_iters11(cum):
     return tot / float(1 << 64)
 
 
-def int_ops(cums, triples, words, iters=lut_search_iters):
+def draws_per_triple(cum):
+    """32-bit words drawn of a random triple (b0, b1, b2): both halves of b0, a
+    half of b1 where b0's has bits, of b2 where b0 & b1's has (a half is 4 bytes
+    of the threshold search; the rotations are left out)."""
+    c = np.asarray(cum, np.uint64).astype(np.float64) / 2.0 ** 64
+    p = np.diff(np.concatenate([[0.0], c]))
+    n = np.arange(256)
+    none01 = float((p[:, None] * p[None, :])[(n[:, None] & n[None, :]) == 0].sum())
+    return 2.0 * (1.0 + (1.0 - p[0] ** 4) + (1.0 - none01 ** 4))
+
+
+def int_ops(cums, triples, words):
     """32-bit integer operations of a launch that draws `triples` random
     triples (spread evenly over the temperatures of `cums`) and updates
     `words` spin words."""
-    e = float(np.mean([iters(c) for c in cums]))
-    return triples * (OPS_TRIPLE_BASE + OPS_PER_ITER * e) + words * OPS_WORD, e
+    e = float(np.mean([lut_search_iters11(c) for c in cums]))
+    draws = float(np.mean([draws_per_triple(c) for c in cums]))
+    return triples * draws * (OPS_DRAW_BASE + OPS_PER_ITER * e) + words * OPS_WORD, e
 
 
 _int_peak = None
@@ -309,8 +289,8 @@ def run_mixed(args, dev, torch, eagb, ns, copies):
     """Batched persistent form vs plain form (one job per launch sequence, every
     job on its own stream, all enqueued before waiting; and the same jobs one
     geometry after another) on the same mixed workload, from twin initial
-    states; one step = one bin of itmax=1 for every job.  Inputs (spins +
-    uniforms) are far larger than L2."""
+    states; one step = one bin of itmax=1 for every job.  Inputs are far
+    larger than L2."""
     su_step = 0
     plain, batched = mixed_jobs(eagb, dev, ns, copies), mixed_jobs(eagb, dev, ns, copies)
     for j in plain:
@@ -371,7 +351,7 @@ def run_mixed(args, dev, torch, eagb, ns, copies):
             "plain_ms_per_step": ms_plain / args.steps, "batched_ms_per_step": ms_batch / args.steps,
             "spin_updates_per_step": su_step, "bit_exact_plain_vs_batched": bool(same), "tile": tile,
             "graph": "sweep/energy/tempering cycle replayed as a CUDA graph",
-            "l2": "inputs larger than L2 (spins ~0.3 GB, uniforms ~9 GB)"}
+            "l2": "inputs larger than L2 (spins ~0.3 GB)"}
 
 
 # serving stream: Poisson arrivals of jobs with L in {8, 16} (the multiples of
@@ -597,14 +577,12 @@ def run_sp(args, dev, torch, eagb):
             # (read + write it, read it once as a neighbour) + 48 B of
             # couplings per (site, sample word); integer ops of the random
             # triples (one per site, replica and slot, shared by the words)
-            # and the word updates, the search iterations of the pass's
-            # pre-search (11 bits for the per-item pass, 8 for tiles)
+            # and the word updates
             hbm, _ = peaks()
             ipk_alu, _ = int_peak(eagb, dev)
             words = V * NR * len(d["betas"]) * nw
             pbytes = words * 24 + V * nw * 48
-            ops, e_it = int_ops(d["cum"], V * NR * len(d["betas"]), words,
-                                lut_search_iters11 if kt == 0 else lut_search_iters)
+            ops, e_it = int_ops(d["cum"], V * NR * len(d["betas"]), words)
             hf = pbytes / (pass_us[0] * 1e-6) / 1e9 / hbm
             inf = ops / (pass_us[0] * 1e-6) / ipk_alu
             rec["pass"] = {"form": "per-item" if kt == 0 else "tiles of %d sites" % kt,
@@ -704,8 +682,7 @@ def run_mixed_sp(args, dev, torch, eagb, nwords=SPMIX_WORDS, steps=2):
 def run_no_cluster(args, dev, torch, eagb):
     """The headline geometry without cluster moves: one step = 5 x (sweep +
     energy + parallel tempering) + the energy measurement, so the fused sweep
-    is most of the step (the cluster uniforms, which bound the full step, are
-    not drawn).  Device-timed, L2 flushed between steps."""
+    is most of the step (no cluster coins are drawn).  Device-timed, L2 flushed between steps."""
     d = np.load(LUT)
     betas, cum = d["betas"], d["cum"]
     NB = len(betas)
@@ -873,8 +850,8 @@ def run_ours(args, rank, world, local):
         step()
     job.sync()
     # timed region: device events on the job's stream around all K steps,
-    # joined with the generator stream at the end so that every uniform drawn
-    # inside the region is counted; the L2 flushes between steps are timed
+    # joined with its other streams at the end so that all work enqueued inside
+    # the region is counted; the L2 flushes between steps are timed
     # by their own events and taken out
     t_beg, t_end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     fl = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
@@ -982,12 +959,12 @@ def run_ours(args, rank, world, local):
     # face merge, compression, selection + flip), per lattice site of the
     # nclust = 16 colder temperatures, 31 samples and 2 replica groups:
     # 3/8 B of overlap bits (two replicas read, one word written), 4 B label
-    # written, 4 B label read at the flip, 8 B uniform of the site's cluster
+    # written, 4 B label read at the flip, 1/8 B coin of the site's cluster
     # (counted for every site: the generator draws one per site), and the two
     # replicas' spin bits read and written (1/2 B)
     nclust = 16
     cl_sites = V * nclust * NS * 2
-    cl_bytes_site = 3.0 / 8 + 4 + 4 + 8 + 0.5
+    cl_bytes_site = 3.0 / 8 + 4 + 4 + 1.0 / 8 + 0.5
     cl_move_ms = cl_ms.value / max(1, args.steps)
     cl_achieved = cl_sites * cl_bytes_site / (cl_move_ms * 1e-3) / 1e9
     roof = {"bound": "int32" if int_frac > hbm_frac else "hbm",
@@ -1026,7 +1003,9 @@ def run_ours(args, rank, world, local):
                         "spins after that step's energies are read (ea_commit_staged_spins)",
                 "serial_value": e2e_serial,
                 "serial_form": "the copy on the job's stream ahead of the step's kernels (ea_upload_spins_async)"},
-        "gpu_launches": args.steps * (HOUFR * 6 + 1 + 2 * 4 + 3),
+        # counters, 5 x (2 half-sweeps + tempering), the move's start and 5
+        # kernels a replica group, the energy and its measurement
+        "gpu_launches": args.steps * (1 + HOUFR * 3 + 1 + 2 * 5 + 2),
         "roofline": roof,
         "kernel_ms": {"sweep": sw_ms.value, "pt": pt_ms.value, "cluster": cl_ms.value,
                       "uniforms_overlapped": rg_ms.value, "step_total": ms},
@@ -1051,8 +1030,8 @@ def run_ours(args, rank, world, local):
 
 
 def main():
-    # more hardware queues, so that the plain form's per-job streams and the
-    # per-job cluster-uniform generators can run side by side
+    # more hardware queues, so that the plain form's per-job streams can run
+    # side by side
     os.environ.setdefault("CUDA_DEVICE_MAX_CONNECTIONS", "32")
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -1066,7 +1045,7 @@ def main():
     ap.add_argument("--mix-only", default="", choices=["", "plain", "batched"],
                     help="only two bins of the 36-job x 32-sample multispin mix in this form (for profilers)")
     ap.add_argument("--rng-sms", type=int, default=-1,
-                    help="SMs of the cluster-uniform generator's partition for the headline job (-1: automatic)")
+                    help="ea_set_rng_sms of the headline job (-1: automatic; the coins are drawn on every SM)")
     ap.add_argument("--small-sp", type=int, default=0, metavar="N",
                     help="only the small sample-packed batching leg with N jobs (prints its record)")
     ap.add_argument("--serve-config5", type=int, default=0, metavar="N",

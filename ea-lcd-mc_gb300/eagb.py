@@ -291,8 +291,9 @@ class Job:
         _ck(lib().ea_join(self.ctx))
 
     def set_rng_sms(self, nsm):
-        """SM split between the cluster-uniform generator and the job (0: none,
-        negative: automatic); before the first cluster move only."""
+        """The SM number ea_get_rng_sms reports (0: none, negative: automatic);
+        before the first cluster move only.  The cluster coins are drawn on
+        every SM whatever it is."""
         _ck(lib().ea_set_rng_sms(self.ctx, int(nsm)))
 
     def rng_sms(self):
