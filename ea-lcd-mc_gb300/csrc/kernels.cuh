@@ -117,7 +117,7 @@ constexpr size_t kSweepMax = 227 * 1024 - 64;  // less the kernel's static SMEM
 // Bits of the pre-search tables, so that two CTAs of a half-sweep fit an SM:
 // the more, the fewer threshold searches (0.22 steps a byte with 8 bits, 0.04
 // with 11, on a ladder of 32 temperatures from 0.7 to 1.6: a half-sweep of the
-// 24^2 x 192 tube takes 104, 100, 96, 93 us with 8, 9, 10, 11 bits, of 8^3
+// 24^2 x 192 tube takes 104, 100, 96, 93 us with 8, 9, 10, 11 bits, of 8^2 x 16
 // 12.5, 11.1, 10.4, 9.5).
 inline int sweep_pre_bits(int NB) { return NB <= 40 ? 11 : NB <= 72 ? 10 : NB <= 128 ? 9 : 8; }
 // Dynamic SMEM of a fused half-sweep CTA: the flip mask's two words of every

@@ -277,12 +277,13 @@ __device__ __forceinline__ void draw_ids(int ntrip, Item &&item, Byte &&byte, u6
 // of each (beta, half-site, replica) once -- they are shared by all samples, as
 // the reference's random buffer has no sample axis (main.cu:1430) -- and then
 // updates every (sample, clone, half-site, replica) word of its tile, picking
-// the words of the clone's current temperature.  What bounds it is the draws,
-// about half of a CTA's time.  Six words a thread one after another through an
+// the words of the clone's current temperature.  What bounds it is issue and
+// latency (ALU pipe 60 % busy, 41 % of the warps); the draws were about half of
+// a CTA's time.  Six words a thread one after another through an
 // 8-bit pre-search, a chain of threshold reads behind most of them, took 104 us
 // a half-sweep of the 24^2 x 192 tube (32 temperatures, 8 replicas, 31
 // samples), draw_ids and 11 bits take 93; 16^2 x 48 with 40 temperatures
-// 27 -> 21 us, 16^2 x 64 with 24 17.4 -> 13.1, 8^3 11.9 -> 9.6.
+// 27 -> 21 us, 16^2 x 64 with 24 17.4 -> 13.1, 8^2 x 16 11.9 -> 9.6.
 // The random word indices
 // depend only on (beta, half-site, replica, counter), never on the launch
 // shape.  A tile of a job too small to fill the GPU is shared by nsplit CTAs,

@@ -31,7 +31,7 @@ __device__ __forceinline__ u64 transpose8(u64 x) {
 //          contacts are still pending in the next round.  A contact whose
 //          labels are equal is done for good: they lie in one tree, or are
 //          joined by the pending contact of the thread that stored one of
-//          them in this round.
+//          them in these rounds of the loop.
 //   jump:  every run walks to its root; roots do not change meanwhile, so one
 //          pass leaves every label a root.
 // until a hook pass finds no difference: 3 passes on overlaps of production
