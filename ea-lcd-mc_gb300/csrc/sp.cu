@@ -953,20 +953,21 @@ __device__ __forceinline__ void sp_slab_merge_body(const SpDev &d, long long t) 
   }
 }
 
-// Roots and their coins: t = unit * V + site.
-__device__ __forceinline__ void sp_slab_roots_body(const SpDev &d, int g, long long t) {
+// Coins of the roots, the sites that are their own label: t = unit * V + site.
+__device__ __forceinline__ void sp_slab_coins_body(const SpDev &d, int g, long long t) {
   const int V = d.V, nc = d.nclust;
   if (t >= (long long)d.nw * nc * 8 * V) return;
   const int unit = (int)(t / V), gi = (int)(t - (long long)unit * V);
   const int grp = unit & 7, lat = unit >> 3, b = lat % nc, w = lat / nc;
+  const uint32_t *Lu = d.slab_lab + (size_t)unit * 8 * V + gi;
+  uint32_t roots = 0, coins = 0;
+#pragma unroll
+  for (int l = 0; l < 8; ++l) roots |= (uint32_t)(Lu[(size_t)l * V] == (uint32_t)gi) << l;
+  if (!roots) return;
   const unsigned long long key = sp_cluster_key(d), mv = *d.move;
-  uint32_t *Lu = d.slab_lab + (size_t)unit * 8 * V;
-  uint32_t coins = 0;
-  for (int l = 0; l < 8; ++l) {
-    const uint32_t r = cc_find(Lu + (size_t)l * V, (uint32_t)gi);
-    Lu[(size_t)l * V + gi] = r;
-    if (r != (uint32_t)gi) continue;
-    const int lane = grp * 8 + l;
+#pragma unroll 1
+  for (uint32_t m = roots; m; m &= m - 1) {
+    const int l = __ffs(m) - 1, lane = grp * 8 + l;
     const uint32_t tag = (((uint32_t)(w * 64 + lane) << 6 | (uint32_t)b) << 1) | (uint32_t)g;
     uint32_t v0 = (uint32_t)mv, v1 = (uint32_t)(mv >> 32), v2 = (uint32_t)gi, v3 = tag;
     philox10(v0, v1, v2, v3, (uint32_t)key, (uint32_t)(key >> 32));
@@ -975,7 +976,12 @@ __device__ __forceinline__ void sp_slab_roots_body(const SpDev &d, int g, long l
   d.slab_coin[(size_t)unit * V + gi] = (uint8_t)coins;
 }
 
-// Flip bytes from the roots' coins, in place of the overlap bytes.
+// Flip bytes from the roots' coins, in place of the overlap bytes: the eight
+// samples' chains of labels followed together.  What bounds it and the coins
+// is the reads of the labels (2 x 453 MB at 24^2 x 192, 16 slots, one word: 133
+// us at the copy rate).  Writing every site's root back first, one chain after
+// another, took 389 us and the flip bytes 93; coins and flip bytes take
+// 101 and 191.
 __device__ __forceinline__ void sp_slab_flip_body(const SpDev &d, long long t) {
   const int V = d.V;
   if (t >= (long long)d.nw * d.nclust * 8 * V) return;
@@ -983,8 +989,23 @@ __device__ __forceinline__ void sp_slab_flip_body(const SpDev &d, long long t) {
   const int grp = unit & 7, lat = unit >> 3;
   const uint32_t *Lu = d.slab_lab + (size_t)unit * 8 * V;
   const uint8_t *Cu = d.slab_coin + (size_t)unit * V;
-  uint32_t f = 0;
-  for (int l = 0; l < 8; ++l) f |= (uint32_t)((Cu[Lu[(size_t)l * V + gi]] >> l) & 1u) << l;
+  uint32_t x[8], f = 0;
+#pragma unroll
+  for (int l = 0; l < 8; ++l) x[l] = Lu[(size_t)l * V + gi];
+  bool more;
+  do {
+    uint32_t y[8];
+    more = false;
+#pragma unroll
+    for (int l = 0; l < 8; ++l) y[l] = Lu[(size_t)l * V + x[l]];
+#pragma unroll
+    for (int l = 0; l < 8; ++l) {
+      more = more || y[l] != x[l];
+      x[l] = y[l];
+    }
+  } while (more);
+#pragma unroll
+  for (int l = 0; l < 8; ++l) f |= (uint32_t)((Cu[x[l]] >> l) & 1u) << l;
   reinterpret_cast<uint8_t *>(d.Q + (size_t)lat * V)[(size_t)gi * 8 + grp] = (uint8_t)f;
 }
 
@@ -1478,8 +1499,8 @@ __global__ void __launch_bounds__(1024, 1) k_sp_slab(const __grid_constant__ SpD
 __global__ void k_sp_slab_merge(const __grid_constant__ SpDev d) {
   sp_slab_merge_body(d, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
-__global__ void k_sp_slab_roots(const __grid_constant__ SpDev d, int g) {
-  sp_slab_roots_body(d, g, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void k_sp_slab_coins(const __grid_constant__ SpDev d, int g) {
+  sp_slab_coins_body(d, g, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void k_sp_slab_flip(const __grid_constant__ SpDev d) {
   sp_slab_flip_body(d, (long long)blockIdx.x * blockDim.x + threadIdx.x);
@@ -1648,7 +1669,7 @@ cudaError_t sp_launch_houdayer(const SpDev &d, cudaStream_t st) {
         default: k_sp_slab<1><<<grid, 1024, sm, st>>>(d);
       }
       k_sp_slab_merge<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d);
-      k_sp_slab_roots<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d, g);
+      k_sp_slab_coins<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d, g);
       k_sp_slab_flip<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d);
     } else {
       k_sp_cluster<<<(unsigned)(d.nw * d.nclust * 8), d.cthreads, sp_cluster_smem(d.L, d.Lz), st>>>(d, g);
