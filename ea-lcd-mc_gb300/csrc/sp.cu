@@ -897,9 +897,8 @@ __device__ __forceinline__ void sp_cluster_runs(const SpDev &d, int g, int blk, 
 // as a global site index into slab_lab [unit = lattice * 8 + group][8][V];
 // then the bonds between slabs joined by the lock-free union of the
 // multispin path (cc_unite: a root hung below the smaller one with
-// atomicMin), the labels compressed to their roots and the roots' coins
-// drawn (slab_coin [unit][V], one bit a sample), and the flip bytes written
-// in place of the overlap bytes.  Labels only decrease and never drop below
+// atomicMin), the roots' coins drawn (slab_coin [unit][V], one bit a sample),
+// and the flip bytes written in place of the overlap bytes.  Labels only decrease and never drop below
 // the smallest site of their cluster, so the roots -- and the coins and
 // flips -- are those of the one-CTA labelling.
 // ---------------------------------------------------------------------------
@@ -933,11 +932,19 @@ __device__ __forceinline__ void sp_slab_body(const SpDev &d, int unit, int sl, u
   }
 }
 
-// Bonds between slabs (each once, from its larger end): t = unit * V + site.
+// Bonds between slabs, each once, from its larger end, which is in a slab's
+// first plane or (the z wrap and the corner bonds between the open planes) in
+// the lattice's last: sp_face_planes of them a unit.  (Over all sites it took
+// 190 us at 24^2 x 192, 128 units, over 13 of its 192 planes 68.)
+__host__ __device__ inline int sp_face_planes(int Lz, int D) { return (Lz + D - 1) / D; }
 __device__ __forceinline__ void sp_slab_merge_body(const SpDev &d, long long t) {
-  const int V = d.V, L2 = d.L * d.L;
-  if (t >= (long long)d.nw * d.nclust * 8 * V) return;
-  const int unit = (int)(t / V), gi = (int)(t - (long long)unit * V);
+  const int V = d.V, L2 = d.L * d.L, nf = sp_face_planes(d.Lz, d.slabD), per = nf * L2;
+  if (t >= (long long)d.nw * d.nclust * 8 * per) return;
+  const int unit = (int)(t / per), e = (int)(t - (long long)unit * per), f = e / L2;
+  // planes D, 2 D, ... and the last one, which may be one of them
+  const int z = f + 1 < nf ? (f + 1) * d.slabD : d.Lz - 1;
+  if (f + 1 == nf && nf > 1 && z == (nf - 1) * d.slabD) return;
+  const int gi = z * L2 + e - f * L2;
   const int grp = unit & 7, lat = unit >> 3;
   const uint8_t *Qb = reinterpret_cast<const uint8_t *>(d.Q + (size_t)lat * V) + grp;
   const int s1 = gi / L2 / d.slabD;
@@ -1668,7 +1675,8 @@ cudaError_t sp_launch_houdayer(const SpDev &d, cudaStream_t st) {
         case 2: k_sp_slab<2><<<grid, 1024, sm, st>>>(d); break;
         default: k_sp_slab<1><<<grid, 1024, sm, st>>>(d);
       }
-      k_sp_slab_merge<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d);
+      const long long nm = (long long)nunits * sp_face_planes(d.Lz, d.slabD) * L2;
+      k_sp_slab_merge<<<(unsigned)((nm + 255) / 256), 256, 0, st>>>(d);
       k_sp_slab_coins<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d, g);
       k_sp_slab_flip<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d);
     } else {
