@@ -345,8 +345,11 @@ __device__ __forceinline__ void sp_pass_any(const SpDev &d, const uint4 *ctr, in
 constexpr int kEnPlanes = 8;
 constexpr int kEnSites = 42;      // sites a lane counts: 6 * 42 < 2^8
 constexpr int kEnMaxThreads = 288;
+constexpr size_t kEnSiteBytes = 80;      // 6 coupling words and 8 indices of a staged site
+constexpr size_t kEnSmem = 64 * 1024;    // of a block, in every form of the count
 
-// Fills the count's launch shape (d.en) for `chunk` sites a lane.
+// Fills the count's launch shape (d.en) for `chunk` sites a lane, fewer where
+// the lane groups of a few columns would stage more sites than kEnSmem holds.
 void sp_energy_shape(SpDev &d, int chunk) {
   EnShape &e = d.en;
   const int G = d.NR * d.NB;
@@ -356,14 +359,14 @@ void sp_energy_shape(SpDev &d, int chunk) {
   e.threads = (e.lanes + 31) / 32 * 32;
   for (int t = e.threads; t <= kEnMaxThreads; t += 32)  // the multiple of 32 that lane groups fill best
     if (t / e.lanes * e.lanes * e.threads >= e.threads / e.lanes * e.lanes * t) e.threads = t;
-  e.tile = std::min(e.threads / e.lanes * chunk, d.esites);
+  e.tile = std::min({e.threads / e.lanes * chunk, d.esites, (int)(kEnSmem / kEnSiteBytes)});
   e.ntile = (d.esites + e.tile - 1) / e.tile;
 }
 inline size_t en_blocks(const SpDev &d) { return (size_t)d.nw * d.en.ntile * d.en.nslice; }
 // The staged sites; then, in the same bytes, the groups' planes.  `threads` of
 // the launch's blocks.
 inline size_t en_smem(const SpDev &d, int threads) {
-  return std::max((size_t)d.en.tile * 80, (size_t)(threads / d.en.lanes) * d.en.lanes * kEnPlanes * 8);
+  return std::max((size_t)d.en.tile * kEnSiteBytes, (size_t)(threads / d.en.lanes) * d.en.lanes * kEnPlanes * 8);
 }
 
 // Sites per lane of the energy count: at most what the counters take, fewer
@@ -1575,7 +1578,7 @@ cudaError_t sp_setup() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, cl);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_sp_permute, cudaFuncAttributeMaxDynamicSharedMemorySize, kPermRows * 65 * 8);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_energy, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_energy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_pt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pt_smem(64));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_slab<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_slab<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
