@@ -422,13 +422,13 @@ __device__ __forceinline__ void sp_energy_body(const SpDev &d, int blk, unsigned
   const int part = blk / e.nslice, sl = blk - part * e.nslice, w = part / e.ntile, tl = part - w * e.ntile;
   const int s0 = tl * e.tile, ns = min(e.tile, d.esites - s0);
   u64 *sJ = reinterpret_cast<u64 *>(sm);                                   // [tile][6]
-  uint32_t *sN = reinterpret_cast<uint32_t *>(sJ + (size_t)6 * e.tile);    // [tile][8]: first words of the 6 neighbours and of the site
+  uint32_t *sN = reinterpret_cast<uint32_t *>(sJ + (size_t)6 * e.tile);    // [tile][8]: the 6 neighbours and the site
   const int32_t *c1 = d.col_sites + d.col_off[1];
   const u64 *Jw = d.J + (size_t)w * V * 6;
   for (int i = threadIdx.x; i < ns * 8; i += blockDim.x) {
     const int k = i >> 3, f = i & 7, site = d.epair ? __ldg(c1 + s0 + k) : s0 + k;
     if (f < 6) sJ[k * 6 + f] = __ldg(Jw + (size_t)site * 6 + f);
-    if (f < 7) sN[i] = (uint32_t)(f < 6 ? __ldg(d.nb + (size_t)site * 6 + f) : site) * (uint32_t)G;
+    if (f < 7) sN[i] = (uint32_t)(f < 6 ? __ldg(d.nb + (size_t)site * 6 + f) : site);
   }
   __syncthreads();
   const int groups = blockDim.x / e.lanes, g = threadIdx.x / e.lanes, ln = threadIdx.x - g * e.lanes;
@@ -437,15 +437,18 @@ __device__ __forceinline__ void sp_energy_body(const SpDev &d, int blk, unsigned
 #pragma unroll
   for (int p = 0; p < kEnPlanes; ++p) n.P[p] = 0;
   if (g < groups && col < G) {
-    const u64 *Sc = d.S + (size_t)w * V * G + col;
+    // a site's words G apart: the product in 64 bits (2^32 words are 34 GB)
+    const char *Sc = reinterpret_cast<const char *>(d.S + (size_t)w * V * G + col);
+    const uint32_t gb = (uint32_t)G * 8u;
+    auto word = [&](uint32_t i) { return *reinterpret_cast<const u64 *>(Sc + (u64)i * gb); };
     auto site = [&](int k) -> u64 {
       const uint4 *nb = reinterpret_cast<const uint4 *>(sN + k * 8);
       const ulonglong2 *J = reinterpret_cast<const ulonglong2 *>(sJ + k * 6);
       const uint4 na = nb[0], nc = nb[1];
-      const u64 sv = Sc[nc.z];
+      const u64 sv = word(nc.z);
       u64 f[6];
-      f[0] = Sc[na.x]; f[1] = Sc[na.y]; f[2] = Sc[na.z];
-      f[3] = Sc[na.w]; f[4] = Sc[nc.x]; f[5] = Sc[nc.y];
+      f[0] = word(na.x); f[1] = word(na.y); f[2] = word(na.z);
+      f[3] = word(na.w); f[4] = word(nc.x); f[5] = word(nc.y);
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const ulonglong2 j = J[q];
