@@ -1371,8 +1371,9 @@ __device__ bool sp_grid_sync(const SpPersistDev &p, unsigned &epoch) {
 
 __global__ void __launch_bounds__(kPersistThreads, 1) k_sp_persist(const __grid_constant__ SpPersistDev p) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ SpDev s_job[kPersistThreads / 64];
-  __shared__ int s_blk[kPersistThreads / 64];
+  // a job a sub-block (SPP_SUB of 256): with the move's kRunSmem they fill the SM
+  __shared__ SpDev s_job[kPersistThreads / 256];
+  __shared__ int s_blk[kPersistThreads / 256];
   const SpBatchDev &b = p.b;
   unsigned epoch = 0;
   auto energy = [&]() -> bool {
