@@ -32,6 +32,8 @@ int fail(int code, const char *fmt, ...) {
   vsnprintf(buf, sizeof(buf), fmt, ap);
   va_end(ap);
   g_err = buf;
+  // reported here: the next launch's check must not meet it again
+  if (code == EA_ERR_CUDA || code == EA_ERR_NOMEM) (void)cudaGetLastError();
   return code;
 }
 

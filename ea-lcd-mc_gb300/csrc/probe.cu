@@ -103,6 +103,7 @@ extern "C" int ea_probe_int32_rate(int32_t device, double *alu_ops_per_s, double
   if (out) cudaFree(out);
   if (e != cudaSuccess) {
     set_last_error(cudaGetErrorString(e));
+    (void)cudaGetLastError();
     return EA_ERR_CUDA;
   }
   return EA_OK;

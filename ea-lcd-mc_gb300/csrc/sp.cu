@@ -1730,6 +1730,7 @@ int spfail(int code, const char *fmt, ...) {
   vsnprintf(buf, sizeof(buf), fmt, ap);
   va_end(ap);
   set_last_error(buf);
+  if (code == EA_ERR_CUDA || code == EA_ERR_NOMEM) (void)cudaGetLastError();  // reported here, not by the next launch
   return code;
 }
 #define SCU(call)                                                                             \

@@ -168,6 +168,12 @@ static int an_fail(const char *m) {
   return EA_ERR_ARG;
 }
 
+static int an_cuda_fail(cudaError_t e) {
+  set_last_error(cudaGetErrorString(e));
+  (void)cudaGetLastError();  // reported here, not by the next launch
+  return EA_ERR_CUDA;
+}
+
 int ea_sp_plane_overlaps(ea_sp *job, int32_t nrep, int32_t *diff) {
   SpDev d;
   cudaStream_t st;
@@ -187,11 +193,7 @@ int ea_sp_plane_overlaps(ea_sp *job, int32_t nrep, int32_t *diff) {
   if (e == cudaSuccess) e = cudaMemcpyAsync(diff, dd, n * 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (dd) cudaFree(dd);
-  if (e != cudaSuccess) {
-    set_last_error(cudaGetErrorString(e));
-    return EA_ERR_CUDA;
-  }
-  return EA_OK;
+  return e == cudaSuccess ? EA_OK : an_cuda_fail(e);
 }
 
 int ea_sp_plane_correlations(ea_sp *job, int32_t nrep, int32_t dmax, double *C) {
@@ -218,11 +220,7 @@ int ea_sp_plane_correlations(ea_sp *job, int32_t nrep, int32_t dmax, double *C) 
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (dx) cudaFree(dx);
   if (dc) cudaFree(dc);
-  if (e != cudaSuccess) {
-    set_last_error(cudaGetErrorString(e));
-    return EA_ERR_CUDA;
-  }
-  return EA_OK;
+  return e == cudaSuccess ? EA_OK : an_cuda_fail(e);
 }
 
 }  // extern "C"
