@@ -710,27 +710,46 @@ int ea_parallel_tempering(ea_ctx *c) {
   return pt(c);
 }
 
+// The coins' buffers of a job, all of them or none.
+static int own_coins(ea_ctx *c) {
+  const Geometry &g = c->g;
+  JobDev &j = c->j;
+  const unsigned long long n = 2ull * g.V * g.NB * g.ns;
+  if (n >> 36) return fail(EA_ERR_NOMEM, "%llu cluster coins a move", n);
+  const int seg = xw_segments(n), w = xw_rows(n, seg);
+  uint32_t *bits = nullptr, *state = nullptr, *mat = nullptr;
+  unsigned long long *pos = nullptr;
+  cudaError_t e = dalloc(bits, xw_words(n));
+  if (e == cudaSuccess) e = dalloc(state, (size_t)seg * 6 * kXwStreams);
+  if (e == cudaSuccess) e = dalloc(pos, 3);
+  if (e == cudaSuccess) e = dalloc(mat, 2 * (size_t)kXwMat);
+  if (e == cudaSuccess && seg > 1) {
+    std::vector<uint32_t> m(2 * (size_t)kXwMat);
+    xw_jump(n / kXwStreams - w, m.data());
+    xw_jump(w, m.data() + kXwMat);
+    e = cudaMemcpy(mat, m.data(), m.size() * 4, cudaMemcpyHostToDevice);
+  }
+  if (e != cudaSuccess) {
+    for (void *p : {(void *)bits, (void *)state, (void *)pos, (void *)mat})
+      if (p) cudaFree(p);
+    return fail(EA_ERR_CUDA, "buffers of the cluster coins: %s", cudaGetErrorString(e));
+  }
+  j.xw_n = n;
+  j.xw_seg = seg;
+  j.xw_w = w;
+  j.xw_bits = bits;
+  j.xw_state = state;
+  j.xw_pos = pos;
+  j.xw_jump = c->xw_mat = mat;
+  return EA_OK;
+}
+
 // st: the stream the move's kernels run on.
 static int ensure_cluster(ea_ctx *c, int nclust, cudaStream_t st) {
   const Geometry &g = c->g;
   JobDev &j = c->j;
-  if (!j.xw_bits) {
-    j.xw_n = 2ull * g.V * g.NB * g.ns;
-    if (j.xw_n >> 36) return fail(EA_ERR_NOMEM, "%llu cluster coins a move", j.xw_n);
-    j.xw_seg = xw_segments(j.xw_n);
-    j.xw_w = xw_rows(j.xw_n, j.xw_seg);
-    CU(dalloc(j.xw_bits, xw_words(j.xw_n)));
-    CU(dalloc(j.xw_state, (size_t)j.xw_seg * 6 * kXwStreams));
-    CU(dalloc(j.xw_pos, 3));
-    CU(dalloc(c->xw_mat, 2 * (size_t)kXwMat));
-    j.xw_jump = c->xw_mat;
-    if (j.xw_seg > 1) {
-      std::vector<uint32_t> m(2 * (size_t)kXwMat);
-      xw_jump(j.xw_n / kXwStreams - j.xw_w, m.data());
-      xw_jump(j.xw_w, m.data() + kXwMat);
-      CU(cudaMemcpy(c->xw_mat, m.data(), m.size() * 4, cudaMemcpyHostToDevice));
-    }
-  }
+  int rc;
+  if (!j.xw_bits && (rc = own_coins(c))) return rc;
   if (nclust > c->nclust_cap) {
     CU(cudaStreamSynchronize(c->st));
     if (c->label) cudaFree(c->label);

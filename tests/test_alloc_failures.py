@@ -53,3 +53,42 @@ def test_a_failure_is_reported_once(fake):
         sp_job(eb)
     job.sweeps(1)
     job.close()
+
+
+def same_buffers(eb, fk, make, calls, last):
+    """Every allocation of `calls` fails once, each on a job of its own.  The
+    calls `last` then leave the buffers of a job that met no failure."""
+    def held(k):
+        live, bytes_ = fk.fake_live(), fk.fake_live_bytes()
+        job = make()
+        failed = 0
+        fk.fake_fail_in(k)
+        for call in calls:
+            try:
+                call(job)
+            except eb.EAError:
+                failed += 1
+        fk.fake_fail_in(-1)
+        for call in last:
+            call(job)
+        got = fk.fake_live() - live, fk.fake_live_bytes() - bytes_
+        job.close()
+        assert (fk.fake_live(), fk.fake_live_bytes()) == (live, bytes_)
+        return got, failed
+
+    want, failed = held(-1)
+    assert not failed
+    k = 0
+    while True:
+        got, failed = held(k)
+        assert got == want, "allocation %d failed" % k
+        if not failed:
+            return k
+        k += 1
+
+
+def test_coins_of_a_move(fake):
+    eb, fk = fake
+    n = same_buffers(eb, fk, lambda: ms_job(eb), [lambda j: j.houdayer()], [lambda j: j.houdayer()])
+    assert n >= 7   # coins, states, positions, jumps; labels, selection, overlaps
+    same_buffers(eb, fk, lambda: ms_job(eb), [lambda j: j.run_bin(1, 1, 1, 1)], [lambda j: j.run_bin(1, 1, 1, 1)])
