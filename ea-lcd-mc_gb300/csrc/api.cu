@@ -756,6 +756,7 @@ static int ensure_cluster(ea_ctx *c, int nclust, cudaStream_t st) {
     if (c->sel) cudaFree(c->sel);
     if (c->Q) cudaFree(c->Q);
     c->label = nullptr; c->sel = nullptr; c->Q = nullptr;
+    c->nclust_cap = 0;  // until all three are there
     CU(dalloc(c->label, (size_t)g.V * nclust * g.ns));
     CU(dalloc(c->sel, (size_t)g.V / 32 * nclust * g.ns));
     CU(dalloc(c->Q, (size_t)2 * g.half * nclust * g.ns));
@@ -842,6 +843,7 @@ int ea_run_bin(ea_ctx *c, const ea_cadence *cad, double *avgE, uint8_t *hist, in
   if (maxit > c->hist_cap) {
     if (c->hist) cudaFree(c->hist);
     c->hist = nullptr;
+    c->hist_cap = 0;
     CU(dalloc(c->hist, nsr * maxit * g.NB));
     c->hist_cap = maxit;
   }
@@ -1336,6 +1338,7 @@ int ea_batch_run_bin(ea_batch *b, const ea_cadence *cad) {
     if (maxit > c->hist_cap) {
       if (c->hist) cudaFree(c->hist);
       c->hist = nullptr;
+      c->hist_cap = 0;
       CU(dalloc(c->hist, nsr * maxit * g.NB));
       c->hist_cap = maxit;
     }

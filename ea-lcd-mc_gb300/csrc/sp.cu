@@ -2332,6 +2332,7 @@ static int sp_cluster_prepare(ea_sp *c, int &nclust) {
     d.slab_lab = nullptr;
     d.slab_coin = nullptr;
     d.slabD = 0;
+    c->q_cap = 0;  // until all of them are there
     SCU(cudaMalloc((void **)&d.Q, sizeof(unsigned long long) * (size_t)d.nw * nclust * d.V));
     if (d.V > kSpClusterMaxV) {
       SCU(cudaMalloc((void **)&d.cscratch, sizeof(uint32_t) * sp_cluster_words(d.V) * (size_t)d.nw * nclust * 8));

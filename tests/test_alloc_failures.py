@@ -92,3 +92,35 @@ def test_coins_of_a_move(fake):
     n = same_buffers(eb, fk, lambda: ms_job(eb), [lambda j: j.houdayer()], [lambda j: j.houdayer()])
     assert n >= 7   # coins, states, positions, jumps; labels, selection, overlaps
     same_buffers(eb, fk, lambda: ms_job(eb), [lambda j: j.run_bin(1, 1, 1, 1)], [lambda j: j.run_bin(1, 1, 1, 1)])
+
+
+def test_buffers_that_grow(fake):
+    """A growth that fails leaves no stale capacity: a smaller move or a
+    shorter bin afterwards has its buffers."""
+    eb, fk = fake
+    for small, large in ((lambda j: j.houdayer(3), lambda j: j.houdayer(9)),
+                         (lambda j: j.run_bin(2, 1, 1, 1, cluster=False), lambda j: j.run_bin(5, 1, 1, 1, cluster=False))):
+        def grown(make):
+            job = make()
+            small(job)
+            return job
+        for make in (lambda: ms_job(eb), lambda: sp_job(eb), lambda: sp_job(eb, 33, 33, 6)):
+            k = 0
+            while True:
+                live, bytes_ = fk.fake_live(), fk.fake_live_bytes()
+                job = grown(make)
+                want = fk.fake_live() - live, fk.fake_live_bytes() - bytes_
+                fk.fake_fail_in(k)
+                try:
+                    large(job)
+                    failed = False
+                except eb.EAError:
+                    failed = True
+                fk.fake_fail_in(-1)
+                small(job)
+                got = fk.fake_live() - live, fk.fake_live_bytes() - bytes_
+                job.close()
+                if not failed:
+                    break
+                assert got == want, "allocation %d failed" % k
+                k += 1
