@@ -430,6 +430,7 @@ int ea_set_temperatures(ea_ctx *c, const double *betas, const uint64_t *cum) {
   CU(cudaMemcpyAsync((void *)c->j.betas, betas, sizeof(double) * g.NB, cudaMemcpyHostToDevice, c->st));
   CU(cudaMemcpyAsync((void *)c->j.expoff, c->expoff.data(), sizeof(int32_t) * g.NB, cudaMemcpyHostToDevice, c->st));
   CU(cudaStreamSynchronize(c->st));
+  c->have_temps = false;  // until the new table is in place
   if (c->exptab) cudaFree(c->exptab);
   c->exptab = nullptr;
   CU(dalloc(c->exptab, tab.size()));

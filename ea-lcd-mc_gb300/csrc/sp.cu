@@ -1996,6 +1996,7 @@ int ea_sp_set_temperatures(ea_sp *c, const double *betas, const uint64_t *cum) {
   pt_exp_table(betas, NB, tab, c->expoff);
   SCU(cudaSetDevice(c->device));
   SCU(cudaStreamSynchronize(c->st));
+  c->have_temps = false;  // until the new tables are in place
   if (c->exptab) cudaFree(c->exptab);
   c->exptab = nullptr;
   SCU(cudaMalloc((void **)&c->exptab, sizeof(double) * std::max<size_t>(1, tab.size())));

@@ -124,3 +124,20 @@ def test_buffers_that_grow(fake):
                     break
                 assert got == want, "allocation %d failed" % k
                 k += 1
+
+
+def test_temperatures_replaced(fake):
+    """New temperatures whose table finds no memory: the job has none, and
+    says so, until they are set again."""
+    eb, fk = fake
+    for job, nb, step in ((ms_job(eb), 24, lambda j: j.monte_carlo(1)), (sp_job(eb), 12, lambda j: j.sweeps(1))):
+        betas, cum = ladder(nb)
+        args = (job.ctx,) if hasattr(job, "ctx") else (job.h,)
+        call = eb.lib().ea_set_temperatures if hasattr(job, "ctx") else eb.lib().ea_sp_set_temperatures
+        fk.fake_fail_in(0)
+        assert call(*args, eb.P(betas), eb.P(cum)) != 0
+        with pytest.raises(eb.EAError, match="temperatures not set"):
+            step(job)
+        eb._ck(call(*args, eb.P(betas), eb.P(cum)))
+        step(job)
+        job.close()
