@@ -2380,10 +2380,10 @@ static bool sp_use_persist(int mode, const SpDev &) { return mode == EA_BIN_PERS
 static int sp_run_persist(ea_sp *c, const ea_cadence *cad) {
   const SpDev &d = c->d;
   if (d.ncol > kSpBatchMaxColours) return spfail(EA_ERR_ARG, "the persistent bin kernel takes up to %d colours", kSpBatchMaxColours);
-  if (!c->p_jobs) {
-    SCU(cudaMalloc((void **)&c->p_jobs, sizeof(SpDev)));
-    SCU(cudaMalloc((void **)&c->p_pre, sizeof(uint32_t) * SPB_COUNT * 2));
-    SCU(cudaMalloc((void **)&c->p_bar, sizeof(unsigned long long)));
+  if (!c->p_jobs) SCU(cudaMalloc((void **)&c->p_jobs, sizeof(SpDev)));
+  if (!c->p_pre) SCU(cudaMalloc((void **)&c->p_pre, sizeof(uint32_t) * SPB_COUNT * 2));
+  if (!c->p_bar) SCU(cudaMalloc((void **)&c->p_bar, sizeof(unsigned long long)));
+  if (!c->p_err) {
     SCU(cudaMalloc((void **)&c->p_err, sizeof(int)));
     SCU(cudaMemsetAsync(c->p_err, 0, sizeof(int), c->st));
   }

@@ -141,3 +141,15 @@ def test_temperatures_replaced(fake):
         eb._ck(call(*args, eb.P(betas), eb.P(cum)))
         step(job)
         job.close()
+
+
+def test_buffers_of_the_persistent_kernel(fake):
+    eb, fk = fake
+
+    def make():
+        job = sp_job(eb)
+        job.set_bin_kernel(eb.EA_BIN_PERSISTENT)
+        return job
+    bin_ = lambda j: j.run_bin(1, 1, 1, 1)
+    assert same_buffers(eb, fk, make, [bin_], [bin_]) >= 4
+    same_buffers(eb, fk, lambda: sp_job(eb), [bin_], [bin_])   # the resident kernel's
