@@ -434,7 +434,8 @@ int ea_set_temperatures(ea_ctx *c, const double *betas, const uint64_t *cum) {
   if (c->exptab) cudaFree(c->exptab);
   c->exptab = nullptr;
   CU(dalloc(c->exptab, tab.size()));
-  CU(cudaMemcpy(c->exptab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
+  CU(cudaMemcpyAsync(c->exptab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c->st));
+  CU(cudaStreamSynchronize(c->st));
   c->j.exptab = c->exptab;
   c->have_temps = true;
   return EA_OK;
@@ -711,7 +712,9 @@ int ea_parallel_tempering(ea_ctx *c) {
   return pt(c);
 }
 
-// The coins' buffers of a job, all of them or none.
+// The coins' buffers of a job, all of them or none.  The jump matrices are on
+// the device when it returns: a batch reads them on a stream of its own, whose
+// earlier bins a job that joins it does not wait for.
 static int own_coins(ea_ctx *c) {
   const Geometry &g = c->g;
   JobDev &j = c->j;
@@ -728,7 +731,8 @@ static int own_coins(ea_ctx *c) {
     std::vector<uint32_t> m(2 * (size_t)kXwMat);
     xw_jump(n / kXwStreams - w, m.data());
     xw_jump(w, m.data() + kXwMat);
-    e = cudaMemcpy(mat, m.data(), m.size() * 4, cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(mat, m.data(), m.size() * 4, cudaMemcpyHostToDevice, c->st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
   }
   if (e != cudaSuccess) {
     for (void *p : {(void *)bits, (void *)state, (void *)pos, (void *)mat})
@@ -1175,7 +1179,7 @@ int ea_batch_create(ea_ctx *const *jobs, int32_t njobs, int32_t tile, ea_batch *
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->up_ev[k], cudaEventDisableTiming);
   }
   if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_ctr, sizeof(uint32_t) * KB_COUNT);
-  if (e == cudaSuccess) e = cudaMemset(b->d_ctr, 0, sizeof(uint32_t) * KB_COUNT);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b->d_ctr, 0, sizeof(uint32_t) * KB_COUNT, b->bs);
   if (e == cudaSuccess && tile) e = batch_setup(b->NR, b->KT);
   if (e != cudaSuccess) { ea_batch_destroy(b); return fail(EA_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(e)); }
   if (!tile) {

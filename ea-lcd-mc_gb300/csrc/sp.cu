@@ -2392,9 +2392,9 @@ static int sp_run_persist(ea_sp *c, const ea_cadence *cad) {
   if (!c->p_valid || std::memcmp(&c->p_up, &d, sizeof(SpDev))) {
     std::vector<uint32_t> pre((size_t)SPB_COUNT * 2);
     for (int k = 0; k < SPB_COUNT; ++k) { pre[2 * k] = 0; pre[2 * k + 1] = cnt[k]; }
+    SCU(cudaMemcpyAsync(c->p_jobs, &d, sizeof(SpDev), cudaMemcpyHostToDevice, c->st));
+    SCU(cudaMemcpyAsync(c->p_pre, pre.data(), sizeof(uint32_t) * pre.size(), cudaMemcpyHostToDevice, c->st));
     SCU(cudaStreamSynchronize(c->st));
-    SCU(cudaMemcpy(c->p_jobs, &d, sizeof(SpDev), cudaMemcpyHostToDevice));
-    SCU(cudaMemcpy(c->p_pre, pre.data(), sizeof(uint32_t) * pre.size(), cudaMemcpyHostToDevice));
     c->p_up = d;
     c->p_valid = true;
   }
@@ -2659,9 +2659,9 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
   }
   if (k.up_jobs.size() != hj.size() || std::memcmp(k.up_jobs.data(), hj.data(), sizeof(SpDev) * n) ||
       k.up_pre != hp) {
+    SCU(cudaMemcpyAsync(k.d_jobs, hj.data(), sizeof(SpDev) * n, cudaMemcpyHostToDevice, bs));
+    SCU(cudaMemcpyAsync(k.d_pre, hp.data(), sizeof(uint32_t) * hp.size(), cudaMemcpyHostToDevice, bs));
     SCU(cudaStreamSynchronize(bs));
-    SCU(cudaMemcpy(k.d_jobs, hj.data(), sizeof(SpDev) * n, cudaMemcpyHostToDevice));
-    SCU(cudaMemcpy(k.d_pre, hp.data(), sizeof(uint32_t) * hp.size(), cudaMemcpyHostToDevice));
     k.up_jobs = hj;
     k.up_pre = hp;
   }
@@ -2752,7 +2752,7 @@ int ea_sp_batch_create(ea_sp *const *jobs, int32_t njobs, ea_sp_batch **out) {
   if (e == cudaSuccess) e = cudaMalloc((void **)&b->all.d_pre, sizeof(uint32_t) * SPB_COUNT * (b->jobs.size() + 1));
   if (e == cudaSuccess) e = cudaMalloc((void **)&b->p_bar, sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMalloc((void **)&b->p_err, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(b->p_err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(b->p_err, 0, sizeof(int), b->bs);
   for (SpClass &k : b->classes) {
     const size_t n = k.jobs.size();
     if (e == cudaSuccess) e = cudaMalloc((void **)&k.d_jobs, sizeof(SpDev) * n);
