@@ -953,8 +953,11 @@ struct ea_batch {
   cudaEvent_t up_ev[2] = {};
   int up_slot = 0;
   BatchDev bd{};
-  cudaGraphExec_t cycle = nullptr;
-  int cycle_ptfr = -1, cycle_n = -1;
+  // graphs of n tempering cycles of ptfr sweeps: the two lengths a bin's
+  // pieces have, or those of two cadences
+  struct Cycles { cudaGraphExec_t exec; int n, ptfr; };
+  Cycles cycles[2] = {};
+  int cycles_used = 0;  // the one launched last
   float tuned_ms = 0.f;  // autotuner: two sweeps of the chosen tile width
 };
 
@@ -992,6 +995,11 @@ static int batch_kt(const ea_batch *b, int forced) {
   for (int i = 2; i >= 0; --i)
     if (fits(c[i])) return c[i];
   return 0;
+}
+
+static void drop_cycles(ea_batch::Cycles &q) {
+  if (q.exec) cudaGraphExecDestroy(q.exec);
+  q.exec = nullptr;
 }
 
 // Uploads the jobs' descriptors and work lists when they changed.
@@ -1052,10 +1060,8 @@ static int batch_upload(ea_batch *b) {
   for (int k = 0; k < KB_COUNT; ++k) b->bd.chunk[k] = chunk[k];
   if (b->bd.total[KB_SWEEP] >= 8u * 304u) b->bd.chunk[KB_SWEEP] = 2;
   // the cycle graph holds the descriptor by value
-  if (std::memcmp(&old_bd, &b->bd, sizeof(BatchDev)) && b->cycle) {
-    cudaGraphExecDestroy(b->cycle);
-    b->cycle = nullptr;
-  }
+  if (std::memcmp(&old_bd, &b->bd, sizeof(BatchDev)))
+    for (auto &q : b->cycles) drop_cycles(q);
   return EA_OK;
 }
 
@@ -1194,7 +1200,7 @@ int ea_batch_destroy(ea_batch *b) {
   if (!b) return EA_OK;
   cudaSetDevice(b->device);
   if (b->bs) cudaStreamSynchronize(b->bs);
-  if (b->cycle) cudaGraphExecDestroy(b->cycle);
+  for (auto &q : b->cycles) drop_cycles(q);
   if (b->d_jobs) cudaFree(b->d_jobs);
   if (b->d_pre) cudaFree(b->d_pre);
   if (b->d_ctr) cudaFree(b->d_ctr);
@@ -1273,25 +1279,38 @@ static int batch_cycle_launch(ea_batch *b, int n, int ptfr) {
   return EA_OK;
 }
 
-// Cycles of one graph launch: long runs between moves go in pieces.
-constexpr int kGraphCycles = 32;
+// The cycles between two moves go in pieces, one graph launch each: at most 32
+// cycles and about 128 kernels, so that a batch whose jobs change captures
+// little, and of two lengths at most, so that nothing is captured again.
+constexpr int kGraphCycles = 32, kGraphLaunches = 128;
+
+static int graph_pieces(int houfr, int ptfr) {
+  const int most = std::max(1, std::min(kGraphCycles, (int)(kGraphLaunches / (2LL * std::max(ptfr, 1) + 1))));
+  return (houfr + most - 1) / most;
+}
 
 static int batch_cycle(ea_batch *b, int n, int ptfr) {
-  if (!b->cycle || b->cycle_ptfr != ptfr || b->cycle_n != n) {
-    if (b->cycle) { cudaGraphExecDestroy(b->cycle); b->cycle = nullptr; }
+  int k = b->cycles_used;
+  for (int i = 0; i < 2; ++i, k ^= 1)
+    if (b->cycles[k].exec && b->cycles[k].n == n && b->cycles[k].ptfr == ptfr) break;
+  ea_batch::Cycles *q = &b->cycles[k];
+  if (!q->exec || q->n != n || q->ptfr != ptfr) {
+    q = &b->cycles[k = b->cycles_used ^ 1];
+    drop_cycles(*q);
     cudaGraph_t graph = nullptr;
     CU(cudaStreamBeginCapture(b->bs, cudaStreamCaptureModeThreadLocal));
     const int rc = batch_cycle_launch(b, n, ptfr);
     const cudaError_t e = cudaStreamEndCapture(b->bs, &graph);
     if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
     CU(e);
-    const cudaError_t ei = cudaGraphInstantiate(&b->cycle, graph, 0);
+    const cudaError_t ei = cudaGraphInstantiate(&q->exec, graph, 0);
     cudaGraphDestroy(graph);
     CU(ei);
-    b->cycle_ptfr = ptfr;
-    b->cycle_n = n;
+    q->n = n;
+    q->ptfr = ptfr;
   }
-  CU(cudaGraphLaunch(b->cycle, b->bs));
+  b->cycles_used = k;
+  CU(cudaGraphLaunch(q->exec, b->bs));
   return EA_OK;
 }
 
@@ -1362,8 +1381,11 @@ int ea_batch_run_bin(ea_batch *b, const ea_cadence *cad) {
     for (int im = 0; im < cad->mesfr; ++im) {
       // with ptfr = 0 the cycle measures the energies before the swaps
       // (measuring energies that are still fresh leaves them unchanged)
-      for (int ih = 0; ih < cad->houfr; ih += kGraphCycles)
-        if ((rc = batch_cycle(b, std::min(kGraphCycles, cad->houfr - ih), cad->ptfr))) return rc;
+      for (int left = cad->houfr, p = graph_pieces(cad->houfr, cad->ptfr); p > 0; --p) {
+        const int piece = (left + p - 1) / p;
+        if ((rc = batch_cycle(b, piece, cad->ptfr))) return rc;
+        left -= piece;
+      }
       if (cad->cluster && (rc = batch_houdayer(b, cad->nclust))) return rc;
     }
     if ((rc = batch_energy(b))) return rc;
