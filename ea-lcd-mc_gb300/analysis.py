@@ -51,7 +51,8 @@ def plane_correlations(diff, L2, pbc, dmax):
     """The correlation matrices of ea_sp_plane_correlations computed on the
     host from plane counts diff[sample][pair][beta][z] (numpy summation
     order): C[sample][beta][d][3][3]."""
-    q = 1.0 - (2.0 / L2) * diff.astype(np.float64)
+    # 0 where half of the plane differs: 2/L^2 times L^2/2 may round to less than 1
+    q = np.where(2 * diff == L2, 0.0, 1.0 - (2.0 / L2) * diff.astype(np.float64))
     F = np.stack([q, q * q * q, np.sign(q)], -1)            # [s][pair][b][z][3]
     Lz = diff.shape[-1]
     ns, _, NB, _ = diff.shape

@@ -79,7 +79,9 @@ __global__ void __launch_bounds__(kDiffThreads) k_sp_plane_diff(const __grid_con
     for (int q = 0; q < 4; ++q) {
       const int n = (int)((acc >> (16 * q)) & 0xFFFFu), smp = s + 16 * q;
       if (xs) {
-        const double x = __dsub_rn(1.0, __dmul_rn(2.0 * inv, (double)n));
+        // 0 where half of the plane differs: 2/L^2 times L^2/2 may round to
+        // less than 1 (L = 14), and sign(x) is read from x
+        const double x = 2 * n == L2 ? 0.0 : __dsub_rn(1.0, __dmul_rn(2.0 * inv, (double)n));
         const size_t o = ((((size_t)w * npairs + k) * NB + slot) * Lz + z) * 64 + smp;
         xs[o] = x;
         xs[tab + o] = __dmul_rn(__dmul_rn(x, x), x);
