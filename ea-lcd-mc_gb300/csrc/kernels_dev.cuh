@@ -458,9 +458,11 @@ __device__ __forceinline__ void pt_body(const JobDev &j, int s, int ry, PtShared
   }
   const uint8_t ip = h->ip, ip1 = h->ip1, ip2 = h->ip2, ip3 = h->ip3;
   u64 zseed = h->zseed, PR = h->PR, fin = h->final;
-  // draws a batch can make at once: no word of it may be read by a later one
+  // draws a batch can make at once: no word of it may be read by a later draw,
+  // nor (ip3, read when all are written) by an earlier one
   auto lag = [](uint8_t d) { return d ? (int)d : 256; };
-  const int most = min(min(32, lag((uint8_t)(ip - ip1))), min(lag((uint8_t)(ip - ip2)), lag((uint8_t)(ip - ip3))));
+  const int most = min(min(min(32, lag((uint8_t)(ip - ip1))), min(lag((uint8_t)(ip - ip2)), lag((uint8_t)(ip - ip3)))),
+                       lag((uint8_t)(ip3 - ip)));
   // lane k: k + 1 steps of z -> a z + 1
   u64 A = 3202034522624059733ULL, C = 1;
 #pragma unroll
