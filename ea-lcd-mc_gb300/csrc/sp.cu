@@ -2150,6 +2150,13 @@ int ea_sp_autotune(ea_sp *c, int32_t *tile, int32_t *echunk, int32_t *cthreads) 
   SCU(cudaSetDevice(c->device));
   SpDev &d = c->d;
   const size_t G = (size_t)d.NR * d.NB;
+  // whatever may be refused comes before the first timing run
+  const bool cluster = d.V <= kSpClusterMaxV;  // lattices labelled in SMEM
+  int nclust = 0;
+  if (cluster) {
+    const int rc = sp_cluster_prepare(c, nclust);
+    if (rc) return rc;
+  }
   struct Part { void *p; size_t n; };
   const Part parts[] = {{d.S, (size_t)d.nw * d.V * G * 8}, {d.iter, 8}, {d.ctr, sizeof(uint4) * d.NR},
                         {d.prc, sizeof(ea_hq) * d.NR}, {d.xo, sizeof(ea_xoshiro) * d.NR},
@@ -2212,12 +2219,9 @@ int ea_sp_autotune(ea_sp *c, int32_t *tile, int32_t *echunk, int32_t *cthreads) 
     if (ms < best) { best = ms; best_ec = ec; }
   }
   sp_energy_shape(d, best_ec);
-  // block size of the labelling (lattices labelled in SMEM)
+  // block size of the labelling
   int best_ct = d.cthreads;
-  if (d.V <= kSpClusterMaxV) {
-    int nclust = 0;
-    int rc = sp_cluster_prepare(c, nclust);
-    if (rc) { cudaFree(save); return rc; }
+  if (cluster) {
     const long long nq = (long long)d.nw * d.nclust * d.V;
     best = 1e30f;
     for (int ct : {256, 512, 1024}) {

@@ -153,3 +153,19 @@ def test_buffers_of_the_persistent_kernel(fake):
     bin_ = lambda j: j.run_bin(1, 1, 1, 1)
     assert same_buffers(eb, fk, make, [bin_], [bin_]) >= 4
     same_buffers(eb, fk, lambda: sp_job(eb), [bin_], [bin_])   # the resident kernel's
+
+
+def test_autotuner_refuses_before_it_times(fake):
+    """A refusal -- no memory, or one replica, which has no moves to label for
+    -- comes before the timing runs change the job's words."""
+    eb, fk = fake
+    for NR, fails in ((2, 2), (1, 1)):
+        job = sp_job(eb, NR=NR)
+        for k in range(fails):
+            fk.fake_reset()
+            fk.fake_fail_in(k)
+            with pytest.raises(eb.EAError):
+                job.autotune()
+            assert fk.fake_calls(b"launch ") == 0
+        fk.fake_reset()
+        job.close()
