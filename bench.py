@@ -849,9 +849,8 @@ def run_ours(args, rank, world, local):
     for _ in range(args.warmup):
         step()
     job.sync()
-    # timed region: device events on the job's stream around all K steps,
-    # joined with its other streams at the end so that all work enqueued inside
-    # the region is counted; the L2 flushes between steps are timed
+    # timed region: device events on the job's stream, which all of its work
+    # runs on, around all K steps; the L2 flushes between steps are timed
     # by their own events and taken out
     t_beg, t_end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     fl = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
@@ -1008,7 +1007,7 @@ def run_ours(args, rank, world, local):
         "gpu_launches": args.steps * (1 + HOUFR * 3 + 1 + 2 * 5 + 2),
         "roofline": roof,
         "kernel_ms": {"sweep": sw_ms.value, "pt": pt_ms.value, "cluster": cl_ms.value,
-                      "uniforms_overlapped": rg_ms.value, "step_total": ms},
+                      "coins": rg_ms.value, "step_total": ms},
         "clocks": clk.summary(),
     }
     line["no_cluster"] = run_no_cluster(args, dev, torch, eagb)
@@ -1045,7 +1044,7 @@ def main():
     ap.add_argument("--mix-only", default="", choices=["", "plain", "batched"],
                     help="only two bins of the 36-job x 32-sample multispin mix in this form (for profilers)")
     ap.add_argument("--rng-sms", type=int, default=-1,
-                    help="ea_set_rng_sms of the headline job (-1: automatic; the coins are drawn on every SM)")
+                    help="ea_set_rng_sms of the headline job (-1: automatic): reported, without effect on the coins, which every SM draws")
     ap.add_argument("--small-sp", type=int, default=0, metavar="N",
                     help="only the small sample-packed batching leg with N jobs (prints its record)")
     ap.add_argument("--serve-config5", type=int, default=0, metavar="N",

@@ -43,12 +43,6 @@ int fail(int code, const char *fmt, ...) {
     if (e_ != cudaSuccess) return fail(EA_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_));     \
   } while (0)
 
-#define CR(call)                                                                                  \
-  do {                                                                                            \
-    curandStatus_t e_ = (call);                                                                   \
-    if (e_ != CURAND_STATUS_SUCCESS) return fail(EA_ERR_CURAND, "%s: curand status %d", #call, (int)e_); \
-  } while (0)
-
 template <class T>
 cudaError_t dalloc(T *&p, size_t n) {
   return cudaMalloc((void **)&p, sizeof(T) * (n ? n : 1));
@@ -963,7 +957,7 @@ struct ea_batch {
 
 extern "C" {
 
-// Tile width of a job's fused sweep; the energy partial sums follow it.
+// Tile width of a job's fused sweep.
 static int set_tile(ea_ctx *c, int kt) {
   JobDev &j = c->j;
   if (kt == j.kt) return EA_OK;

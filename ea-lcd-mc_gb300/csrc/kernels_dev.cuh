@@ -103,7 +103,8 @@ __device__ __forceinline__ void fill_bits_body(const JobDev &j, int parity) {
 // main.cu:1045-1060, and for each of the four 64-bit keys the first byte n with
 // R < cum[n] (the heat-bath thresholds); this is the function the reference's
 // pre-search + bisection computes (main.cu:1063-1078).  Here the pre-search is
-// indexed by the top 8 bits so that every temperature's table fits in SMEM.
+// indexed by the top 8 to 11 bits, so that every temperature's table fits in
+// SMEM.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void philox10(uint32_t &v0, uint32_t &v1, uint32_t &v2, uint32_t &v3, uint32_t k0,
                                          uint32_t k1) {
@@ -296,9 +297,9 @@ __device__ __forceinline__ void draw_ids(int ntrip, Item &&item, Byte &&byte, u6
 // Per-tile partial sums and a reduction kernel took 34 us a sweep on the large
 // tube and a link of 3 to 10 us in a small job's chain.
 // ---------------------------------------------------------------------------
+// stage = false: the pre-search tables of this job are already in SMEM (the
+// block's previous tile was of the same job).
 template <int NR, int KT, bool UPDATE>
-// stage = false: the thresholds of this job are already in SMEM (the block's
-// previous tile was of the same job).
 __device__ __forceinline__ void sweep_body(const JobDev &j, const uint4 *ctr, int blk, int parity, int energy,
                                            unsigned char *smem, bool stage = true) {
   const int tile = blk / j.nsplit, part = blk - tile * j.nsplit;

@@ -24,8 +24,8 @@ namespace eagb {
 namespace {
 
 // Limits: at most kMaxHalf half-sites per parity (e.g. L = 32, Lz = 256: the
-// scratch tables) and kMaxPartials tile energies (the entry point's bound on the
-// job, from when they were kept).
+// scratch tables) and kMaxPartials tile sums (the documented bound on a job; the
+// sums are added up in place and take no scratch).
 constexpr size_t kMaxPartials = (size_t)1 << 20;
 constexpr int kMaxHalf = 8192;
 constexpr size_t kIdxBytes = (size_t)12 * kMaxHalf * 4;

@@ -40,8 +40,8 @@ __device__ __forceinline__ u64 transpose8(u64 x) {
 // NS samples at a time (lanes: NS samples of 32 / NS neighbouring columns, so
 // one 2 NS-byte label slot serves the NS lanes of a column).
 //
-// Bound by instruction issue (63 % of the slots busy, 38 % of the SMEM path, 21
-// of 32 lanes active in the walks).  The forms it replaces labelled every
+// Bound by instruction issue (61 % of the slots busy with 37 % of the warps, 44 %
+// of the SMEM path, 19 of 32 lanes active; 83 % and 78 % of the warps in slabs).  The forms it replaces labelled every
 // site, 8 samples in lock step with vector label slots, at 72 % of the SMEM
 // path.  A launch on 6144 x 8 lattices of 12 x 12 x 48: 5.08 -> 2.27 ms; one
 // word of it (96 blocks): 155 -> 62 us; 24 x 24 x 192 in slabs: 1.83 -> 0.83

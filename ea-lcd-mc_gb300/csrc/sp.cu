@@ -175,7 +175,7 @@ __device__ __forceinline__ void sp_pass_body(const SpDev &d, const uint4 *ctr, i
 // item's 6 words on T in [0.6, 1.6] and [0.7, 1.6] (the draws are
 // counter-based, so the ones made are the same).  The loops stay rolled: the
 // three copies of a draw are most of the code, and unrolled by item they
-// missed the instruction cache.  The pass is bound by instruction issue (65 % of
+// missed the instruction cache.  The pass is bound by instruction issue (67 % of
 // the slots), mostly of these draws: 24 x 24 x 192, 32 temperatures, 4
 // replicas, one word: 760 -> 559 us a sweep; 12 x 12 x 48, 24 temperatures: 62
 // -> 55.
@@ -736,9 +736,12 @@ __device__ __forceinline__ void sp_overlap_body(const SpDev &d, int g, long long
   d.Q[t] = p[(size_t)r1 * d.NB] ^ p[(size_t)r2 * d.NB];
 }
 
-// One CTA per (word, slot, group of 8 samples): the CTA reads its byte of
-// every site's overlap word into SMEM and labels the 8 samples' lattices one
-// after the other with lock-step rounds -- each site hooks the labels of its
+// The labelling of lattices that the runs (runs.cuh) do not take: wide flat
+// ones, whose run words pass the SMEM, and in batches and the persistent kernel
+// those above kSpClusterMaxV sites.  One CTA per (word, slot, group of 8
+// samples): the CTA reads its byte of every site's overlap word into SMEM and
+// labels the 8 samples' lattices one after the other with lock-step rounds --
+// each site hooks the labels of its
 // equal-q neighbours of smaller index with atomicMin, then labels are
 // pointer-jumped until stable, until a round hooks nothing.  Labels only
 // decrease and stay inside the cluster, so each cluster ends labelled by its
