@@ -2438,13 +2438,11 @@ static bool sp_use_resident(ea_sp *c, const ea_cadence *cad) {
   return sp_res_launch_sweeps(c->d.V, (size_t)c->d.NR * c->d.NB, cad) > 0 && sp_res_ok(c);
 }
 
-static int sp_run_resident(ea_sp *c, const ea_cadence *cad) {
+// The resident path's buffers for such bins: counters, random words, draws.
+static int sp_res_buffers(ea_sp *c, const ea_cadence *cad) {
   const SpDev &d = c->d;
-  const SpResPlan &pl = c->r_plan;
-  const int spi = cad->mesfr * cad->houfr * cad->ptfr;  // sweeps per iteration
   const size_t words_sweep = (size_t)2 * d.V * d.NR * d.NB;
   const size_t nsweep = sp_res_launch_sweeps(d.V, (size_t)d.NR * d.NB, cad), npass = nsweep * d.ncol;
-  const int ipl = cad->cluster ? 1 : (int)(nsweep / spi);  // iterations per launch
   const size_t npt = nsweep / cad->ptfr;                    // tempering steps per launch
   if (npass > c->r_cap_pass || nsweep > c->r_cap_sweep || npt > c->r_cap_pt) {
     SCU(cudaStreamSynchronize(c->st));
@@ -2462,6 +2460,15 @@ static int sp_run_resident(ea_sp *c, const ea_cadence *cad) {
     c->r_cap_sweep = nsweep;
     c->r_cap_pt = npt;
   }
+  return EA_OK;
+}
+
+static int sp_run_resident(ea_sp *c, const ea_cadence *cad) {
+  const SpDev &d = c->d;
+  const SpResPlan &pl = c->r_plan;
+  const int spi = cad->mesfr * cad->houfr * cad->ptfr;  // sweeps per iteration
+  const size_t nsweep = sp_res_launch_sweeps(d.V, (size_t)d.NR * d.NB, cad);
+  const int ipl = cad->cluster ? 1 : (int)(nsweep / spi);  // iterations per launch
   SpResDev p{};
   p.d = d;
   p.R = c->r_R;
@@ -2521,12 +2528,16 @@ int ea_sp_run(ea_sp *c, const ea_cadence *cad, double *avgE) {
   const SpDev &d = c->d;
   const size_t n = (size_t)d.nw * 64 * d.NR * d.NB;
   SCU(cudaMemsetAsync(d.avgE, 0, n * 8, c->st));
-  int rc, nclust = cad->nclust;
+  int rc = EA_OK, nclust = cad->nclust;
   if (cad->cluster && (rc = sp_cluster_prepare(c, nclust))) return rc;
   if (c->bin_mode == EA_BIN_RESIDENT && !sp_use_resident(c, cad))
     return spfail(EA_ERR_ARG, "the resident bin kernel takes jobs whose words fit one thread-block cluster, bins "
                               "without cluster moves or with at least %d sweeps between moves", kResMinBlock);
-  if (sp_use_resident(c, cad)) {
+  // without memory for the resident path's buffers the graph takes the bin,
+  // unless the caller asked for the resident kernel
+  const bool resident = sp_use_resident(c, cad);
+  if (resident && (rc = sp_res_buffers(c, cad)) && c->bin_mode == EA_BIN_RESIDENT) return rc;
+  if (resident && !rc) {
     if ((rc = sp_run_resident(c, cad))) return rc;
     c->last_itmax = cad->itmax;
     if (avgE) return ea_sp_bin_results(c, avgE);

@@ -169,3 +169,28 @@ def test_autotuner_refuses_before_it_times(fake):
             assert fk.fake_calls(b"launch ") == 0
         fk.fake_reset()
         job.close()
+
+
+@pytest.mark.parametrize("cluster", [False, True])
+def test_a_bin_without_room_for_the_resident_buffers(fake, cluster):
+    """The default takes the graph, which needs none of them; the resident
+    kernel, when asked for by name, says that they are missing."""
+    eb, fk = fake
+    for k in range(3):
+        for mode in (eb.EA_BIN_AUTO, eb.EA_BIN_RESIDENT):
+            job = sp_job(eb)
+            job.set_bin_kernel(mode)
+            assert job.bin_kernel_for(3, 4, cluster=cluster) == eb.EA_BIN_RESIDENT
+            fk.fake_reset()
+            fk.fake_fail_in(k + int(cluster))     # after the overlap words of a move
+            if mode == eb.EA_BIN_AUTO:
+                job.run_bin(3, 4, cluster=cluster)
+                assert fk.fake_calls(b"cudaGraphLaunch") == 3 and not fk.fake_calls(b"launch _ZN4eagb13k_sp_resident")
+                job.run_bin(3, 4, cluster=cluster)
+            else:
+                with pytest.raises(eb.EAError, match="out of memory"):
+                    job.run_bin(3, 4, cluster=cluster)
+                job.run_bin(3, 4, cluster=cluster)
+            assert fk.fake_calls(b"launch _ZN4eagb13k_sp_resident") > 0
+            job.close()
+            fk.fake_reset()
