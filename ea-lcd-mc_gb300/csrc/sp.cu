@@ -2347,11 +2347,18 @@ static int sp_cluster_prepare(ea_sp *c, int &nclust) {
       int ns = 0;
       const int D = sp_slab_planes(d.L, d.Lz, d.nw, nclust, &ns);
       if (D > 0) {
+        // without memory for the slabs' labels: in the scratch, one CTA a unit
         const size_t units = (size_t)d.nw * nclust * 8;
-        SCU(cudaMalloc((void **)&d.slab_lab, sizeof(uint32_t) * units * 8 * d.V));
-        SCU(cudaMalloc((void **)&d.slab_coin, units * d.V));
-        d.slabD = D;
-        d.slabNS = ns;
+        if (cudaMalloc((void **)&d.slab_lab, sizeof(uint32_t) * units * 8 * d.V) == cudaSuccess &&
+            cudaMalloc((void **)&d.slab_coin, units * d.V) == cudaSuccess) {
+          d.slabD = D;
+          d.slabNS = ns;
+        } else {
+          (void)cudaGetLastError();
+          if (d.slab_lab) cudaFree(d.slab_lab);
+          d.slab_lab = nullptr;
+          d.slab_coin = nullptr;
+        }
       }
     }
     c->q_cap = nclust;

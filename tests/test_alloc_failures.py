@@ -194,3 +194,22 @@ def test_a_bin_without_room_for_the_resident_buffers(fake, cluster):
             assert fk.fake_calls(b"launch _ZN4eagb13k_sp_resident") > 0
             job.close()
             fk.fake_reset()
+
+
+def test_a_move_without_room_for_slab_labels(fake):
+    """Wide planes (100 x 100) and a long tube: the scratch that every large
+    lattice has is enough for a move."""
+    eb, fk = fake
+    for L, Lz in ((100, 4), (24, 60)):
+        for k in (2, 3):   # overlap words, scratch; slab labels, their coins
+            job = sp_job(eb, L, Lz, 4)
+            fk.fake_reset()
+            fk.fake_fail_in(k)
+            job.houdayer(2)
+            assert fk.fake_calls(b"launch _ZN4eagb12k_sp_cluster") == 1
+            assert fk.fake_calls(b"launch _ZN4eagb9k_sp_slab") == 0
+            fk.fake_fail_in(-1)
+            job.houdayer(4)    # a larger move asks again
+            assert fk.fake_calls(b"launch _ZN4eagb9k_sp_slab") > 0
+            job.close()
+            fk.fake_reset()
