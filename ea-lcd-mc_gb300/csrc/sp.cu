@@ -1349,21 +1349,23 @@ __device__ bool sp_grid_sync(const SpPersistDev &p, unsigned &epoch) {
   }
 
 // Kinds whose one-job blocks have SUB threads and no barrier: each thread
-// block takes kPersistThreads / SUB of them at a time.
+// block takes kPersistThreads / SUB of them at a time.  They use no dynamic
+// SMEM, so their job descriptors lie there.
 #define SPP_SUB(KIND, SUB, BODY)                                                      \
   for (uint32_t vb0 = blockIdx.x * (kPersistThreads / SUB); vb0 < b.total[KIND];      \
        vb0 += gridDim.x * (kPersistThreads / SUB)) {                                 \
     const int sub = threadIdx.x / SUB, ltid = threadIdx.x % SUB;                      \
+    SpDev *const sjob = reinterpret_cast<SpDev *>(smem);                              \
     const uint32_t vb = vb0 + sub;                                                    \
     __syncthreads();                                                                  \
     if (ltid == 0 && vb < b.total[KIND]) {                                            \
       const int jb_ = spb_job(b.pre[KIND], b.njobs, vb);                              \
-      s_job[sub] = b.jobs[jb_];                                                       \
+      sjob[sub] = b.jobs[jb_];                                                        \
       s_blk[sub] = (int)(vb - __ldg(b.pre[KIND] + jb_));                              \
     }                                                                                 \
     __syncthreads();                                                                  \
     if (vb < b.total[KIND]) {                                                         \
-      const SpDev &d = s_job[sub];                                                    \
+      const SpDev &d = sjob[sub];                                                     \
       const int blk = s_blk[sub];                                                     \
       BODY;                                                                           \
     }                                                                                 \
@@ -1374,8 +1376,8 @@ __device__ bool sp_grid_sync(const SpPersistDev &p, unsigned &epoch) {
 
 __global__ void __launch_bounds__(kPersistThreads, 1) k_sp_persist(const __grid_constant__ SpPersistDev p) {
   extern __shared__ __align__(16) unsigned char smem[];
-  // a job a sub-block (SPP_SUB of 256): with the move's kRunSmem they fill the SM
-  __shared__ SpDev s_job[kPersistThreads / 256];
+  // at most 512 bytes of static SMEM beside the widest tiles (sp_kt)
+  __shared__ SpDev s_job[1];
   __shared__ int s_blk[kPersistThreads / 256];
   const SpBatchDev &b = p.b;
   unsigned epoch = 0;
