@@ -405,9 +405,13 @@ __device__ __forceinline__ void res_count_add(u64 *P, int npl, const u64 f[6]) {
 // A warp (one slot) sums its bit-sliced counters: in each round a lane keeps
 // half of its samples and gives the other half's planes to its partner, so that
 // lane l ends with samples 2 l and 2 l + 1.  Their counts go into this CTA's
-// part of every CTA's Pt, or are added to its U2s.  (Loops kept rolled: the kernel runs through all its
-// code once a step, and what is unrolled comes from the instruction cache
-// again each time.)
+// part of every CTA's Pt, or, on ladders whose Pt would not fit (61 temperatures
+// in 16 CTAs), are added to the U2s of the slot's CTA, b mod ncta, where
+// res_tempering fetches the sums.  (Added to every CTA's U2s, 16 times the
+// atomics, 8 sweeps of the 6^2 x 30 tube with 61 temperatures and one replica
+// took 530 us, now 308.)  Loops are kept rolled: the kernel runs through all its
+// code once a step, and what is unrolled comes from the instruction cache again
+// each time.
 template <int NPL>
 __device__ __forceinline__ void res_count_flush(const SpResDev &p, const ResCta &me, const ResShared &s, const u64 *P,
                                                 int b, int scale) {
@@ -439,12 +443,11 @@ __device__ __forceinline__ void res_count_flush(const SpResDev &p, const ResCta 
 #pragma unroll
   for (int q = 0; q < NPL; ++q) v |= ((H[q] & 1u) | (H[q] & 2u) << 15) << q;
   if (!p.parts) {
-    const uint32_t to = smem_addr(s.U2s + b * 64 + 2 * lane);
-    for (int c = 0; c < p.ncta; ++c)
-      for (int j = 0; j < 2; ++j)
-        asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(mapa(to + 4 * j, c)),
-                     "r"(scale * (j ? v >> 16 : v & 0xFFFFu))
-                     : "memory");
+    const uint32_t to = mapa(smem_addr(s.U2s + b * 64 + 2 * lane), b % p.ncta);
+    for (int j = 0; j < 2; ++j)
+      asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(to + 4 * j),
+                   "r"(scale * (j ? v >> 16 : v & 0xFFFFu))
+                   : "memory");
     return;
   }
   const uint32_t own = smem_addr(s.Pt + ((size_t)me.rank * p.d.NB + b) * 64 + 2 * lane);
@@ -534,6 +537,10 @@ __device__ __forceinline__ void res_tempering(const SpResDev &p, const ResCta &m
         hi += (int)(v >> 16);
       }
       U2 = make_int2(scale * lo, scale * hi);
+    } else if (const int own = (i >> 5) % ncta; own != me.rank) {  // the others stay as they are
+      int x, y;
+      asm volatile("ld.shared::cluster.v2.s32 {%0, %1}, [%2];" : "=r"(x), "=r"(y) : "r"(mapa(smem_addr(&U2), own)) : "memory");
+      U2 = make_int2(x, y);
     }
     if (last && me.rank == 0) {
       const int smp = 2 * (i & 31), b = i >> 5;
@@ -596,8 +603,14 @@ __device__ __forceinline__ void res_state(const SpResDev &p, const ResShared &s,
   s.Es[NP * 64 + lane] = carry_e;
   s.Ps[NP * 64 + lane] = (uint8_t)carry_p;
   if (measure) s.Av[NP * 64 + lane] += carry_e;
-  if (!p.parts)  // the next counts come after another barrier (two colours, or the energy's own phase)
-    for (int i = 0; i <= NP; ++i) s.U2s[i * 64 + lane] = 0;
+}
+
+// The sums of this CTA's slots cleared, when every CTA has fetched them (behind
+// the barrier of the permute).  The next counts come after another barrier: two
+// colours, or the energy's own phase.
+__device__ __forceinline__ void res_clear(const SpResDev &p, const ResCta &me, const ResShared &s) {
+  for (int i = threadIdx.x; i < p.d.NB * 64; i += blockDim.x)
+    if ((i >> 6) % p.ncta == me.rank) s.U2s[i] = 0;
 }
 
 // The accepted swaps applied to the CTA's sites (sp_permute_body), four slots
@@ -721,6 +734,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sp_resident(const __grid_con
         cluster_arrive();
         res_state(p, s, p.measure && lastpt);
         cluster_wait();
+        if (!p.parts) {
+          __syncthreads();  // res_state's reads
+          res_clear(p, me, s);
+        }
         ++ptj;
       }
 
