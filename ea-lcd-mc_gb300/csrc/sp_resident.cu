@@ -412,7 +412,7 @@ __device__ __forceinline__ void res_count_add(u64 *P, int npl, const u64 f[6]) {
 // took 530 us, now 308.)  Loops are kept rolled: the kernel runs through all its
 // code once a step, and what is unrolled comes from the instruction cache again
 // each time.
-template <int NPL>
+template <int NPL, bool PARTS>
 __device__ __forceinline__ void res_count_flush(const SpResDev &p, const ResCta &me, const ResShared &s, const u64 *P,
                                                 int b, int scale) {
   const int lane = threadIdx.x & 31;
@@ -442,7 +442,7 @@ __device__ __forceinline__ void res_count_flush(const SpResDev &p, const ResCta 
   uint32_t v = 0;
 #pragma unroll
   for (int q = 0; q < NPL; ++q) v |= ((H[q] & 1u) | (H[q] & 2u) << 15) << q;
-  if (!p.parts) {
+  if (!PARTS) {
     const uint32_t to = mapa(smem_addr(s.U2s + b * 64 + 2 * lane), b % p.ncta);
     for (int j = 0; j < 2; ++j)
       asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(to + 4 * j),
@@ -462,7 +462,7 @@ __device__ __forceinline__ void res_count_flush(const SpResDev &p, const ResCta 
 // so U2 is twice the unsatisfied half-edges of the colour-1 sites, all final
 // once their pass has flipped them (f ^= flip).  A warp per (word, column),
 // lanes over the colour's sites.
-template <int NPL>
+template <int NPL, bool PARTS>
 __device__ __forceinline__ void res_pass_count(const SpResDev &p, const ResCta &me, const ResShared &s,
                                                const ResColour &q, int sweep, int k, u64 r[2]) {
   const ResPass a = res_pass_at(p, me, q, sweep, k);
@@ -489,13 +489,13 @@ __device__ __forceinline__ void res_pass_count(const SpResDev &p, const ResCta &
       for (int j = 0; j < 2; ++j) r[j] = x[j];
     }
     res_fetch(a, q, b + nwarp, lane, b + nwarp < NB && lane < q.nkc, r);
-    res_count_flush<NPL>(p, me, s, P, b, 2);
+    res_count_flush<NPL, PARTS>(p, me, s, P, b, 2);
   }
 }
 
 // Unsatisfied half-edges per (sample, slot) of the CTA's sites
 // (sp_energy_body's count).
-template <int NPL>
+template <int NPL, bool PARTS>
 __device__ __forceinline__ void res_energy(const SpResDev &p, const ResCta &me, const ResShared &s) {
   const int NB = p.d.NB, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
 #pragma unroll 1
@@ -509,7 +509,7 @@ __device__ __forceinline__ void res_energy(const SpResDev &p, const ResCta &me, 
       res_bonds(p, s, b, i, s.S[b * p.nslm + i], f);
       res_count_add(P, NPL, f);
     }
-    res_count_flush<NPL>(p, me, s, P, b, 1);
+    res_count_flush<NPL, PARTS>(p, me, s, P, b, 1);
   }
 }
 
@@ -521,6 +521,7 @@ __device__ __forceinline__ void res_energy(const SpResDev &p, const ResCta &me, 
 // is accepted up to the m = -dE / 2 that k_sp_pt_draw found.  The walk finds the
 // lanes that swap and nothing more; res_permute applies them.  `last`: the
 // counts are handed back.
+template <bool PARTS>
 __device__ __forceinline__ void res_tempering(const SpResDev &p, const ResCta &me, const ResShared &s, bool last) {
   const SpDev &d = p.d;
   const int NB = d.NB, NP = NB - 1, ncta = p.ncta;
@@ -528,7 +529,7 @@ __device__ __forceinline__ void res_tempering(const SpResDev &p, const ResCta &m
   const uint32_t *Pw = reinterpret_cast<const uint32_t *>(s.Pt);
   for (int i = threadIdx.x; i < n2; i += blockDim.x) {
     int2 &U2 = reinterpret_cast<int2 *>(s.U2s)[i];
-    if (p.parts) {
+    if (PARTS) {
       int lo = 0, hi = 0;
 #pragma unroll 4
       for (int c = 0; c < ncta; ++c) {
@@ -642,7 +643,7 @@ __device__ __forceinline__ void res_permute(const SpResDev &p, const ResCta &me,
 }
 
 // NPL: bit planes of a warp's per-sample count, 6 * nslm < 2^NPL.
-template <int NPL>
+template <int NPL, bool PARTS>
 __global__ void __launch_bounds__(kResThreads, 1) k_sp_resident(const __grid_constant__ SpResDev p) {
   const cg::cluster_group cl = cg::this_cluster();
   const SpDev &d = p.d;
@@ -714,7 +715,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sp_resident(const __grid_con
         res_stage_x(p, me, s, ptj);
         for (int sw = 0; sw < p.ptfr; ++sw, ++sweep)
           for (int k = 0; k < ncol; ++k) {
-            if (res_counts(p, sw, k)) res_pass_count<NPL>(p, me, s, col[k], sweep, k, words);
+            if (res_counts(p, sw, k)) res_pass_count<NPL, PARTS>(p, me, s, col[k], sweep, k, words);
             else res_pass(p, me, s, col[k], sweep, k, words);
             const bool wrap = k == ncol - 1;
             if (wrap && sw == p.ptfr - 1) cp_async_wait_all();  // the step's draws
@@ -724,17 +725,17 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sp_resident(const __grid_con
             cluster_wait();
           }
         if (!p.pair_energy) {
-          res_energy<NPL>(p, me, s);
+          res_energy<NPL, PARTS>(p, me, s);
           cluster_arrive();
           cluster_wait();
         }
         const bool lastpt = im == p.mesfr - 1 && ih == p.houfr - 1;
-        res_tempering(p, me, s, lastpt && it == p.nit - 1);
+        res_tempering<PARTS>(p, me, s, lastpt && it == p.nit - 1);
         res_permute(p, me, s);
         cluster_arrive();
         res_state(p, s, p.measure && lastpt);
         cluster_wait();
-        if (!p.parts) {
+        if (!PARTS) {
           __syncthreads();  // res_state's reads
           res_clear(p, me, s);
         }
@@ -766,16 +767,20 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sp_resident(const __grid_con
 // Counter planes of the energy phase's warp sums: 6 * nslm < 2^NPL.
 static int res_npl(int nslm) { return 6 * nslm < (1 << 10) ? 10 : kResPlanes; }
 
-template <int NPL>
-static cudaError_t res_attrs() {
-  cudaError_t e = cudaFuncSetAttribute(k_sp_resident<NPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sp_resident<NPL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  return e;
+using ResKernel = void (*)(SpResDev);
+static ResKernel res_kernel(int npl, bool parts) {
+  if (npl == 10) return parts ? k_sp_resident<10, true> : k_sp_resident<10, false>;
+  return parts ? k_sp_resident<kResPlanes, true> : k_sp_resident<kResPlanes, false>;
 }
 
 cudaError_t sp_res_setup() {
-  cudaError_t e = res_attrs<10>();
-  if (e == cudaSuccess) e = res_attrs<kResPlanes>();
+  cudaError_t e = cudaSuccess;
+  for (int npl : {10, kResPlanes})
+    for (bool parts : {false, true}) {
+      const ResKernel k = res_kernel(npl, parts);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_sp_ctr_chain, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              64 * (int)(sizeof(ea_hq) + sizeof(ea_xoshiro)));
@@ -828,8 +833,7 @@ bool sp_res_plan(const SpDev &d, const int32_t *col_sites, SpResPlan &pl) {
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = res_config(ncta, units, smem, nullptr, &at);
     int nclusters = 0;
-    const cudaError_t e = npl == 10 ? cudaOccupancyMaxActiveClusters(&nclusters, k_sp_resident<10>, &cfg)
-                                    : cudaOccupancyMaxActiveClusters(&nclusters, k_sp_resident<kResPlanes>, &cfg);
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, res_kernel(npl, parts > 0), &cfg);
     if (e != cudaSuccess) {
       cudaGetLastError();
       continue;
@@ -877,8 +881,7 @@ cudaError_t sp_res_chunk(const SpResDev &p, const SpResPlan &pl, int npass, uint
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute at;
   const cudaLaunchConfig_t cfg = res_config(pl.ncta, d.nw * d.NR, pl.smem, st, &at);
-  return pl.npl == 10 ? cudaLaunchKernelEx(&cfg, k_sp_resident<10>, p)
-                      : cudaLaunchKernelEx(&cfg, k_sp_resident<kResPlanes>, p);
+  return cudaLaunchKernelEx(&cfg, res_kernel(pl.npl, pl.parts > 0), p);
 }
 
 }  // namespace eagb
