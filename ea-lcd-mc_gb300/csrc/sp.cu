@@ -1635,15 +1635,33 @@ size_t sp_cluster_smem(int L, int Lz) {
   return ns ? run_smem(run_shape(L, Lz), ns) : V <= kSpClusterMaxV ? (size_t)V * 7 : 0;
 }
 
-// Block size of the cluster labelling: its (column chunk, sample) items spread
-// evenly over the fewest passes of at most 1024 threads (12 x 12 x 48: 768
-// threads 4.91 ms a move, 1024 4.96, 512 6.51; 8 x 8 x 16: 512 threads 31 us,
-// 256 40; 7 x 7 x 21: 512 threads 38 us, 256 47).
-int sp_cluster_threads(int L, int Lz) {
+// Block size of the cluster labelling for a launch of `blocks` CTAs: its
+// (column chunk, sample) items spread evenly over some passes, so that an SM's
+// CTAs -- as many as SMEM, registers (56 a thread) and the launch leave it --
+// take the most items side by side; of equal ones the smallest blocks, whose
+// barriers hide behind other CTAs.  12 x 12 x 48: 768 threads (one CTA an SM, the
+// passes that 1024 threads take) 4.91 ms a move, 512 6.51.  11 x 11 x 3, 24
+// temperatures, 15 words: 224 threads 99 us a move, 992 (the fewest passes) 134;
+// 15 x 15 x 3, 40 words: 384 272, 928 352; 10 x 10 x 10, 8 words: 288 85, 800 103.
+// One word's launches of fewer CTAs than SMs keep the fewest passes.
+int sp_cluster_threads(int L, int Lz, size_t blocks) {
   const int ns = run_samples(L, Lz);
   if (!ns) return 1024;
-  const int items = run_shape(L, Lz).nseg * ns, passes = (items + 1023) / 1024;
-  return std::min(1024, ((items + passes - 1) / passes + 31) / 32 * 32);
+  const int items = run_shape(L, Lz).nseg * ns, few = (items + 1023) / 1024;
+  const double smem = (double)sp_cluster_smem(L, Lz), most = std::max(1.0, blocks / 152.0);
+  int best = 0;
+  double rate = 0;  // items of an SM side by side, over all of a CTA's
+  for (int p = few; p <= 3 * few + 4; ++p) {
+    const int t = std::min(1024, ((items + p - 1) / p + 31) / 32 * 32);
+    const double ctas = std::floor(std::min({227 * 1024 / (smem + 1024), 65536.0 / (56 * t), 2048.0 / t}));
+    const double r = std::min(std::max(ctas, 1.0), most) / p;
+    if (r >= 0.999 * rate) {
+      best = t;
+      rate = std::max(rate, r);
+    }
+    if (t <= 96) break;
+  }
+  return best;
 }
 
 // Planes per slab of the slab labelling of lattices above kSpClusterMaxV
@@ -1692,7 +1710,9 @@ cudaError_t sp_launch_houdayer(const SpDev &d, cudaStream_t st) {
       k_sp_slab_coins<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d, g);
       k_sp_slab_flip<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(d);
     } else {
-      k_sp_cluster<<<(unsigned)(d.nw * d.nclust * 8), d.cthreads, sp_cluster_smem(d.L, d.Lz), st>>>(d, g);
+      const size_t blocks = (size_t)d.nw * d.nclust * 8;
+      const int threads = d.cthreads ? d.cthreads : sp_cluster_threads(d.L, d.Lz, blocks);
+      k_sp_cluster<<<(unsigned)blocks, threads, sp_cluster_smem(d.L, d.Lz), st>>>(d, g);
     }
     k_sp_flip<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, g);
   }
@@ -1841,7 +1861,6 @@ int ea_sp_create(const ea_sp_geom *gp, int32_t device, ea_sp **out) {
   int maxc = 0;
   for (int k = 0; k < g.ncol; ++k) maxc = std::max(maxc, g.col_off[k + 1] - g.col_off[k]);
   d.kt = sp_kt(d.NB, d.NR, maxc);
-  d.cthreads = sp_cluster_threads(d.L, d.Lz);
   d.fd_NB.set((uint32_t)d.NB);
   d.esites = d.V;
   d.epair = 0;
@@ -2250,7 +2269,7 @@ int ea_sp_autotune(ea_sp *c, int32_t *tile, int32_t *echunk, int32_t *cthreads) 
   SCU(e);
   if (tile) *tile = d.pgrid ? 0 : d.kt;
   if (echunk) *echunk = d.echunk;
-  if (cthreads) *cthreads = d.cthreads;
+  if (cthreads) *cthreads = d.cthreads ? d.cthreads : 1024;
   return EA_OK;
 }
 
@@ -2635,7 +2654,7 @@ int ea_sp_bin_results(ea_sp *c, double *avgE) {
 // geometries into one launch costs more than the launches it saves.)
 struct SpClass {
   std::vector<ea_sp *> jobs;
-  int ncol_max = 0, cl_threads = 0;
+  int ncol_max = 0;
   SpDev *d_jobs = nullptr;
   uint32_t *d_pre = nullptr;
   std::vector<SpDev> up_jobs;
@@ -2669,7 +2688,7 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
   const int n = (int)k.jobs.size();
   std::vector<SpDev> hj(n);
   std::vector<uint32_t> hp((size_t)SPB_COUNT * (n + 1), 0);
-  int pass_smem = 0, prm_smem = 0, cl_smem = 0, e_smem = 0, t_smem = 0, e_threads = 32, nrep = 1;
+  int pass_smem = 0, prm_smem = 0, cl_smem = 0, e_smem = 0, t_smem = 0, e_threads = 32, nrep = 1, cl_threads = 32;
   for (int i = 0; i < n; ++i) {
     hj[i] = k.jobs[i]->d;
     uint32_t cnt[SPB_COUNT];
@@ -2682,7 +2701,10 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
     e_threads = std::max(e_threads, hj[i].en.threads);
     e_smem = std::max(e_smem, (int)en_smem(hj[i], kPersistThreads));  // a persistent launch's blocks are the larger
     t_smem = std::max(t_smem, (int)pt_smem(hj[i].NB));
-    if (cluster) cl_smem = std::max(cl_smem, (int)sp_cluster_smem(hj[i].L, hj[i].Lz));
+    if (cluster) {
+      cl_smem = std::max(cl_smem, (int)sp_cluster_smem(hj[i].L, hj[i].Lz));
+      cl_threads = std::max(cl_threads, sp_cluster_threads(hj[i].L, hj[i].Lz, cnt[SPB_CL0]));
+    }
   }
   if (k.up_jobs.size() != hj.size() || std::memcmp(k.up_jobs.data(), hj.data(), sizeof(SpDev) * n) ||
       k.up_pre != hp) {
@@ -2707,7 +2729,7 @@ static int spb_upload(SpClass &k, bool cluster, cudaStream_t bs) {
   bd.nrep = nrep;
   bd.pt_smem = t_smem;
   bd.cluster_smem = cl_smem;
-  bd.cluster_threads = k.cl_threads;
+  bd.cluster_threads = cl_threads;
   return EA_OK;
 }
 
@@ -2767,7 +2789,6 @@ int ea_sp_batch_create(ea_sp *const *jobs, int32_t njobs, ea_sp_batch **out) {
     SpClass &k = b->classes[q];
     k.jobs.push_back(c);
     k.ncol_max = std::max(k.ncol_max, c->d.ncol);
-    k.cl_threads = std::max(k.cl_threads, sp_cluster_threads(c->d.L, c->d.Lz));
   }
   cudaError_t e = cudaSetDevice(b->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->bs, cudaStreamNonBlocking);

@@ -51,7 +51,7 @@ struct SpDev {
   int echunk;                        // sites per thread of the energy count
   EnShape en;
   int esites, epair;                 // sites the count walks: all V, or (epair = 1) the colour-1 sites, counted twice
-  int cthreads;                      // block size of the one-job cluster labelling
+  int cthreads;                      // block size of the one-job cluster labelling (0: sp_cluster_threads)
   int pgrid;                         // > 0: one-job colour passes as the per-item pass on this many CTAs
   int col_off[9];                    // colour c owns col_sites[col_off[c] .. col_off[c+1])
   const int32_t *nb;                 // [V][6]
