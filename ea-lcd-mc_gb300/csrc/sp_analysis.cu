@@ -32,6 +32,14 @@ void set_last_error(const char *msg);  // api.cu
 constexpr int kPlanePlanes = 12;  // bit planes of a plane's count: L^2 < 4096
 
 constexpr int kDiffThreads = 256;
+// Lane groups of a block: every group's bit planes are summed by a few lanes, so
+// a small plane has one group for 4 sites (3667 planes of 3 x 3 sites, 2 slots:
+// ea_sp_plane_overlaps took 232 us with all 128 groups, 135 with 3; 4 x 10, 2
+// slots, one word 37 and 29).
+__host__ __device__ inline int plane_groups(int NB, int L2) {
+  const int most = kDiffThreads / NB, few = (L2 + 3) / 4;
+  return few < most ? few : most;
+}
 
 // Spins that differ between the pair's two replicas on plane z, for every slot
 // and sample: one block per (word, pair, plane), lane groups of one lane per
@@ -45,7 +53,7 @@ __global__ void __launch_bounds__(kDiffThreads) k_sp_plane_diff(const __grid_con
   extern __shared__ u64 pl[];  // [group][bit plane][slot]
   const int NB = d.NB, NR = d.NR, G = NR * NB, Lz = d.Lz, L2 = d.L * d.L;
   const int z = blockIdx.x % Lz, k = (blockIdx.x / Lz) % npairs, w = blockIdx.x / (Lz * npairs);
-  const int groups = kDiffThreads / NB, g = threadIdx.x / NB, b = threadIdx.x - g * NB;
+  const int groups = plane_groups(NB, L2), g = threadIdx.x / NB, b = threadIdx.x - g * NB;
   if (g < groups) {
     const u64 *Sa = d.S + ((size_t)w * d.V + (size_t)z * L2) * G + (size_t)(2 * k) * NB + b;
     u64 P[kPlanePlanes];
@@ -161,7 +169,7 @@ extern "C" {
 int ea_sp_device_view(ea_sp *job, SpDev *d, cudaStream_t *st);
 
 static void launch_plane_diff(const SpDev &d, int npairs, int32_t *diff, double *xs, cudaStream_t st) {
-  const size_t sm = (size_t)(kDiffThreads / d.NB) * d.NB * kPlanePlanes * 8;
+  const size_t sm = (size_t)plane_groups(d.NB, d.L * d.L) * d.NB * kPlanePlanes * 8;
   k_sp_plane_diff<<<(unsigned)((size_t)d.nw * npairs * d.Lz), kDiffThreads, sm, st>>>(d, npairs, diff, xs);
 }
 
