@@ -339,7 +339,7 @@ __device__ __forceinline__ void sp_pass_any(const SpDev &d, const uint4 *ctr, in
 // DRAM once (340 MB on 64 words of 12 x 12 x 48, 24 temperatures, 4 replicas:
 // 50 us at the copy rate).  One thread a column and run of sites, each ending
 // in 64 global atomic additions, took 257 us there (190 instructions a word)
-// and 28 us on one word; this form 167 and 12.  Two columns a lane (16-byte loads)
+// and 28 us on one word; this form 160 and 12.  Two columns a lane (16-byte loads)
 // took 181 us: 115 registers leave 16 warps an SM.
 // ---------------------------------------------------------------------------
 constexpr int kEnPlanes = 8;
@@ -350,15 +350,18 @@ constexpr size_t kEnSmem = 64 * 1024;    // of a block, in every form of the cou
 
 // Fills the count's launch shape (d.en) for `chunk` sites a lane, fewer where
 // the lane groups of a few columns would stage more sites than kEnSmem holds.
-void sp_energy_shape(SpDev &d, int chunk) {
-  EnShape &e = d.en;
+static void en_threads(const SpDev &d, EnShape &e) {
   const int G = d.NR * d.NB;
-  d.echunk = chunk;
   e.nslice = (G + kEnMaxThreads - 1) / kEnMaxThreads;
   e.lanes = (G + e.nslice - 1) / e.nslice;
   e.threads = (e.lanes + 31) / 32 * 32;
   for (int t = e.threads; t <= kEnMaxThreads; t += 32)  // the multiple of 32 that lane groups fill best
     if (t / e.lanes * e.lanes * e.threads >= e.threads / e.lanes * e.lanes * t) e.threads = t;
+}
+void sp_energy_shape(SpDev &d, int chunk) {
+  EnShape &e = d.en;
+  en_threads(d, e);
+  d.echunk = chunk;
   e.tile = std::min({e.threads / e.lanes * chunk, d.esites, (int)(kEnSmem / kEnSiteBytes)});
   e.ntile = (d.esites + e.tile - 1) / e.tile;
 }
@@ -369,13 +372,20 @@ inline size_t en_smem(const SpDev &d, int threads) {
   return std::max((size_t)d.en.tile * kEnSiteBytes, (size_t)(threads / d.en.lanes) * d.en.lanes * kEnPlanes * 8);
 }
 
-// Sites per lane of the energy count: at most what the counters take, fewer
-// when the GPU would otherwise get less than about three waves of blocks, at
-// least 4 (the counters take 4 at a time).
+// Sites per lane of the energy count, a multiple of the 4 that the counters take
+// at a time, at most what they hold.  A block ends with an atomic addition a (column,
+// sample), so n sites a lane cost a / n in additions (a = 64 columns x sites /
+// lane groups, some 2 us a million) and about half a microsecond each: the sum
+// is least at sqrt(4e-6 a).  us a count with the sites of three waves of blocks
+// / with these, and of the form without blocks: 12^2 x 48, 96 columns, 64
+// words 175 / 160, 262; 24^2 x 192, 128 columns 84 / 74, 123; 10^2 x 80, 240
+// columns, 3 words 80 / 33, 62; 18^2 x 55, 189 columns 99 / 43, 68.
 int sp_energy_chunk(const SpDev &d) {
-  const double words = (double)d.nw * d.esites * d.NR * d.NB;
-  const int c = (int)(words / (3 * 152.0 * 1152.0));
-  return c < 4 ? 4 : (c > kEnSites ? kEnSites : c);
+  EnShape e{};
+  en_threads(d, e);
+  const double a = 64.0 * d.nw * d.esites * d.NR * d.NB / (e.threads / e.lanes);
+  const double n = std::sqrt(4e-6 * a);
+  return n >= kEnSites ? kEnSites : std::max(4, 4 * (int)std::lround(n / 4));
 }
 
 // Bit-sliced counters of 64 samples.  site() takes a site's six unsatisfied
