@@ -299,8 +299,17 @@ int scalar_energy(const Geometry &g, const uint8_t *u, const uint8_t *J6) {
 void prefault(void *p, size_t n) {
 #ifdef MADV_POPULATE_WRITE
   const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p & ~(page - 1);
-  if (!p || n < page) return;  // small results lie among the caller's other data
+  if (!p || n < 2 * page) return;  // small results lie among the caller's other data
   const int err = errno;
+  // a large array used before has its pages: two of them tell
+  auto present = [&](uintptr_t q) {
+    unsigned char v = 0;
+    return mincore((void *)(q & ~(page - 1)), page, &v) == 0 && (v & 1);
+  };
+  if (n >= (1u << 20) && present((uintptr_t)p + n / 2) && present((uintptr_t)p + n - 1)) {
+    errno = err;
+    return;
+  }
   (void)madvise((void *)a, (uintptr_t)p + n - a, MADV_POPULATE_WRITE);
   errno = err;
 #else

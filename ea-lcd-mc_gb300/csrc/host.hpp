@@ -64,7 +64,8 @@ int scalar_energy(const Geometry &g, const uint8_t *u, const uint8_t *J6);
 // copy into pages that nobody has touched (a new array of the caller's) takes
 // the device's fault path, one page at a time: 110 MB of new 64 KiB pages took
 // 90 ms to fill on the GB300, 5 ms with this.  Pages that are there already
-// cost a walk of the page table.  Nothing is written and no error is raised: a
+// cost a walk of the page table (some 40 ns a page), so arrays of 1 MB and more
+// whose middle and last page are present are left alone.  Nothing is written and no error is raised: a
 // range that is not the host's is left to the copy to refuse.
 void prefault(void *p, size_t n);
 
